@@ -7,17 +7,19 @@
 // the row exchanged with row i at step i, 0-based) on the row-major matrix
 // as the reference stores it.
 //
-// getrf: one CTA per matrix, right-looking by panels of PW columns.  The
-// panel (rows k..N-1) is factored in shared memory by the whole CTA (block
-// argmax for the pivot, row exchange, scaling, rank-1 update of the panel),
-// written back; the CTA then applies the panel's exchanges to the other
-// columns, forms U12 = L11^-1 A12 (a thread per column) and updates
-// A22 -= L21 U12 with U12 staged in shared memory in chunks of 128 columns.
-// The matrix itself stays in global memory (L2-resident for these sizes).
-// getrs: one warp per system, dot-product substitutions over the contiguous
-// rows (exchange, L y = P b, U x = y).
+// getrf, N <= 64: one CTA per matrix with the matrix in shared memory
+// (getrf_small_kernel).  Above: a cluster of C CTAs per matrix
+// (getrf_cluster_kernel), right-looking by panels of PW columns held in
+// registers; while CTA 0 brings the next panel up to date and factors it, the
+// others update the remaining columns, one cluster barrier per panel.
+// getrs: one warp per system with the factors in shared memory up to N = 64,
+// one CTA per system by blocks of 32 unknowns above.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <math.h>
+
+#include <atomic>
 
 #include "qg_batchlu.h"
 #include "qg_internal.h"
@@ -26,17 +28,23 @@
 namespace qg {
 namespace {
 
+namespace cg = cooperative_groups;
+
+// PW: panel columns.  CT: columns of an update tile (256 bytes of a row).
+// PT: threads that factor a panel, each with kBatchLuMaxN / PT rows of it in
+// registers; complex128 takes half the threads, because every warp of them
+// forms the pivot's reciprocal and FP64 instructions cost 64 times FP32's.
 template <typename T>
 struct BL;
 template <>
 struct BL<float2> {
   typedef float R;
-  static constexpr int PW = 32;
+  static constexpr int PW = 16, CT = 32, PT = 256;
 };
 template <>
 struct BL<double2> {
   typedef double R;
-  static constexpr int PW = 16;
+  static constexpr int PW = 8, CT = 16, PT = 128;
 };
 
 template <typename T>
@@ -46,231 +54,791 @@ __device__ __forceinline__ T cmk(typename BL<T>::R r, typename BL<T>::R i) {
   z.y = i;
   return z;
 }
+__device__ __forceinline__ float fmar(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fmar(double a, double b, double c) { return fma(a, b, c); }
 template <typename T>
 __device__ __forceinline__ T cfma(T acc, T a, T b) {
-  return cmk<T>(acc.x + a.x * b.x - a.y * b.y, acc.y + a.x * b.y + a.y * b.x);
+  return cmk<T>(fmar(-a.y, b.y, fmar(a.x, b.x, acc.x)), fmar(a.y, b.x, fmar(a.x, b.y, acc.y)));
 }
 template <typename T>
 __device__ __forceinline__ T cfms(T acc, T a, T b) {  // acc - a b
-  return cmk<T>(acc.x - a.x * b.x + a.y * b.y, acc.y - a.x * b.y - a.y * b.x);
+  return cmk<T>(fmar(a.y, b.y, fmar(-a.x, b.x, acc.x)), fmar(-a.y, b.x, fmar(-a.x, b.y, acc.y)));
 }
 template <typename T>
-__device__ __forceinline__ T cdiv(T a, T b) {
+__device__ __forceinline__ T cmul(T a, T b) {
+  return cmk<T>(fmar(-a.y, b.y, a.x * b.x), fmar(a.y, b.x, a.x * b.y));
+}
+template <typename T>
+__device__ __forceinline__ T crcp(T b) {
   typedef typename BL<T>::R R;
-  const R d = b.x * b.x + b.y * b.y;
-  return cmk<T>((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
-}
-template <typename T>
-__device__ __forceinline__ double cabs1(T a) {  // |Re| + |Im|, LAPACK's izamax measure
-  return fabs((double)a.x) + fabs((double)a.y);
+  const R s = R(1) / fmar(b.x, b.x, b.y * b.y);
+  return cmk<T>(b.x * s, -b.y * s);
 }
 
-constexpr int kThreads = 256;
-constexpr int kChunk = 128;  // trailing-update columns staged per pass
+// Pivot search over |Re| + |Im| (LAPACK's izamax measure), first of equals.
+// A key orders candidates as unsigned integers: 0 for a NaN, else the bits of
+// the measure plus one.
+template <typename T>
+struct PivKey;
+template <>
+struct PivKey<float2> {
+  typedef unsigned K;
+  static __device__ __forceinline__ K key(float2 a) {
+    const float v = fabsf(a.x) + fabsf(a.y);
+    return v >= 0 ? __float_as_uint(v) + 1u : 0u;
+  }
+  static __device__ __forceinline__ K warp_max(K k) { return __reduce_max_sync(0xffffffffu, k); }
+};
+template <>
+struct PivKey<double2> {
+  typedef unsigned long long K;
+  static __device__ __forceinline__ K key(double2 a) {
+    const double v = fabs(a.x) + fabs(a.y);
+    return v >= 0 ? (unsigned long long)__double_as_longlong(v) + 1ull : 0ull;
+  }
+  static __device__ __forceinline__ K warp_max(K k) {
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(k >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(k >> 32) == hi ? (unsigned)k : 0u);
+    return ((unsigned long long)hi << 32) | lo;
+  }
+};
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads) getrf_kernel(int N, T *A_all, int *piv_all, int *info_all) {
-  constexpr int PW = BL<T>::PW;
+__device__ __forceinline__ T shfl_c(T v, int lane) {
+  return cmk<T>(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
+}
+
+// ---------------- N <= 64: the matrix in shared memory ----------------
+// Unblocked right-looking elimination, a rank-1 update per column: the FP64
+// pipe (two FMAs per clock and SM) is the bound of the complex128 update
+// whether its operands come from registers or shared memory, so nothing is
+// gained from blocking here, and several CTAs share an SM to cover each
+// other's pivot searches and barriers (three per column).
+// Measured, complex128 (one CTA of 256 threads with panels of 16 columns through
+// global memory before -> now): 4,096 matrices of N = 30 2,410 -> 455 us,
+// 1,005 of N = 60 1,724 -> 863 us (0.29 and 0.58 GFLOP: 235 and 463 us at the
+// FP64 pipes' 1.25 TFLOP/s).
+constexpr int kSmallN = 64, kSmallThreads = 128;
+
+template <typename T>
+__global__ void __launch_bounds__(kSmallThreads) getrf_small_kernel(int N, T *A_all, int *piv_all, int *info_all) {
   extern __shared__ __align__(16) unsigned char sm[];
-  T *P = reinterpret_cast<T *>(sm);  // panel [N][PW] (rows k..N-1 used, row r at P[(r - k) * PW])
-  T *U = P + (size_t)N * PW;         // U12 chunk [PW][kChunk]
-  __shared__ double red_v[kThreads / 32];
-  __shared__ int red_i[kThreads / 32];
-  __shared__ int s_piv;
+  T *S = reinterpret_cast<T *>(sm);
+  const int LD = N + 1;
+  __shared__ T lcol[kSmallN];
+  __shared__ T s_rinv, s_piv, s_old;
+  __shared__ int s_p;
   T *A = A_all + (size_t)blockIdx.x * N * N;
-  int *piv = piv_all + (size_t)blockIdx.x * N;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int t = tid, r = t / N, c = t - r * N; t < N * N; t += kSmallThreads) {
+    S[r * LD + c] = A[t];
+    c += kSmallThreads;
+    while (c >= N) {
+      c -= N;
+      ++r;
+    }
+  }
+  __syncthreads();
   int info = 0;
-  for (int k = 0; k < N; k += PW) {
-    const int pw = min(PW, N - k), rows = N - k;
-    // load the panel
-    for (int t = tid; t < rows * pw; t += kThreads) {
-      const int r = t / pw, c = t - r * pw;
-      P[r * PW + c] = A[(size_t)(k + r) * N + k + c];
-    }
-    __syncthreads();
-    for (int c = 0; c < pw; ++c) {
-      // pivot: argmax |Re| + |Im| over panel rows c..rows-1 of column c (first of equals)
-      double bv = -1;
-      int bi = c;
-      for (int r = c + tid; r < rows; r += kThreads) {
-        const double v = cabs1(P[r * PW + c]);
-        if (v > bv) {
-          bv = v;
-          bi = r;
-        }
-      }
-      for (int o = 16; o; o >>= 1) {
-        const double ov = __shfl_xor_sync(0xffffffffu, bv, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov > bv || (ov == bv && oi < bi)) {
-          bv = ov;
-          bi = oi;
-        }
-      }
+  for (int c = 0; c < N; ++c) {
+    if (tid < 32) {
+      typename PivKey<T>::K k0 = 0, k1 = 0;
+      const int r0 = c + lane, r1 = r0 + 32;
+      if (r0 < N) k0 = PivKey<T>::key(S[r0 * LD + c]);
+      if (r1 < N) k1 = PivKey<T>::key(S[r1 * LD + c]);
+      const bool second = k1 > k0;
+      const typename PivKey<T>::K best = PivKey<T>::warp_max(second ? k1 : k0);
+      unsigned r = INT_MAX;
+      if (r0 < N && k0 == best)
+        r = r0;
+      else if (r1 < N && k1 == best)
+        r = r1;
+      const int p = (int)__reduce_min_sync(0xffffffffu, r);
       if (lane == 0) {
-        red_v[warp] = bv;
-        red_i[warp] = bi;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        double v = red_v[0];
-        int i = red_i[0];
-        for (int w = 1; w < kThreads / 32; ++w)
-          if (red_v[w] > v || (red_v[w] == v && red_i[w] < i)) {
-            v = red_v[w];
-            i = red_i[w];
-          }
-        s_piv = i;
-        piv[k + c] = k + i;
-      }
-      __syncthreads();
-      const int p = s_piv;
-      if (p != c && tid < pw) {  // exchange panel rows c and p
-        const T a = P[c * PW + tid];
-        P[c * PW + tid] = P[p * PW + tid];
-        P[p * PW + tid] = a;
-      }
-      __syncthreads();
-      const T d = P[c * PW + c];
-      const bool zero = (d.x == 0 && d.y == 0);
-      if (zero && info == 0) info = k + c + 1;
-      // scale the column below the diagonal, then the rank-1 update of the panel
-      if (!zero)
-        for (int r = c + 1 + tid; r < rows; r += kThreads) P[r * PW + c] = cdiv(P[r * PW + c], d);
-      __syncthreads();
-      const int nc = pw - c - 1;
-      if (nc > 0 && !zero)
-        for (int t = tid; t < (rows - c - 1) * nc; t += kThreads) {
-          const int r = c + 1 + t / nc, j = c + 1 + t % nc;
-          P[r * PW + j] = cfms(P[r * PW + j], P[r * PW + c], P[c * PW + j]);
-        }
-      __syncthreads();
-    }
-    // write the panel back
-    for (int t = tid; t < rows * pw; t += kThreads) {
-      const int r = t / pw, c = t - r * pw;
-      A[(size_t)(k + r) * N + k + c] = P[r * PW + c];
-    }
-    // the panel's row exchanges on the columns outside it, in order, a thread per column
-    for (int j = tid; j < N - pw; j += kThreads) {
-      const int col = j < k ? j : j + pw;
-      for (int c = 0; c < pw; ++c) {
-        const int p = piv[k + c];
-        if (p != k + c) {
-          const T a = A[(size_t)(k + c) * N + col];
-          A[(size_t)(k + c) * N + col] = A[(size_t)p * N + col];
-          A[(size_t)p * N + col] = a;
-        }
+        const T d = S[p * LD + c];
+        s_p = p;
+        s_piv = d;
+        s_old = S[c * LD + c];
+        if (!(d.x == 0 && d.y == 0)) s_rinv = crcp(d);
+        piv_all[(size_t)blockIdx.x * N + c] = p;
       }
     }
     __syncthreads();
-    const int k2 = k + pw;
-    if (k2 >= N) break;
-    // U12 = L11^-1 A12 (unit lower), a thread per column
-    for (int col = k2 + tid; col < N; col += kThreads) {
-      T x[PW];
-#pragma unroll
-      for (int r = 0; r < PW; ++r)
-        if (r < pw) x[r] = A[(size_t)(k + r) * N + col];
-#pragma unroll
-      for (int r = 1; r < PW; ++r)
-        if (r < pw)
-#pragma unroll
-          for (int s = 0; s < PW; ++s)
-            if (s < r) x[r] = cfms(x[r], P[r * PW + s], x[s]);
-#pragma unroll
-      for (int r = 0; r < PW; ++r)
-        if (r < pw) A[(size_t)(k + r) * N + col] = x[r];
+    const int p = s_p;
+    const T d = s_piv;
+    const bool zero = (d.x == 0 && d.y == 0);
+    if (zero && info == 0) info = c + 1;
+    if (tid < 64) {  // column c: the pivot on the diagonal, multipliers below
+      const int r = c + tid;
+      if (r < N) {
+        T v = r == c ? d : (r == p ? s_old : S[r * LD + c]);
+        if (r > c) {
+          if (!zero) v = cmul(v, s_rinv);
+          lcol[r] = v;
+        }
+        S[r * LD + c] = v;
+      }
+    } else {  // exchange rows c and p in the other columns
+      const int j = tid - 64;
+      if (p != c && j < N && j != c) {
+        const T a = S[c * LD + j];
+        S[c * LD + j] = S[p * LD + j];
+        S[p * LD + j] = a;
+      }
     }
     __syncthreads();
-    // A22 -= L21 U12, U12 staged by column chunks
-    for (int c0 = k2; c0 < N; c0 += kChunk) {
-      const int cw = min(kChunk, N - c0);
-      for (int t = tid; t < pw * cw; t += kThreads) {
-        const int r = t / cw, j = t - r * cw;
-        U[r * kChunk + j] = A[(size_t)(k + r) * N + c0 + j];
+    const int m = N - c - 1;
+    if (!zero && m > 0) {
+      const float im = 1.0f / m;
+      for (int t = tid; t < m * m; t += kSmallThreads) {
+        const int i = (int)((t + 0.5f) * im), j = t - i * m;  // exact: m * m <= 4096
+        T *x = S + (c + 1 + i) * LD + c + 1 + j;
+        *x = cfms(*x, lcol[c + 1 + i], S[c * LD + c + 1 + j]);
       }
-      __syncthreads();
-      const int nr = N - k2;
-      for (int t = tid; t < nr * cw; t += kThreads) {
-        const int i = t / cw, j = t - i * cw;
-        const T *l = P + (size_t)(pw + i) * PW;
-        T acc = A[(size_t)(k2 + i) * N + c0 + j];
-#pragma unroll 8
-        for (int s = 0; s < pw; ++s) acc = cfms(acc, l[s], U[s * kChunk + j]);
-        A[(size_t)(k2 + i) * N + c0 + j] = acc;
-      }
-      __syncthreads();
+    }
+    __syncthreads();
+  }
+  for (int t = tid, r = t / N, c = t - r * N; t < N * N; t += kSmallThreads) {
+    A[t] = S[r * LD + c];
+    c += kSmallThreads;
+    while (c >= N) {
+      c -= N;
+      ++r;
     }
   }
   if (tid == 0 && info_all) info_all[blockIdx.x] = info;
 }
 
-// One warp per system: x = (P M)^-1 b in place on b (one right-hand side).
+// ---------------- 64 < N <= 512: a cluster of CTAs per matrix ----------------
+constexpr int kThreads = 256;
+
 template <typename T>
-__global__ void getrs_kernel(int nm, int N, const T *LU_all, const int *piv_all, T *b_all) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= nm) return;
-  const T *A = LU_all + (size_t)w * N * N;
-  const int *piv = piv_all + (size_t)w * N;
-  T *b = b_all + (size_t)w * N;
-  if (lane == 0)
-    for (int i = 0; i < N; ++i) {
-      const int p = piv[i];
-      if (p != i) {
-        const T a = b[i];
-        b[i] = b[p];
-        b[p] = a;
-      }
-    }
+struct ClusterSmem {
+  static constexpr int PW = BL<T>::PW, CT = BL<T>::CT;
+  static constexpr int LDP = PW + 16 / (int)sizeof(T);  // panel row stride: 16 bytes of padding
+  static size_t bytes(int N) { return (2 * (size_t)N * LDP + (size_t)PW * CT) * sizeof(T); }
+};
+
+// The panel's row exchanges as one permutation of the rows it touches:
+// row dst[e] receives row src[e].  The first pw entries are the panel's own
+// rows, in order.
+struct SwapList {
+  int src[32], dst[32];
+  int cnt;    // entries
+  int moved;  // whether any row moves
+};
+
+// Called by warp 0.
+__device__ __forceinline__ void build_swaps(SwapList &s, const int *piv, int k, int pw) {
+  const int lane = threadIdx.x & 31;
+  const int p0 = lane < pw ? piv[k + lane] : k + lane;
+  const unsigned moved = __ballot_sync(0xffffffffu, p0 != k + lane);
+  if (lane < pw) s.src[lane] = s.dst[lane] = k + lane;
   __syncwarp();
-  for (int i = 1; i < N; ++i) {  // L y = P b, unit lower
-    T acc = cmk<T>(0, 0);
-    for (int j = lane; j < i; j += 32) acc = cfma(acc, A[(size_t)i * N + j], b[j]);
-    for (int o = 16; o; o >>= 1) {
-      acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
-      acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+  int cnt = pw;
+  for (unsigned left = moved; left; left &= left - 1) {  // uniform: the exchanges in order
+    const int c = __ffs(left) - 1, p = __shfl_sync(0xffffffffu, p0, c);
+    if (lane == 0) {
+      int e = p - k;
+      if (e >= pw) {
+        for (e = pw; e < cnt && s.dst[e] != p; ++e) {
+        }
+        if (e == cnt) {
+          s.src[e] = s.dst[e] = p;
+          ++cnt;
+        }
+      }
+      const int a = s.src[c];
+      s.src[c] = s.src[e];
+      s.src[e] = a;
     }
-    if (lane == 0) b[i] = cmk<T>(b[i].x - acc.x, b[i].y - acc.y);
-    __syncwarp();
   }
-  for (int i = N - 1; i >= 0; --i) {  // U x = y
-    T acc = cmk<T>(0, 0);
-    for (int j = i + 1 + lane; j < N; j += 32) acc = cfma(acc, A[(size_t)i * N + j], b[j]);
-    for (int o = 16; o; o >>= 1) {
-      acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
-      acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
-    }
-    if (lane == 0) b[i] = cdiv(cmk<T>(b[i].x - acc.x, b[i].y - acc.y), A[(size_t)i * N + i]);
-    __syncwarp();
+  if (lane == 0) {
+    s.cnt = cnt;
+    s.moved = moved != 0;
   }
 }
 
+// Factors the panel of columns [k, k + pw): rows k..N-1 in registers (row
+// k + tid + PT i in thread tid), one barrier per column.  Each warp offers its
+// best row; the warp's winner and the owner of the diagonal row put these rows
+// into one of two alternating slots, and after the barrier every thread picks
+// the winner itself, exchanges and eliminates.  The panel comes from and goes
+// back to Lp (a thread's row is strided in global memory: read and written
+// from there it took as long as the elimination); the pivots (0-based rows of
+// the matrix) go to piv.
 template <typename T>
-size_t getrf_smem(int N) {
-  return ((size_t)N * BL<T>::PW + (size_t)BL<T>::PW * kChunk) * sizeof(T);
+__device__ __forceinline__ void factor_panel(int N, int k, int pw, T *Lp, int *piv, int &info) {
+  constexpr int PW = BL<T>::PW, PT = BL<T>::PT, RPT = kBatchLuMaxN / PT, NW = PT / 32;
+  constexpr int LDP = ClusterSmem<T>::LDP;
+  __shared__ T s_row[2][NW + 1][PW];
+  __shared__ typename PivKey<T>::K s_key[2][NW];
+  __shared__ int s_r[2][NW];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid >= PT) return;
+  const int rows = N - k;
+  T a[RPT][PW];
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int r = tid + PT * i;
+#pragma unroll
+    for (int c = 0; c < PW; ++c) a[i][c] = (r < rows && c < pw) ? Lp[r * LDP + c] : cmk<T>(0, 0);
+  }
+#pragma unroll
+  for (int c = 0; c < PW; ++c) {
+    if (c < pw) {  // uniform
+      const int buf = c & 1;
+      typename PivKey<T>::K key = 0;
+      int br = INT_MAX;
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) {
+        const int r = tid + PT * i;
+        if (r >= c && r < rows) {
+          const typename PivKey<T>::K q = PivKey<T>::key(a[i][c]);
+          if (br == INT_MAX || q > key) {
+            key = q;
+            br = r;
+          }
+        }
+      }
+      const typename PivKey<T>::K best = PivKey<T>::warp_max(key);
+      const int rmin = (int)__reduce_min_sync(0xffffffffu, key == best ? (unsigned)br : (unsigned)INT_MAX);
+      if (lane == 0) {
+        s_key[buf][warp] = best;
+        s_r[buf][warp] = rmin;
+      }
+      if (br == rmin && br != INT_MAX) {
+#pragma unroll
+        for (int i = 0; i < RPT; ++i)
+          if (tid + PT * i == rmin)
+#pragma unroll
+            for (int j = 0; j < PW; ++j) s_row[buf][warp][j] = a[i][j];
+      }
+      if (tid == c) {
+#pragma unroll
+        for (int j = 0; j < PW; ++j) s_row[buf][NW][j] = a[0][j];
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(PT) : "memory");
+      const int wl = min(lane, NW - 1);
+      const typename PivKey<T>::K wk = s_key[buf][wl], bk = PivKey<T>::warp_max(wk);
+      const unsigned wr = wk == bk ? (unsigned)s_r[buf][wl] : (unsigned)INT_MAX;
+      const int p = (int)__reduce_min_sync(0xffffffffu, wr);
+      const int win = __ffs(__ballot_sync(0xffffffffu, wr == (unsigned)p)) - 1;
+      T u[PW];
+#pragma unroll
+      for (int j = 0; j < PW; ++j) u[j] = s_row[buf][win][j];
+      if (tid == 0) piv[k + c] = k + p;
+      if (p != c) {
+        if (tid == c) {
+#pragma unroll
+          for (int j = 0; j < PW; ++j) a[0][j] = u[j];
+        }
+#pragma unroll
+        for (int i = 0; i < RPT; ++i)
+          if (tid + PT * i == p)
+#pragma unroll
+            for (int j = 0; j < PW; ++j) a[i][j] = s_row[buf][NW][j];
+      }
+      const bool zero = (u[c].x == 0 && u[c].y == 0);
+      if (zero) {
+        if (info == 0) info = k + c + 1;
+      } else {
+        const T rinv = crcp(u[c]);
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+          const int r = tid + PT * i;
+          if (PT * i < rows && r > c) {  // rows past the matrix hold zeros
+            const T l = cmul(a[i][c], rinv);
+            a[i][c] = l;
+#pragma unroll
+            for (int j = c + 1; j < PW; ++j) a[i][j] = cfms(a[i][j], l, u[j]);
+          }
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int r = tid + PT * i;
+    if (r < rows) {
+#pragma unroll
+      for (int c = 0; c < PW; ++c) Lp[r * LDP + c] = a[i][c];
+    }
+  }
+}
+
+// The panel of columns [k, k + pw), rows k..N-1, between the matrix and shared memory.
+template <typename T, bool STORE>
+__device__ __forceinline__ void copy_panel(int N, int k, int pw, T *A, T *Lp) {
+  constexpr int PW = BL<T>::PW, LDP = ClusterSmem<T>::LDP;
+  const int c = threadIdx.x % PW;
+  if (c >= pw) return;
+#pragma unroll 4
+  for (int r = threadIdx.x / PW; r < N - k; r += kThreads / PW) {
+    if (STORE)
+      A[(size_t)(k + r) * N + k + c] = Lp[r * LDP + c];
+    else
+      Lp[r * LDP + c] = A[(size_t)(k + r) * N + k + c];
+  }
+}
+
+// Columns [c0, c0 + cw), cw <= CW, right of a full panel at k: row exchanges,
+// U12 = L11^-1 A12 and A22 -= L21 U12.  Called by the whole CTA.  With `next`,
+// A22's rows go there (the next panel, row stride LDP) and not to the matrix.
+template <typename T, int CW>
+__device__ __forceinline__ void update_tile(int N, int k, int c0, int cw, T *A, const T *Lp, T *Us,
+                                            const SwapList &sw, T *next) {
+  constexpr int PW = BL<T>::PW, LDP = ClusterSmem<T>::LDP;
+  constexpr int PER = (2 * PW * CW + kThreads - 1) / kThreads;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  T v[PER];
+  const int cnt = sw.cnt;
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int e = (tid + kThreads * q) / CW, j = tid % CW;
+    if (e < cnt && j < cw) v[q] = A[(size_t)sw.src[e] * N + c0 + j];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int e = (tid + kThreads * q) / CW, j = tid % CW;
+    if (e < cnt && j < cw) {
+      if (e < PW)
+        Us[e * CW + j] = v[q];
+      else
+        A[(size_t)sw.dst[e] * N + c0 + j] = v[q];
+    }
+  }
+  __syncthreads();
+  // forward substitution with the unit lower L11: a lane per (row, column)
+  for (int j0 = warp * (32 / PW); j0 < CW; j0 += (kThreads / 32) * (32 / PW)) {
+    const int rr = lane % PW, cc = lane / PW, j = j0 + cc;
+    T x = Us[rr * CW + j];
+#pragma unroll
+    for (int s = 0; s < PW - 1; ++s) {
+      const T xs = shfl_c(x, cc * PW + s);
+      if (rr > s) x = cfms(x, Lp[rr * LDP + s], xs);
+    }
+    Us[rr * CW + j] = x;
+    if (j < cw) A[(size_t)(k + rr) * N + c0 + j] = x;
+  }
+  __syncthreads();
+  {
+    constexpr int RS = 32 / CW;  // rows of one warp step
+    const int j = lane % CW, sub = lane / CW;
+    T u[PW];
+#pragma unroll
+    for (int s = 0; s < PW; ++s) u[s] = Us[s * CW + j];
+    if (j < cw) {
+      constexpr int step = (kThreads / 32) * RS, UB = 4;  // UB rows in flight per thread
+      for (int r = PW + warp * RS + sub; r < N - k; r += UB * step) {
+        T acc[UB];
+#pragma unroll
+        for (int i = 0; i < UB; ++i)
+          if (r + i * step < N - k) acc[i] = A[(size_t)(k + r + i * step) * N + c0 + j];
+#pragma unroll
+        for (int i = 0; i < UB; ++i) {
+          if (r + i * step < N - k) {
+            const T *l = Lp + (r + i * step) * LDP;
+#pragma unroll
+            for (int s = 0; s < PW; ++s) acc[i] = cfms(acc[i], l[s], u[s]);
+            if (next)
+              next[(r + i * step - PW) * LDP + j] = acc[i];
+            else
+              A[(size_t)(k + r + i * step) * N + c0 + j] = acc[i];
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// Row exchanges of the columns [c0, c0 + cw) left of the panel.
+template <typename T>
+__device__ __forceinline__ void swap_tile(int N, int c0, int cw, T *A, const SwapList &sw) {
+  constexpr int PW = BL<T>::PW, CW = BL<T>::CT;
+  constexpr int PER = (2 * PW * CW + kThreads - 1) / kThreads;
+  const int tid = threadIdx.x;
+  T v[PER];
+  const int cnt = sw.cnt;
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int e = (tid + kThreads * q) / CW, j = tid % CW;
+    if (e < cnt && j < cw) v[q] = A[(size_t)sw.src[e] * N + c0 + j];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int e = (tid + kThreads * q) / CW, j = tid % CW;
+    if (e < cnt && j < cw) A[(size_t)sw.dst[e] * N + c0 + j] = v[q];
+  }
+  __syncthreads();
+}
+
+// C CTAs (one cluster) per matrix, C = 1 or >= 4.  Per panel: CTA 0 updates the
+// next panel's columns and factors it (the serial chain), the other CTAs update
+// the remaining tiles of CT columns and exchange rows on the left; with C = 1
+// the one CTA does both.  All panel data pass through the matrix in global
+// memory (L2); the cluster barrier orders them.  Every CTA runs the same
+// number of barriers.
+template <typename T>
+__global__ void __launch_bounds__(kThreads) getrf_cluster_kernel(int N, int C, T *A_all, int *piv_all, int *info_all) {
+  constexpr int PW = BL<T>::PW, CT = BL<T>::CT, LDP = ClusterSmem<T>::LDP;
+  extern __shared__ __align__(16) unsigned char sm[];
+  T *Lp = reinterpret_cast<T *>(sm);  // panel rows k..N-1, row stride LDP
+  T *Ln = Lp + (size_t)N * LDP;       // CTA 0: the next panel
+  T *Us = Ln + (size_t)N * LDP;       // U12 tile [PW][CT]
+  __shared__ SwapList sw;
+  const int m = blockIdx.x / C, cr = blockIdx.x - m * C;
+  T *A = A_all + (size_t)m * N * N;
+  int *piv = piv_all + (size_t)m * N;
+  const int tid = threadIdx.x;
+  cg::cluster_group cl = cg::this_cluster();
+  int info = 0;
+  if (cr == 0) {
+    copy_panel<T, false>(N, 0, min(PW, N), A, Lp);
+    __syncthreads();
+    factor_panel(N, 0, min(PW, N), Lp, piv, info);
+    __syncthreads();
+    copy_panel<T, true>(N, 0, min(PW, N), A, Lp);
+  }
+  if (C > 1)
+    cl.sync();
+  else
+    __syncthreads();
+  for (int k = 0; k < N; k += PW) {
+    const int pw = min(PW, N - k), k2 = k + pw, pn = min(PW, N - k2);
+    if (tid < 32) build_swaps(sw, piv, k, pw);
+    if (cr != 0 && pn > 0) copy_panel<T, false>(N, k, pw, A, Lp);
+    __syncthreads();
+    if (cr == 0 && pn > 0) update_tile<T, PW>(N, k, k2, pn, A, Lp, Us, sw, Ln);
+    if (cr != 0 || C == 1) {
+      const int first = C == 1 ? 0 : cr - 1, step = C == 1 ? 1 : C - 1;
+      const int nt = pn > 0 ? (N - k2 - pn + CT - 1) / CT : 0;
+      for (int t = first; t < nt; t += step) {
+        const int c0 = k2 + pn + t * CT;
+        update_tile<T, CT>(N, k, c0, min(CT, N - c0), A, Lp, Us, sw, (T *)nullptr);
+      }
+      if (sw.moved)
+        for (int t = first; t * CT < k; t += step) swap_tile<T>(N, t * CT, min(CT, k - t * CT), A, sw);
+    }
+    if (cr == 0 && pn > 0) {
+      T *t = Lp;
+      Lp = Ln;
+      Ln = t;
+      factor_panel(N, k2, pn, Lp, piv, info);
+      __syncthreads();
+      copy_panel<T, true>(N, k2, pn, A, Lp);
+    }
+    if (C > 1)
+      cl.sync();
+    else
+      __syncthreads();
+  }
+  if (cr == 0 && tid == 0 && info_all) info_all[m] = info;
+}
+
+// ---------------- substitutions, one right-hand side ----------------
+// N <= 64: one warp per system, the factors staged in shared memory, lane l
+// holding unknowns l and l + 32.
+template <typename T>
+__global__ void __launch_bounds__(32) getrs_small_kernel(int N, const T *LU_all, const int *piv_all, T *b_all) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  T *S = reinterpret_cast<T *>(sm);
+  const int LD = N + 1, lane = threadIdx.x;
+  T *xs = S + N * LD;  // [kSmallN]
+  const T *A = LU_all + (size_t)blockIdx.x * N * N;
+  const int *piv = piv_all + (size_t)blockIdx.x * N;
+  T *b = b_all + (size_t)blockIdx.x * N;
+  for (int t = lane, r = t / N, c = t - r * N; t < N * N; t += 32) {
+    S[r * LD + c] = A[t];
+    c += 32;
+    while (c >= N) {
+      c -= N;
+      ++r;
+    }
+  }
+  const int r0 = lane, r1 = lane + 32;
+  if (r0 < N) xs[r0] = b[r0];
+  if (r1 < N) xs[r1] = b[r1];
+  const int p0 = r0 < N ? piv[r0] : 0, p1 = r1 < N ? piv[r1] : 0;
+  __syncwarp();
+  for (int i = 0; i < N; ++i) {
+    const int p = __shfl_sync(0xffffffffu, i < 32 ? p0 : p1, i & 31);
+    if (lane == 0 && p != i) {
+      const T a = xs[i];
+      xs[i] = xs[p];
+      xs[p] = a;
+    }
+  }
+  __syncwarp();
+  const T z = cmk<T>(0, 0);
+  T x0 = r0 < N ? xs[r0] : z, x1 = r1 < N ? xs[r1] : z;
+  const int q0 = min(r0, N - 1), q1 = min(r1, N - 1);
+  const T d0 = crcp(S[q0 * LD + q0]), d1 = N > 32 ? crcp(S[q1 * LD + q1]) : z;
+  for (int j = 0; j < N; ++j) {  // L y = P b, unit lower
+    const T y = shfl_c(j < 32 ? x0 : x1, j & 31);
+    if (j < 31 && r0 > j) x0 = cfms(x0, S[q0 * LD + j], y);
+    if (N > 32 && r1 > j) x1 = cfms(x1, S[q1 * LD + j], y);
+  }
+  for (int j = N - 1; j >= 0; --j) {  // U x = y
+    if (j < 32) {
+      if (r0 == j) x0 = cmul(x0, d0);
+    } else if (r1 == j) {
+      x1 = cmul(x1, d1);
+    }
+    const T y = shfl_c(j < 32 ? x0 : x1, j & 31);
+    if (r0 < j) x0 = cfms(x0, S[q0 * LD + j], y);
+    if (j > 32 && r1 < j) x1 = cfms(x1, S[q1 * LD + j], y);
+  }
+  if (r0 < N) b[r0] = x0;
+  if (r1 < N) b[r1] = x1;
+}
+
+// Above: one CTA per system, blocks of 32 unknowns.  Warp 0 solves a block's
+// 32 x 32 triangle with a lane per row; meanwhile the other warps form the next
+// block rows' products with the unknowns known before this block (coalesced
+// along the rows) and stage the next triangle and the square beside it, so
+// that between two triangles only the 32 new unknowns' products remain.
+constexpr int kRsB = 32;
+
+constexpr int kRsFar = 8, kRsThreads = 32 * (1 + kRsFar), kRsRows = kRsB / kRsFar;
+
+// Sums of the 8 values over the warp's lanes, folded so that each exchange
+// halves the values (9 additions instead of 40; FP64 additions are the cost):
+// returns the sum of v[lane >> 2 & 7] (bits 4, 3, 2 of the lane).
+template <typename R>
+__device__ __forceinline__ R fold8(R (&v)[8], int lane) {
+#pragma unroll
+  for (int h = 4, o = 16; h; h >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const R keep = up ? v[i + h] : v[i], give = up ? v[i] : v[i + h];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kRsThreads) getrs_block_kernel(int N, const T *LU_all, const int *piv_all, T *b_all) {
+  typedef typename BL<T>::R R;
+  __shared__ T x[kBatchLuMaxN], dinv[kBatchLuMaxN];
+  __shared__ T tri[2][kRsB][kRsB + 1], near[kRsB][kRsB + 1], part[kRsB];
+  __shared__ int sp[kBatchLuMaxN];
+  const T *A = LU_all + (size_t)blockIdx.x * N * N;
+  T *b = b_all + (size_t)blockIdx.x * N;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int moved = 0;
+  for (int i = tid; i < N; i += kRsThreads) {
+    x[i] = b[i];
+    sp[i] = piv_all[(size_t)blockIdx.x * N + i];
+    moved |= sp[i] != i;
+    dinv[i] = crcp(A[(size_t)i * N + i]);
+  }
+  const int nb = (N + kRsB - 1) / kRsB;
+  // stage q of 2 nb: the forward blocks in order, then the backward blocks
+  auto block = [&](int q) { return (q < nb ? q : 2 * nb - 1 - q) * kRsB; };
+  for (int t = tid; t < kRsB * kRsB; t += kRsThreads) {
+    const int r = t / kRsB, c = t % kRsB;
+    if (r < N && c < N) tri[0][r][c] = A[(size_t)r * N + c];
+  }
+  if (tid < kRsB) part[tid] = cmk<T>(0, 0);
+  if (__syncthreads_or(moved)) {
+    if (tid == 0)
+      for (int i = 0; i < N; ++i) {
+        const int p = sp[i];
+        if (p != i) {
+          const T a = x[i];
+          x[i] = x[p];
+          x[p] = a;
+        }
+      }
+    __syncthreads();
+  }
+  for (int q = 0; q < 2 * nb; ++q) {
+    const int i0 = block(q), bs = min(kRsB, N - i0);
+    const bool more = q + 1 < 2 * nb, back = q + 1 >= nb;  // the next stage: is there one, is it backward
+    const int n0 = more ? block(q + 1) : 0, ns = min(kRsB, N - n0);
+    T acc[kRsRows];
+    if (warp == 0) {
+      const int r = min(lane, bs - 1);
+      T v = x[i0 + r];
+      v = cmk<T>(v.x - part[r].x, v.y - part[r].y);
+      const T(*tl)[kRsB + 1] = tri[q & 1];
+      if (q < nb) {
+        for (int j = 0; j < bs; ++j) {
+          const T y = shfl_c(v, j);
+          if (r > j) v = cfms(v, tl[r][j], y);
+        }
+      } else {
+        const T di = dinv[i0 + r];
+        for (int j = bs - 1; j >= 0; --j) {
+          if (r == j) v = cmul(v, di);
+          const T y = shfl_c(v, j);
+          if (r < j) v = cfms(v, tl[r][j], y);
+        }
+      }
+      if (lane < bs) x[i0 + lane] = v;
+    } else if (more) {
+      // the next triangle and the square beside it: lane = column, loads in flight together
+      const int w0 = (warp - 1) * kRsRows;
+      T vt[kRsRows], vn[kRsRows];
+#pragma unroll
+      for (int r = 0; r < kRsRows; ++r) {
+        if (w0 + r < ns && lane < ns) vt[r] = A[(size_t)(n0 + w0 + r) * N + n0 + lane];
+        if (w0 + r < ns && lane < bs) vn[r] = A[(size_t)(n0 + w0 + r) * N + i0 + lane];
+      }
+      // products with the unknowns of the stages before this one
+      const int j0 = back ? i0 + bs : 0, j1 = back ? N : i0;
+#pragma unroll
+      for (int r = 0; r < kRsRows; ++r) acc[r] = cmk<T>(0, 0);
+#pragma unroll 2
+      for (int j = j0 + lane; j < j1; j += 32) {
+        const T y = x[j];
+#pragma unroll
+        for (int r = 0; r < kRsRows; ++r) {
+          const int i = n0 + min(w0 + r, ns - 1);
+          acc[r] = cfma(acc[r], A[(size_t)i * N + j], y);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < kRsRows; ++r) {
+        if (w0 + r < ns && lane < ns) tri[(q + 1) & 1][w0 + r][lane] = vt[r];
+        if (w0 + r < ns && lane < bs) near[w0 + r][lane] = vn[r];
+      }
+    }
+    __syncthreads();
+    if (warp != 0 && more) {
+      // the 32 new unknowns (none where the sweep turns round: the last forward
+      // block is the first backward one)
+      const int w0 = (warp - 1) * kRsRows;
+      R v[8];
+#pragma unroll
+      for (int r = 0; r < kRsRows; ++r) {
+        if (n0 != i0 && lane < bs && w0 + r < ns) acc[r] = cfma(acc[r], near[w0 + r][lane], x[i0 + lane]);
+        v[2 * r] = acc[r].x;
+        v[2 * r + 1] = acc[r].y;
+      }
+      const R sum = fold8(v, lane);
+      if ((lane & 3) == 0) reinterpret_cast<R *>(part)[2 * w0 + (lane >> 2)] = sum;
+    }
+    __syncthreads();
+  }
+  for (int i = tid; i < N; i += kRsThreads) b[i] = x[i];
+}
+
+template <typename T>
+void cluster_config(int C, int nm, int N, cudaStream_t st, cudaLaunchConfig_t *cfg, cudaLaunchAttribute *at) {
+  *cfg = {};
+  cfg->gridDim = dim3((unsigned)nm * C);
+  cfg->blockDim = dim3(kThreads);
+  cfg->dynamicSmemBytes = ClusterSmem<T>::bytes(N);
+  cfg->stream = st;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = C;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cfg->attrs = at;
+  cfg->numAttrs = 1;
+}
+
+// CTAs per matrix above N = 64.  The time of a matrix against its time on one
+// CTA, measured (us, GB300):
+//                            C = 1     4     8    16
+//   complex128, N 512, 2     47321 15949  7695  4321   (FP64 pipes of C - 1 SMs)
+//   complex128, N 390, 9     21790  7349  3724  4714   (two waves at 16)
+//   complex64,  N 512, 2      2788  1000   660   580   (the panels' serial chain)
+//   complex64,  N 256, 32      574   271   750  1268   (two and four waves)
+// so the choice is the least waves x relative time, a wave being the clusters
+// that the GPU holds at once (a cluster lies within one group of SMs, so 16
+// clusters of 8 no longer fit), among sizes whose CTAs all get a tile of the
+// first update.  The counts are asked for once per device.
+template <typename T>
+int cluster_size(int nm, int N, int *C_out) {
+  constexpr int kN = 4, kC[kN] = {1, 4, 8, 16}, kMaxDev = 64;
+  constexpr double kCost[kN] = {1.0, sizeof(T) == 16 ? 0.34 : 0.45, sizeof(T) == 16 ? 0.17 : 0.30,
+                                sizeof(T) == 16 ? 0.10 : 0.25};
+  static std::atomic<int> active[kMaxDev][kN];  // 0: not asked yet
+  int dev = 0;
+  QG_CUDA_TRY(cudaGetDevice(&dev));
+  const int tiles = (N - 2 * BL<T>::PW + BL<T>::CT - 1) / BL<T>::CT;
+  double best = 0;
+  *C_out = 1;
+  for (int i = 0; i < kN; ++i) {
+    if (kC[i] > 1 && tiles < kC[i] - 1) break;
+    int n = dev < kMaxDev ? active[dev][i].load() : 0;
+    if (!n) {
+      cudaLaunchConfig_t cfg;
+      cudaLaunchAttribute at[1];
+      cluster_config<T>(kC[i], 1, kBatchLuMaxN, 0, &cfg, at);
+      QG_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, getrf_cluster_kernel<T>, &cfg));
+      if (n < 1) n = -1;  // this size does not fit
+      if (dev < kMaxDev) active[dev][i].store(n);
+    }
+    if (n < 1) continue;
+    const double t = ((nm + n - 1) / n) * kCost[i];
+    if (i == 0 || t < best) {
+      best = t;
+      *C_out = kC[i];
+    }
+  }
+  return QPMS_SUCCESS;
+}
+
+template <typename T>
+int cluster_launch(int nm, int N, T *A, int *piv, int *info, cudaStream_t st) {
+  auto kern = getrf_cluster_kernel<T>;
+  QG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)ClusterSmem<T>::bytes(kBatchLuMaxN)));
+  QG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  int C = 1;
+  const int e = cluster_size<T>(nm, N, &C);
+  if (e) return e;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[1];
+  cluster_config<T>(C, nm, N, st, &cfg, at);
+  QG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, N, C, A, piv, info));
+  return QPMS_SUCCESS;
 }
 
 template <typename T>
 int getrf_launch(int nm, int N, T *A, int *piv, int *info, cudaStream_t st) {
-  const size_t smem = getrf_smem<T>(N);
   if (N > kBatchLuMaxN) {
     set_error("batched LU: N = %d above %d", N, kBatchLuMaxN);
     return QPMS_EINVAL;
   }
-  QG_CUDA_TRY(cudaFuncSetAttribute(getrf_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   KtScope kt(KT_BATCHLU, st, nm * 8.0 * N * (double)N * N / 3.0);
-  getrf_kernel<T><<<nm, kThreads, smem, st>>>(N, A, piv, info);
-  QG_CUDA_TRY(cudaGetLastError());
+  if (N <= kSmallN) {
+    const size_t smem = (size_t)N * (N + 1) * sizeof(T);
+    QG_CUDA_TRY(cudaFuncSetAttribute(getrf_small_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     kSmallN * (kSmallN + 1) * (int)sizeof(T)));
+    getrf_small_kernel<T><<<nm, kSmallThreads, smem, st>>>(N, A, piv, info);
+    QG_CUDA_TRY(cudaGetLastError());
+  } else {
+    const int e = cluster_launch<T>(nm, N, A, piv, info, st);
+    if (e) return e;
+  }
   g_launches.fetch_add(1);
   return QPMS_SUCCESS;
 }
 
 template <typename T>
 int getrs_launch(int nm, int N, const T *LU, const int *piv, T *b, cudaStream_t st) {
-  const int wpb = 4;
-  getrs_kernel<T><<<(nm + wpb - 1) / wpb, 32 * wpb, 0, st>>>(nm, N, LU, piv, b);
+  if (N > kBatchLuMaxN) {
+    set_error("batched LU: N = %d above %d", N, kBatchLuMaxN);
+    return QPMS_EINVAL;
+  }
+  if (N <= kSmallN) {
+    const size_t smem = ((size_t)N * (N + 1) + kSmallN) * sizeof(T);
+    QG_CUDA_TRY(cudaFuncSetAttribute(getrs_small_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (kSmallN * (kSmallN + 1) + kSmallN) * (int)sizeof(T)));
+    getrs_small_kernel<T><<<nm, 32, smem, st>>>(N, LU, piv, b);
+  } else {
+    getrs_block_kernel<T><<<nm, kRsThreads, 0, st>>>(N, LU, piv, b);
+  }
   QG_CUDA_TRY(cudaGetLastError());
   g_launches.fetch_add(1);
   return QPMS_SUCCESS;
