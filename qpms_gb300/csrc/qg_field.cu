@@ -9,17 +9,30 @@
 // components by csphvec2ccart (vectors.h:272-303).  Default normalisation
 // (qpms_types.h:167): Condon-Shortley phase, e^{i m phi}, factors 1.
 //
-// Layout: one thread per evaluation point, all threads of a block walk the
-// same particles, so positions and coefficient vectors are warp-uniform loads
-// (L1 broadcasts).  grid.y splits the particle list when the points alone do
-// not fill the GPU; the partial sums [split][point][3] are then added in a
-// fixed order by a second kernel, so the result does not depend on timing.
+// The sum over the waves of one particle is evaluated through its cartesian
+// components.  M_lm = -r x grad(psi_lm) / sqrt(l(l+1)) and N = rot M / k, with
+// psi_lm = z_l(kr) Y_lm: the angular momentum and gradient formulas for solid
+// waves (e.g. Edmonds, Angular Momentum in Quantum Mechanics, 5.7-5.9) give
+//   E_c = sum_{l' <= L+1, m'} C_c(l',m') psi_{l'm'}(k (r - r_p)),   c = x, y, z,
+// where C is a fixed sparse linear map of f (three real coefficients per
+// entry, FieldTables).  +-m' are paired into real harmonics
+//   Q_lm(cos th) Re / Im (u_x + i u_y)^m,  u = (r - r_p) / |r - r_p|,
+// Q_lm = P_l^m / sin^m th scaled to be monic, by Q_l = x Q_{l-1} - c Q_{l-2};
+// no angle, no pole and no division by sin th appears.  Per pair that is a
+// square root, a sine and cosine, two operations per recurrence step and six
+// FMAs per real harmonic.
 //
-// Per (point, particle) pair: one complex reciprocal, the Hankel/Bessel
-// recurrence (L + 1 orders), the normalised Legendre recurrence in l for all m
-// at once (registers), and per (l, |m|) four complex products with the
-// coefficients.  The work is FP64 arithmetic on data that stays in L1/L2: the
-// kernel is bound by the FP64 pipe, not by HBM.
+// Layout: one thread per evaluation point, all threads of a block walk the
+// same particles.  A block maps the f of kTile particles to C in shared memory
+// (about 2 % of the arithmetic) and its threads read C as broadcasts.  grid.y
+// splits the particle list when the points alone do not fill the GPU; the
+// partial sums [split][point][3] are then added in a fixed order by a second
+// kernel, so the result does not depend on timing.
+//
+// Bound: the FP64 pipe (1/64 of the FP32 rate), so the FP64 instructions per
+// pair count.  Through spherical components (radial, polar and azimuthal parts
+// of N and M per (l, m), a complex product per coefficient) lMax 3 took 790 of
+// them and @MEAS@
 #include <math.h>
 #include <string.h>
 
@@ -35,187 +48,219 @@ int scatsys_lmax(const qpms_scatsys_t *ss);
 
 namespace {
 
-constexpr int kFieldLMax = 8;
+constexpr int kFieldLMax = 6;  // the systems' largest
 constexpr int kFieldThreads = 128;
-constexpr int kFieldT = (kFieldLMax + 1) * (kFieldLMax + 2) / 2;  // (l, m >= 0) pairs
+constexpr int kTile = 8;  // particles whose coefficients are staged together
 
-// Normalised associated Legendre recurrences (GSL_SF_LEGENDRE_SPHARM with the
-// Condon-Shortley phase), index t = l (l + 1) / 2 + m:
-//   Pbar_m^m     = mm[m] sin(theta) Pbar_{m-1}^{m-1},   mm[m] = -sqrt((2m+1)/(2m))
-//   Pbar_{m+1}^m = sub[m] x Pbar_m^m,                   sub[m] = sqrt(2m+3)
-//   Pbar_l^m     = a[t] (x Pbar_{l-1}^m - b[t] Pbar_{l-2}^m)
-//   (x^2 - 1) dPbar_l^m/dx = l x Pbar_l^m - e[t] Pbar_{l-1}^m,  e = sqrt((2l+1)(l^2-m^2)/(2l-1))
-// il[l] = 1/sqrt(l(l+1)) is the power-normalisation factor (legendre.c:65-117).
+// C_c(l', m') = -i al f_M(l', m' + d) + bm f_N(l' - 1, m' + d) + bp f_N(l' + 1, m' + d)
+// for the components c = + (E_x + i E_y, d = -1), - (E_x - i E_y, d = 1) and z
+// (d = 0), index l'(l'+1) + m'.  The scale of the monic harmonics and, for
+// m' < 0, the sign of Y_{l',m'} against its conjugate are included.
+template <int L>
 struct FieldTables {
-  double y00;
-  double mm[kFieldLMax + 1], sub[kFieldLMax + 1], il[kFieldLMax + 1];
-  double a[kFieldT], b[kFieldT], e[kFieldT];
-  double pole_leg[kFieldLMax + 1], pole_f[kFieldLMax + 1];
+  double al[3][(L + 2) * (L + 2)], bm[3][(L + 2) * (L + 2)], bp[3][(L + 2) * (L + 2)];
 };
 
+template <int L>
 struct FieldArgs {
   int npts, np, chunk, J;
-  qg_c k;
+  qg_c k, ik;  // wavenumber and its reciprocal
   const double *where;  // [npts][3]
   const double *pos;    // [np][3]
   const qg_c *cvf;      // [np][2 nelem]: electric block, then magnetic
   qg_c *out;            // [split][npts][3]
-  FieldTables tb;
+  FieldTables<L> tb;
 };
 
-const FieldTables &field_tables() {
-  static FieldTables t;
+template <int L>
+const FieldTables<L> &field_tables() {
+  static FieldTables<L> t;
   static std::once_flag once;
   std::call_once(once, [] {
-    memset(&t, 0, sizeof t);
     typedef long double ld;
-    t.y00 = (double)(1.0L / sqrtl(4.0L * 3.14159265358979323846264338327950288L));
-    for (int m = 1; m <= kFieldLMax; ++m) t.mm[m] = (double)(-sqrtl((2.0L * m + 1) / (2.0L * m)));
-    for (int m = 0; m <= kFieldLMax; ++m) t.sub[m] = (double)sqrtl(2.0L * m + 3);
-    for (int l = 1; l <= kFieldLMax; ++l) {
-      t.il[l] = (double)(1.0L / sqrtl((ld)l * (l + 1)));
-      const ld pi_l = 3.14159265358979323846264338327950288L;
-      t.pole_leg[l] = (double)sqrtl((2.0L * l + 1) / (4 * pi_l * l * (l + 1)));
-      t.pole_f[l] = (double)(0.25L * sqrtl((2.0L * l + 1) / pi_l));
-      for (int m = 0; m <= l; ++m) {
-        const int ti = l * (l + 1) / 2 + m;
-        const ld L2 = (ld)l * l, M2 = (ld)m * m;
-        if (l >= m + 2) {
-          t.a[ti] = (double)sqrtl((4 * L2 - 1) / (L2 - M2));
-          t.b[ti] = (double)sqrtl((((ld)l - 1) * (l - 1) - M2) / (4 * ((ld)l - 1) * (l - 1) - 1));
-        }
-        t.e[ti] = (double)sqrtl((2.0L * l + 1) * (L2 - M2) / (2.0L * l - 1));
+    memset(&t, 0, sizeof t);
+    auto fact = [](int n) {
+      ld f = 1;
+      for (int i = 2; i <= n; ++i) f *= i;
+      return f;
+    };
+    // Y_lm = scale(l, m) Q_l|m| (u_x +- i u_y)^|m|
+    auto scale = [&](int l, int m) {
+      const int am = abs(m);
+      const ld s = sqrtl((2 * l + 1) / (4 * 3.14159265358979323846264338327950288L) * fact(l - am) / fact(l + am)) *
+                   fact(2 * l) / (powl(2, l) * fact(l) * fact(l - am));
+      return (m > 0 && (am & 1)) ? -s : s;
+    };
+    // grad psi_lm / k: z component -a(l+1,m) psi_{l+1,m} + a(l,m) psi_{l-1,m}, x + iy component
+    // g(l,m) psi_{l+1,m+1} + h(l,m) psi_{l-1,m+1}, x - iy component -g(l,-m) psi_{l+1,m-1} - h(l,-m) psi_{l-1,m-1}
+    auto aa = [](int l, int m) { return abs(m) > l ? (ld)0 : sqrtl((ld)(l * l - m * m) / (4 * l * l - 1)); };
+    auto g = [](int l, int m) { return sqrtl((ld)((l + m + 1) * (l + m + 2)) / ((2 * l + 1) * (2 * l + 3))); };
+    auto h = [](int l, int m) { return sqrtl((ld)((l - m) * (l - m - 1)) / ((2 * l - 1) * (2 * l + 1))); };
+    for (int l = 1; l <= L; ++l)
+      for (int m = -l; m <= l; ++m) {
+        const ld s = sqrtl((ld)l * (l + 1));
+        const ld m0 = m / s, mp = sqrtl((ld)(l - m) * (l + m + 1)) / s, mm = sqrtl((ld)(l + m) * (l - m + 1)) / s;
+        auto put = [&](double *row, int l2, int m2, ld v) {
+          if (abs(m2) <= l2) row[l2 * (l2 + 1) + m2] = (double)(v * scale(l2, m2));
+        };
+        put(t.al[0], l, m + 1, mp);
+        put(t.al[1], l, m - 1, mm);
+        put(t.al[2], l, m, m0);
+        put(t.bm[0], l + 1, m + 1, -mp * aa(l + 1, m + 1) - m0 * g(l, m));
+        put(t.bm[1], l + 1, m - 1, mm * aa(l + 1, m - 1) - m0 * g(l, -m));
+        put(t.bm[2], l + 1, m, (mp * g(l, -m - 1) + mm * g(l, m - 1)) / 2);
+        put(t.bp[0], l - 1, m + 1, mp * aa(l, m + 1) - m0 * h(l, m));
+        put(t.bp[1], l - 1, m - 1, -(mm * aa(l, m - 1) + m0 * h(l, -m)));
+        put(t.bp[2], l - 1, m, (mp * h(l, -m - 1) + mm * h(l, m - 1)) / 2);
       }
-    }
   });
   return t;
 }
 
-__device__ __forceinline__ qg_c ldg_c(const qg_c *p) {
-  const double2 v = __ldg(reinterpret_cast<const double2 *>(p));
-  return cmk(v.x, v.y);
+// Cartesian components (x, y, z) of C(l, m) from one particle's f.
+template <int L>
+__device__ __forceinline__ void field_coef(const FieldTables<L> &t, const qg_c *f, int l, int m, qg_c C[3]) {
+  constexpr int NE = L * (L + 2);
+  const int i = l * (l + 1) + m;
+  qg_c v[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const int m2 = m + (c == 0 ? -1 : c == 1 ? 1 : 0), am = abs(m2);
+    v[c] = cmk(0, 0);
+    if (l >= 1 && l <= L && am <= l) {
+      const qg_c x = f[NE + l * (l + 1) + m2 - 1];
+      v[c] = cmk(t.al[c][i] * x.im, -t.al[c][i] * x.re);
+    }
+    if (l >= 2 && am <= l - 1) {
+      const qg_c x = f[(l - 1) * l + m2 - 1];
+      v[c] = cmk(fma(t.bm[c][i], x.re, v[c].re), fma(t.bm[c][i], x.im, v[c].im));
+    }
+    if (l <= L - 1 && am <= l + 1) {
+      const qg_c x = f[(l + 1) * (l + 2) + m2 - 1];
+      v[c] = cmk(fma(t.bp[c][i], x.re, v[c].re), fma(t.bp[c][i], x.im, v[c].im));
+    }
+  }
+  C[0] = cscale(cadd(v[0], v[1]), 0.5);
+  C[1] = cmk(0.5 * (v[0].im - v[1].im), -0.5 * (v[0].re - v[1].re));
+  C[2] = v[2];
 }
 
-template <int L>
-__global__ void __launch_bounds__(kFieldThreads) scattered_field_kernel(const FieldArgs a) {
+// KIND 0: outgoing waves, real wavenumber; 1: outgoing waves, complex
+// wavenumber; 2: any Bessel kind.
+template <int L, int KIND>
+__global__ void __launch_bounds__(kFieldThreads) scattered_field_kernel(const FieldArgs<L> a) {
+  constexpr int LP = L + 1;                           // highest order of the cartesian waves
+  constexpr int NH = (LP + 1) * (LP + 1);             // real harmonics
+  constexpr int NP = (LP + 1) * (LP + 2) / 2;         // (l, m >= 0)
   constexpr int NE = L * (L + 2);
-  const int q = blockIdx.x * kFieldThreads + threadIdx.x;
-  if (q >= a.npts) return;
-  const double wx = a.where[3 * q], wy = a.where[3 * q + 1], wz = a.where[3 * q + 2];
+  // [particle][harmonic][component]; harmonic l^2 is m = 0, l^2 + 2m - 1 and l^2 + 2m the cosine and sine of m
+  __shared__ qg_c sC[kTile][NH][3];
+  const int q0 = blockIdx.x * kFieldThreads + threadIdx.x;
+  const int q = min(q0, a.npts - 1);
+  const double wx = a.where[3 * (size_t)q], wy = a.where[3 * (size_t)q + 1], wz = a.where[3 * (size_t)q + 2];
   const int p0 = blockIdx.y * a.chunk;
   const int p1 = min(a.np, p0 + a.chunk);
-  qg_c Ex = cmk(0, 0), Ey = cmk(0, 0), Ez = cmk(0, 0);
-  for (int p = p0; p < p1; ++p) {
-    const double dx = wx - __ldg(a.pos + 3 * p), dy = wy - __ldg(a.pos + 3 * p + 1),
-                 dz = wz - __ldg(a.pos + 3 * p + 2);
-    const double rho2 = dx * dx + dy * dy;
-    const double r = sqrt(rho2 + dz * dz);
-    // cart2sph: theta = pi/2, phi = atan2(0, 0) = 0 at r = 0
-    double ct = 0.0, st = 1.0, cf = 1.0, sf = 0.0;
-    if (r > 0.0) {
-      // true divisions: z / r is exactly +-1 on the polar axis, which selects
-      // the |cos theta| = 1 branch as acos/cos do in the reference
-      const double rho = sqrt(rho2);
-      ct = dz / r;
-      st = rho / r;
-      if (rho > 0.0) {
-        const double ir = 1.0 / rho;
-        cf = dx * ir;
-        sf = dy * ir;
-      }
-    }
-    const bool pole = (fabs(ct) == 1.0);  // legendre.c:72-86 branch
-    const qg_c kr = cscale(a.k, r);
-    qg_c z[L + 1];
-    if (a.J == 3) {  // h+_l by forward recurrence from h_0, h_1 (real or complex kr)
-      const qg_c ri = crecip(kr);
-      const qg_c ex = cexpi(kr);
-      const qg_c h0 = cmul(cmk(0.0, -1.0), cmul(ex, ri));
-      const qg_c h1 = cscale(cmul(cmul(ex, cadd(kr, cmk(0.0, 1.0))), cmul(ri, ri)), -1.0);
-      sph_forward<L>(ri, h0, h1, z);
-    } else {
-      sph_bessel<L>(a.J, kr, z);
-    }
-    const qg_c rkr = (r > 0.0) ? crecip(kr) : cmk(0, 0);
-    // e^{i m phi}, m = 0..L
-    qg_c em[L + 1];
-    em[0] = cmk(1.0, 0.0);
-#pragma unroll
-    for (int m = 1; m <= L; ++m) em[m] = cmul(em[m - 1], cmk(cf, sf));
-    const double ist = pole ? 0.0 : 1.0 / st;
-    const qg_c *cv = a.cvf + (size_t)p * 2 * NE;
-    double P1[L + 1], P2[L + 1];  // Pbar_{l-1}^m, Pbar_{l-2}^m
-#pragma unroll
-    for (int m = 0; m <= L; ++m) P1[m] = P2[m] = 0.0;
-    P1[0] = a.tb.y00;
-    qg_c sr = cmk(0, 0), sth = cmk(0, 0), sph = cmk(0, 0);
-#pragma unroll
-    for (int l = 1; l <= L; ++l) {
-      qg_c R = cmk(0, 0), T = cmk(0, 0), Pp = cmk(0, 0), TM = cmk(0, 0), PM = cmk(0, 0);
-      double Pc[L + 1];
-#pragma unroll
-      for (int m = 0; m <= l; ++m) {
-        const int ti = l * (l + 1) / 2 + m;
-        double Pl;
-        if (m == l) Pl = a.tb.mm[l] * st * P1[l - 1];
-        else if (m == l - 1) Pl = a.tb.sub[m] * ct * P1[m];
-        else Pl = a.tb.a[ti] * (ct * P1[m] - a.tb.b[ti] * P2[m]);
-        Pc[m] = Pl;
-        double leg, pi, tau;
-        if (!pole) {
-          const double Pm1 = (m <= l - 1) ? P1[m] : 0.0;
-          leg = Pl * a.tb.il[l];
-          pi = m * leg * ist;
-          tau = (l * ct * Pl - a.tb.e[ti] * Pm1) * a.tb.il[l] * ist;
-        } else {
-          const double lpar = (l & 1) ? -1.0 : 1.0;
-          leg = (m == 0) ? ((l & 1) ? ct : 1.0) * a.tb.pole_leg[l] : 0.0;
-          pi = (m == 1) ? ((ct > 0) ? -1.0 : lpar) * a.tb.pole_f[l] : 0.0;
-          tau = (m == 1) ? -((ct > 0) ? 1.0 : lpar) * a.tb.pole_f[l] : 0.0;
-        }
-        const int yp = l * (l + 1) + m - 1;
-        const qg_c SNp = cmul(ldg_c(cv + yp), em[m]);
-        const qg_c SMp = cmul(ldg_c(cv + NE + yp), em[m]);
+  qg_c E[3] = {cmk(0, 0), cmk(0, 0), cmk(0, 0)};
+  for (int pt = p0; pt < p1; pt += kTile) {
+    const int nt = min(kTile, p1 - pt);
+    __syncthreads();
+    for (int t = threadIdx.x; t < nt * NP; t += kFieldThreads) {
+      const int p = t / NP, i = t - p * NP;
+      int l = (int)((sqrtf(8.0f * i + 1.0f) - 1.0f) * 0.5f);
+      if ((l + 1) * (l + 2) / 2 <= i) ++l;
+      if (l * (l + 1) / 2 > i) --l;
+      const int m = i - l * (l + 1) / 2;
+      const qg_c *f = a.cvf + (size_t)(pt + p) * 2 * NE;
+      qg_c Cp[3], Cm[3];
+      field_coef<L>(a.tb, f, l, m, Cp);
+      if (m) field_coef<L>(a.tb, f, l, -m, Cm);
+      for (int c = 0; c < 3; ++c) {
         if (m == 0) {
-          R = cadd(R, cscale(SNp, leg));
-          T = cadd(T, cscale(SNp, tau));
-          PM = cadd(PM, cscale(SMp, tau));
+          sC[p][l * l][c] = Cp[c];
         } else {
-          const int ym = l * (l + 1) - m - 1;
-          const double sg = (m & 1) ? -1.0 : 1.0;
-          const qg_c SNm = cscale(cmul(ldg_c(cv + ym), cconj(em[m])), sg);
-          const qg_c SMm = cscale(cmul(ldg_c(cv + NE + ym), cconj(em[m])), sg);
-          // y(l, -m): leg, tau times (-1)^m, pi times -(-1)^m
-          const qg_c U = cadd(SNp, SNm), V = csub(SNp, SNm), W = csub(SMp, SMm), X = cadd(SMp, SMm);
-          R = cadd(R, cscale(U, leg));
-          T = cadd(T, cscale(U, tau));
-          Pp = cadd(Pp, cscale(V, pi));
-          TM = cadd(TM, cscale(W, pi));
-          PM = cadd(PM, cscale(X, tau));
+          sC[p][l * l + 2 * m - 1][c] = cadd(Cp[c], Cm[c]);
+          sC[p][l * l + 2 * m][c] = cmk(Cm[c].im - Cp[c].im, Cp[c].re - Cm[c].re);  // i (Cp - Cm)
         }
       }
-#pragma unroll
-      for (int m = 0; m <= L; ++m) {
-        P2[m] = P1[m];
-        P1[m] = (m <= l) ? Pc[m] : 0.0;
-      }
-      // qpms_vswf_fill_csph: besfac = z_l / kr (1/3 for l = 1 at r = 0), besderfac = z_{l-1} - l besfac
-      const qg_c besfac = (r > 0.0) ? cmul(z[l], rkr) : cmk((l == 1) ? 1.0 / 3.0 : 0.0, 0.0);
-      const qg_c besder = csub(z[l - 1], cscale(besfac, (double)l));
-      const qg_c iPp = cmk(-Pp.im, Pp.re), iTM = cmk(-TM.im, TM.re);  // the i of d(e^{im phi})/dphi / m
-      sr = cadd(sr, cscale(cmul(besfac, R), (double)(l * (l + 1))));
-      sth = cadd(sth, cadd(cmul(besder, T), cmul(z[l], iTM)));
-      sph = cadd(sph, csub(cmul(besder, iPp), cmul(z[l], PM)));
     }
-    // csphvec2ccart
-    Ex = cadd(Ex, cadd(cadd(cscale(sr, st * cf), cscale(sth, ct * cf)), cscale(sph, -sf)));
-    Ey = cadd(Ey, cadd(cadd(cscale(sr, st * sf), cscale(sth, ct * sf)), cscale(sph, cf)));
-    Ez = cadd(Ez, csub(cscale(sr, ct), cscale(sth, st)));
+    __syncthreads();
+    for (int p = 0; p < nt; ++p) {
+      const double *pp = a.pos + 3 * (size_t)(pt + p);
+      const double dx = wx - __ldg(pp), dy = wy - __ldg(pp + 1), dz = wz - __ldg(pp + 2);
+      const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+      const double ir = r2 > 0 ? rsqrt(r2) : 0.0;  // at r = 0 only l = 0 is left of a regular wave
+      // one Newton step: the phase k r carries r's error times k r
+      const double rs = r2 * ir, r = fma(0.5 * ir, fma(-rs, rs, r2), rs);
+      const double ux = dx * ir, uy = dy * ir, ct = dz * ir;
+      qg_c z[LP + 1];
+      if (KIND == 0) {  // h+_l(x), x real: e^{ix} once, forward recurrence
+        const double ri = r2 > 0 ? ir * a.ik.re : __longlong_as_double(0x7ff8000000000000ULL);
+        double sn, cs;
+        sincos(a.k.re * r, &sn, &cs);
+        z[0] = cmk(sn * ri, -cs * ri);
+        z[1] = cmk(fma(z[0].re, ri, z[0].im), fma(z[0].im, ri, -z[0].re));
+#pragma unroll
+        for (int l = 1; l < LP; ++l) {
+          const double f = (2 * l + 1) * ri;
+          z[l + 1] = cmk(fma(f, z[l].re, -z[l - 1].re), fma(f, z[l].im, -z[l - 1].im));
+        }
+      } else if (KIND == 1) {
+        const double nan = __longlong_as_double(0x7ff8000000000000ULL);
+        const qg_c kr = cscale(a.k, r), ri = r2 > 0 ? cscale(a.ik, ir) : cmk(nan, nan);
+        const qg_c ex = cexpi(kr);
+        const qg_c h0 = cmul(cmk(ex.im, -ex.re), ri);
+        const qg_c h1 = cadd(cmul(h0, ri), cmk(h0.im, -h0.re));  // h_1 = h_0 / x - i h_0
+        sph_forward<LP>(ri, h0, h1, z);
+      } else {
+        sph_bessel<LP>(a.J, cscale(a.k, r), z);
+      }
+      double Q1[LP + 1], Q2[LP + 1], A[LP + 1], B[LP + 1];  // Q_{l-1,m}, Q_{l-2,m}; (u_x + i u_y)^m
+      A[0] = 1.0;
+      B[0] = 0.0;
+      const qg_c(*C)[3] = sC[p];
+#pragma unroll
+      for (int l = 0; l <= LP; ++l) {
+        if (l == 1) {
+          A[1] = ux;
+          B[1] = uy;
+        } else if (l > 1) {
+          A[l] = fma(A[l - 1], ux, -B[l - 1] * uy);
+          B[l] = fma(A[l - 1], uy, B[l - 1] * ux);
+        }
+        qg_c S[3] = {cmk(0, 0), cmk(0, 0), cmk(0, 0)};
+#pragma unroll
+        for (int m = 0; m <= l; ++m) {
+          double Q;
+          if (m == l)
+            Q = 1.0;
+          else if (m == l - 1)
+            Q = ct;
+          else
+            Q = fma(ct, Q1[m], -((l - 1) * (l - 1) - m * m) / (4.0 * (l - 1) * (l - 1) - 1) * Q2[m]);
+          if (m < l) Q2[m] = Q1[m];
+          Q1[m] = Q;
+          const double R = m == l ? A[m] : (m == 0 ? Q : Q * A[m]);
+          const int i = m == 0 ? l * l : l * l + 2 * m - 1;
+#pragma unroll
+          for (int c = 0; c < 3; ++c) S[c] = cmk(fma(R, C[i][c].re, S[c].re), fma(R, C[i][c].im, S[c].im));
+          if (m) {
+            const double I = m == l ? B[m] : Q * B[m];
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+              S[c] = cmk(fma(I, C[i + 1][c].re, S[c].re), fma(I, C[i + 1][c].im, S[c].im));
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          E[c] = cmk(fma(-z[l].im, S[c].im, fma(z[l].re, S[c].re, E[c].re)),
+                     fma(z[l].im, S[c].re, fma(z[l].re, S[c].im, E[c].im)));
+      }
+    }
   }
+  if (q0 >= a.npts) return;
   qg_c *o = a.out + ((size_t)blockIdx.y * a.npts + q) * 3;
-  o[0] = Ex;
-  o[1] = Ey;
-  o[2] = Ez;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) o[c] = E[c];
 }
 
 // out[q][c] = sum over s of part[s][q][c], s in increasing order.
@@ -227,54 +272,84 @@ __global__ void field_reduce_kernel(const qg_c *__restrict__ part, int nsplit, s
   out[i] = s;
 }
 
-// Resident blocks of the lMax kernel on the whole device (one wave).
-template <int L>
-long field_wave_L() {
+// What one evaluation needs beside the tables of its lMax.
+struct FieldCall {
+  int npts, np, J;
+  qg_c k;
+  const double *where, *pos;
+  const qg_c *cvf;
+  qg_c *out;
+};
+
+template <int L, int KIND>
+int run_field(const FieldCall &f, cudaStream_t st) {
+  FieldArgs<L> a;
+  a.npts = f.npts;
+  a.np = f.np;
+  a.J = f.J;
+  a.k = f.k;
+  a.ik = crecip(f.k);
+  a.where = f.where;
+  a.pos = f.pos;
+  a.cvf = f.cvf;
+  a.tb = field_tables<L>();
+  // Split the particles over grid.y so that the grid fills whole waves of
+  // resident blocks (at least two waves), with >= 8 particles per split.
   int dev = 0, nsm = 152, per = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, scattered_field_kernel<L>, kFieldThreads, 0) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, scattered_field_kernel<L, KIND>, kFieldThreads, 0) !=
           cudaSuccess ||
       per < 1) {
     cudaGetLastError();
     per = 1;
   }
-  return (long)nsm * per;
-}
-
-long field_wave(int lMax) {
-  switch (lMax) {
-    case 1: return field_wave_L<1>();
-    case 2: return field_wave_L<2>();
-    case 3: return field_wave_L<3>();
-    case 4: return field_wave_L<4>();
-    case 5: return field_wave_L<5>();
-    case 6: return field_wave_L<6>();
-    case 7: return field_wave_L<7>();
-    default: return field_wave_L<8>();
+  const long bx = ((long)f.npts + kFieldThreads - 1) / kFieldThreads;
+  const long wave = (long)nsm * per;
+  const long maxsplit = std::max(1, std::min(a.np / 8, 65535));
+  long nsplit = 1;
+  double best = 2.0;
+  for (long sp = 1; sp <= maxsplit; ++sp) {
+    const long tot = bx * sp, waves = (tot + wave - 1) / wave;
+    if (waves < 2 && sp < maxsplit) continue;
+    const double idle = (double)(waves * wave - tot) / (double)(waves * wave);
+    if (idle < best - 0.02) {  // a smaller split unless a larger one idles clearly less
+      best = idle;
+      nsplit = sp;
+    }
+    if (tot >= 16 * wave) break;
   }
+  a.chunk = (int)((a.np + nsplit - 1) / nsplit);
+  nsplit = (a.np + a.chunk - 1) / a.chunk;
+  const dim3 grid((unsigned)bx, (unsigned)nsplit);
+  if (nsplit == 1) {
+    a.out = f.out;
+    scattered_field_kernel<L, KIND><<<grid, kFieldThreads, 0, st>>>(a);
+    g_launches.fetch_add(1);
+    QG_CUDA_TRY(cudaGetLastError());
+    return QPMS_SUCCESS;
+  }
+  qg_c *part = nullptr;
+  const size_t n = 3 * (size_t)f.npts;
+  QG_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void **>(&part), (size_t)nsplit * n * sizeof(qg_c), st));
+  a.out = part;
+  scattered_field_kernel<L, KIND><<<grid, kFieldThreads, 0, st>>>(a);
+  g_launches.fetch_add(1);
+  cudaError_t le = cudaGetLastError();
+  if (le == cudaSuccess) {
+    field_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part, (int)nsplit, n, f.out);
+    g_launches.fetch_add(1);
+    le = cudaGetLastError();
+  }
+  cudaFreeAsync(part, st);
+  QG_CUDA_TRY(le);
+  return QPMS_SUCCESS;
 }
 
 template <int L>
-cudaError_t launch_field_L(const FieldArgs &a, int nsplit, cudaStream_t st) {
-  dim3 grid((a.npts + kFieldThreads - 1) / kFieldThreads, nsplit);
-  scattered_field_kernel<L><<<grid, kFieldThreads, 0, st>>>(a);
-  g_launches.fetch_add(1);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_field(int lMax, const FieldArgs &a, int nsplit, cudaStream_t st) {
-  switch (lMax) {
-    case 1: return launch_field_L<1>(a, nsplit, st);
-    case 2: return launch_field_L<2>(a, nsplit, st);
-    case 3: return launch_field_L<3>(a, nsplit, st);
-    case 4: return launch_field_L<4>(a, nsplit, st);
-    case 5: return launch_field_L<5>(a, nsplit, st);
-    case 6: return launch_field_L<6>(a, nsplit, st);
-    case 7: return launch_field_L<7>(a, nsplit, st);
-    case 8: return launch_field_L<8>(a, nsplit, st);
-    default: return cudaErrorInvalidValue;
-  }
+int run_field_L(const FieldCall &f, cudaStream_t st) {
+  if (f.J != 3) return run_field<L, 2>(f, st);
+  return f.k.im == 0.0 ? run_field<L, 0>(f, st) : run_field<L, 1>(f, st);
 }
 
 // Device positions of a system, uploaded once and kept with it.
@@ -348,52 +423,15 @@ int field_device(const qpms_scatsys_t *ss, int btyp, qg_c k, const qg_c *d_cvf, 
   const double *d_pos = nullptr;
   int e;
   if ((e = device_positions(ss, &d_pos))) return e;
-  FieldArgs a;
-  a.npts = (int)npoints;
-  a.np = ss->p_count;
-  a.J = btyp;
-  a.k = k;
-  a.where = d_where;
-  a.pos = d_pos;
-  a.cvf = d_cvf;
-  a.tb = field_tables();
-  // Split the particles over grid.y so that the grid fills whole waves of
-  // resident blocks (at least two waves), with >= 8 particles per split.
-  const long bx = ((long)npoints + kFieldThreads - 1) / kFieldThreads;
-  const long wave = field_wave(lMax);
-  const long maxsplit = std::max(1, std::min(a.np / 8, 65535));
-  long nsplit = 1;
-  double best = 2.0;
-  for (long sp = 1; sp <= maxsplit; ++sp) {
-    const long tot = bx * sp, waves = (tot + wave - 1) / wave;
-    if (waves < 2 && sp < maxsplit) continue;
-    const double idle = (double)(waves * wave - tot) / (double)(waves * wave);
-    if (idle < best - 0.02) {  // a smaller split unless a larger one idles clearly less
-      best = idle;
-      nsplit = sp;
-    }
-    if (tot >= 16 * wave) break;
+  const FieldCall f = {(int)npoints, (int)ss->p_count, btyp, k, d_where, d_pos, d_cvf, d_E};
+  switch (lMax) {
+    case 1: return run_field_L<1>(f, st);
+    case 2: return run_field_L<2>(f, st);
+    case 3: return run_field_L<3>(f, st);
+    case 4: return run_field_L<4>(f, st);
+    case 5: return run_field_L<5>(f, st);
+    default: return run_field_L<6>(f, st);
   }
-  a.chunk = (int)((a.np + nsplit - 1) / nsplit);
-  nsplit = (a.np + a.chunk - 1) / a.chunk;
-  if (nsplit == 1) {
-    a.out = d_E;
-    QG_CUDA_TRY(launch_field(lMax, a, 1, st));
-    return QPMS_SUCCESS;
-  }
-  qg_c *part = nullptr;
-  const size_t n = 3 * npoints;
-  QG_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void **>(&part), (size_t)nsplit * n * sizeof(qg_c), st));
-  a.out = part;
-  cudaError_t le = launch_field(lMax, a, (int)nsplit, st);
-  if (le == cudaSuccess) {
-    field_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part, (int)nsplit, n, d_E);
-    g_launches.fetch_add(1);
-    le = cudaGetLastError();
-  }
-  cudaFreeAsync(part, st);
-  QG_CUDA_TRY(le);
-  return QPMS_SUCCESS;
 }
 
 }  // namespace
