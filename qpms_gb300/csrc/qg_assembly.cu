@@ -151,28 +151,34 @@ __global__ void __launch_bounds__(kAThreads) assemble_kernel(AsmArgs a, TransDev
         const uint8_t *cnt = which ? T.cntB : T.cntA;
         const double *coef = which ? T.coefB : T.coefA;
         const uint16_t *slot = which ? T.slotB : T.slotA;
-        const int32_t *perm = which ? T.permB : T.perm;
-        for (int k = tid; k < NE2; k += kAThreads) {
+        const uint32_t *pair = which ? T.pairB : T.pairA;
+        const int nk = which ? T.nB : T.nA;
+        for (int k = tid; k < nk; k += kAThreads) {
           const int c = cnt[k];
           double sr = 0, si = 0;
           for (int q = 0; q < c; ++q) {
-            const double cf = __ldg(coef + q * NE2 + k);
-            const qg_c x = wv[__ldg(slot + q * NE2 + k)];
+            const double cf = __ldg(coef + q * nk + k);
+            const qg_c x = wv[__ldg(slot + q * nk + k)];
             sr = fma(cf, x.re, sr);
             si = fma(cf, x.im, si);
           }
-          const qg_c v = which ? cmk(-si, sr) : cmk(sr, si);  // B multipliers are imaginary
-          const int e = __ldg(perm + k);
-          const int yi = e / NE, yj = e - yi * NE;
-          // A: (E <- E) and (M <- M) blocks; B: (E <- M) and (M <- E) blocks
-          const int r1 = yi, c1 = which ? NE + yj : yj;
-          const int r2 = NE + yi, c2 = which ? yj : NE + yj;
-          if (DENSE) {
-            sblk[r1 * NB + c1] = v;
-            sblk[r2 * NB + c2] = v;
-          } else {
-            M[(row0 + r1) * N + col0 + c1] = cscale(cmul(TR[r1], v), -1.0);
-            M[(row0 + r2) * N + col0 + c2] = cscale(cmul(TR[r2], v), -1.0);
+          qg_c v = which ? cmk(xor_sign(si, kSignBit), sr) : cmk(sr, si);  // B multipliers are imaginary
+          const uint32_t pr = __ldg(pair + k);
+          const int ends = pair_second(pr) == pair_first(pr) ? 1 : 2;
+          for (int h = 0; h < ends; ++h) {  // the two elements that share the dot product
+            const int e = h ? pair_second(pr) : pair_first(pr);
+            if (h && pair_negated(pr)) v = cmk(xor_sign(v.re, kSignBit), xor_sign(v.im, kSignBit));
+            const int yi = e / NE, yj = e - yi * NE;
+            // A: (E <- E) and (M <- M) blocks; B: (E <- M) and (M <- E) blocks
+            const int r1 = yi, c1 = which ? NE + yj : yj;
+            const int r2 = NE + yi, c2 = which ? yj : NE + yj;
+            if (DENSE) {
+              sblk[r1 * NB + c1] = v;
+              sblk[r2 * NB + c2] = v;
+            } else {
+              M[(row0 + r1) * N + col0 + c1] = cmul_neg(TR[r1], v);
+              M[(row0 + r2) * N + col0 + c2] = cmul_neg(TR[r2], v);
+            }
           }
         }
       }

@@ -20,8 +20,21 @@ QG_HD qg_c csub(qg_c a, qg_c b) { return cmk(a.re - b.re, a.im - b.im); }
 QG_HD qg_c cmul(qg_c a, qg_c b) {
   return cmk(fma(a.re, b.re, -a.im * b.im), fma(a.re, b.im, a.im * b.re));
 }
+// -(a b)
+QG_HD qg_c cmul_neg(qg_c a, qg_c b) {
+  return cmk(fma(-a.re, b.re, a.im * b.im), fma(-a.re, b.im, -(a.im * b.re)));
+}
 QG_HD qg_c cscale(qg_c a, double s) { return cmk(a.re * s, a.im * s); }
 QG_HD qg_c cconj(qg_c a) { return cmk(a.re, -a.im); }
+#if defined(__CUDACC__)
+// x with its sign flipped where bit 63 of `mask` is set.  A negation that is
+// stored and not folded into an arithmetic instruction's operand is an FP64
+// addition otherwise.
+__device__ __forceinline__ double xor_sign(double x, unsigned long long mask) {
+  return __longlong_as_double(__double_as_longlong(x) ^ (long long)mask);
+}
+constexpr unsigned long long kSignBit = 0x8000000000000000ull;
+#endif
 QG_HD double cabs2(qg_c a) { return a.re * a.re + a.im * a.im; }
 QG_HD double cabsd(qg_c a) { return hypot(a.re, a.im); }
 // Smith's algorithm for a / b.

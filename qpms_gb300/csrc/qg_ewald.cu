@@ -128,7 +128,6 @@ struct EwShape {
   static constexpr int LE = 2 * LMAX + 1;
   static constexpr int S = (LE + 1) * (LE + 1);  // nelem_sc
   static constexpr int NE = LMAX * (LMAX + 2);
-  static constexpr int NE2 = NE * NE;
   static constexpr int NB = 2 * NE;
   static constexpr int NEVEN = (LE + 1) * (LE + 2) / 2;  // (n, m) with n + m even
   static constexpr int ZP = S < 36 ? S : 36;               // accumulators per shifted pass
@@ -453,7 +452,7 @@ template <int LMAX>
 __device__ __forceinline__ void contract_block(const EwaldArgs &a, const TransDevTables &T, const qg_c *sig,
                                                size_t wk, size_t per, int pr, int R, int C, int iw) {
   using Sh = EwShape<LMAX>;
-  constexpr int NE = Sh::NE, NE2 = Sh::NE2, NB = Sh::NB;
+  constexpr int NE = Sh::NE, NB = Sh::NB;
   const int tid = threadIdx.x;
   const size_t N = (size_t)a.np * NB;
   // full matrix: block (R, C) of the N x N matrix wk; pair list: block pr alone (ld NB)
@@ -466,24 +465,30 @@ __device__ __forceinline__ void contract_block(const EwaldArgs &a, const TransDe
     const uint8_t *cnt = which ? T.cntBe : T.cntA;
     const double *coef = which ? T.coefB : T.coefA;
     const uint16_t *slot = which ? T.slotB : T.slotA;
-    const int32_t *perm = which ? T.permB : T.perm;
-    for (int kx = tid; kx < NE2; kx += kEThreads) {
+    const uint32_t *pair = which ? T.pairB : T.pairA;
+    const int nk = which ? T.nB : T.nA;
+    for (int kx = tid; kx < nk; kx += kEThreads) {
       const int c = cnt[kx];
       double sr = 0, si = 0;
       for (int q = 0; q < c; ++q) {
-        const double cf = __ldg(coef + q * NE2 + kx);
-        const qg_c x = sig[__ldg(slot + q * NE2 + kx)];
+        const double cf = __ldg(coef + q * nk + kx);
+        const qg_c x = sig[__ldg(slot + q * nk + kx)];
         sr = fma(cf, x.re, sr);
         si = fma(cf, x.im, si);
       }
-      const qg_c v = which ? cmk(-si, sr) : cmk(sr, si);
-      const int e = __ldg(perm + kx);
-      const int yi = e / NE, yj = e - yi * NE;
-      const int r1 = yi, c1 = which ? NE + yj : yj;
-      const int r2 = NE + yi, c2 = which ? yj : NE + yj;
-      const qg_c m1 = cscale(cmul(TR[r1], v), -1.0), m2 = cscale(cmul(TR[r2], v), -1.0);
-      M[(row0 + r1) * ldm + col0 + c1] = (R == C && r1 == c1) ? cadd(m1, cmk(1, 0)) : m1;
-      M[(row0 + r2) * ldm + col0 + c2] = (R == C && r2 == c2) ? cadd(m2, cmk(1, 0)) : m2;
+      qg_c v = which ? cmk(xor_sign(si, kSignBit), sr) : cmk(sr, si);
+      const uint32_t pr2 = __ldg(pair + kx);
+      const int ends = pair_second(pr2) == pair_first(pr2) ? 1 : 2;
+      for (int h = 0; h < ends; ++h) {  // the two elements that share the dot product
+        const int e = h ? pair_second(pr2) : pair_first(pr2);
+        if (h && pair_negated(pr2)) v = cmk(xor_sign(v.re, kSignBit), xor_sign(v.im, kSignBit));
+        const int yi = e / NE, yj = e - yi * NE;
+        const int r1 = yi, c1 = which ? NE + yj : yj;
+        const int r2 = NE + yi, c2 = which ? yj : NE + yj;
+        const qg_c m1 = cmul_neg(TR[r1], v), m2 = cmul_neg(TR[r2], v);
+        M[(row0 + r1) * ldm + col0 + c1] = (R == C && r1 == c1) ? cadd(m1, cmk(1, 0)) : m1;
+        M[(row0 + r2) * ldm + col0 + c2] = (R == C && r2 == c2) ? cadd(m2, cmk(1, 0)) : m2;
+      }
     }
   }
   __syncthreads();

@@ -47,15 +47,23 @@ struct TransHostTables {
   // reference-layout ragged multipliers (complex), row-major over (y, yu)
   std::vector<qg_c> A_mult, B_mult;
   std::vector<size_t> A_off, B_off;  // nelem^2 + 1 offsets
-  // kernel tables, element e = y * nelem + yu; A and B each in their own
-  // term-count order k (permA / permB: k -> e)
-  std::vector<int32_t> perm, permB;
-  std::vector<uint8_t> cntA, cntB;   // per k
-  std::vector<uint8_t> cntBe;        // B order: min(cntB, cntA of the same element), the
-                                     // q <= qmax_A bound of the lattice-sum contraction
-  std::vector<double> coefA, coefB;  // [q][k]: A real part, B imaginary part
+  // kernel tables: one entry k per pair of elements with a common dot product,
+  // A and B each in their own term-count order
+  std::vector<uint32_t> pairA, pairB;  // trans_pair(e, f, neg), elements e = y * nelem + yu
+  std::vector<uint8_t> cntA, cntB;     // terms
+  std::vector<uint8_t> cntBe;          // B's terms within A's q <= qmax_A, the lattice sums' bound
+  std::vector<double> coefA, coefB;    // [q][k]: A real part, B imaginary part
   std::vector<uint16_t> slotA, slotB;  // [q][k]: w-table slot p^2 + p + d
 };
+
+// Elements e and f = +-e that share a dot product (f == e: none), 14 bits each
+// (nelem^2 <= 14,400).
+inline uint32_t trans_pair(int e, int f, int neg) {
+  return (uint32_t)e | ((uint32_t)f << 14) | ((uint32_t)neg << 28);
+}
+QG_HD int pair_first(uint32_t p) { return (int)(p & 0x3fffu); }
+QG_HD int pair_second(uint32_t p) { return (int)((p >> 14) & 0x3fffu); }
+QG_HD bool pair_negated(uint32_t p) { return (p >> 28) & 1u; }
 
 // Builds the tables for (lMax, normalisation); returns false on bad input.
 bool build_trans_tables(int lMax, int normalisation, TransHostTables *t);
@@ -63,7 +71,8 @@ bool build_trans_tables(int lMax, int normalisation, TransHostTables *t);
 // Device copy of the kernel tables.
 struct TransDevTables {
   int lMax, nelem, ne2, tq;
-  const int32_t *perm, *permB;
+  int nA, nB;  // entries of A's and B's lists
+  const uint32_t *pairA, *pairB;
   const uint8_t *cntA, *cntB, *cntBe;
   const double *coefA, *coefB;
   const uint16_t *slotA, *slotB;

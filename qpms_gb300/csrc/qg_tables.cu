@@ -230,36 +230,71 @@ bool build_trans_tables(int lMax, int norm, TransHostTables *t) {
     for (ld v : cA[e]) t->A_mult.push_back(cmk((double)v, 0.0));
     for (ld v : cB[e]) t->B_mult.push_back(cmk(0.0, (double)v));
   }
-  // kernel order: A and B elements each sorted by their own term count
-  // (descending), so the lanes of a warp share trip counts
-  t->perm.resize(ne2);
-  t->permB.resize(ne2);
-  std::iota(t->perm.begin(), t->perm.end(), 0);
-  std::iota(t->permB.begin(), t->permB.end(), 0);
-  std::stable_sort(t->perm.begin(), t->perm.end(), [&](int a, int b) { return cA[a].size() > cA[b].size(); });
-  std::stable_sort(t->permB.begin(), t->permB.end(), [&](int a, int b) { return cB[a].size() > cB[b].size(); });
+  // Kernel tables.  Terms with a zero coefficient are left out (B's first term
+  // always is one; an element of zeros keeps its last, so that NaN inputs give
+  // NaN).  Reciprocity pairs the elements: A[(n,m),(nu,mu)] and
+  // A[(nu,-mu),(n,-m)] (and B's) have the same slots and, up to a common sign,
+  // the same coefficients, so one dot product serves both.  Elements are paired
+  // where the computed coefficients agree to a few units of rounding, and each
+  // list is sorted by term count (descending), so the lanes of a warp share trip
+  // counts.
   const int tq = t->tq;
-  t->cntA.assign(ne2, 0);
-  t->cntB.assign(ne2, 0);
-  t->cntBe.assign(ne2, 0);
-  t->coefA.assign((size_t)tq * ne2, 0.0);
-  t->coefB.assign((size_t)tq * ne2, 0.0);
-  t->slotA.assign((size_t)tq * ne2, 0);
-  t->slotB.assign((size_t)tq * ne2, 0);
-  for (int k = 0; k < ne2; ++k) {
-    const int e = t->perm[k], eb = t->permB[k];
-    t->cntA[k] = (uint8_t)cA[e].size();
-    t->cntB[k] = (uint8_t)cB[eb].size();
-    t->cntBe[k] = (uint8_t)std::min(cB[eb].size(), cA[eb].size());
-    for (size_t q = 0; q < cA[e].size(); ++q) {
-      t->coefA[q * ne2 + k] = (double)cA[e][q];
-      t->slotA[q * ne2 + k] = (uint16_t)sA[e][q];
+  auto build = [&](const std::vector<std::vector<ld>> &c, const std::vector<std::vector<int>> &slot,
+                   const std::vector<std::vector<ld>> &cA_, std::vector<uint32_t> &pair, std::vector<uint8_t> &cnt,
+                   std::vector<uint8_t> *cntE, std::vector<double> &coef, std::vector<uint16_t> &sl) {
+    std::vector<std::vector<int>> keep(ne2);  // kept term indices
+    for (int e = 0; e < ne2; ++e) {
+      for (size_t q = 0; q < c[e].size(); ++q)
+        if ((double)c[e][q] != 0) keep[e].push_back((int)q);
+      if (keep[e].empty()) keep[e].push_back((int)c[e].size() - 1);
     }
-    for (size_t q = 0; q < cB[eb].size(); ++q) {
-      t->coefB[q * ne2 + k] = (double)cB[eb][q];
-      t->slotB[q * ne2 + k] = (uint16_t)sB[eb][q];
+    struct Item {
+      int e, f, neg;
+    };
+    std::vector<Item> items;
+    std::vector<char> done(ne2, 0);
+    for (int y = 0; y < ne; ++y)
+      for (int yu = 0; yu < ne; ++yu) {
+        const int e = y * ne + yu;
+        if (done[e]) continue;
+        const int n = (int)sqrt((double)y + 1), m = y - (n * (n + 1) - 1);
+        const int nu = (int)sqrt((double)yu + 1), mu = yu - (nu * (nu + 1) - 1);
+        const int f = (nu * (nu + 1) - 1 - mu) * ne + (n * (n + 1) - 1 - m);
+        Item it = {e, e, 0};
+        if (f != e && !done[f] && keep[e] == keep[f] && slot[e] == slot[f] && cA_[e].size() == cA_[f].size())
+          for (int neg = 0; neg < 2 && it.f == e; ++neg) {
+            bool same = true;
+            for (int q : keep[e]) {
+              const ld a = c[e][q], b = neg ? -c[f][q] : c[f][q];
+              same = same && fabsl(a - b) <= 1e-15L * fabsl(a);
+            }
+            if (same) it = {e, f, neg};
+          }
+        done[it.e] = done[it.f] = 1;
+        items.push_back(it);
+      }
+    std::stable_sort(items.begin(), items.end(),
+                     [&](const Item &a, const Item &b) { return keep[a.e].size() > keep[b.e].size(); });
+    const int nu_ = (int)items.size();
+    pair.assign(nu_, 0);
+    cnt.assign(nu_, 0);
+    if (cntE) cntE->assign(nu_, 0);
+    coef.assign((size_t)tq * nu_, 0.0);
+    sl.assign((size_t)tq * nu_, 0);
+    for (int k = 0; k < nu_; ++k) {
+      const Item &it = items[k];
+      pair[k] = trans_pair(it.e, it.f, it.neg);
+      cnt[k] = (uint8_t)keep[it.e].size();
+      for (size_t i = 0; i < keep[it.e].size(); ++i) {
+        const int q = keep[it.e][i];
+        coef[i * nu_ + k] = (double)c[it.e][q];
+        sl[i * nu_ + k] = (uint16_t)slot[it.e][q];
+        if (cntE && q < (int)cA_[it.e].size()) (*cntE)[k] = (uint8_t)(i + 1);
+      }
     }
-  }
+  };
+  build(cA, sA, cA, t->pairA, t->cntA, nullptr, t->coefA, t->slotA);
+  build(cB, sB, cA, t->pairB, t->cntB, &t->cntBe, t->coefB, t->slotB);
   return true;
 }
 

@@ -37,8 +37,8 @@ int upload_tables(TransCalcPriv *p) {
   const TransHostTables &h = p->host;
   size_t total = 0;
   auto add = [&](size_t bytes) { total = ((total + 255) & ~size_t(255)) + bytes; };
-  add(h.perm.size() * 4);
-  add(h.permB.size() * 4);
+  add(h.pairA.size() * 4);
+  add(h.pairB.size() * 4);
   add(h.cntA.size());
   add(h.cntB.size());
   add(h.cntBe.size());
@@ -64,8 +64,10 @@ int upload_tables(TransCalcPriv *p) {
     off += bytes;
     return (char *)d + o;
   };
-  T.perm = (const int32_t *)put(h.perm.data(), h.perm.size() * 4);
-  T.permB = (const int32_t *)put(h.permB.data(), h.permB.size() * 4);
+  T.nA = (int)h.pairA.size();
+  T.nB = (int)h.pairB.size();
+  T.pairA = (const uint32_t *)put(h.pairA.data(), h.pairA.size() * 4);
+  T.pairB = (const uint32_t *)put(h.pairB.data(), h.pairB.size() * 4);
   T.cntA = (const uint8_t *)put(h.cntA.data(), h.cntA.size());
   T.cntB = (const uint8_t *)put(h.cntB.data(), h.cntB.size());
   T.cntBe = (const uint8_t *)put(h.cntBe.data(), h.cntBe.size());

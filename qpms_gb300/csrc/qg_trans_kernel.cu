@@ -10,32 +10,32 @@
 // then a short real-coefficient dot product over w (A multipliers are real,
 // B multipliers purely imaginary), i.e. two FP64 FMAs per term.
 //
-// Work layout: a persistent CTA of 256 threads owns a chunk of V
+// Reciprocity makes A[(n,m),(nu,mu)] and A[(nu,-mu),(n,-m)] equal up to sign (B
+// likewise), with the same slots of w: the tables list such pairs, and a thread
+// writes both elements of one dot product.  Terms that are identically zero
+// (the first of every B element) are not listed.  At lMax 6 that leaves 13,200
+// of 31,300 FP64 operations a translation.
+//
+// Work layout: a persistent CTA owns chunks of up to V
 // translations.  Phase 1 (setup): one thread per translation runs the Bessel
 // recurrence, one thread per (translation, m) a Legendre column, all threads
 // fill w.  Phase 2 (contraction): threads walk the elements in term-count
 // order (uniform trip counts per warp) and write each output row (one A or B
 // matrix, nelem^2 complex128, contiguous in HBM) to a shared-memory stage;
 // one elected thread then writes the row to HBM with a TMA bulk copy
-// (cp.async.bulk.global.shared::cta), double-buffered so the copy overlaps
-// the next row's arithmetic.
+// (cp.async.bulk.global.shared::cta).
+// Bound: the FP64 pipe (two FMAs per clock and SM); 150,001 translations at
+// lMax 6, 11 GB of output, take 6.6 ms (12.8 ms with a dot product per element).
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "qg_internal.h"
 #include "qg_specfunc.cuh"
 
 namespace qg {
 namespace {
-
-constexpr int kThreads = 256;
-// Output-row stage buffers: 2 overlaps the TMA store of one row with the next
-// row's arithmetic; 1 frees shared memory for the L1 that caches the
-// multiplier tables.
-#ifndef QG_TRANS_STAGES
-#define QG_TRANS_STAGES 2
-#endif
-constexpr int kStages = QG_TRANS_STAGES;
 
 template <int LMAX>
 struct TransShape {
@@ -44,8 +44,17 @@ struct TransShape {
   static constexpr int NL = (L + 1) * (L + 2) / 2;  // Legendre entries
   static constexpr int NE = LMAX * (LMAX + 2);
   static constexpr int NE2 = NE * NE;
-  // translations per chunk: keep the w tables ~25-40 KB
-  static constexpr int V = LMAX <= 3 ? 32 : (LMAX <= 5 ? 16 : (LMAX <= 7 ? 8 : 4));
+  // The per-translation set-up is a chain of dependent FP64 operations in one
+  // warp, so what counts is how many CTAs an SM holds to cover each other's
+  // (registers and shared memory), against the lanes that the set-up fills (V
+  // translations per chunk).  One output stage and small CTAs won for each lMax
+  // (us, 256 threads with two stages and V = 32, 16, 16, 8 -> now): lMax 2, 10^6
+  // translations 6,134 -> 2,744; lMax 3, 2 * 10^5 1,690 -> 1,119; lMax 4, 10^5
+  // 1,508 -> 1,209; lMax 5, 10^5 2,326 -> 2,150; lMax 6, 150,001 7,911 -> 6,640.
+  static constexpr int V = LMAX <= 2 ? 32 : (LMAX <= 4 ? 16 : (LMAX == 5 || LMAX == 7 ? 8 : 4));
+  static constexpr int kThreads = LMAX <= 5 ? 128 : (LMAX == 6 ? 192 : 256);
+  static constexpr int kMinCtas = LMAX <= 4 ? 6 : (LMAX <= 6 ? 3 : 1);
+  static constexpr int kStages = LMAX <= 6 ? 1 : 2;  // output-row buffers: 2 overlap the store with the next row
   static constexpr bool kStaged = (kStages * NE2 * 16 + V * (S * 16 + 2 * (L + 1) * 16 + NL * 8 + 16)) <= 200 * 1024;
 };
 
@@ -59,7 +68,7 @@ template <int LMAX>
 constexpr size_t trans_smem_bytes(bool staged) {
   using Sh = TransShape<LMAX>;
   return (size_t)Sh::V * Sh::S * 16 + (size_t)Sh::V * (Sh::L + 1) * 16 * 2 + (size_t)Sh::V * Sh::NL * 8 +
-         (size_t)Sh::V * sizeof(VecInfo) + (staged ? (size_t)kStages * Sh::NE2 * 16 : 0);
+         (size_t)Sh::V * sizeof(VecInfo) + (staged ? (size_t)Sh::kStages * Sh::NE2 * 16 : 0);
 }
 
 __device__ __forceinline__ void bulk_store_row(void *gdst, const void *ssrc, uint32_t bytes) {
@@ -80,13 +89,15 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 }
 
 template <int LMAX, bool STAGED>
-__global__ void __launch_bounds__(kThreads) trans_ab_kernel(TransDevTables T, size_t n, const qg_c *__restrict__ kr,
+__global__ void __launch_bounds__(TransShape<LMAX>::kThreads, TransShape<LMAX>::kMinCtas)
+    trans_ab_kernel(TransDevTables T, size_t n, int vc, const qg_c *__restrict__ kr,
                                                             const double *__restrict__ theta,
                                                             const double *__restrict__ phi,
                                                             const unsigned char *__restrict__ r_ge_d, int J,
                                                             qg_c *__restrict__ A, qg_c *__restrict__ B) {
   using Sh = TransShape<LMAX>;
   constexpr int L = Sh::L, S = Sh::S, NL = Sh::NL, NE2 = Sh::NE2, V = Sh::V;
+  constexpr int kThreads = Sh::kThreads, kStages = Sh::kStages;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   qg_c *w = reinterpret_cast<qg_c *>(smem_raw);  // [V][S]
   qg_c *zb = w + V * S;                           // [V][L+1]
@@ -96,13 +107,13 @@ __global__ void __launch_bounds__(kThreads) trans_ab_kernel(TransDevTables T, si
   qg_c *stage = reinterpret_cast<qg_c *>(info + V);             // [kStages][NE2] if STAGED
 
   const int tid = threadIdx.x;
-  const size_t nchunks = (n + V - 1) / V;
+  const size_t nchunks = (n + vc - 1) / vc;  // vc <= V translations per chunk
   int row_counter = 0;  // rows issued by this CTA (selects the stage buffer)
 
   for (size_t chunk = blockIdx.x; chunk < nchunks; chunk += gridDim.x) {
-    const size_t base = chunk * V;
+    const size_t base = chunk * vc;
     // ---------------- phase 1: per-translation factors ----------------
-    if (tid < V) {
+    if (tid < vc) {
       const size_t i = base + tid;
       VecInfo inf;
       inf.valid = (i < n);
@@ -133,14 +144,14 @@ __global__ void __launch_bounds__(kThreads) trans_ab_kernel(TransDevTables T, si
       info[tid] = inf;
     }
     __syncthreads();
-    for (int t = tid; t < V * (L + 1); t += kThreads) {
+    for (int t = tid; t < vc * (L + 1); t += kThreads) {
       const int v = t / (L + 1), m = t - v * (L + 1);
       legendre_column_rt(L, m, info[v].ct, leg + v * NL);
     }
     __syncthreads();
     // w[p^2+p+d] and w[p^2+p-d] share P_p^{|d|} z_p; the phases are conjugate
     constexpr int NPD = (L + 1) * (L + 2) / 2;  // (p, |d|) pairs
-    for (int t = tid; t < V * NPD; t += kThreads) {
+    for (int t = tid; t < vc * NPD; t += kThreads) {
       const int v = t / NPD, i = t - v * NPD;
       int p = (int)((sqrtf(8.0f * i + 1.0f) - 1.0f) * 0.5f);
       if ((p + 1) * (p + 2) / 2 <= i) ++p;
@@ -160,7 +171,7 @@ __global__ void __launch_bounds__(kThreads) trans_ab_kernel(TransDevTables T, si
     __syncthreads();
 
     // ---------------- phase 2: contraction ----------------
-    const int vmax = (int)((n - base) < (size_t)V ? (n - base) : (size_t)V);
+    const int vmax = (int)((n - base) < (size_t)vc ? (n - base) : (size_t)vc);
     for (int v = 0; v < vmax; ++v) {
       const qg_c *wv = w + v * S;
 #pragma unroll 1
@@ -168,7 +179,8 @@ __global__ void __launch_bounds__(kThreads) trans_ab_kernel(TransDevTables T, si
         const uint8_t *cnt = which ? T.cntB : T.cntA;
         const double *coef = which ? T.coefB : T.coefA;
         const uint16_t *slot = which ? T.slotB : T.slotA;
-        const int32_t *perm = which ? T.permB : T.perm;
+        const uint32_t *pair = which ? T.pairB : T.pairA;
+        const int nk = which ? T.nB : T.nA;
         qg_c *out = (which ? B : A) + (base + v) * (size_t)NE2;
         qg_c *buf = nullptr;
         if (STAGED) {
@@ -181,7 +193,7 @@ __global__ void __launch_bounds__(kThreads) trans_ab_kernel(TransDevTables T, si
           }
           __syncthreads();
         }
-        for (int k = tid; k < NE2; k += kThreads) {
+        for (int k = tid; k < nk; k += kThreads) {
           // term counts are sorted, so the trip count is (nearly) warp-uniform
           const int c = cnt[k];
           double sr = 0.0, si = 0.0;
@@ -189,17 +201,17 @@ __global__ void __launch_bounds__(kThreads) trans_ab_kernel(TransDevTables T, si
           const uint16_t *sq = slot + k;
 #pragma unroll 2
           for (int q = 0; q < c; ++q) {
-            const double a = __ldg(cq + q * NE2);
-            const qg_c x = wv[__ldg(sq + q * NE2)];
+            const double a = __ldg(cq + q * nk);
+            const qg_c x = wv[__ldg(sq + q * nk)];
             sr = fma(a, x.re, sr);
             si = fma(a, x.im, si);
           }
-          const qg_c r = which ? cmk(-si, sr) : cmk(sr, si);
-          const int e = __ldg(perm + k);
-          if (STAGED)
-            buf[e] = r;
-          else
-            out[e] = r;
+          const qg_c r = which ? cmk(xor_sign(si, kSignBit), sr) : cmk(sr, si);
+          const uint32_t pr = __ldg(pair + k);
+          const unsigned long long flip = pair_negated(pr) ? kSignBit : 0ull;
+          qg_c *o = STAGED ? buf : out;
+          o[pair_first(pr)] = r;
+          if (pair_second(pr) != pair_first(pr)) o[pair_second(pr)] = cmk(xor_sign(r.re, flip), xor_sign(r.im, flip));
         }
         if (STAGED) {
           fence_proxy_async_smem();
@@ -223,24 +235,18 @@ int launch_lmax(const TransDevTables &T, size_t n, const qg_c *kr, const double 
   int dev = 0, nsm = 0, per_sm = 0;
   QG_CUDA_TRY(cudaGetDevice(&dev));
   QG_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const size_t nchunks = (n + Sh::V - 1) / Sh::V;
-  if (staged) {
-    auto k = trans_ab_kernel<LMAX, Sh::kStaged>;
+  auto run = [&](auto k) -> int {
     QG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    QG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem));
-    if (per_sm < 1) per_sm = 1;
-    size_t grid = (size_t)nsm * per_sm;
-    if (grid > nchunks) grid = nchunks;
-    k<<<(unsigned)grid, kThreads, smem, st>>>(T, n, kr, th, ph, rgd, J, A, B);
-  } else {
-    auto k = trans_ab_kernel<LMAX, false>;
-    QG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    QG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem));
-    if (per_sm < 1) per_sm = 1;
-    size_t grid = (size_t)nsm * per_sm;
-    if (grid > nchunks) grid = nchunks;
-    k<<<(unsigned)grid, kThreads, smem, st>>>(T, n, kr, th, ph, rgd, J, A, B);
-  }
+    QG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, Sh::kThreads, smem));
+    const size_t resident = (size_t)nsm * std::max(per_sm, 1);
+    // few translations: fewer in a chunk, so that every resident CTA has one
+    const int vc = (int)std::min<size_t>(Sh::V, (n + resident - 1) / resident);
+    const size_t grid = std::min(resident, (n + vc - 1) / vc);
+    k<<<(unsigned)grid, Sh::kThreads, smem, st>>>(T, n, vc, kr, th, ph, rgd, J, A, B);
+    return QPMS_SUCCESS;
+  };
+  const int e = staged ? run(trans_ab_kernel<LMAX, Sh::kStaged>) : run(trans_ab_kernel<LMAX, false>);
+  if (e) return e;
   QG_CUDA_TRY(cudaGetLastError());
   g_launches.fetch_add(1);
   return QPMS_SUCCESS;
