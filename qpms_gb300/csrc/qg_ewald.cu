@@ -143,12 +143,233 @@ __device__ __forceinline__ void even_nm(int k, int &n, int &m) {
 }
 
 
+// Class of a reciprocal point |beta + K| = rb: 0 past the cutoff (x^2 > 56),
+// 1 evanescent at real k (gamma and x real), 2 otherwise; gamma and the branch
+// of x = gamma k / 2 eta (clilgamma, ewald.h:157-170, and ewald.c:390-393).
+__device__ __forceinline__ int lr_class(qg_c k, bool kreal, double eta, double rb, qg_c &gam, qg_c &uu) {
+  if (kreal) {
+    // clilgamma(rb / k) for real k: sqrt(t - 1) sqrt(t + 1) with t - 1 exact;
+    // near a Rayleigh anomaly (t -> 1) the 1/gamma terms dominate, so gamma is
+    // formed from the exact differences as there
+    const double tt = rb / k.re;
+    if (tt >= 1.0) {
+      gam = cmk(sqrt(tt - 1.0) * sqrt(tt + 1.0), 0.0);
+      const double x = gam.re * k.re / (2 * eta);
+      if (x * x > 56.0) return 0;
+      uu = cmk(x, 0.0);
+      return 1;
+    }
+    const double g = sqrt(1.0 - tt) * sqrt(1.0 + tt);
+    gam = cmk(0.0, -g);  // -i sqrt(1 - t^2)
+    // x^2 = -(g k / 2 eta)^2, approached from below the negative axis: sqrt -> -i c
+    uu = cmk(0.0, -g * k.re / (2 * eta));
+    return 2;
+  }
+  // z = rb / k as C's real / complex division forms it: (rb + 0i)(conj k) / |k|^2.
+  // The sign of a zero imaginary part (rb = 0, i.e. beta on a reciprocal
+  // lattice point) picks the branch of a1 below, so it must be +0 as there.
+  const double kk2 = k.re * k.re + k.im * k.im;
+  const qg_c z = cmk((rb * k.re + 0.0 * k.im) / kk2, (0.0 * k.re - rb * k.im) / kk2);
+  qg_c a1 = cmk(z.re - 1, z.im), a2 = cmk(z.re + 1, z.im);
+  a2 = (a2.re < 0 && a2.im <= 0) ? cscale(csqrt_(a2), -1.0) : csqrt_(a2);
+  a1 = (a1.re < 0 && a1.im >= 0) ? cscale(csqrt_(a1), -1.0) : csqrt_(a1);
+  gam = cmul(a1, a2);
+  const qg_c x = cscale(cmul(gam, k), 1.0 / (2 * eta));
+  const qg_c x2 = cmul(x, x);
+  if (x2.re > 56.0) return 0;
+  uu = csqrt_(x2);
+  if (x2.re < 0 && !signbit(x2.im)) uu = cscale(uu, -1.0);  // branch m = -1 (ewald.c:390-393)
+  return 2;
+}
+
+// ---------------- layers apart: the reciprocal-lattice sum ----------------
+// eta -> infinity for a shift w = -shift.z off the plane: every order is a plane
+// or evanescent wave of complex direction, at which the spherical harmonic has
+// a closed form.  With q = beta + K, gamma = sqrt(q^2 / k^2 - 1) on the branch
+// of clilgamma, cos(theta) = i sgn(w) gamma and sin(theta) = q / k,
+//   sigma_nm = (-i)^(n+1) 2 pi / (k^2 A) sum_K e^{iK.s} e^{-gamma k |w|} / gamma
+//              P_n^|m|(i sgn(w) gamma) (-1)^m e^{i m alpha}
+// (and the reference's sign (-1)^m for m < 0; P with the Condon-Shortley phase).  P_n^m / sin^m, scaled to be monic,
+// obeys Q_{j+1} = x Q_j - c Q_{j-1}; at x = i sgn(w) gamma it is
+// (i sgn w)^j q_j with q_{j+1} = gamma q_j + c q_{j-1}, a sum of positive real
+// numbers for the evanescent orders of a real k (all but a few), two FP64
+// operations per (n, m).  The terms are taken up to q |w| = C(lMax), past which
+// q^(2 lMax + 1) e^{-q |w|} sums to less than 1e-20 of the whole.
+//
+// Bound: the FP64 pipe, about 220 operations per reciprocal point at lMax 2
+// against some 2,700 for Kambe's double sum over (j, s) at each point.
+template <int LMAX>
+struct SpecShape {
+  static constexpr int LE = 2 * LMAX + 1;
+  static constexpr double kCut = LMAX == 1 ? 58 : (LMAX == 2 ? 63 : (LMAX == 3 ? 68 : 72));
+  // accumulators of the orders |m| = m0 .. m1
+  static constexpr __host__ __device__ int count(int m0, int m1) {
+    int c = 0;
+    for (int m = m0; m <= m1; ++m) c += (LE - m + 1) * (m ? 2 : 1);
+    return c;
+  }
+  // last |m| of the pass that starts at m0: at most 36 accumulators
+  static constexpr __host__ __device__ int last(int m0) {
+    int m1 = m0;
+    while (m1 < LE && count(m0, m1 + 1) <= 36) ++m1;
+    return m1;
+  }
+};
+
+// 2D lattice phases e^{iK.s}, K = i rb1 + j rb2, as products of two rows of
+// factors in shared memory (kSpecTab / 2 each; longer rows are not tabulated)
+constexpr int kSpecTab = 512;
+constexpr double kSpecPoints = 4000;
+
+struct SpecUnit {
+  qg_c k;
+  double bx, by, sx, sy, w, pmax;
+  int I1, I2;  // index ranges of K; W1 W2 <= kEwMaxPoints
+  bool tab;    // the factor rows are in use
+};
+
+template <int LMAX, int M0>
+__device__ __forceinline__ void spectral_passes(const SpecUnit &u, const qg_c *tab, qg_c *sig,
+                                                qg_c (*red)[EwShape<LMAX>::RED]) {
+  constexpr int LE = EwShape<LMAX>::LE, M1 = SpecShape<LMAX>::last(M0), NA = SpecShape<LMAX>::count(M0, M1);
+  static_assert(NA <= EwShape<LMAX>::RED, "reduction buffer");
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const qg_c k = u.k, rk = crecip(k);
+  const double aw = fabs(u.w), pmax2 = u.pmax * u.pmax, k2 = k.re * k.re;
+  const bool kreal = k.im == 0.0 && k.re > 0;
+  const int W1 = 2 * u.I1 + 1, W2 = 2 * u.I2 + 1;
+  qg_c acc[NA];
+#pragma unroll
+  for (int i = 0; i < NA; ++i) acc[i] = cmk(0, 0);
+  for (int t = tid; t < W1 * W2; t += kEThreads) {
+    const int i = t / W2, j = t - i * W2;
+    const double Kx = (i - u.I1) * c_ew.rb[0] + (j - u.I2) * c_ew.rb[2];
+    const double Ky = (i - u.I1) * c_ew.rb[1] + (j - u.I2) * c_ew.rb[3];
+    const double qx = Kx + u.bx, qy = Ky + u.by, q2 = fma(qx, qx, qy * qy);
+    if (q2 > pmax2) continue;
+    qg_c ph;
+    if (u.tab) {
+      ph = cmul(tab[i], tab[kSpecTab / 2 + j]);
+    } else {
+      double sn, cs;
+      sincos(Kx * u.sx + Ky * u.sy, &sn, &cs);
+      ph = cmk(cs, sn);
+    }
+    if (kreal && q2 > k2) {
+      // gamma from the exact difference q/k - 1 (near a Rayleigh anomaly 1 / gamma dominates)
+      const double tt = sqrt(q2) / k.re, g2 = (tt - 1.0) * (tt + 1.0), rg = rsqrt(g2), g = g2 * rg;
+      ph = cscale(ph, exp(-g * k.re * aw) * rg);
+      const double px = qx * rk.re, py = qy * rk.re;
+      double a = 1.0, b = 0.0;  // ((q_x + i q_y) / k)^m
+#pragma unroll
+      for (int m = 1; m < M0; ++m) {
+        const double a1 = fma(a, px, -b * py);
+        b = fma(a, py, b * px);
+        a = a1;
+      }
+      int e = 0;
+#pragma unroll
+      for (int m = M0; m <= M1; ++m) {
+        if (m > 0) {
+          const double a1 = fma(a, px, -b * py);
+          b = fma(a, py, b * px);
+          a = a1;
+        }
+        const qg_c vp = m ? cmk(fma(ph.re, a, -ph.im * b), fma(ph.re, b, ph.im * a)) : ph;
+        const qg_c vm = cmk(fma(ph.re, a, ph.im * b), fma(-ph.re, b, ph.im * a));
+        double q0 = 0.0, q1 = 1.0;
+#pragma unroll
+        for (int n = m; n <= LE; ++n) {
+          if (n > m) {
+            const double c = ((n - 1) * (n - 1) - m * m) / (4.0 * (n - 1) * (n - 1) - 1);
+            const double qn = n == m + 1 ? g : fma(g, q1, c * q0);
+            q0 = q1;
+            q1 = qn;
+          }
+          acc[e] = cmk(fma(q1, vp.re, acc[e].re), fma(q1, vp.im, acc[e].im));
+          ++e;
+          if (m) {
+            acc[e] = cmk(fma(q1, vm.re, acc[e].re), fma(q1, vm.im, acc[e].im));
+            ++e;
+          }
+        }
+      }
+    } else {
+      qg_c gam, uu;
+      lr_class(k, k.im == 0.0, 1e300, sqrt(q2), gam, uu);  // the branch of gamma; no cutoff
+      const qg_c ga = cscale(cmul(gam, k), aw);
+      ph = cmul(cmul(ph, cexpi(cmk(-ga.im, ga.re))), crecip(gam));
+      const qg_c fp = cmul(cmk(qx, qy), rk), fm = cmul(cmk(qx, -qy), rk);
+      qg_c vp = ph, vm = ph;
+#pragma unroll
+      for (int m = 1; m < M0; ++m) {
+        vp = cmul(vp, fp);
+        vm = cmul(vm, fm);
+      }
+      int e = 0;
+#pragma unroll
+      for (int m = M0; m <= M1; ++m) {
+        if (m > 0) {
+          vp = cmul(vp, fp);
+          vm = cmul(vm, fm);
+        }
+        qg_c q0 = cmk(0, 0), q1 = cmk(1.0, 0.0);
+#pragma unroll
+        for (int n = m; n <= LE; ++n) {
+          if (n > m) {
+            const double c = ((n - 1) * (n - 1) - m * m) / (4.0 * (n - 1) * (n - 1) - 1);
+            const qg_c qn = cadd(cmul(gam, q1), cscale(q0, c));
+            q0 = q1;
+            q1 = qn;
+          }
+          acc[e] = cadd(acc[e], cmul(q1, vp));
+          ++e;
+          if (m) {
+            acc[e] = cadd(acc[e], cmul(q1, vm));
+            ++e;
+          }
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NA; ++i) {
+    double re = acc[i].re, im = acc[i].im;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      re += __shfl_xor_sync(0xffffffffu, re, o);
+      im += __shfl_xor_sync(0xffffffffu, im, o);
+    }
+    if (lane == 0) red[warp][i] = cmk(re, im);
+  }
+  __syncthreads();
+  if (tid < NA) {
+    qg_c v = cmk(0, 0);
+    for (int wq = 0; wq < kEThreads / 32; ++wq) v = cadd(v, red[wq][tid]);
+    // which (n, m) this accumulator is
+    int m = M0, e = tid;
+    for (int c; e >= (c = (LE - m + 1) * (m ? 2 : 1)); ++m) e -= c;
+    const int n = m + (m ? e / 2 : e);
+    const bool neg = m && (e & 1);
+    double f = 2 * 3.14159265358979323846 / c_ew.area;  // times (2n)! / (2^n n! (n - m)!)
+    for (int x = 1; x <= n; ++x) f *= 2 * x - 1;
+    for (int x = 2; x <= n - m; ++x) f /= x;
+    // (-i)^(n+1) (i sgn w)^(n-m); legs: (-1)^m for m < 0 and the normalisation's phase
+    const int y = n * (n + 1) + (neg ? -m : m);
+    int quarter = -(n + 1) + (n - m) + (u.w < 0 ? 2 * (n - m) : 0);
+    v = cscale(cmul(v, cmul(rk, rk)), f * c_ew.legs[y]);
+    for (quarter = ((quarter % 4) + 4) % 4; quarter; --quarter) v = cmk(-v.im, v.re);
+    sig[y] = v;
+  }
+  __syncthreads();
+  if constexpr (M1 < LE) spectral_passes<LMAX, M1 + 1>(u, tab, sig, red);
+}
+
 // Unit data shared by the passes of one shifted pair.
 struct ZUnit {
   qg_c k;
   double eta, bx, by, sx, sy, w;
   int KM;         // terms of the Delta series
-  int spectral;   // 1: pure reciprocal-lattice sum (distant layers, |k w| >= 2.5)
 };
 
 // One pass of the shifted sums: sigma_y for Y0 <= y < Y0 + NY into sig[].
@@ -166,8 +387,8 @@ __device__ __forceinline__ void shifted_pass(const ZUnit &u, const qg_c *s1u, co
   for (int i = 0; i < NY; ++i) acc[i] = cmk(0, 0);
   const double sqpi = 1.7724538509055160273;
 
-  // ---------------- short range (none for the reciprocal-lattice sum) ----------------
-  if (!u.spectral) {
+  // ---------------- short range ----------------
+  {
     const double rc = 7.5 / eta;
     const double smax = sqrt(u.sx * u.sx + u.sy * u.sy);
     const int I1 = (int)ceil((rc + smax) * c_ew.rbn[0] / (2 * M_PI)) + 1;
@@ -254,11 +475,8 @@ __device__ __forceinline__ void shifted_pass(const ZUnit &u, const qg_c *s1u, co
   // ---------------- long range ----------------
   {
     const double kap2 = k.re * k.re + k.im * k.im;
-    const double aw = fabs(w);
-    // Ewald: terms below e^-56 past x^2 = 56; reciprocal-lattice sum: the terms
-    // fall like e^(-|beta + K| |w|) (|beta + K|/k)^(2 lMax + 1), below 1e-17 past |beta + K| |w| = 80
-    const double pmax = u.spectral ? 80.0 / aw : sqrt(kap2 + 56.0 * 4 * eta * eta);
-    const double Kc = pmax + sqrt(u.bx * u.bx + u.by * u.by);
+    // terms below e^-56 past x^2 = 56
+    const double Kc = sqrt(kap2 + 56.0 * 4 * eta * eta) + sqrt(u.bx * u.bx + u.by * u.by);
     const int I1 = (int)ceil(Kc * c_ew.bn[0] / (2 * M_PI)) + 1;
     const int I2 = (int)ceil(Kc * c_ew.bn[1] / (2 * M_PI)) + 1;
     const int W1 = 2 * I1 + 1, W2 = 2 * I2 + 1;
@@ -266,59 +484,16 @@ __device__ __forceinline__ void shifted_pass(const ZUnit &u, const qg_c *s1u, co
     if (!lr_ok && tid == 0) atomicOr(errflag, 1);
     const qg_c rk = crecip(k);
     const qg_c lrfac = crecip(cscale(cmul(k, k), c_ew.area));
-    const qg_c kaw = cscale(k, aw);
-    const qg_c rkaw = crecip(kaw);
     const int KM = u.KM;
     for (int t = tid; lr_ok && t < W1 * W2; t += kEThreads) {
       const int i = t / W2 - I1, j = t % W2 - I2;
       const double Kx = i * c_ew.rb[0] + j * c_ew.rb[2], Ky = i * c_ew.rb[1] + j * c_ew.rb[3];
       const double qx = Kx + u.bx, qy = Ky + u.by;
       const double rb = sqrt(qx * qx + qy * qy);
-      if (u.spectral && rb > pmax) continue;
       qg_c gam, uu;
-      if (kreal) {
-        const double tt = rb / k.re;
-        if (tt >= 1.0) {
-          gam = cmk(sqrt(tt - 1.0) * sqrt(tt + 1.0), 0.0);
-          const double x = gam.re * k.re / (2 * eta);
-          if (!u.spectral && x * x > 56.0) continue;
-          uu = cmk(x, 0.0);
-        } else {
-          const double g = sqrt(1.0 - tt) * sqrt(1.0 + tt);
-          gam = cmk(0.0, -g);
-          uu = cmk(0.0, -g * k.re / (2 * eta));
-        }
-      } else {
-        const double kk2 = k.re * k.re + k.im * k.im;
-        const qg_c z = cmk((rb * k.re + 0.0 * k.im) / kk2, (0.0 * k.re - rb * k.im) / kk2);
-        qg_c a1 = cmk(z.re - 1, z.im), a2 = cmk(z.re + 1, z.im);
-        a2 = (a2.re < 0 && a2.im <= 0) ? cscale(csqrt_(a2), -1.0) : csqrt_(a2);
-        a1 = (a1.re < 0 && a1.im >= 0) ? cscale(csqrt_(a1), -1.0) : csqrt_(a1);
-        gam = cmul(a1, a2);
-        const qg_c x = cscale(cmul(gam, k), 1.0 / (2 * eta));
-        const qg_c x2 = cmul(x, x);
-        if (!u.spectral && x2.re > 56.0) continue;
-        uu = csqrt_(x2);
-        if (x2.re < 0 && !signbit(x2.im)) uu = cscale(uu, -1.0);
-      }
+      if (!lr_class(k, kreal, eta, rb, gam, uu)) continue;
       qg_c D[LE + 1];
-      if (u.spectral) {
-        // gamma^(2j-1) Delta_j(0, z) = sqrt(pi) 2^j (k|w|)^-j e^-a Kt_j, a = gamma k |w|,
-        // Kt_j = gamma^(j-1) kappa_j(a) (half-integer Bessel K); sqrt(pi) 2^j (k|w|)^-j is in s1u
-        const qg_c a = cmul(gam, kaw);
-        const qg_c ea = cexpi(cmk(-a.im, a.re));  // e^-a
-        const qg_c g2 = cmul(gam, gam);
-        qg_c km1 = crecip(gam), kc = cmk(1.0, 0.0);
-        D[0] = cmul(km1, ea);
-        if (LE >= 1) D[1] = ea;
-#pragma unroll
-        for (int jq = 1; jq < LE; ++jq) {
-          const qg_c kn = cadd(cmul(g2, km1), cscale(cmul(kc, rkaw), 2 * jq - 1));
-          km1 = kc;
-          kc = kn;
-          D[jq + 1] = cmul(kn, ea);
-        }
-      } else {
+      {
         // D_a = sum_q r_q g_(a+q), g_i = X^i Gamma(1/2 - i, X)
         const qg_c X = cmul(uu, uu);
         const qg_c emX = cexpi(cmk(-X.im, X.re));
@@ -406,45 +581,6 @@ __device__ __forceinline__ void shifted_passes(const ZUnit &u, const qg_c *s1u, 
 }
 
 constexpr int kELChunks = 8;  // reciprocal-point chunks classified per batch
-
-// Class of a reciprocal point |beta + K| = rb: 0 past the cutoff (x^2 > 56),
-// 1 evanescent at real k (gamma and x real), 2 otherwise; gamma and the branch
-// of x = gamma k / 2 eta (clilgamma, ewald.h:157-170, and ewald.c:390-393).
-__device__ __forceinline__ int lr_class(qg_c k, bool kreal, double eta, double rb, qg_c &gam, qg_c &uu) {
-  if (kreal) {
-    // clilgamma(rb / k) for real k: sqrt(t - 1) sqrt(t + 1) with t - 1 exact;
-    // near a Rayleigh anomaly (t -> 1) the 1/gamma terms dominate, so gamma is
-    // formed from the exact differences as there
-    const double tt = rb / k.re;
-    if (tt >= 1.0) {
-      gam = cmk(sqrt(tt - 1.0) * sqrt(tt + 1.0), 0.0);
-      const double x = gam.re * k.re / (2 * eta);
-      if (x * x > 56.0) return 0;
-      uu = cmk(x, 0.0);
-      return 1;
-    }
-    const double g = sqrt(1.0 - tt) * sqrt(1.0 + tt);
-    gam = cmk(0.0, -g);  // -i sqrt(1 - t^2)
-    // x^2 = -(g k / 2 eta)^2, approached from below the negative axis: sqrt -> -i c
-    uu = cmk(0.0, -g * k.re / (2 * eta));
-    return 2;
-  }
-  // z = rb / k as C's real / complex division forms it: (rb + 0i)(conj k) / |k|^2.
-  // The sign of a zero imaginary part (rb = 0, i.e. beta on a reciprocal
-  // lattice point) picks the branch of a1 below, so it must be +0 as there.
-  const double kk2 = k.re * k.re + k.im * k.im;
-  const qg_c z = cmk((rb * k.re + 0.0 * k.im) / kk2, (0.0 * k.re - rb * k.im) / kk2);
-  qg_c a1 = cmk(z.re - 1, z.im), a2 = cmk(z.re + 1, z.im);
-  a2 = (a2.re < 0 && a2.im <= 0) ? cscale(csqrt_(a2), -1.0) : csqrt_(a2);
-  a1 = (a1.re < 0 && a1.im >= 0) ? cscale(csqrt_(a1), -1.0) : csqrt_(a1);
-  gam = cmul(a1, a2);
-  const qg_c x = cscale(cmul(gam, k), 1.0 / (2 * eta));
-  const qg_c x2 = cmul(x, x);
-  if (x2.re > 56.0) return 0;
-  uu = csqrt_(x2);
-  if (x2.re < 0 && !signbit(x2.im)) uu = cscale(uu, -1.0);  // branch m = -1 (ewald.c:390-393)
-  return 2;
-}
 
 // M[R, C] = delta_RC I - T_R W(R <- C) from sigma in shared memory
 // (translations.c:926-1078 contraction; the B sum runs over q <= qmax_A).
@@ -1004,6 +1140,7 @@ __global__ void __launch_bounds__(kEThreads) ewald_layers_kernel(EwaldArgs a, Tr
   __shared__ qg_c sig[S];
   __shared__ qg_c red[kEThreads / 32][Sh::RED];
   __shared__ qg_c s1u[kEwZ];
+  __shared__ qg_c tab[kSpecTab];
   __shared__ double rr[48];
   const int tid = threadIdx.x;
   const int np = a.np;
@@ -1022,12 +1159,47 @@ __global__ void __launch_bounds__(kEThreads) ewald_layers_kernel(EwaldArgs a, Tr
     const double sz = a.pos[3 * R + 2] - a.pos[3 * C + 2];
     if (sz == 0.0) continue;  // ewald_assemble_kernel
     // ---------------- layers at different heights ----------------
+    // The reciprocal-lattice sum for distant layers (|k sz| >= 2.5, where the Ewald sums
+    // cancel) and wherever it takes at most kSpecPoints points; else Ewald with
+    // eta <= 1 / |sz| for the Delta series, which keeps k / (2 eta) <= 1.25.  A scan of
+    // 100 (omega, k), reciprocal sum against Ewald (ms): lMax 2, 4,752 points 1.62 : 1.57,
+    // 7,425 1.99 : 1.56; lMax 4, 6,236 4.57 : 4.72, 17,324 8.9 : 6.0.
+    const double pcut = SpecShape<LMAX>::kCut / fabs(sz);
+    const bool spectral = hypot(k.re, k.im) * fabs(sz) >= 2.5 || pcut * pcut * c_ew.area <= kSpecPoints * 4 * M_PI;
+    if (spectral) {
+      SpecUnit su;
+      su.k = k;
+      su.bx = bx;
+      su.by = by;
+      su.sx = sx;
+      su.sy = sy;
+      su.w = -sz;
+      su.pmax = pcut;
+      const double Kc = pcut + sqrt(bx * bx + by * by);
+      su.I1 = (int)ceil(Kc * c_ew.bn[0] / (2 * M_PI)) + 1;
+      su.I2 = (int)ceil(Kc * c_ew.bn[1] / (2 * M_PI)) + 1;
+      const int W1 = 2 * su.I1 + 1, W2 = 2 * su.I2 + 1;
+      if (!((long)W1 * W2 <= kEwMaxPoints && su.I1 >= 0 && su.I2 >= 0)) {
+        if (tid == 0) atomicOr(a.err, 1);
+        su.I1 = su.I2 = 0;
+      }
+      su.tab = W1 <= kSpecTab / 2 && W2 <= kSpecTab / 2;
+      if (su.tab)
+        for (int t = tid; t < W1 + W2; t += kEThreads) {
+          const int d = t < W1 ? 0 : 2, i = t < W1 ? t - su.I1 : t - W1 - su.I2;
+          double sn, cs;
+          sincos(i * (c_ew.rb[d] * sx + c_ew.rb[d + 1] * sy), &sn, &cs);
+          tab[t < W1 ? t : kSpecTab / 2 + t - W1] = cmk(cs, sn);
+        }
+      __syncthreads();
+      spectral_passes<LMAX, 0>(su, tab, sig, red);
+      contract_block<LMAX>(a, T, sig, wk, per, pr, R, C, iw);
+      __syncthreads();
+      continue;
+    }
     ZUnit zu;
     zu.k = k;
     zu.w = -sz;
-    // distant layers (|k sz| >= 2.5): the pure reciprocal-lattice sum; else
-    // eta <= 1 / |sz| for the Delta series, which keeps k / (2 eta) <= 1.25
-    zu.spectral = hypot(k.re, k.im) * fabs(sz) >= 2.5;
     zu.eta = fmin(eta, 1.0 / fabs(sz));
     zu.bx = bx;
     zu.by = by;
@@ -1051,21 +1223,14 @@ __global__ void __launch_bounds__(kEThreads) ewald_layers_kernel(EwaldArgs a, Tr
       }
     }
     {
-      // Ewald: S1 (k w)^(2j - s) (2 eta / k)^(2j);
-      // reciprocal-lattice sum: S1 sqrt(pi) 2^j sgn(w)^s (k |w|)^(j - s)
+      // S1 (k w)^(2j - s) (2 eta / k)^(2j)
       const qg_c kw = cscale(k, zu.w), te = cscale(crecip(k), 2 * zu.eta);
       const qg_c te2 = cmul(te, te);
-      const qg_c rkaw = crecip(cscale(k, fabs(zu.w)));
       for (int e = tid; e < c_ew.zoff[S]; e += kEThreads) {
         const int jq = c_ew.zj[e], sv = c_ew.zsv[e];
         qg_c f = c_ew.zs1[e];
-        if (zu.spectral) {
-          f = cscale(f, 1.7724538509055160273 * (double)(1 << jq) * ((zu.w < 0 && (sv & 1)) ? -1.0 : 1.0));
-          for (int q = 0; q < sv - jq; ++q) f = cmul(f, rkaw);
-        } else {
-          for (int q = 0; q < 2 * jq - sv; ++q) f = cmul(f, kw);
-          for (int q = 0; q < jq; ++q) f = cmul(f, te2);
-        }
+        for (int q = 0; q < 2 * jq - sv; ++q) f = cmul(f, kw);
+        for (int q = 0; q < jq; ++q) f = cmul(f, te2);
         s1u[e] = f;
       }
     }
