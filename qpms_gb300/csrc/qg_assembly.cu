@@ -249,15 +249,98 @@ __global__ void incident_kernel(int nw, int np, int n, const qg_c *coef, size_t 
   }
 }
 
-// b[w][p*n + i] = sum_j T_w,tm(p)[i][j] a[w][p*n + j]  (diag: T[i] a[i])
-__global__ void apply_t_kernel(int nw, int np, int n, int ntm, int dense, const int *tmid, const qg_c *T,
+// Incidence of the lattice scan, one thread per (frequency w, Bloch vector k):
+// the plane wave of in-plane wavevector k and E along x made transverse (x at
+// normal incidence), kvec its wavevector, coef its regular-wave coefficients
+// (electric, then magnetic; vswf.c:445-467 with the dual harmonics, as
+// planewave_coeffs of the host), all zero where the order is evanescent
+// (|k| >= Re kappa_w), kk the medium wavenumber.  pi = m P / sin th comes from
+// P / sin th's own recurrence and tau = dP/dth from neighbouring orders, so the
+// polar axis needs no branch.  4,096 wavevectors took 4 ms on the host.
+constexpr int kIncLMax = 6;
+struct IncTables {
+  double nf[(kIncLMax + 1) * (kIncLMax + 2) / 2];  // sqrt((2l+1)/(4 pi l(l+1)) (l-m)!/(l+m)!)
+};
+
+__global__ void __launch_bounds__(128) scan_incidence_kernel(int nw, int nk, int lMax, IncTables tb, const qg_c *kappa,
+                                                             const double *beta, qg_c *coef, double *kvec, qg_c *kk) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nw * nk) return;
+  const int w = t / nk, ik = t - w * nk, ne = lMax * (lMax + 2);
+  const double kap = kappa[w].re, bx = beta[2 * ik], by = beta[2 * ik + 1], b2 = bx * bx + by * by;
+  const bool prop = kap * kap > b2;
+  const double kz = prop ? sqrt(kap * kap - b2) : 0.0, kn = sqrt(b2 + kz * kz);
+  kk[t] = kappa[w];
+  kvec[3 * t] = bx;
+  kvec[3 * t + 1] = by;
+  kvec[3 * t + 2] = kz;
+  qg_c *el = coef + (size_t)t * 2 * ne, *mg = el + ne;
+  if (!prop) {
+    for (int y = 0; y < 2 * ne; ++y) el[y] = cmk(0, 0);
+    return;
+  }
+  const double rho = sqrt(b2), ct = kz / kn, st = rho / kn, cf = rho > 0 ? bx / rho : 1.0, sf = rho > 0 ? by / rho : 0.0;
+  const double ux = bx / kn;
+  double E[3] = {1.0 - ux * bx / kn, -ux * by / kn, -ux * kz / kn};
+  const double En = sqrt(E[0] * E[0] + E[1] * E[1] + E[2] * E[2]);
+  const double Et = (E[0] * ct * cf + E[1] * ct * sf - E[2] * st) / En, Ep = (E[1] * cf - E[0] * sf) / En;
+  // columns m - 1, m, m + 1 of P_l^m, and P_l^m / sin for m
+  double Pm[kIncLMax + 2], P0[kIncLMax + 2], Pp[kIncLMax + 2], R[kIncLMax + 2];
+  auto column = [&](int m, double first, double *out) {  // out[l], l = m .. lMax + 1, from its first entry
+    double a = 0.0, b = first;
+    for (int l = 0; l < m && l <= lMax + 1; ++l) out[l] = 0.0;
+    for (int l = m; l <= lMax + 1; ++l) {
+      out[l] = b;
+      const double nx = ((2 * l + 1) * ct * b - (l + m) * a) / (l + 1 - m);
+      a = b;
+      b = nx;
+    }
+  };
+  double pmm = 1.0;  // P_m^m
+  column(0, 1.0, P0);
+  column(1, -st, Pp);
+  qg_c em = cmk(1.0, 0.0);  // e^{-i m phi}
+  for (int m = 0; m <= lMax; ++m) {
+    if (m > 0) {
+      for (int l = 0; l <= lMax + 1; ++l) {
+        Pm[l] = P0[l];
+        P0[l] = Pp[l];
+      }
+      column(m, m == 1 ? -1.0 : -(2 * m - 1) * pmm, R);  // P / sin: its first entry is -(2m - 1) P_{m-1}^{m-1}
+      pmm *= -(2 * m - 1) * st;
+      column(m + 1, -(2 * m + 1) * st * pmm, Pp);
+      em = cmul(em, cmk(cf, -sf));
+    }
+    for (int l = m > 1 ? m : 1; l <= lMax; ++l) {
+      const double nf = 4 * 3.14159265358979323846 * tb.nf[l * (l + 1) / 2 + m];
+      const double pi = m ? nf * m * R[l] : 0.0;
+      const double tau = m ? -0.5 * nf * ((l + m) * (l - m + 1) * Pm[l] - Pp[l]) : nf * Pp[l];
+      for (int sg = 0; sg < (m ? 2 : 1); ++sg) {
+        // order -m: pi (-1)^(m+1), tau (-1)^m, conjugate phase
+        const double f = (sg && (m & 1)) ? -1.0 : 1.0, pl = sg ? -f * pi : pi, tl = f * tau;
+        const qg_c e = sg ? cconj(em) : em;
+        qg_c a = cmul(cmk(-tl * Ep, -pl * Et), e), b = cmul(cmk(-tl * Et, pl * Ep), e);
+        // a i^l (magnetic), b i^(l+1) (electric)
+        for (int q = 0; q < (l & 3); ++q) a = cmk(-a.im, a.re);
+        for (int q = 0; q < ((l + 1) & 3); ++q) b = cmk(-b.im, b.re);
+        const int y = l * (l + 1) + (sg ? -m : m) - 1;
+        mg[y] = a;
+        el[y] = b;
+      }
+    }
+  }
+}
+
+// b[w][p*n + i] = sum_j T_w,tm(p)[i][j] a[w][p*n + j]  (diag: T[i] a[i]); tper
+// consecutive w share a T
+__global__ void apply_t_kernel(int nw, int np, int n, int ntm, int dense, int tper, const int *tmid, const qg_c *T,
                                const qg_c *a, qg_c *b) {
   const size_t N = (size_t)np * n, tot = (size_t)nw * N;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < tot; t += (size_t)gridDim.x * blockDim.x) {
     const int w = (int)(t / N);
     const size_t r = t - (size_t)w * N;
     const int p = (int)(r / n), i = (int)(r - (size_t)p * n);
-    const qg_c *Tp = T + ((size_t)w * ntm + tmid[p]) * (dense ? (size_t)n * n : n);
+    const qg_c *Tp = T + ((size_t)(w / tper) * ntm + tmid[p]) * (dense ? (size_t)n * n : n);
     if (!dense) {
       b[t] = cmul(Tp[i], a[t]);
     } else {
@@ -389,9 +472,29 @@ int launch_incident(int nw, int np, int n, const qg_c *coef, const double *kvec,
   return QPMS_SUCCESS;
 }
 
+int launch_scan_incidence(int nw, int nk, int lMax, const qg_c *kappa, const double *beta, qg_c *coef, double *kvec,
+                          qg_c *kk, cudaStream_t st) {
+  if (lMax < 1 || lMax > kIncLMax) {
+    set_error("scan incidence: lMax %d", lMax);
+    return QPMS_EINVAL;
+  }
+  IncTables tb;
+  for (int l = 0; l <= kIncLMax; ++l)
+    for (int m = 0; m <= l; ++m) {
+      double f = l ? (2 * l + 1) / (4 * M_PI * l * (l + 1)) : 0.0;
+      for (int x = l - m + 1; x <= l + m; ++x) f /= x;
+      tb.nf[l * (l + 1) / 2 + m] = sqrt(f);
+    }
+  scan_incidence_kernel<<<(unsigned)(((size_t)nw * nk + 127) / 128), 128, 0, st>>>(nw, nk, lMax, tb, kappa, beta, coef,
+                                                                                   kvec, kk);
+  QG_CUDA_TRY(cudaGetLastError());
+  g_launches.fetch_add(1);
+  return QPMS_SUCCESS;
+}
+
 int launch_apply_t(int nw, int np, int n, int ntm, int dense, const int *tmid, const qg_c *T, const qg_c *a,
-                   qg_c *b, cudaStream_t st) {
-  apply_t_kernel<<<grid_for((size_t)nw * np * n, 256), 256, 0, st>>>(nw, np, n, ntm, dense, tmid, T, a, b);
+                   qg_c *b, cudaStream_t st, int tper) {
+  apply_t_kernel<<<grid_for((size_t)nw * np * n, 256), 256, 0, st>>>(nw, np, n, ntm, dense, tper, tmid, T, a, b);
   QG_CUDA_TRY(cudaGetLastError());
   g_launches.fetch_add(1);
   return QPMS_SUCCESS;

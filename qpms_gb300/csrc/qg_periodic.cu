@@ -11,6 +11,7 @@
 #include <mutex>
 #include <vector>
 
+#include "qg_arena.h"
 #include "qg_assembly.h"
 #include "qg_batched.h"
 #include "qg_ewald.h"
@@ -22,8 +23,6 @@ bool scatsys_is_own(const qpms_scatsys_t *ss);
 int scatsys_lmax(const qpms_scatsys_t *ss);
 void scatsys_tdiag(const qpms_scatsys_t *ss, int t, double om_re, double om_im, std::vector<qg_c> &out);
 qg_c scatsys_wavenumber(const qpms_scatsys_t *ss, double om_re, double om_im);
-void planewave_direction_coeffs(int lMax, const double k_dir[3], const qpms_complex_t E_cart[3],
-                                std::vector<qg_c> &coef);
 int blas_handle_get(cublasHandle_t *h);
 bool scatsys_dense(const qpms_scatsys_t *ss);
 
@@ -617,90 +616,62 @@ int qpms_gpu_periodic_scan(const qpms_scatsys_t *ss, size_t nw, const double *om
     pos[3 * i + 2] = ss->p[i].pos.z;
     tm[i] = ss->p[i].tmatrix_id;
   }
-  Dev dM, dscr, dlog, dT, dtm, dpos, dk, dkv, dcf, da, db, dx, dsig;
-  const size_t nmat = (size_t)wchunk * nk;
-  if ((e = dalloc(dM, nmat * N2 * 16)) || (e = dalloc(dscr, batched_solve_bytes((int)nmat, N, mode))) ||
-      (e = dalloc(dlog, nmat * 8)) || (e = dalloc(dtm, np * 4)) || (e = dalloc(dpos, np * 24)) ||
-      (e = dalloc(da, nmat * N * 16)) || (e = dalloc(db, nmat * N * 16)) || (e = dalloc(dx, nmat * N * 16)) ||
-      (e = dalloc(dsig, nmat * 8)) || (e = dalloc(dk, nmat * 16)) || (e = dalloc(dkv, nmat * 24)) ||
-      (e = dalloc(dT, nmat * ntm * (scatsys_dense(ss) ? (size_t)n * n : n) * 16)) ||
-      (e = dalloc(dcf, nmat * n * 16)))
-    return e;
-  QG_CUDA_TRY(cudaMemcpy(dtm.p, tm.data(), np * 4, cudaMemcpyHostToDevice));
-  QG_CUDA_TRY(cudaMemcpy(dpos.p, pos.data(), np * 24, cudaMemcpyHostToDevice));
+  const size_t nmat = (size_t)wchunk * nk, tsz = scatsys_dense(ss) ? (size_t)n * n : (size_t)n;
+  std::vector<qg_c> kall(nw), Tall;
+  for (size_t w = 0; w < nw; ++w) {
+    kall[w] = scatsys_wavenumber(ss, omegas[w], 0.0);
+    for (int t = 0; t < ntm; ++t) {
+      std::vector<qg_c> d;
+      scatsys_tdiag(ss, t, omegas[w], 0.0, d);
+      Tall.insert(Tall.end(), d.begin(), d.end());
+    }
+  }
+  DevArena ar;
+  const size_t otm = ar.upload(tm.data(), np * 4), opos = ar.upload(pos.data(), np * 24),
+               okap = ar.upload(kall.data(), nw * 16), obeta = ar.upload(kvecs, nk * 16),
+               oT = ar.upload(Tall.data(), Tall.size() * 16), ok = ar.add(nmat * 16), okv = ar.add(nmat * 24),
+               ocf = ar.add(nmat * n * 16), oa = ar.add(nmat * N * 16), ob = ar.add(nmat * N * 16),
+               ox = ar.add(nmat * N * 16), osig = ar.add(nmat * 8), olog = ar.add(nmat * 8),
+               oM = ar.add(nmat * N2 * 16), oscr = ar.add(batched_solve_bytes((int)nmat, N, mode));
+  if ((e = ar.alloc(0))) return e;
+  const int *dtm = ar.at<int>(otm);
+  const double *dpos = ar.at<double>(opos);
+  qg_c *dM = ar.at<qg_c>(oM), *da = ar.at<qg_c>(oa), *db = ar.at<qg_c>(ob), *dx = ar.at<qg_c>(ox),
+       *dk = ar.at<qg_c>(ok), *dcf = ar.at<qg_c>(ocf);
+  double *dlog = ar.at<double>(olog), *dsig = ar.at<double>(osig), *dkv = ar.at<double>(okv);
   std::vector<double> res(nmat);
   std::vector<int> its(nmat), info(nmat);
   for (size_t w0 = 0; w0 < nw; w0 += wchunk) {
     const int W = (int)std::min<size_t>(wchunk, nw - w0);
     const size_t nm = (size_t)W * nk;
-    std::vector<qg_c> T, k(W), kk(nm), Tm;
-    std::vector<double> eta(nm), kvec(3 * nm);
-    std::vector<qg_c> coefs(nm * n);
+    const qg_c *dTw = ar.at<qg_c>(oT) + w0 * ntm * tsz;
+    const std::vector<qg_c> T(Tall.begin() + w0 * ntm * tsz, Tall.begin() + (w0 + W) * ntm * tsz);
+    std::vector<double> eta(nm);
     for (int w = 0; w < W; ++w) {
-      for (int t = 0; t < ntm; ++t) {
-        std::vector<qg_c> d;
-        scatsys_tdiag(ss, t, omegas[w0 + w], 0.0, d);
-        T.insert(T.end(), d.begin(), d.end());
-      }
-      k[w] = scatsys_wavenumber(ss, omegas[w0 + w], 0.0);
-      const double kap = k[w].re;
       // one eta per frequency, the largest adjusted eta of its Bloch vectors
       // (the sums do not depend on eta; a larger one only moves work to the
       // long-range sum), so the short-range terms are shared by all of them
       double eta_w = 0;
       for (size_t ik = 0; ik < nk; ++ik) {
         const double kv[3] = {kvecs[2 * ik], kvecs[2 * ik + 1], 0.0};
-        eta_w = std::max(eta_w, qpms_ss_adjusted_eta(ss, *(const qpms_complex_t *)&k[w], kv));
+        eta_w = std::max(eta_w, qpms_ss_adjusted_eta(ss, *(const qpms_complex_t *)&kall[w0 + w], kv));
       }
-      for (size_t ik = 0; ik < nk; ++ik) {
-        const size_t m = (size_t)w * nk + ik;
-        const double kv[3] = {kvecs[2 * ik], kvecs[2 * ik + 1], 0.0};
-        eta[m] = eta_w;
-        kk[m] = k[w];
-        // incident plane wave with in-plane wavevector beta, E along x projected
-        // perpendicular to k (x-polarised at normal incidence)
-        const double b2 = kv[0] * kv[0] + kv[1] * kv[1];
-        const double kz = kap * kap > b2 ? sqrt(kap * kap - b2) : 0.0;
-        const double kd[3] = {kv[0], kv[1], kz};
-        const double kn = sqrt(b2 + kz * kz);
-        double E[3] = {1, 0, 0};
-        const double ex = kd[0] / kn;
-        for (int c = 0; c < 3; ++c) E[c] -= ex * kd[c] / kn;
-        const double En = sqrt(E[0] * E[0] + E[1] * E[1] + E[2] * E[2]);
-        qpms_complex_t Ec[3];
-        for (int c = 0; c < 3; ++c) Ec[c] = {E[c] / En, 0.0};
-        std::vector<qg_c> cf;
-        planewave_direction_coeffs(lMax, kd, Ec, cf);
-        const bool prop = kap * kap > b2;
-        for (int i = 0; i < n; ++i) coefs[m * n + i] = prop ? cf[i] : cmk(0, 0);
-        for (int c = 0; c < 3; ++c) kvec[3 * m + c] = kd[c];
-        const size_t tsz = scatsys_dense(ss) ? (size_t)n * n : (size_t)n;
-        for (int t = 0; t < ntm; ++t) Tm.insert(Tm.end(), T.begin() + ((size_t)w * ntm + t) * tsz,
-                                                T.begin() + ((size_t)w * ntm + t + 1) * tsz);
-      }
+      std::fill(eta.begin() + (size_t)w * nk, eta.begin() + (size_t)(w + 1) * nk, eta_w);
     }
-    if ((e = periodic_assemble_device_ex(ss, W, k.data(), T, (int)nk, kvecs, eta.data(), dM.as<qg_c>(), 0, true)))
-      return e;
+    if ((e = periodic_assemble_device_ex(ss, W, &kall[w0], T, (int)nk, kvecs, eta.data(), dM, 0, true))) return e;
     // per-matrix incidence (coefficients and phases differ per (w, k)), b = T a
-    QG_CUDA_TRY(cudaMemcpy(dcf.p, coefs.data(), coefs.size() * 16, cudaMemcpyHostToDevice));
-    QG_CUDA_TRY(cudaMemcpy(dkv.p, kvec.data(), nm * 24, cudaMemcpyHostToDevice));
-    QG_CUDA_TRY(cudaMemcpy(dk.p, kk.data(), nm * 16, cudaMemcpyHostToDevice));
-    QG_CUDA_TRY(cudaMemcpy(dT.p, Tm.data(), Tm.size() * 16, cudaMemcpyHostToDevice));
-    if ((e = launch_incident((int)nm, np, n, dcf.as<qg_c>(), dkv.as<double>(), dpos.as<double>(), da.as<qg_c>(), 0,
-                             (size_t)n)))
-      return e;
-    if ((e = launch_apply_t((int)nm, np, n, ntm, scatsys_dense(ss) ? 1 : 0, dtm.as<int>(), dT.as<qg_c>(),
-                            da.as<qg_c>(), db.as<qg_c>(), 0)))
+    if ((e = launch_scan_incidence(W, (int)nk, lMax, ar.at<qg_c>(okap) + w0, ar.at<double>(obeta), dcf, dkv, dk, 0)) ||
+        (e = launch_incident((int)nm, np, n, dcf, dkv, dpos, da, 0, (size_t)n)) ||
+        (e = launch_apply_t((int)nm, np, n, ntm, scatsys_dense(ss) ? 1 : 0, dtm, dTw, da, db, 0, (int)nk)))
       return e;
     // LU (complex128, or complex64 + FP64 refinement), log|det| from the factors
-    if ((e = batched_solve(h, 0, (int)nm, N, dM.as<qg_c>(), db.as<qg_c>(), dx.as<qg_c>(), mode, 1e-13, 12, dscr.p,
-                           res.data(), its.data(), info.data(), dlog.as<double>())))
+    if ((e = batched_solve(h, 0, (int)nm, N, dM, db, dx, mode, 1e-13, 12, ar.at<char>(oscr), res.data(), its.data(),
+                           info.data(), dlog)))
       return e;
-    QG_CUDA_TRY(cudaMemcpy(logdet + w0 * nk, dlog.p, nm * 8, cudaMemcpyDeviceToHost));
-    if ((e = launch_sigma_ext((int)nm, N, da.as<qg_c>(), dx.as<qg_c>(), dk.as<qg_c>(), dsig.as<double>(), 0)))
-      return e;
-    if (sigma_ext) QG_CUDA_TRY(cudaMemcpy(sigma_ext + w0 * nk, dsig.p, nm * 8, cudaMemcpyDeviceToHost));
-    if (f_out) QG_CUDA_TRY(cudaMemcpy(f_out + w0 * nk * N, dx.p, nm * N * 16, cudaMemcpyDeviceToHost));
+    QG_CUDA_TRY(cudaMemcpy(logdet + w0 * nk, dlog, nm * 8, cudaMemcpyDeviceToHost));
+    if ((e = launch_sigma_ext((int)nm, N, da, dx, dk, dsig, 0))) return e;
+    if (sigma_ext) QG_CUDA_TRY(cudaMemcpy(sigma_ext + w0 * nk, dsig, nm * 8, cudaMemcpyDeviceToHost));
+    if (f_out) QG_CUDA_TRY(cudaMemcpy(f_out + w0 * nk * N, dx, nm * N * 16, cudaMemcpyDeviceToHost));
     for (size_t m = 0; m < nm; ++m) {
       if (resid_out) resid_out[w0 * nk + m] = res[m];
       if (iters_out) iters_out[w0 * nk + m] = its[m];

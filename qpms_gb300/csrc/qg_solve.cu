@@ -16,6 +16,7 @@
 #include <memory>
 #include <vector>
 
+#include "qg_arena.h"
 #include "qg_assembly.h"
 #include "qg_batched.h"
 #include "qg_batchlu.h"
@@ -474,14 +475,6 @@ int qpms_gpu_finite_planewave_scatter_ext(const qpms_scatsys_t *ss, size_t nw, c
   int e;
   if ((e = blas_handle_get(&h))) return e;
   QG_BLAS_TRY(cublasSetStream(h, st));
-  Dev dM, dLU, dpiv, dinfo, dT, dtm, dpos, dk, dkv, dcoef, da, db, dx, dr, dn, dsig, dcb;
-  if ((e = dalloc(dM, N2 * W * 16)) || (e = dalloc(dLU, N2 * W * (mode ? 8 : 16))) ||
-      (e = dalloc(dpiv, N * W * 4)) || (e = dalloc(dinfo, W * 4)) || (e = dalloc(dT, T.size() * 16)) ||
-      (e = dalloc(dtm, np * 4)) || (e = dalloc(dpos, np * 24)) || (e = dalloc(dk, W * 16)) ||
-      (e = dalloc(dkv, W * 24)) || (e = dalloc(dcoef, n * 16)) || (e = dalloc(da, N * W * 16)) ||
-      (e = dalloc(db, N * W * 16)) || (e = dalloc(dx, N * W * 16)) || (e = dalloc(dr, N * W * 16)) ||
-      (e = dalloc(dn, W * 16)) || (e = dalloc(dsig, W * 8)) || (e = dalloc(dcb, N * W * 8)))
-    return e;
   std::vector<double> pos(3 * np);
   std::vector<int> tm(np);
   for (int i = 0; i < np; ++i) {
@@ -490,57 +483,66 @@ int qpms_gpu_finite_planewave_scatter_ext(const qpms_scatsys_t *ss, size_t nw, c
     pos[3 * i + 2] = ss->p[i].pos.z;
     tm[i] = ss->p[i].tmatrix_id;
   }
-  QG_CUDA_TRY(cudaMemcpy(dT.p, T.data(), T.size() * 16, cudaMemcpyHostToDevice));
-  QG_CUDA_TRY(cudaMemcpy(dtm.p, tm.data(), np * 4, cudaMemcpyHostToDevice));
-  QG_CUDA_TRY(cudaMemcpy(dpos.p, pos.data(), np * 24, cudaMemcpyHostToDevice));
-  QG_CUDA_TRY(cudaMemcpy(dk.p, k.data(), W * 16, cudaMemcpyHostToDevice));
-  QG_CUDA_TRY(cudaMemcpy(dkv.p, kvec.data(), W * 24, cudaMemcpyHostToDevice));
-  QG_CUDA_TRY(cudaMemcpy(dcoef.p, coef.data(), n * 16, cudaMemcpyHostToDevice));
+  const bool dense = scatsys_dense(ss);
+  DevArena ar;
+  const size_t oT = ar.upload(T.data(), T.size() * 16), otm = ar.upload(tm.data(), np * 4),
+               opos = ar.upload(pos.data(), np * 24), ok = ar.upload(k.data(), W * 16),
+               okv = ar.upload(kvec.data(), W * 24), ocoef = ar.upload(coef.data(), n * 16),
+               opiv = ar.add(N * W * 4), oinfo = ar.add(W * 4),
+               oa = ar.add(N * W * 16), ob = ar.add(N * W * 16), ox = ar.add(N * W * 16), orr = ar.add(N * W * 16),
+               on = ar.add(W * 16), osig = ar.add(W * 8), ocb = ar.add(N * W * 8), oM = ar.add(N2 * W * 16),
+               oLU = ar.add(N2 * W * (mode ? 8 : 16));
+  if ((e = ar.alloc(st))) return e;
+  qg_c *dT = ar.at<qg_c>(oT), *dk = ar.at<qg_c>(ok), *da = ar.at<qg_c>(oa), *db = ar.at<qg_c>(ob),
+       *dx = ar.at<qg_c>(ox), *dr = ar.at<qg_c>(orr), *dM = ar.at<qg_c>(oM);
+  int *dtm = ar.at<int>(otm), *dpiv = ar.at<int>(opiv), *dinfo = ar.at<int>(oinfo);
+  double *dpos = ar.at<double>(opos), *dsig = ar.at<double>(osig);
+  void *dLU = ar.at<char>(oLU), *dcb = ar.at<char>(ocb);
   // assemble M_w = I - T_w S_w (FP64)
   {
     AsmArgs a;
     a.nw = W;
     a.np = np;
     a.ntm = ntm;
-    a.dense = scatsys_dense(ss) ? 1 : 0;
+    a.dense = dense ? 1 : 0;
     a.J = 3;
-    a.pos = dpos.as<double>();
-    a.tmid = dtm.as<int>();
-    a.T = dT.as<qg_c>();
-    a.k = dk.as<qg_c>();
-    a.M = dM.as<qg_c>();
+    a.pos = dpos;
+    a.tmid = dtm;
+    a.T = dT;
+    a.k = dk;
+    a.M = dM;
     if ((e = launch_assemble(a, priv(ss->c)->dev, st))) return e;
   }
-  if ((e = launch_incident(W, np, n, dcoef.as<qg_c>(), dkv.as<double>(), dpos.as<double>(), da.as<qg_c>(), st)))
+  if ((e = launch_incident(W, np, n, ar.at<qg_c>(ocoef), ar.at<double>(okv), dpos, da, st)))
     return e;
-  if ((e = launch_apply_t(W, np, n, ntm, scatsys_dense(ss) ? 1 : 0, dtm.as<int>(), dT.as<qg_c>(), da.as<qg_c>(),
-                          db.as<qg_c>(), st)))
+  if ((e = launch_apply_t(W, np, n, ntm, dense ? 1 : 0, dtm, dT, da,
+                          db, st)))
     return e;
-  double *rn2 = dn.as<double>(), *bn2 = rn2 + W;
+  double *rn2 = ar.at<double>(on), *bn2 = rn2 + W;
   std::vector<double> hr(W), hb(W);
   std::vector<int> iters(W, 0);
   int info = 0;
   if (mode == 0) {
-    QG_CUDA_TRY(cudaMemcpyAsync(dLU.p, dM.p, N2 * W * 16, cudaMemcpyDeviceToDevice, st));
-    QG_CUDA_TRY(cudaMemcpyAsync(dx.p, db.p, N * W * 16, cudaMemcpyDeviceToDevice, st));
-    if ((e = batch_getrf_c128(W, (int)N, dLU.p, dpiv.as<int>(), dinfo.as<int>(), st))) return e;
-    if ((e = batch_getrs_c128(W, (int)N, dLU.p, dpiv.as<int>(), dx.p, st))) return e;
-    if ((e = launch_residual(W, N, dM.as<qg_c>(), dx.as<qg_c>(), db.as<qg_c>(), dr.as<qg_c>(), rn2, bn2, st)))
+    QG_CUDA_TRY(cudaMemcpyAsync(dLU, dM, N2 * W * 16, cudaMemcpyDeviceToDevice, st));
+    QG_CUDA_TRY(cudaMemcpyAsync(dx, db, N * W * 16, cudaMemcpyDeviceToDevice, st));
+    if ((e = batch_getrf_c128(W, (int)N, dLU, dpiv, dinfo, st))) return e;
+    if ((e = batch_getrs_c128(W, (int)N, dLU, dpiv, dx, st))) return e;
+    if ((e = launch_residual(W, N, dM, dx, db, dr, rn2, bn2, st)))
       return e;
     QG_CUDA_TRY(cudaMemcpy(hr.data(), rn2, W * 8, cudaMemcpyDeviceToHost));
     QG_CUDA_TRY(cudaMemcpy(hb.data(), bn2, W * 8, cudaMemcpyDeviceToHost));
   } else {
-    if ((e = launch_c128_to_c64(N2 * W, dM.as<qg_c>(), dLU.p, st))) return e;
-    if ((e = batch_getrf_c64(W, (int)N, dLU.p, dpiv.as<int>(), dinfo.as<int>(), st))) return e;
+    if ((e = launch_c128_to_c64(N2 * W, dM, dLU, st))) return e;
+    if ((e = batch_getrf_c64(W, (int)N, dLU, dpiv, dinfo, st))) return e;
     // x0 = LU32^{-1} b, then refine: r = b - M x (FP64), x += LU32^{-1} r
-    QG_CUDA_TRY(cudaMemcpyAsync(dr.p, db.p, N * W * 16, cudaMemcpyDeviceToDevice, st));
+    QG_CUDA_TRY(cudaMemcpyAsync(dr, db, N * W * 16, cudaMemcpyDeviceToDevice, st));
     const int kMaxIter = max_refine_steps(12);
     double prev = 1e300;
     for (int it = 0; it <= kMaxIter; ++it) {
-      if ((e = launch_c128_to_c64(N * W, dr.as<qg_c>(), dcb.p, st))) return e;
-      if ((e = batch_getrs_c64(W, (int)N, dLU.p, dpiv.as<int>(), dcb.p, st))) return e;
-      if ((e = launch_add_c64(N * W, dcb.p, dx.as<qg_c>(), it == 0, st))) return e;
-      if ((e = launch_residual(W, N, dM.as<qg_c>(), dx.as<qg_c>(), db.as<qg_c>(), dr.as<qg_c>(), rn2, bn2, st)))
+      if ((e = launch_c128_to_c64(N * W, dr, dcb, st))) return e;
+      if ((e = batch_getrs_c64(W, (int)N, dLU, dpiv, dcb, st))) return e;
+      if ((e = launch_add_c64(N * W, dcb, dx, it == 0, st))) return e;
+      if ((e = launch_residual(W, N, dM, dx, db, dr, rn2, bn2, st)))
         return e;
       QG_CUDA_TRY(cudaMemcpy(hr.data(), rn2, W * 8, cudaMemcpyDeviceToHost));
       QG_CUDA_TRY(cudaMemcpy(hb.data(), bn2, W * 8, cudaMemcpyDeviceToHost));
@@ -558,47 +560,47 @@ int qpms_gpu_finite_planewave_scatter_ext(const qpms_scatsys_t *ss, size_t nw, c
     for (int w = 0; w < W; ++w)
       if (sqrt(hr[w] / (hb[w] > 0 ? hb[w] : 1)) > 1e-13) bad.push_back(w);
     if (!bad.empty()) {
-      if ((e = resolve_fp64(st, bad, N, dM.as<qg_c>(), db.as<qg_c>(), dx.as<qg_c>()))) return e;
-      if ((e = launch_residual(W, N, dM.as<qg_c>(), dx.as<qg_c>(), db.as<qg_c>(), dr.as<qg_c>(), rn2, bn2, st)))
+      if ((e = resolve_fp64(st, bad, N, dM, db, dx))) return e;
+      if ((e = launch_residual(W, N, dM, dx, db, dr, rn2, bn2, st)))
         return e;
       QG_CUDA_TRY(cudaMemcpy(hr.data(), rn2, W * 8, cudaMemcpyDeviceToHost));
       QG_CUDA_TRY(cudaMemcpy(hb.data(), bn2, W * 8, cudaMemcpyDeviceToHost));
     }
   }
-  if ((e = launch_sigma_ext(W, N, da.as<qg_c>(), dx.as<qg_c>(), dk.as<qg_c>(), dsig.as<double>(), st))) return e;
-  QG_CUDA_TRY(cudaMemcpy(sigma_ext, dsig.p, W * 8, cudaMemcpyDeviceToHost));
+  if ((e = launch_sigma_ext(W, N, da, dx, dk, dsig, st))) return e;
+  QG_CUDA_TRY(cudaMemcpy(sigma_ext, dsig, W * 8, cudaMemcpyDeviceToHost));
   if (sigma_scat) {
     // sigma_scat = Re(f^H (I + R) f) / k^2 with R the regular-wave translation
     // matrix, zero self blocks (misc/finiterectlat-scatter.py:98-111): the
     // assembly with J = 1 and T = -1 builds I + R in place of M
     std::vector<qg_c> mone((size_t)W * ntm * n, cmk(-1.0, 0.0));  // diagonal -1 (dT holds at least this)
-    QG_CUDA_TRY(cudaMemcpy(dT.p, mone.data(), mone.size() * 16, cudaMemcpyHostToDevice));
+    QG_CUDA_TRY(cudaMemcpy(dT, mone.data(), mone.size() * 16, cudaMemcpyHostToDevice));
     AsmArgs a;
     a.nw = W;
     a.np = np;
     a.ntm = ntm;
     a.dense = 0;
     a.J = 1;
-    a.pos = dpos.as<double>();
-    a.tmid = dtm.as<int>();
-    a.T = dT.as<qg_c>();
-    a.k = dk.as<qg_c>();
-    a.M = dM.as<qg_c>();
+    a.pos = dpos;
+    a.tmid = dtm;
+    a.T = dT;
+    a.k = dk;
+    a.M = dM;
     if ((e = launch_assemble(a, priv(ss->c)->dev, st))) return e;
     // r = 0 - (I + R) f, then -Re(f^H r) / k^2
-    QG_CUDA_TRY(cudaMemsetAsync(db.p, 0, N * W * 16, st));
-    if ((e = launch_residual(W, N, dM.as<qg_c>(), dx.as<qg_c>(), db.as<qg_c>(), dr.as<qg_c>(), rn2, bn2, st)))
+    QG_CUDA_TRY(cudaMemsetAsync(db, 0, N * W * 16, st));
+    if ((e = launch_residual(W, N, dM, dx, db, dr, rn2, bn2, st)))
       return e;
-    if ((e = launch_sigma_ext(W, N, dx.as<qg_c>(), dr.as<qg_c>(), dk.as<qg_c>(), dsig.as<double>(), st))) return e;
-    QG_CUDA_TRY(cudaMemcpy(sigma_scat, dsig.p, W * 8, cudaMemcpyDeviceToHost));
+    if ((e = launch_sigma_ext(W, N, dx, dr, dk, dsig, st))) return e;
+    QG_CUDA_TRY(cudaMemcpy(sigma_scat, dsig, W * 8, cudaMemcpyDeviceToHost));
   }
-  if (f_out) QG_CUDA_TRY(cudaMemcpy(f_out, dx.p, N * W * 16, cudaMemcpyDeviceToHost));
+  if (f_out) QG_CUDA_TRY(cudaMemcpy(f_out, dx, N * W * 16, cudaMemcpyDeviceToHost));
   for (int w = 0; w < W; ++w) {
     if (resid_out) resid_out[w] = sqrt(hr[w] / (hb[w] > 0 ? hb[w] : 1));
     if (iters_out) iters_out[w] = mode ? iters[w] + 1 : 0;
   }
   std::vector<int> hinfo(W);
-  QG_CUDA_TRY(cudaMemcpy(hinfo.data(), dinfo.p, W * 4, cudaMemcpyDeviceToHost));
+  QG_CUDA_TRY(cudaMemcpy(hinfo.data(), dinfo, W * 4, cudaMemcpyDeviceToHost));
   for (int w = 0; w < W; ++w)
     if (hinfo[w] != 0) {
       set_error("singular matrix at frequency %d (info %d)", w, hinfo[w]);
