@@ -1,15 +1,22 @@
 // Mode-problem assembly and the small-system solve pipeline on sm_103a.
 //
-// assemble_kernel: for every (frequency w, particle pair R, C) unit of a batch
-// it writes the fecv x fecv block M_w[R, C] = delta_RC I - T_R S_w(R <- C)
-// straight into the row-major complex128 matrix M_w (the reference's
-// qpms_scatsysw_build_modeproblem_matrix_full, scatsystem.c:1283-1343, with
-// the finite semantics S(R <- R) = 0).  S comes from the translation tables
-// of the calculator: the per-pair factor table w (Hankel+ Bessel, Legendre,
-// azimuthal phases) is built in shared memory, every (y, yu) element of A and
-// B is one short FP64 dot product, and each A/B value lands in two blocks of
-// the 2x2 (electric, magnetic) type structure (translations_inlines.h:213-240).
-// Diagonal T (Mie spheres) scales rows; a dense T is applied from shared memory.
+// assemble_kernel writes the fecv x fecv blocks M_w[R, C] = delta_RC I - T_R
+// S_w(R <- C) straight into the row-major complex128 matrix M_w (the
+// reference's qpms_scatsysw_build_modeproblem_matrix_full,
+// scatsystem.c:1283-1343, with the finite semantics S(R <- R) = 0).  S comes
+// from the translation tables of the calculator: the per-pair factor table w
+// (Hankel+ Bessel, Legendre, azimuthal phases) is built in shared memory, the
+// elements of A and B are short FP64 dot products, one for each pair of
+// elements that reciprocity makes equal up to sign, and each value lands in two
+// blocks of the 2x2 (electric, magnetic) type structure
+// (translations_inlines.h:213-240).  Diagonal T (Mie spheres) scales rows: a
+// unit is then an unordered particle pair, because the opposite translation
+// only changes signs, (-1)^(n + nu) for A and -(-1)^(n + nu) for B, and the
+// dot products of a chunk's pairs form one list, so the lanes are full at every
+// lMax.  A dense T is applied from shared memory, an ordered pair at a time.
+// Bound: the FP64 pipe; the row scaling alone is four FMAs per element of M.
+// 900 spheres at lMax 2 (14,400 unknowns, 3.3 GB): 2.9 ms, against 8.3 ms with
+// a dot product per element and ordered pairs on CTAs of 256 threads.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -21,17 +28,19 @@
 namespace qg {
 namespace {
 
-constexpr int kAThreads = 256;
-
 template <int LMAX>
 struct AsmShape {
   static constexpr int L = 2 * LMAX + 1;
   static constexpr int S = (L + 1) * (L + 1);
   static constexpr int NL = (L + 1) * (L + 2) / 2;
   static constexpr int NE = LMAX * (LMAX + 2);
-  static constexpr int NE2 = NE * NE;
   static constexpr int NB = 2 * NE;  // block side
-  static constexpr int V = LMAX <= 2 ? 16 : (LMAX <= 4 ? 8 : 4);
+  // As in the translation kernel, small CTAs cover each other's set-up; V fills
+  // the set-up's lanes where the pairs are cheap (us, one 14,400-unknown matrix
+  // at lMax 2: V = 8 3,398, 16 3,013, 32 2,909; 14,400 at lMax 4: 2,404, 2,498,
+  // 2,737).
+  static constexpr int V = LMAX <= 2 ? 32 : (LMAX == 3 ? 16 : 8);
+  static constexpr int kThreads = 128, kMinCtas = 5;
 };
 
 template <int LMAX>
@@ -41,6 +50,9 @@ constexpr size_t asm_smem_bytes(bool dense) {
          (size_t)Sh::V * 32 + (dense ? (size_t)Sh::NB * Sh::NB * 16 : 0);
 }
 
+// degree n of the wave y = n(n+1) + m - 1
+__device__ __forceinline__ int ydeg(int y) { return (int)sqrtf((float)y + 1.0f); }
+
 struct __align__(16) PairInfo {
   double ct;
   int diag;   // R == C: identity block, no translation
@@ -49,9 +61,11 @@ struct __align__(16) PairInfo {
 };
 
 template <int LMAX, bool DENSE>
-__global__ void __launch_bounds__(kAThreads) assemble_kernel(AsmArgs a, TransDevTables T) {
+__global__ void __launch_bounds__(AsmShape<LMAX>::kThreads, AsmShape<LMAX>::kMinCtas)
+    assemble_kernel(AsmArgs a, TransDevTables T, int vc) {
   using Sh = AsmShape<LMAX>;
-  constexpr int L = Sh::L, S = Sh::S, NL = Sh::NL, NE = Sh::NE, NE2 = Sh::NE2, NB = Sh::NB, V = Sh::V;
+  constexpr int L = Sh::L, S = Sh::S, NL = Sh::NL, NE = Sh::NE, NB = Sh::NB, V = Sh::V;
+  constexpr int kAThreads = Sh::kThreads;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   qg_c *w = reinterpret_cast<qg_c *>(smem_raw);
   qg_c *zb = w + V * S;
@@ -61,12 +75,13 @@ __global__ void __launch_bounds__(kAThreads) assemble_kernel(AsmArgs a, TransDev
   qg_c *sblk = reinterpret_cast<qg_c *>(info + V);  // [NB][NB] if DENSE
 
   const int tid = threadIdx.x;
-  const size_t np = (size_t)a.np, units = (size_t)a.nw * np * np;
+  // a unit: the pair (R, C) of a frequency; unordered (C <= R) for a diagonal T
+  const size_t np = (size_t)a.np, per = DENSE ? np * np : np * (np + 1) / 2, units = (size_t)a.nw * per;
   const size_t N = np * NB;
-  const size_t nchunks = (units + V - 1) / V;
+  const size_t nchunks = (units + vc - 1) / vc;  // vc <= V units per chunk
   for (size_t chunk = blockIdx.x; chunk < nchunks; chunk += gridDim.x) {
-    const size_t base = chunk * V;
-    if (tid < V) {
+    const size_t base = chunk * vc;
+    if (tid < vc) {
       const size_t u = base + tid;
       PairInfo inf;
       inf.valid = u < units;
@@ -77,26 +92,33 @@ __global__ void __launch_bounds__(kAThreads) assemble_kernel(AsmArgs a, TransDev
 #pragma unroll
       for (int l = 0; l <= L; ++l) z[l] = cmk(0.0, 0.0);
       if (inf.valid) {
-        const int wi = (int)(u / (np * np));
-        const size_t pr = u - (size_t)wi * np * np;
+        const int wi = (int)(u / per);
+        const size_t pr = u - (size_t)wi * per;
         inf.w = wi;
-        inf.R = (int)(pr / np);
-        inf.C = (int)(pr - (size_t)inf.R * np);
+        if (DENSE) {
+          inf.R = (int)(pr / np);
+          inf.C = (int)(pr - (size_t)inf.R * np);
+        } else {
+          size_t r = (size_t)((sqrt(8.0 * (double)pr + 1.0) - 1.0) * 0.5);
+          while ((r + 1) * (r + 2) / 2 <= pr) ++r;
+          while (r * (r + 1) / 2 > pr) --r;
+          inf.R = (int)r;
+          inf.C = (int)(pr - r * (r + 1) / 2);
+        }
         inf.diag = inf.R == inf.C;
         if (!inf.diag) {
           const double dx = a.pos[3 * inf.R] - a.pos[3 * inf.C];
           const double dy = a.pos[3 * inf.R + 1] - a.pos[3 * inf.C + 1];
           const double dz = a.pos[3 * inf.R + 2] - a.pos[3 * inf.C + 2];
           const double r = sqrt(dx * dx + dy * dy + dz * dz);
-          // cart2sph (vectors.h:134-140), then kd.r *= k (translations.c:808-809)
-          const double th = r > 0 ? acos(dz / r) : 1.5707963267948966;
-          const double ph = atan2(dy, dx);
+          // cart2sph (vectors.h:134-140), then kd.r *= k (translations.c:808-809); only
+          // cos(theta) and e^{i phi} of the angles are needed (theta = pi/2, phi = 0 at r = 0)
+          const double rho = sqrt(dx * dx + dy * dy);
           const qg_c k = a.k[wi];
           sph_bessel<L>(a.J, cmk(k.re * r, k.im * r), z);
-          inf.ct = cos(th);
-          double s1, c1;
-          sincos(ph, &s1, &c1);
-          qg_c e1 = cmk(c1, s1), e = cmk(1.0, 0.0);
+          inf.ct = r > 0 ? dz / r : 0.0;
+          const qg_c e1 = rho > 0 ? cmk(dx / rho, dy / rho) : cmk(1.0, 0.0);
+          qg_c e = cmk(1.0, 0.0);
 #pragma unroll
           for (int d = 0; d <= L; ++d) {
             eph[tid * (L + 1) + d] = e;
@@ -109,12 +131,12 @@ __global__ void __launch_bounds__(kAThreads) assemble_kernel(AsmArgs a, TransDev
       info[tid] = inf;
     }
     __syncthreads();
-    for (int t = tid; t < V * (L + 1); t += kAThreads) {
+    for (int t = tid; t < vc * (L + 1); t += kAThreads) {
       const int v = t / (L + 1), m = t - v * (L + 1);
       if (!info[v].diag) legendre_column_rt(L, m, info[v].ct, leg + v * NL);
     }
     __syncthreads();
-    for (int t = tid; t < V * NL; t += kAThreads) {
+    for (int t = tid; t < vc * NL; t += kAThreads) {
       const int v = t / NL, i = t - v * NL;
       if (info[v].diag) continue;
       int p = (int)((sqrtf(8.0f * i + 1.0f) - 1.0f) * 0.5f);
@@ -129,7 +151,51 @@ __global__ void __launch_bounds__(kAThreads) assemble_kernel(AsmArgs a, TransDev
     }
     __syncthreads();
 
-    for (int v = 0; v < V; ++v) {
+    if (!DENSE) {
+      // all elements of the chunk's pairs in one list, so that the lanes stay full
+      // at small lMax (36 dot products of A and 36 of B at lMax 2)
+      const int nAB = T.nA + T.nB;
+      for (int t = tid; t < vc * nAB; t += kAThreads) {
+        const int v = t / nAB, kk = t - v * nAB, which = kk >= T.nA, k = which ? kk - T.nA : kk;
+        const PairInfo inf = info[v];
+        if (!inf.valid || inf.diag) continue;
+        const int nk = which ? T.nB : T.nA, c = which ? T.cntB[k] : T.cntA[k];
+        const double *coef = (which ? T.coefB : T.coefA) + k;
+        const uint16_t *slot = (which ? T.slotB : T.slotA) + k;
+        const qg_c *wv = w + v * S;
+        double sr = 0, si = 0;
+        for (int q = 0; q < c; ++q) {
+          const double cf = __ldg(coef + q * nk);
+          const qg_c x = wv[__ldg(slot + q * nk)];
+          sr = fma(cf, x.re, sr);
+          si = fma(cf, x.im, si);
+        }
+        qg_c val = which ? cmk(xor_sign(si, kSignBit), sr) : cmk(sr, si);  // B multipliers are imaginary
+        const uint32_t pr = __ldg((which ? T.pairB : T.pairA) + k);
+        qg_c *M = a.M + (size_t)inf.w * N * N;
+        const size_t row0 = (size_t)inf.R * NB, col0 = (size_t)inf.C * NB;
+        const qg_c *TR = a.T + ((size_t)inf.w * a.ntm + a.tmid[inf.R]) * NB;
+        const qg_c *TC = a.T + ((size_t)inf.w * a.ntm + a.tmid[inf.C]) * NB;
+        const int ends = pair_second(pr) == pair_first(pr) ? 1 : 2;
+        for (int h = 0; h < ends; ++h) {  // the two elements that share the dot product
+          const int e = h ? pair_second(pr) : pair_first(pr);
+          if (h && pair_negated(pr)) val = cmk(xor_sign(val.re, kSignBit), xor_sign(val.im, kSignBit));
+          const int yi = e / NE, yj = e - yi * NE;
+          // A: (E <- E) and (M <- M) blocks; B: (E <- M) and (M <- E) blocks
+          const int r1 = yi, c1 = which ? NE + yj : yj;
+          const int r2 = NE + yi, c2 = which ? yj : NE + yj;
+          M[(row0 + r1) * N + col0 + c1] = cmul_neg(TR[r1], val);
+          M[(row0 + r2) * N + col0 + c2] = cmul_neg(TR[r2], val);
+          // (C, R): the opposite translation flips the waves of odd order,
+          // S(C <- R) = (-1)^(n + nu) A, -(-1)^(n + nu) B
+          const unsigned long long odd = ((ydeg(yi) + ydeg(yj) + which) & 1) ? kSignBit : 0ull;
+          const qg_c u = cmk(xor_sign(val.re, odd), xor_sign(val.im, odd));
+          M[(col0 + r1) * N + row0 + c1] = cmul_neg(TC[r1], u);
+          M[(col0 + r2) * N + row0 + c2] = cmul_neg(TC[r2], u);
+        }
+      }
+    }
+    for (int v = 0; v < vc; ++v) {
       const PairInfo inf = info[v];
       if (!inf.valid) break;
       qg_c *M = a.M + (size_t)inf.w * N * N;
@@ -141,11 +207,9 @@ __global__ void __launch_bounds__(kAThreads) assemble_kernel(AsmArgs a, TransDev
         }
         continue;
       }
+      if (!DENSE) continue;
       const qg_c *wv = w + v * S;
-      const int tmR = a.tmid[inf.R];
-      const qg_c *TR = a.T + ((size_t)inf.w * a.ntm + tmR) * (DENSE ? NB * NB : NB);
-      // A and B each in their own term-count order; each value lands in two
-      // blocks of the (electric, magnetic) type structure
+      const qg_c *TR = a.T + ((size_t)inf.w * a.ntm + a.tmid[inf.R]) * NB * NB;
 #pragma unroll 1
       for (int which = 0; which < 2; ++which) {
         const uint8_t *cnt = which ? T.cntB : T.cntA;
@@ -162,40 +226,30 @@ __global__ void __launch_bounds__(kAThreads) assemble_kernel(AsmArgs a, TransDev
             sr = fma(cf, x.re, sr);
             si = fma(cf, x.im, si);
           }
-          qg_c v = which ? cmk(xor_sign(si, kSignBit), sr) : cmk(sr, si);  // B multipliers are imaginary
+          qg_c val = which ? cmk(xor_sign(si, kSignBit), sr) : cmk(sr, si);
           const uint32_t pr = __ldg(pair + k);
           const int ends = pair_second(pr) == pair_first(pr) ? 1 : 2;
-          for (int h = 0; h < ends; ++h) {  // the two elements that share the dot product
+          for (int h = 0; h < ends; ++h) {
             const int e = h ? pair_second(pr) : pair_first(pr);
-            if (h && pair_negated(pr)) v = cmk(xor_sign(v.re, kSignBit), xor_sign(v.im, kSignBit));
+            if (h && pair_negated(pr)) val = cmk(xor_sign(val.re, kSignBit), xor_sign(val.im, kSignBit));
             const int yi = e / NE, yj = e - yi * NE;
-            // A: (E <- E) and (M <- M) blocks; B: (E <- M) and (M <- E) blocks
-            const int r1 = yi, c1 = which ? NE + yj : yj;
-            const int r2 = NE + yi, c2 = which ? yj : NE + yj;
-            if (DENSE) {
-              sblk[r1 * NB + c1] = v;
-              sblk[r2 * NB + c2] = v;
-            } else {
-              M[(row0 + r1) * N + col0 + c1] = cmul_neg(TR[r1], v);
-              M[(row0 + r2) * N + col0 + c2] = cmul_neg(TR[r2], v);
-            }
+            sblk[yi * NB + (which ? NE + yj : yj)] = val;
+            sblk[(NE + yi) * NB + (which ? yj : NE + yj)] = val;
           }
         }
       }
-      if (DENSE) {
-        __syncthreads();
-        for (int t = tid; t < NB * NB; t += kAThreads) {
-          const int i = t / NB, j = t - i * NB;
-          double sr = 0, si = 0;
-          for (int q = 0; q < NB; ++q) {
-            const qg_c tq = TR[i * NB + q], sq = sblk[q * NB + j];
-            sr = fma(tq.re, sq.re, fma(-tq.im, sq.im, sr));
-            si = fma(tq.re, sq.im, fma(tq.im, sq.re, si));
-          }
-          M[(row0 + i) * N + col0 + j] = cmk(-sr, -si);
+      __syncthreads();
+      for (int t = tid; t < NB * NB; t += kAThreads) {
+        const int i = t / NB, j = t - i * NB;
+        double sr = 0, si = 0;
+        for (int q = 0; q < NB; ++q) {
+          const qg_c tq = TR[i * NB + q], sq = sblk[q * NB + j];
+          sr = fma(tq.re, sq.re, fma(-tq.im, sq.im, sr));
+          si = fma(tq.re, sq.im, fma(tq.im, sq.re, si));
         }
-        __syncthreads();
+        M[(row0 + i) * N + col0 + j] = cmk(-sr, -si);
       }
+      __syncthreads();
     }
     __syncthreads();
   }
@@ -207,26 +261,22 @@ int launch_asm(const AsmArgs &a, const TransDevTables &T, cudaStream_t st) {
   int dev = 0, nsm = 0, per_sm = 0;
   QG_CUDA_TRY(cudaGetDevice(&dev));
   QG_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const size_t units = (size_t)a.nw * a.np * a.np;
-  const size_t nchunks = (units + Sh::V - 1) / Sh::V;
-  if (nchunks == 0) return QPMS_SUCCESS;
+  const size_t np = (size_t)a.np, units = (size_t)a.nw * (a.dense ? np * np : np * (np + 1) / 2);
+  if (units == 0) return QPMS_SUCCESS;
   const double nrow = (double)a.np * 2 * LMAX * (LMAX + 2);
   KtScope kt(KT_ASSEMBLE, st, 16.0 * a.nw * nrow * nrow);
-  if (a.dense) {
-    auto k = assemble_kernel<LMAX, true>;
-    const size_t smem = asm_smem_bytes<LMAX>(true);
+  const size_t smem = asm_smem_bytes<LMAX>(a.dense);
+  auto run = [&](auto k) -> int {
     QG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    QG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kAThreads, smem));
-    size_t grid = std::min<size_t>((size_t)nsm * std::max(per_sm, 1), nchunks);
-    k<<<(unsigned)grid, kAThreads, smem, st>>>(a, T);
-  } else {
-    auto k = assemble_kernel<LMAX, false>;
-    const size_t smem = asm_smem_bytes<LMAX>(false);
-    QG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    QG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kAThreads, smem));
-    size_t grid = std::min<size_t>((size_t)nsm * std::max(per_sm, 1), nchunks);
-    k<<<(unsigned)grid, kAThreads, smem, st>>>(a, T);
-  }
+    QG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, Sh::kThreads, smem));
+    const size_t resident = (size_t)nsm * std::max(per_sm, 1);
+    // few pairs: fewer in a chunk, so that every resident CTA has one
+    const int vc = (int)std::min<size_t>(Sh::V, (units + resident - 1) / resident);
+    k<<<(unsigned)std::min(resident, (units + vc - 1) / vc), Sh::kThreads, smem, st>>>(a, T, vc);
+    return QPMS_SUCCESS;
+  };
+  const int e = a.dense ? run(assemble_kernel<LMAX, true>) : run(assemble_kernel<LMAX, false>);
+  if (e) return e;
   QG_CUDA_TRY(cudaGetLastError());
   g_launches.fetch_add(1);
   return QPMS_SUCCESS;

@@ -240,61 +240,70 @@ bool build_trans_tables(int lMax, int norm, TransHostTables *t) {
   // counts.
   const int tq = t->tq;
   auto build = [&](const std::vector<std::vector<ld>> &c, const std::vector<std::vector<int>> &slot,
-                   const std::vector<std::vector<ld>> &cA_, std::vector<uint32_t> &pair, std::vector<uint8_t> &cnt,
-                   std::vector<uint8_t> *cntE, std::vector<double> &coef, std::vector<uint16_t> &sl) {
-    std::vector<std::vector<int>> keep(ne2);  // kept term indices
+                   std::vector<uint32_t> &pair, std::vector<uint8_t> &cnt, std::vector<uint8_t> *cntE,
+                   std::vector<double> &coef, std::vector<uint16_t> &sl) {
+    std::vector<double> v((size_t)ne2 * tq);    // kept terms' coefficients
+    std::vector<uint8_t> idx((size_t)ne2 * tq);  // and their indices
+    std::vector<uint8_t> nk(ne2);
     for (int e = 0; e < ne2; ++e) {
-      for (size_t q = 0; q < c[e].size(); ++q)
-        if ((double)c[e][q] != 0) keep[e].push_back((int)q);
-      if (keep[e].empty()) keep[e].push_back((int)c[e].size() - 1);
+      int k = 0;
+      const int nq = (int)c[e].size();
+      for (int q = 0; q < nq; ++q) {
+        const double x = (double)c[e][q];
+        if (x == 0 && !(q == nq - 1 && k == 0)) continue;
+        v[(size_t)e * tq + k] = x;
+        idx[(size_t)e * tq + k++] = (uint8_t)q;
+      }
+      nk[e] = (uint8_t)k;
     }
     struct Item {
       int e, f, neg;
     };
     std::vector<Item> items;
+    items.reserve(ne2);
     std::vector<char> done(ne2, 0);
-    for (int y = 0; y < ne; ++y)
-      for (int yu = 0; yu < ne; ++yu) {
-        const int e = y * ne + yu;
-        if (done[e]) continue;
-        const int n = (int)sqrt((double)y + 1), m = y - (n * (n + 1) - 1);
-        const int nu = (int)sqrt((double)yu + 1), mu = yu - (nu * (nu + 1) - 1);
-        const int f = (nu * (nu + 1) - 1 - mu) * ne + (n * (n + 1) - 1 - m);
-        Item it = {e, e, 0};
-        if (f != e && !done[f] && keep[e] == keep[f] && slot[e] == slot[f] && cA_[e].size() == cA_[f].size())
-          for (int neg = 0; neg < 2 && it.f == e; ++neg) {
-            bool same = true;
-            for (int q : keep[e]) {
-              const ld a = c[e][q], b = neg ? -c[f][q] : c[f][q];
-              same = same && fabsl(a - b) <= 1e-15L * fabsl(a);
+    for (int n = 1, y = 0; n <= lMax; ++n)
+      for (int m = -n; m <= n; ++m, ++y)
+        for (int nu = 1, yu = 0; nu <= lMax; ++nu)
+          for (int mu = -nu; mu <= nu; ++mu, ++yu) {
+            const int e = y * ne + yu;
+            if (done[e]) continue;
+            const int f = (nu * (nu + 1) - 1 - mu) * ne + (n * (n + 1) - 1 - m);
+            Item it = {e, e, 0};
+            if (f != e && !done[f] && nk[e] == nk[f] && slot[e] == slot[f] && cA[e].size() == cA[f].size()) {
+              bool same[2] = {true, true};
+              for (int k = 0; k < nk[e]; ++k) {
+                const double a = v[(size_t)e * tq + k], b = v[(size_t)f * tq + k];
+                const bool at = idx[(size_t)e * tq + k] == idx[(size_t)f * tq + k];
+                same[0] = same[0] && at && fabs(a - b) <= 1e-15 * fabs(a);
+                same[1] = same[1] && at && fabs(a + b) <= 1e-15 * fabs(a);
+              }
+              if (same[0] || same[1]) it = {e, f, same[0] ? 0 : 1};
             }
-            if (same) it = {e, f, neg};
+            done[it.e] = done[it.f] = 1;
+            items.push_back(it);
           }
-        done[it.e] = done[it.f] = 1;
-        items.push_back(it);
-      }
-    std::stable_sort(items.begin(), items.end(),
-                     [&](const Item &a, const Item &b) { return keep[a.e].size() > keep[b.e].size(); });
-    const int nu_ = (int)items.size();
-    pair.assign(nu_, 0);
-    cnt.assign(nu_, 0);
-    if (cntE) cntE->assign(nu_, 0);
-    coef.assign((size_t)tq * nu_, 0.0);
-    sl.assign((size_t)tq * nu_, 0);
-    for (int k = 0; k < nu_; ++k) {
+    std::stable_sort(items.begin(), items.end(), [&](const Item &a, const Item &b) { return nk[a.e] > nk[b.e]; });
+    const int np = (int)items.size();
+    pair.assign(np, 0);
+    cnt.assign(np, 0);
+    if (cntE) cntE->assign(np, 0);
+    coef.assign((size_t)tq * np, 0.0);
+    sl.assign((size_t)tq * np, 0);
+    for (int k = 0; k < np; ++k) {
       const Item &it = items[k];
       pair[k] = trans_pair(it.e, it.f, it.neg);
-      cnt[k] = (uint8_t)keep[it.e].size();
-      for (size_t i = 0; i < keep[it.e].size(); ++i) {
-        const int q = keep[it.e][i];
-        coef[i * nu_ + k] = (double)c[it.e][q];
-        sl[i * nu_ + k] = (uint16_t)slot[it.e][q];
-        if (cntE && q < (int)cA_[it.e].size()) (*cntE)[k] = (uint8_t)(i + 1);
+      cnt[k] = nk[it.e];
+      for (int i = 0; i < nk[it.e]; ++i) {
+        const int q = idx[(size_t)it.e * tq + i];
+        coef[(size_t)i * np + k] = v[(size_t)it.e * tq + i];
+        sl[(size_t)i * np + k] = (uint16_t)slot[it.e][q];
+        if (cntE && q < (int)cA[it.e].size()) (*cntE)[k] = (uint8_t)(i + 1);
       }
     }
   };
-  build(cA, sA, cA, t->pairA, t->cntA, nullptr, t->coefA, t->slotA);
-  build(cB, sB, cA, t->pairB, t->cntB, &t->cntBe, t->coefB, t->slotB);
+  build(cA, sA, t->pairA, t->cntA, nullptr, t->coefA, t->slotA);
+  build(cB, sB, t->pairB, t->cntB, &t->cntBe, t->coefB, t->slotB);
   return true;
 }
 
