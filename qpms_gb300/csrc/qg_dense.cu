@@ -1117,12 +1117,16 @@ size_t tc_plane_bytes(int Np, int nrhs_max, int nb) {
 // Block size of the LU: complex128 factors use 64; complex64 factors use 128
 // for large systems (the trailing updates carry the time) and 64 below the
 // tuned size kTunedNb64Below (the chain of diagonal-block inversions carries
-// it there: an inversion costs nb^3).  QPMS_GB300_LU_NB = 64 / 128 overrides.
-int lu_block_size(int N, int mode) {
+// it there: an inversion costs nb^3).  With many right-hand sides the
+// substitutions' chain, two launches per block and sweep, is the longer one:
+// 128 at every size (six contour nodes with 64 columns at 5,776 unknowns 119.7 ms
+// with 64-wide blocks, 108.5 with 128; 32 columns at 1,600 unknowns 24.2 : 22.7).
+// QPMS_GB300_LU_NB = 64 / 128 overrides.
+int lu_block_size(int N, int mode, int nrhs) {
   if (!mode) return 64;
   const char *ev = getenv("QPMS_GB300_LU_NB");
   if (ev && (!strcmp(ev, "64") || !strcmp(ev, "128"))) return atoi(ev);
-  return N < kTunedNb64Below ? 64 : 128;
+  return N < kTunedNb64Below && nrhs <= kSmallRhs ? 64 : 128;
 }
 
 int DenseSolver::init(int N_, int nrhs_max_, int mode_, unsigned long long seed, cudaMemPool_t pool_,
@@ -1144,7 +1148,7 @@ int DenseSolver::init(int N_, int nrhs_max_, int mode_, unsigned long long seed,
   base_mode = mode;
   base_trail = trail_ct;
   base_tc = tc_split;
-  nb = (mode && (nb_pref == 64 || nb_pref == 128)) ? nb_pref : lu_block_size(N, mode);
+  nb = (mode && (nb_pref == 64 || nb_pref == 128)) ? nb_pref : lu_block_size(N, mode, nrhs_max);
   const size_t esz = mode ? 8 : 16;
   const size_t NN = (size_t)Np * Np;
   const int nblk = (Np + nb - 1) / nb;
@@ -1152,28 +1156,41 @@ int DenseSolver::init(int N_, int nrhs_max_, int mode_, unsigned long long seed,
   // a mixed solver that falls back to complex128 factors uses the same work
   // buffer for nb = 64 complex128 column blocks (N x 64 x 16 bytes)
   if (mode) wsz = std::max<size_t>(wsz, (size_t)std::max(Np, nrhs_max) * 64 * 16);
-  if (mode)
-    QG_CUDA_TRY(dev_alloc(&A, NN * esz));  // complex64 factors; the FP64 transform is fused into their fill
-  else
-    QG_CUDA_TRY(dev_alloc(&T64, NN * 16));
-  QG_CUDA_TRY(dev_alloc(&Dinv, (size_t)nblk * 2 * nb * nb * esz));
-  QG_CUDA_TRY(dev_alloc(&work, wsz));
-  QG_CUDA_TRY(dev_alloc(&rhs_lo, (size_t)Np * nrhs_max * 8));
-  QG_CUDA_TRY(dev_alloc(&rp, (size_t)Np * nrhs_max * 16));
-  QG_CUDA_TRY(dev_alloc(&r64, (size_t)N * nrhs_max * 16));
-  QG_CUDA_TRY(dev_alloc(&y64, (size_t)N * nrhs_max * 16));
-  QG_CUDA_TRY(dev_alloc(&dinfo, 16));
-  QG_CUDA_TRY(dev_alloc(&rs, (size_t)4 * Np * sizeof(double)));
-  QG_CUDA_TRY(dev_alloc(&res_nrm, (size_t)2 * kOzakiMinRhs * sizeof(double)));
   // sized for 64-wide blocks (the complex128 fallback's), the larger count
   const size_t sweep_bytes = sweep_words((Np + 63) / 64) * sizeof(unsigned);
-  QG_CUDA_TRY(dev_alloc(&sweep, sweep_bytes));
+  // K up to group x nb: the combined update of a group of blocks
+  const int kmax = lu_group() * nb;
+  // one allocation for all buffers that every solver of this mode has (each by
+  // itself costs a driver call, and its release a wait for the whole device)
+  struct Part {
+    void **p;
+    size_t bytes;
+  };
+  const Part parts[] = {
+      {mode ? &A : &T64, NN * esz},  // mixed: complex64 factors; the FP64 transform is fused into their fill
+      {&Dinv, (size_t)nblk * 2 * nb * nb * esz},
+      {&work, wsz},
+      {&rhs_lo, (size_t)Np * nrhs_max * 8},
+      {&rp, (size_t)Np * nrhs_max * 16},
+      {&r64, (size_t)N * nrhs_max * 16},
+      {&y64, (size_t)N * nrhs_max * 16},
+      {(void **)&dinfo, 16},
+      {(void **)&rs, (size_t)4 * Np * sizeof(double)},
+      {(void **)&res_nrm, (size_t)2 * kOzakiMinRhs * sizeof(double)},
+      {(void **)&sweep, sweep_bytes},
+      {&tc_pa, tc_split ? tc_planes_bytes_a(Np, kmax, 3) : 0},
+      {&tc_pb, tc_split ? tc_planes_bytes_b(std::max(Np, nrhs_max), kmax, 3) : 0},
+  };
+  size_t total = 0;
+  for (const Part &q : parts) total += (q.bytes + 255) / 256 * 256;
+  QG_CUDA_TRY(dev_alloc(&block, total));
+  size_t off = 0;
+  for (const Part &q : parts) {
+    *q.p = q.bytes ? (char *)block + off : nullptr;
+    off += (q.bytes + 255) / 256 * 256;
+  }
   QG_CUDA_TRY(cudaMemsetAsync(sweep, 0, sweep_bytes, ast));
   if (tc_split) {
-    // K up to group x nb: the combined update of a group of blocks
-    const int kmax = lu_group() * nb;
-    QG_CUDA_TRY(dev_alloc(&tc_pa, tc_planes_bytes_a(Np, kmax, 3)));
-    QG_CUDA_TRY(dev_alloc(&tc_pb, tc_planes_bytes_b(std::max(Np, nrhs_max), kmax, 3)));
     const char *la = getenv("QPMS_GB300_LOOKAHEAD");
     if (lookahead && !(la && !strcmp(la, "0")) && Np > nb) {
       int lo = 0, hi = 0;
@@ -1247,9 +1264,8 @@ cudaError_t DenseSolver::dev_alloc(void *ptr, size_t bytes) {
 
 void DenseSolver::release() {
   if (side) cudaStreamSynchronize(side);  // its last inversion reads buffers freed below
-  for (void *p : {(void *)A, (void *)T64, (void *)Dinv, (void *)work, (void *)rhs_lo, (void *)rp, (void *)r64,
-                  (void *)y64, (void *)dinfo, (void *)rs, (void *)res_nrm, (void *)sweep, oz_mat, oz_work, tc_pa,
-                  tc_pb, fac_planes})
+  // the fallback's T64 of a mixed solver has an allocation of its own
+  for (void *p : {block, base_mode ? T64 : nullptr, oz_mat, oz_work, fac_planes})
     if (p) {
       if (pool)
         cudaFreeAsync(p, ast);
@@ -1265,7 +1281,7 @@ void DenseSolver::release() {
   if (ev_d) cudaEventDestroy(ev_d);
   side = nullptr;
   ev_a = ev_d = nullptr;
-  A = T64 = Dinv = work = rhs_lo = rp = nullptr;
+  block = A = T64 = Dinv = work = rhs_lo = rp = nullptr;
   r64 = y64 = nullptr;
   dinfo = nullptr;
   rs = nullptr;
@@ -1350,7 +1366,7 @@ int DenseSolver::factorize(const void *M64, size_t ldm, cudaStream_t st, bool ro
   mode = base_mode;
   trail_ct = base_trail;
   tc_split = base_tc;
-  nb = (mode && (nb_pref == 64 || nb_pref == 128)) ? nb_pref : lu_block_size(N, mode);
+  nb = (mode && (nb_pref == 64 || nb_pref == 128)) ? nb_pref : lu_block_size(N, mode, nrhs_max);
   const unsigned long long key[6] = {(unsigned long long)(uintptr_t)M64, ldm, rowmaj ? 1ull : 0ull,
                                      (unsigned long long)mode, (unsigned long long)tc_split,
                                      use_ozaki ? 1ull : 0ull};
@@ -1372,10 +1388,12 @@ int DenseSolver::factorize_current(const void *M64, size_t ldm, cudaStream_t st)
 int DenseSolver::factor_launch(const void *M64, size_t ldm, cudaStream_t st) {
   const bool rowmaj = row_major;
   const size_t NN = (size_t)Np * Np;
-  cublasHandle_t h;
+  cublasHandle_t h = nullptr;  // the tensor-core path needs none (a thread's first handle takes milliseconds)
   int e;
-  if ((e = blas_handle_get(&h))) return e;
-  QG_BLAS_TRY(cublasSetStream(h, st));
+  if (!(mode && tc_split)) {
+    if ((e = blas_handle_get(&h))) return e;
+    QG_BLAS_TRY(cublasSetStream(h, st));
+  }
   QG_CUDA_TRY(cudaMemsetAsync(dinfo, 0, 4, st));
   if (mode) {
     // complex64 A = W_u^T diag(M, I) W_v in one pass over M
@@ -1457,10 +1475,12 @@ int DenseSolver::apply_inverse(const void *R, size_t ldr, void *Y, size_t ldy, i
 }
 
 int DenseSolver::apply_launch(const void *R, size_t ldr, void *Y, size_t ldy, int nrhs, cudaStream_t st) {
-  cublasHandle_t h;
+  cublasHandle_t h = nullptr;
   int e;
-  if ((e = blas_handle_get(&h))) return e;
-  QG_BLAS_TRY(cublasSetStream(h, st));
+  if (nrhs > kSmallRhs && !(mode && tc_split)) {
+    if ((e = blas_handle_get(&h))) return e;
+    QG_BLAS_TRY(cublasSetStream(h, st));
+  }
   const size_t n = (size_t)Np * nrhs;
   if (Np != N) QG_CUDA_TRY(cudaMemsetAsync(rp, 0, n * 16, st));
   QG_CUDA_TRY(cudaMemcpy2DAsync(rp, (size_t)Np * 16, R, ldr * 16, (size_t)N * 16, nrhs, cudaMemcpyDeviceToDevice,
@@ -1519,10 +1539,7 @@ int DenseSolver::solve(const void *M64, size_t ldm, const void *B, void *X, int 
     return QPMS_EINVAL;
   }
   max_iter = max_refine_steps(max_iter);
-  cublasHandle_t h;
   int e;
-  if ((e = blas_handle_get(&h))) return e;
-  QG_BLAS_TRY(cublasSetStream(h, st));
   const size_t n = (size_t)N * nrhs;
   double *nrm = (double *)dinfo + 1;  // two doubles after the info word
   double hb = 0, hr = 0;
@@ -1552,6 +1569,9 @@ int DenseSolver::solve(const void *M64, size_t ldm, const void *B, void *X, int 
     } else {
       QG_CUDA_TRY(cudaMemcpyAsync(r64, B, n * 16, cudaMemcpyDeviceToDevice, st));
       // a row-major M read column-major is M^T: multiply with OP_T
+      cublasHandle_t h;
+      if ((e = blas_handle_get(&h))) return e;
+      QG_BLAS_TRY(cublasSetStream(h, st));
       QG_BLAS_TRY(cublasZgemm(h, row_major ? CUBLAS_OP_T : CUBLAS_OP_N, CUBLAS_OP_N, N, nrhs, N, &mone,
                               (const cuDoubleComplex *)M64, (int)ldm, (const cuDoubleComplex *)X, N, &one,
                               (cuDoubleComplex *)r64, N));
@@ -1587,8 +1607,6 @@ int DenseSolver::solve(const void *M64, size_t ldm, const void *B, void *X, int 
         }
         ++refactors;
         if ((e = factorize_current(M64, ldm, st))) return e;
-        if ((e = blas_handle_get(&h))) return e;
-        QG_BLAS_TRY(cublasSetStream(h, st));
         prev = 1e300;
         extra = it + 1;
         continue;

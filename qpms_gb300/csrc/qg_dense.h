@@ -23,6 +23,7 @@ bool fac_planes_wanted();
 // padding), the size the two butterfly levels halve.
 struct DenseSolver {
   int N = 0, Np = 0, nrhs_max = 0, mode = 0, nb = 64;
+  void *block = nullptr;   // the allocation that holds the buffers below
   void *A = nullptr;       // mode 1: complex64 LU factors, Np x Np (mode 0 factors T64 in place)
   void *T64 = nullptr;     // complex128 Np x Np: W_u^T diag(M, I) W_v (mode 0; mode 1 at its first fallback)
   void *Dinv = nullptr;    // per diagonal block: L^-1 and U^-1 (nb x nb each)
