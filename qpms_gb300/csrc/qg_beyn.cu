@@ -19,12 +19,15 @@
 
 #include <chrono>
 #include <complex>
+#include <memory>
 #include <vector>
 
+#include "qg_arena.h"
 #include "qg_assembly.h"
 #include "qg_dense.h"
 #include "qg_hostla.h"
 #include "qg_internal.h"
+#include "qg_lanes.h"
 
 namespace qg {
 bool scatsys_is_own(const qpms_scatsys_t *ss);
@@ -93,6 +96,18 @@ __global__ void beyn_accumulate_kernel(size_t n, const double2 *X, double2 dz, d
   }
 }
 
+// y += x: the sums of another lane of nodes
+__global__ void beyn_add_kernel(size_t n, const double2 *x, double2 *y) {
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
+    y[t] = make_double2(y[t].x + x[t].x, y[t].y + x[t].y);
+}
+
+// Nodes solved side by side: the substitutions' chains of one overlap the
+// products of the other.  ms for 6 nodes on 1, 2, 3, 4 lanes: 544 unknowns x 16
+// columns 9.4, 6.9, 7.6, 8.4; 1,600 x 32 22.4, 15.6, 15.6, 16.6; 5,776 x 64
+// 109.0, 84.1, 90.4, 83.0; 8 nodes of 14,400 x 64 615, 533, 561, 554.
+constexpr int kBeynLanes = 2;
+
 // ---------------- sources of M(z), built column-major on the device ----------------
 struct MSource {
   size_t m = 0;
@@ -106,6 +121,9 @@ struct MSource {
   }
   // fills stage (row-major, the reference's layout)
   virtual int build_rowmajor(cd z, cudaStream_t st) = 0;
+  // A source of the same matrix for another lane of nodes, with buffers of its
+  // own (init_stage still to be called); null: nodes are built one at a time.
+  virtual MSource *clone() const { return nullptr; }
   int build(cd z, qg_c *dM, cudaStream_t st) {
     int e;
     if ((e = build_rowmajor(z, st))) return e;
@@ -144,8 +162,17 @@ struct FiniteSource : MSource {
   const qpms_scatsys_t *ss = nullptr;
   int iri = -1;
   qg_c *full = nullptr;  // N x N when packing
+  std::unique_ptr<DevArena> in;  // particles, then this node's T-matrices and wavenumber
+  size_t otm = 0, opos = 0, oT = 0, ok = 0;
   ~FiniteSource() override {
     if (full) cudaFree(full);
+  }
+  MSource *clone() const override {
+    if (iri >= 0) return nullptr;
+    FiniteSource *f = new FiniteSource;
+    f->ss = ss;
+    f->m = m;
+    return f;
   }
   int build_rowmajor(cd z, cudaStream_t st) override {
     std::vector<qg_c> T, d;
@@ -153,13 +180,41 @@ struct FiniteSource : MSource {
       scatsys_tdiag(ss, t, z.real(), z.imag(), d);
       T.insert(T.end(), d.begin(), d.end());
     }
-    std::vector<qg_c> k(1, scatsys_wavenumber(ss, z.real(), z.imag()));
-    if (iri < 0) return assemble_modeproblem_device(ss, 1, T, scatsys_dense(ss), k, QPMS_HANKEL_PLUS, stage, st);
-    const size_t N = ss->fecv_size;
-    if (!full) QG_CUDA_TRY(cudaMalloc(&full, N * N * 16));
+    const qg_c k = scatsys_wavenumber(ss, z.real(), z.imag());
     int e;
-    if ((e = assemble_modeproblem_device(ss, 1, T, scatsys_dense(ss), k, QPMS_HANKEL_PLUS, full, st))) return e;
-    return sym_pack_matrix_device(ss, iri, full, N, stage, st);
+    if (!in) {
+      std::vector<double> pos(3 * ss->p_count);
+      std::vector<int> tm(ss->p_count);
+      for (int i = 0; i < ss->p_count; ++i) {
+        pos[3 * i] = ss->p[i].pos.x;
+        pos[3 * i + 1] = ss->p[i].pos.y;
+        pos[3 * i + 2] = ss->p[i].pos.z;
+        tm[i] = ss->p[i].tmatrix_id;
+      }
+      in.reset(new DevArena);
+      otm = in->upload(tm.data(), tm.size() * 4);
+      opos = in->upload(pos.data(), pos.size() * 8);
+      oT = in->add(T.size() * 16);
+      ok = in->add(16);
+      if ((e = in->alloc(st))) return e;
+    }
+    const size_t N = ss->fecv_size;
+    if (iri >= 0 && !full) QG_CUDA_TRY(cudaMalloc(&full, N * N * 16));
+    QG_CUDA_TRY(cudaMemcpyAsync(in->at<qg_c>(oT), T.data(), T.size() * 16, cudaMemcpyHostToDevice, st));
+    QG_CUDA_TRY(cudaMemcpyAsync(in->at<qg_c>(ok), &k, 16, cudaMemcpyHostToDevice, st));
+    AsmArgs a;
+    a.nw = 1;
+    a.np = (int)ss->p_count;
+    a.ntm = (int)ss->tm_count;
+    a.dense = scatsys_dense(ss) ? 1 : 0;
+    a.J = QPMS_HANKEL_PLUS;
+    a.pos = in->at<double>(opos);
+    a.tmid = in->at<int>(otm);
+    a.T = in->at<qg_c>(oT);
+    a.k = in->at<qg_c>(ok);
+    a.M = iri < 0 ? stage : full;
+    if ((e = launch_assemble(a, priv(ss->c)->dev, st))) return e;
+    return iri < 0 ? QPMS_SUCCESS : sym_pack_matrix_device(ss, iri, full, N, stage, st);
   }
 };
 
@@ -295,77 +350,120 @@ int beyn_quadrature(MSource &src, beyn_function_M_inv_Vhat_t minv, void *minv_pa
   std::vector<cd> Vc(nml);
   for (size_t i = 0; i < m; ++i)
     for (size_t j = 0; j < l; ++j) Vc[i + j * m] = Vh[i * l + j];
-  DevPtr dV, dX, dA[4];
-  if (cudaMalloc(&dV.p, nml * 16) != cudaSuccess || cudaMalloc(&dX.p, nml * 16) != cudaSuccess) {
+  DevPtr dV;
+  if (cudaMalloc(&dV.p, nml * 16) != cudaSuccess) {
     set_error("Beyn: out of device memory (m = %zu, l = %zu)", m, l);
     return QPMS_ENOMEM;
   }
-  for (auto &a : dA)
-    if (cudaMalloc(&a.p, nml * 16) != cudaSuccess || cudaMemset(a.p, 0, nml * 16) != cudaSuccess) {
-      set_error("Beyn: out of device memory (m = %zu, l = %zu)", m, l);
-      return QPMS_ENOMEM;
-    }
   if (cudaMemcpy(dV.p, Vc.data(), nml * 16, cudaMemcpyHostToDevice) != cudaSuccess) {
     set_error("Beyn: host to device copy failed");
     return QPMS_ERROR;
   }
-  // the nodes run on a stream of their own (ordered with the legacy default
-  // stream), so that the solver's repeated launch sequences can be captured
-  // as CUDA graphs and replayed node after node
-  struct Stream {
-    cudaStream_t s = nullptr;
-    ~Stream() {
-      if (s) cudaStreamDestroy(s);
+  // lanes of nodes, each with a source, solver, stream and sums of its own
+  int lanes = 1;
+  std::vector<std::unique_ptr<MSource>> clones;
+  if (!minv && mode == 1 && ne - nb > 1) {
+    lanes = lanes_that_fit((int)std::min<size_t>(kBeynLanes, ne - nb),
+                           m * m * 16 + DenseSolver::footprint((int)m, (int)l, mode) + 5 * nml * 16);
+    for (int i = 1; i < lanes; ++i) {
+      clones.emplace_back(src.clone());
+      if (!clones.back()) {
+        clones.clear();
+        lanes = 1;
+      }
     }
-  } ns;
-  if (cudaStreamCreate(&ns.s) != cudaSuccess) {
-    set_error("Beyn: stream creation failed");
-    return QPMS_ERROR;
   }
-  const cudaStream_t st = ns.s;
-  DenseSolver ds;
-  int e;
-  if (!minv && (e = ds.init((int)m, (int)l, mode, seed ^ 0x9e3779b97f4a7c15ULL))) return e;
-  ds.graphs = true;
-  std::vector<qpms_complex_t> hx;
-  double max_res = 0;
-  int max_it = 0;
+  struct Sums {
+    DevPtr dX, dA[4];
+    double max_res = 0;
+    int max_it = 0;
+  };
+  std::vector<Sums> sums(lanes);
   const cd z0 = to_cd(contour->centre);
-  for (size_t i = nb; i < ne; ++i) {
-    const cd z = to_cd(contour->z_dz[i][0]), dz = to_cd(contour->z_dz[i][1]);
-    if (minv) {  // user-supplied M(z)^-1 Vhat (row-major m x l)
-      hx.resize(nml);
-      const int rc = minv(hx.data(), m, l, (const qpms_complex_t *)Vh.data(), from_cd(z), minv_params);
-      if (rc) {
-        set_error("M^-1 Vhat callback returned %d", rc);
-        return rc;
+  if (lanes > 1) QG_CUDA_TRY(cudaStreamSynchronize(0));  // dV is there for every lane's stream
+  auto run = [&](int lane) -> int {
+    // the nodes run on a stream of their own, so that the solver's repeated
+    // launch sequences can be captured as CUDA graphs and replayed node after
+    // node (a single lane's stream is ordered with the legacy default stream)
+    struct Stream {
+      cudaStream_t s = nullptr;
+      ~Stream() {
+        if (s) cudaStreamDestroy(s);
       }
-      for (size_t r = 0; r < m; ++r)
-        for (size_t c = 0; c < l; ++c) Vc[r + c * m] = to_cd(hx[r * l + c]);
-      if (cudaMemcpy(dX.p, Vc.data(), nml * 16, cudaMemcpyHostToDevice) != cudaSuccess) {
-        set_error("Beyn: host to device copy failed");
-        return QPMS_ERROR;
-      }
-    } else {
-      double res = 0;
-      int it = 0;
-      if ((e = src.build_rowmajor(z, st))) return e;
-      // the staged row-major M(z) goes straight to the solver (transposed on the fly)
-      if ((e = ds.factorize(src.stage, m, st, true))) return e;
-      if ((e = ds.solve(src.stage, m, dV.p, dX.p, (int)l, refine_tol, kMaxRefine, &res, &it, st))) return e;
-      if (!(res <= max_res)) max_res = res;  // NaN-propagating max
-      if (it > max_it) max_it = it;
-    }
-    beyn_accumulate_kernel<<<grid1(nml), 256, 0, st>>>(nml, (const double2 *)dX.p, make_double2(dz.real(), dz.imag()),
-                                                make_double2((z - z0).real(), (z - z0).imag()), (i % 2) == 0,
-                                                (double2 *)dA[0].p, (double2 *)dA[1].p, (double2 *)dA[2].p,
-                                                (double2 *)dA[3].p);
-    if (cudaGetLastError() != cudaSuccess) {
-      set_error("Beyn: accumulation kernel launch failed");
+    } ns;
+    if (cudaStreamCreateWithFlags(&ns.s, lanes > 1 ? cudaStreamNonBlocking : cudaStreamDefault) != cudaSuccess) {
+      set_error("Beyn: stream creation failed");
       return QPMS_ERROR;
     }
-    g_launches.fetch_add(1);
+    const cudaStream_t st = ns.s;
+    Sums &S = sums[lane];
+    if (cudaMalloc(&S.dX.p, nml * 16) != cudaSuccess) {
+      set_error("Beyn: out of device memory (m = %zu, l = %zu)", m, l);
+      return QPMS_ENOMEM;
+    }
+    for (auto &a : S.dA)
+      if (cudaMalloc(&a.p, nml * 16) != cudaSuccess || cudaMemsetAsync(a.p, 0, nml * 16, st) != cudaSuccess) {
+        set_error("Beyn: out of device memory (m = %zu, l = %zu)", m, l);
+        return QPMS_ENOMEM;
+      }
+    MSource &so = lane ? *clones[lane - 1] : src;
+    int e;
+    if (lane && (e = so.init_stage())) return e;
+    DenseSolver ds;
+    if (!minv && (e = ds.init((int)m, (int)l, mode, seed ^ 0x9e3779b97f4a7c15ULL, nullptr, st))) return e;
+    ds.graphs = true;
+    std::vector<qpms_complex_t> hx;
+    for (size_t i = nb + lane; i < ne; i += lanes) {
+      const cd z = to_cd(contour->z_dz[i][0]), dz = to_cd(contour->z_dz[i][1]);
+      if (minv) {  // user-supplied M(z)^-1 Vhat (row-major m x l)
+        hx.resize(nml);
+        const int rc = minv(hx.data(), m, l, (const qpms_complex_t *)Vh.data(), from_cd(z), minv_params);
+        if (rc) {
+          set_error("M^-1 Vhat callback returned %d", rc);
+          return rc;
+        }
+        for (size_t r = 0; r < m; ++r)
+          for (size_t c = 0; c < l; ++c) Vc[r + c * m] = to_cd(hx[r * l + c]);
+        if (cudaMemcpy(S.dX.p, Vc.data(), nml * 16, cudaMemcpyHostToDevice) != cudaSuccess) {
+          set_error("Beyn: host to device copy failed");
+          return QPMS_ERROR;
+        }
+      } else {
+        double res = 0;
+        int it = 0;
+        if ((e = so.build_rowmajor(z, st))) return e;
+        // the staged row-major M(z) goes straight to the solver (transposed on the fly)
+        if ((e = ds.factorize(so.stage, m, st, true))) return e;
+        if ((e = ds.solve(so.stage, m, dV.p, S.dX.p, (int)l, refine_tol, kMaxRefine, &res, &it, st))) return e;
+        if (!(res <= S.max_res)) S.max_res = res;  // NaN-propagating max
+        if (it > S.max_it) S.max_it = it;
+      }
+      beyn_accumulate_kernel<<<grid1(nml), 256, 0, st>>>(
+          nml, (const double2 *)S.dX.p, make_double2(dz.real(), dz.imag()),
+          make_double2((z - z0).real(), (z - z0).imag()), (i % 2) == 0, (double2 *)S.dA[0].p, (double2 *)S.dA[1].p,
+          (double2 *)S.dA[2].p, (double2 *)S.dA[3].p);
+      if (cudaGetLastError() != cudaSuccess) {
+        set_error("Beyn: accumulation kernel launch failed");
+        return QPMS_ERROR;
+      }
+      g_launches.fetch_add(1);
+    }
+    QG_CUDA_TRY(cudaStreamSynchronize(st));
+    return QPMS_SUCCESS;
+  };
+  int e;
+  if ((e = run_lanes(lanes, run))) return e;
+  for (int i = 1; i < lanes; ++i) {  // in the lanes' order
+    for (int c = 0; c < 4; ++c)
+      beyn_add_kernel<<<grid1(nml), 256>>>(nml, (const double2 *)sums[i].dA[c].p, (double2 *)sums[0].dA[c].p);
+    QG_CUDA_TRY(cudaGetLastError());
+    g_launches.fetch_add(4);
+    if (!(sums[i].max_res <= sums[0].max_res)) sums[0].max_res = sums[i].max_res;
+    sums[0].max_it = std::max(sums[0].max_it, sums[i].max_it);
   }
+  DevPtr(&dA)[4] = sums[0].dA;
+  const double max_res = sums[0].max_res;
+  const int max_it = sums[0].max_it;
   A0.resize(nml);
   A1.resize(nml);
   A0c.resize(nml);

@@ -22,6 +22,7 @@
 #include "qg_batchlu.h"
 #include "qg_dense.h"
 #include "qg_internal.h"
+#include "qg_lanes.h"
 
 namespace qg {
 bool scatsys_is_own(const qpms_scatsys_t *ss);
@@ -76,9 +77,16 @@ int ptr_array(Dev &arr, void *base, size_t stride_bytes, int nb) {
 // each frequency runs through the dense solver (RBT + blocked LU) instead.
 constexpr size_t kBatchedMaxN = 512;
 
-// The finite plane-wave scatter for large systems: one frequency at a time
-// (one N x N matrix resident), assembly -> incidence -> T a -> dense solve
-// with FP64 refinement -> sigma_ext (and sigma_scat).
+// Frequencies solved side by side: a solve is a chain of small kernels (the
+// inversions of the diagonal blocks, narrow products, substitutions) that leaves
+// most of the GPU idle, the more so the smaller the system.  ms for 4 (14,400
+// unknowns: 2) frequencies on 1, 2, 3, 4 lanes: 600 unknowns 4.8, 3.3, 3.5, 3.3;
+// 1,350 9.0, 5.5, 5.9, 4.6; 7,500 58.1, 40.4, 42.0, 34.9; 14,400 97.5, 81.3.
+int scatter_lanes(size_t N, int W) { return std::min(W, N <= 8192 ? 4 : 2); }
+
+// The finite plane-wave scatter for large systems, an N x N matrix resident per
+// lane of frequencies: assembly -> incidence -> T a -> dense solve with FP64
+// refinement -> sigma_ext (and sigma_scat).
 int finite_scatter_dense(const qpms_scatsys_t *ss, int W, const std::vector<qg_c> &T, const std::vector<qg_c> &k,
                          const std::vector<double> &kvec, const std::vector<qg_c> &coef, int mode, qpms_complex_t *f_out,
                          double *sigma_ext, double *sigma_scat, double *resid_out, int *iters_out) {
@@ -86,14 +94,6 @@ int finite_scatter_dense(const qpms_scatsys_t *ss, int W, const std::vector<qg_c
   const int n = 2 * lMax * (lMax + 2);
   const size_t N = ss->fecv_size, N2 = N * N;
   const size_t tper = T.size() / W;
-  cudaStream_t st = 0;
-  int e;
-  Dev dM, dT, dtm, dpos, dk, dkv, dcoef, da, db, dx, dr, dn, dsig;
-  if ((e = dalloc(dM, N2 * 16)) || (e = dalloc(dT, tper * 16)) || (e = dalloc(dtm, np * 4)) ||
-      (e = dalloc(dpos, np * 24)) || (e = dalloc(dk, 16)) || (e = dalloc(dkv, 24)) || (e = dalloc(dcoef, n * 16)) ||
-      (e = dalloc(da, N * 16)) || (e = dalloc(db, N * 16)) || (e = dalloc(dx, N * 16)) || (e = dalloc(dr, N * 16)) ||
-      (e = dalloc(dn, 16)) || (e = dalloc(dsig, 8)))
-    return e;
   std::vector<double> pos(3 * np);
   std::vector<int> tm(np);
   for (int i = 0; i < np; ++i) {
@@ -102,99 +102,119 @@ int finite_scatter_dense(const qpms_scatsys_t *ss, int W, const std::vector<qg_c
     pos[3 * i + 2] = ss->p[i].pos.z;
     tm[i] = ss->p[i].tmatrix_id;
   }
-  QG_CUDA_TRY(cudaMemcpy(dtm.p, tm.data(), np * 4, cudaMemcpyHostToDevice));
-  QG_CUDA_TRY(cudaMemcpy(dpos.p, pos.data(), np * 24, cudaMemcpyHostToDevice));
-  QG_CUDA_TRY(cudaMemcpy(dcoef.p, coef.data(), n * 16, cudaMemcpyHostToDevice));
+  const bool dense = scatsys_dense(ss);
+  const std::vector<qg_c> mone(sigma_scat ? (size_t)ntm * n : 0, cmk(-1.0, 0.0));  // diagonal -1
+  DevArena in;
+  const size_t oT = in.upload(T.data(), T.size() * 16), otm = in.upload(tm.data(), np * 4),
+               opos = in.upload(pos.data(), np * 24), ok = in.upload(k.data(), W * 16),
+               okv = in.upload(kvec.data(), W * 24), ocoef = in.upload(coef.data(), n * 16),
+               omone = in.upload(mone.data(), mone.size() * 16);
+  int e;
+  if ((e = in.alloc(0))) return e;
   // With a point symmetry the system splits into one independent system per
   // irrep (about N / |G| unknowns each: |G|^2 fewer LU flops): M and T a are
   // packed on the device, each irrep is solved, and the solutions unpacked.
   const int nir = sym_nirreps(ss);
-  DenseSolver ds;
-  std::vector<std::unique_ptr<DenseSolver>> dsi(nir);
-  Dev dMp, dbp, dxp;
   size_t namax = 0;
   for (int i = 0; i < nir; ++i) namax = std::max(namax, sym_size(ss, i));
-  if (nir == 0) {
-    if ((e = ds.init((int)N, 1, mode, 0x5eedbe11))) return e;
-  } else {
-    if ((e = dalloc(dMp, namax * namax * 16)) || (e = dalloc(dbp, namax * 16)) || (e = dalloc(dxp, namax * 16)))
-      return e;
-    for (int i = 0; i < nir; ++i) {
-      const size_t na = sym_size(ss, i);
-      if (!na) continue;
-      dsi[i].reset(new DenseSolver());
-      if ((e = dsi[i]->init((int)na, 1, mode, 0x5eedbe11 + i))) return e;
-    }
-  }
-  const bool dense = scatsys_dense(ss);
-  auto assemble = [&](int J, const qg_c *Tsrc, size_t count, bool dn) -> int {
-    QG_CUDA_TRY(cudaMemcpy(dT.p, Tsrc, count * 16, cudaMemcpyHostToDevice));
-    AsmArgs a;
-    a.nw = 1;
-    a.np = np;
-    a.ntm = ntm;
-    a.dense = dn ? 1 : 0;
-    a.J = J;
-    a.pos = dpos.as<double>();
-    a.tmid = dtm.as<int>();
-    a.T = dT.as<qg_c>();
-    a.k = dk.as<qg_c>();
-    a.M = dM.as<qg_c>();
-    return launch_assemble(a, priv(ss->c)->dev, st);
-  };
-  const std::vector<qg_c> mone((size_t)ntm * n, cmk(-1.0, 0.0));  // diagonal -1
-  for (int w = 0; w < W; ++w) {
-    QG_CUDA_TRY(cudaMemcpy(dk.p, &k[w], 16, cudaMemcpyHostToDevice));
-    QG_CUDA_TRY(cudaMemcpy(dkv.p, &kvec[3 * w], 24, cudaMemcpyHostToDevice));
-    if ((e = assemble(3, T.data() + w * tper, tper, dense))) return e;  // row-major M = I - T S
-    if ((e = launch_incident(1, np, n, dcoef.as<qg_c>(), dkv.as<double>(), dpos.as<double>(), da.as<qg_c>(), st)))
-      return e;
-    if ((e = launch_apply_t(1, np, n, ntm, dense ? 1 : 0, dtm.as<int>(), dT.as<qg_c>(), da.as<qg_c>(),
-                            db.as<qg_c>(), st)))
-      return e;
-    double res = 0;
-    int it = 0;
+  // the complex128 path fills the GPU by itself
+  const int lanes = nir == 0 && mode == 1 ? lanes_that_fit(scatter_lanes(N, W), N2 * 16 + DenseSolver::footprint((int)N, 1, 1)) : 1;
+  if (lanes > 1) QG_CUDA_TRY(cudaStreamSynchronize(0));  // the inputs are there for every lane's stream
+  auto run = [&](int lane) -> int {
+    LaneStream ls;
+    int e;
+    if (lanes > 1 && (e = ls.create())) return e;
+    const cudaStream_t st = ls.s;
+    DevArena ar;
+    const size_t oM = ar.add(N2 * 16), oa = ar.add(N * 16), ob = ar.add(N * 16), ox = ar.add(N * 16),
+                 orr = ar.add(N * 16), on = ar.add(16), osig = ar.add(16), oMp = ar.add(namax * namax * 16),
+                 obp = ar.add(namax * 16), oxp = ar.add(namax * 16);
+    if ((e = ar.alloc(st))) return e;
+    qg_c *dM = ar.at<qg_c>(oM), *da = ar.at<qg_c>(oa), *db = ar.at<qg_c>(ob), *dx = ar.at<qg_c>(ox),
+         *dr = ar.at<qg_c>(orr);
+    double *rn2 = ar.at<double>(on), *dsig = ar.at<double>(osig);
+    const int *dtm = in.at<int>(otm);
+    const double *dpos = in.at<double>(opos);
+    DenseSolver ds;
+    std::vector<std::unique_ptr<DenseSolver>> dsi(nir);
     if (nir == 0) {
-      if ((e = ds.factorize(dM.p, N, st, true))) return e;
-      if ((e = ds.solve(dM.p, N, db.p, dx.p, 1, 1e-13, 12, &res, &it, st))) return e;
+      if ((e = ds.init((int)N, 1, mode, 0x5eedbe11, nullptr, st))) return e;
     } else {
-      QG_CUDA_TRY(cudaMemsetAsync(dx.p, 0, N * 16, st));
       for (int i = 0; i < nir; ++i) {
         const size_t na = sym_size(ss, i);
         if (!na) continue;
-        double ri = 0;
-        int iti = 0;
-        if ((e = sym_pack_matrix_device(ss, i, dM.as<qg_c>(), N, dMp.as<qg_c>(), st)) ||
-            (e = sym_pack_vectors_device(ss, i, db.as<qg_c>(), 1, N, dbp.as<qg_c>(), na, st)) ||
-            (e = dsi[i]->factorize(dMp.p, na, st, true)) ||
-            (e = dsi[i]->solve(dMp.p, na, dbp.p, dxp.p, 1, 1e-13, 12, &ri, &iti, st)) ||
-            (e = sym_unpack_add_vectors_device(ss, i, dxp.as<qg_c>(), 1, na, dx.as<qg_c>(), N, st)))
-          return e;
-        it = std::max(it, iti);
+        dsi[i].reset(new DenseSolver());
+        if ((e = dsi[i]->init((int)na, 1, mode, 0x5eedbe11 + i, nullptr, st))) return e;
       }
-      // the residual of the unpacked solution in the full system (FP64)
-      double *rn2 = dn.as<double>(), h2[2];
-      if ((e = launch_residual(1, N, dM.as<qg_c>(), dx.as<qg_c>(), db.as<qg_c>(), dr.as<qg_c>(), rn2, rn2 + 1, st)))
-        return e;
-      QG_CUDA_TRY(cudaMemcpy(h2, rn2, 16, cudaMemcpyDeviceToHost));
-      res = sqrt(h2[0] / (h2[1] > 0 ? h2[1] : 1));
     }
-    if (resid_out) resid_out[w] = res;
-    if (iters_out) iters_out[w] = it;
-    if ((e = launch_sigma_ext(1, N, da.as<qg_c>(), dx.as<qg_c>(), dk.as<qg_c>(), dsig.as<double>(), st))) return e;
-    QG_CUDA_TRY(cudaMemcpy(sigma_ext + w, dsig.p, 8, cudaMemcpyDeviceToHost));
-    if (sigma_scat) {
-      if ((e = assemble(1, mone.data(), mone.size(), false))) return e;  // I + R (regular waves, zero self blocks)
-      QG_CUDA_TRY(cudaMemsetAsync(db.p, 0, N * 16, st));
-      double *rn2 = dn.as<double>();
-      if ((e = launch_residual(1, N, dM.as<qg_c>(), dx.as<qg_c>(), db.as<qg_c>(), dr.as<qg_c>(), rn2, rn2 + 1, st)))
+    for (int w = lane; w < W; w += lanes) {
+      const qg_c *dT = in.at<qg_c>(oT) + w * tper, *dk = in.at<qg_c>(ok) + w;
+      auto assemble = [&](int J, const qg_c *Td, bool dn) -> int {
+        AsmArgs a;
+        a.nw = 1;
+        a.np = np;
+        a.ntm = ntm;
+        a.dense = dn ? 1 : 0;
+        a.J = J;
+        a.pos = dpos;
+        a.tmid = dtm;
+        a.T = Td;
+        a.k = dk;
+        a.M = dM;
+        return launch_assemble(a, priv(ss->c)->dev, st);
+      };
+      if ((e = assemble(3, dT, dense)) ||  // row-major M = I - T S
+          (e = launch_incident(1, np, n, in.at<qg_c>(ocoef), in.at<double>(okv) + 3 * w, dpos, da, st)) ||
+          (e = launch_apply_t(1, np, n, ntm, dense ? 1 : 0, dtm, dT, da, db, st)))
         return e;
-      if ((e = launch_sigma_ext(1, N, dx.as<qg_c>(), dr.as<qg_c>(), dk.as<qg_c>(), dsig.as<double>(), st))) return e;
-      QG_CUDA_TRY(cudaMemcpy(sigma_scat + w, dsig.p, 8, cudaMemcpyDeviceToHost));
+      double res = 0;
+      int it = 0;
+      if (nir == 0) {
+        if ((e = ds.factorize(dM, N, st, true))) return e;
+        if ((e = ds.solve(dM, N, db, dx, 1, 1e-13, 12, &res, &it, st))) return e;
+      } else {
+        QG_CUDA_TRY(cudaMemsetAsync(dx, 0, N * 16, st));
+        for (int i = 0; i < nir; ++i) {
+          const size_t na = sym_size(ss, i);
+          if (!na) continue;
+          double ri = 0;
+          int iti = 0;
+          qg_c *dMp = ar.at<qg_c>(oMp), *dbp = ar.at<qg_c>(obp), *dxp = ar.at<qg_c>(oxp);
+          if ((e = sym_pack_matrix_device(ss, i, dM, N, dMp, st)) ||
+              (e = sym_pack_vectors_device(ss, i, db, 1, N, dbp, na, st)) ||
+              (e = dsi[i]->factorize(dMp, na, st, true)) ||
+              (e = dsi[i]->solve(dMp, na, dbp, dxp, 1, 1e-13, 12, &ri, &iti, st)) ||
+              (e = sym_unpack_add_vectors_device(ss, i, dxp, 1, na, dx, N, st)))
+            return e;
+          it = std::max(it, iti);
+        }
+        // the residual of the unpacked solution in the full system (FP64)
+        double h2[2];
+        if ((e = launch_residual(1, N, dM, dx, db, dr, rn2, rn2 + 1, st))) return e;
+        QG_CUDA_TRY(cudaMemcpyAsync(h2, rn2, 16, cudaMemcpyDeviceToHost, st));
+        QG_CUDA_TRY(cudaStreamSynchronize(st));
+        res = sqrt(h2[0] / (h2[1] > 0 ? h2[1] : 1));
+      }
+      if (resid_out) resid_out[w] = res;
+      if (iters_out) iters_out[w] = it;
+      if ((e = launch_sigma_ext(1, N, da, dx, dk, dsig, st))) return e;
+      if (sigma_scat) {
+        if ((e = assemble(1, in.at<qg_c>(omone), false))) return e;  // I + R (regular waves, zero self blocks)
+        QG_CUDA_TRY(cudaMemsetAsync(db, 0, N * 16, st));
+        if ((e = launch_residual(1, N, dM, dx, db, dr, rn2, rn2 + 1, st)) ||
+            (e = launch_sigma_ext(1, N, dx, dr, dk, dsig + 1, st)))
+          return e;
+      }
+      double hs[2];
+      QG_CUDA_TRY(cudaMemcpyAsync(hs, dsig, 16, cudaMemcpyDeviceToHost, st));
+      if (f_out) QG_CUDA_TRY(cudaMemcpyAsync(f_out + w * N, dx, N * 16, cudaMemcpyDeviceToHost, st));
+      QG_CUDA_TRY(cudaStreamSynchronize(st));
+      sigma_ext[w] = hs[0];
+      if (sigma_scat) sigma_scat[w] = hs[1];
     }
-    if (f_out) QG_CUDA_TRY(cudaMemcpy(f_out + w * N, dx.p, N * 16, cudaMemcpyDeviceToHost));
-  }
-  return QPMS_SUCCESS;
+    return QPMS_SUCCESS;
+  };
+  return run_lanes(lanes, run);
 }
 
 }  // namespace
