@@ -1007,10 +1007,344 @@ __global__ void __launch_bounds__(kEThreads) ewald_assemble_kernel(EwaldArgs a, 
   }
 }
 
+// ---------------- scans at real wavenumbers ----------------
+// ewald_assemble_kernel's sums where k is real and the short-range terms come
+// from tables, with everything that is real kept real:
+//  * short range: prefac_n I_n is -i times a real number, so a point adds the
+//    four real products of (cos, sin)(m phi) and (cos, sin)(beta.(R - s)) times
+//    a tabulated real number, for n, +m and -m together: accumulators CC, CS,
+//    SC, SS with sigma_{n,+-m} = -i [(CC -+ SS) + i (CS +- SC)] (and (-1)^m for -m);
+//  * long range: Gamma and gamma are real for evanescent orders, and for
+//    propagating ones real numbers times a known power of i (Gamma(1/2 - j, -c^2)
+//    has the imaginary recurrence (G - (-1)^(j+1) c^(1-2j) e^(c^2)) / (1/2 - j));
+//    e^{i m alpha} (q/k)^m = ((q_x + i q_y) / k)^m needs no angle; i^(n+1) turns
+//    into a static permutation of the same four accumulators;
+//  * a class test without square roots, evanescent and propagating points in
+//    different warps, reductions folded over 8 values at a time, the self term
+//    once per frequency from the table kernel.
+// Bound: the FP64 pipe, about a quarter of the instructions of the general kernel.
+// 16 x 256 points of the square lattice at lMax 3: 3.35 -> 1.52 ms; 5 x 201 of the
+// honeycomb lattice 3.06 -> 1.45 ms (pipe 80 % busy).
+template <int LMAX>
+struct ScanShape {
+  static constexpr int LE = 2 * LMAX + 1;
+  static constexpr int NEV = (LE + 1) * (LE + 2) / 2;  // (n, m) with n + m even: also tabulated numbers per point
+  static constexpr int NR = 2 * NEV;                   // accumulators
+  static constexpr int NG = (NR + 7) / 8;              // reduction groups
+  static constexpr int NH = LE / 2 + 1;                // (n - |m|) / 2 + 1 at most
+};
+
+// Sums of the 8 values over the warp's lanes; lane l gets the sum of v[l >> 2].
+__device__ __forceinline__ double fold8(double (&v)[8], int lane) {
+#pragma unroll
+  for (int h = 4, o = 16; h; h >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const double keep = up ? v[i + h] : v[i], give = up ? v[i] : v[i + h];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// acc[e..] += i^r j (p1, p2, p3, p4): the products of order m's phase
+template <int R>
+__device__ __forceinline__ void acc4(double *acc, double j, double p1, double p2, double p3, double p4) {
+  // i (CC, CS, SC, SS) = (-CS, CC, -SS, SC)
+  if constexpr (R == 0) {
+    acc[0] = fma(j, p1, acc[0]);
+    acc[1] = fma(j, p2, acc[1]);
+    acc[2] = fma(j, p3, acc[2]);
+    acc[3] = fma(j, p4, acc[3]);
+  } else if constexpr (R == 1) {
+    acc[0] = fma(-j, p2, acc[0]);
+    acc[1] = fma(j, p1, acc[1]);
+    acc[2] = fma(-j, p4, acc[2]);
+    acc[3] = fma(j, p3, acc[3]);
+  } else {
+    acc4<R - 2>(acc, -j, p1, p2, p3, p4);
+  }
+}
+template <int R>
+__device__ __forceinline__ void acc2(double *acc, double j, double p1, double p2) {
+  if constexpr (R == 0) {
+    acc[0] = fma(j, p1, acc[0]);
+    acc[1] = fma(j, p2, acc[1]);
+  } else if constexpr (R == 1) {
+    acc[0] = fma(-j, p2, acc[0]);
+    acc[1] = fma(j, p1, acc[1]);
+  } else {
+    acc2<R - 2>(acc, -j, p1, p2);
+  }
+}
+
+// One reciprocal point's terms of order m = M and above: Pr, Pi [h (h + 1) / 2 + j]
+// = (q/k)^(2 (h - j)) gamma^(2j - 1) Gamma_j (Pi: propagating points only).
+template <int LMAX, bool PROP, int M, int E>
+__device__ __forceinline__ void scan_orders(double (&acc)[ScanShape<LMAX>::NR], const double *Pr, const double *Pi,
+                                            double pr, double pi, double px, double py, double a, double b) {
+  constexpr int LE = ScanShape<LMAX>::LE;
+  const double p1 = pr * a, p2 = pi * a, p3 = pr * b, p4 = pi * b;
+#pragma unroll
+  for (int n = M; n <= LE; n += 2) {
+    const int h = (n - M) / 2, y = n * (n + 1) + M;
+    constexpr int W = M ? 4 : 2;
+    double jr = 0, ji = 0;
+#pragma unroll
+    for (int j = 0; j <= h; ++j) {
+      const double c = c_ew.s1r[c_ew.s1off[y] + j];
+      jr = fma(c, Pr[h * (h + 1) / 2 + j], jr);
+      if (PROP) ji = fma(c, Pi[h * (h + 1) / 2 + j], ji);
+    }
+    double *x = acc + E + W * h;
+    // i^(n+1) (jr + i ji) in units of -i: i^(n+2); n = M, M + 2, ...: i^(M+2) (-1)^h
+    if (h & 1) {
+      jr = -jr;
+      ji = -ji;
+    }
+    if constexpr (M > 0) {
+      acc4<(M + 2) & 3>(x, jr, p1, p2, p3, p4);
+      if (PROP) acc4<(M + 3) & 3>(x, ji, p1, p2, p3, p4);
+    } else {
+      acc2<2>(x, jr, p1, p2);
+      if (PROP) acc2<3>(x, ji, p1, p2);
+    }
+  }
+  if constexpr (M < LE)
+    scan_orders<LMAX, PROP, M + 1, E + (M ? 4 : 2) * ((LE - M) / 2 + 1)>(acc, Pr, Pi, pr, pi, px, py,
+                                                                        fma(a, px, -b * py), fma(a, py, b * px));
+}
+
+
+template <int LMAX>
+__global__ void __launch_bounds__(kEThreads) ewald_scan_kernel(EwaldArgs a, TransDevTables T) {
+  using Sc = ScanShape<LMAX>;
+  constexpr int LE = Sc::LE, NEV = Sc::NEV, NR = Sc::NR, NG = Sc::NG, NH = Sc::NH, S = EwShape<LMAX>::S;
+  __shared__ qg_c sig[S];
+  __shared__ double red[kEThreads / 32][NG * 8];
+  __shared__ int lstA[kEThreads * kELChunks], lstB[kEThreads * kELChunks];
+  __shared__ int lw[2][kEThreads / 32], lcnt[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int np = a.np;
+  const size_t per = (size_t)np * np, units = (size_t)a.nw * a.nk * per;
+  const double sqpi = 1.7724538509055160273;
+  for (size_t u = blockIdx.x; u < units; u += gridDim.x) {
+    const int pr = (int)(u % per);
+    const size_t wk = u / per;
+    const int iw = (int)(wk / a.nk), ik = (int)(wk % a.nk);
+    const int R = pr / np, C = pr - R * np;
+    const double k = a.k[iw].re, eta = a.eta[wk], bx = a.beta[2 * ik], by = a.beta[2 * ik + 1];
+    const double sx = a.pos[3 * R] - a.pos[3 * C], sy = a.pos[3 * R + 1] - a.pos[3 * C + 1];
+    if (a.pos[3 * R + 2] != a.pos[3 * C + 2]) {  // a pair of layers: ewald_layers_kernel forms it
+      if (!a.layered && tid == 0) atomicOr(a.err, 2);
+      continue;
+    }
+    const bool self = sx == 0.0 && sy == 0.0;
+    double acc[NR];
+#pragma unroll
+    for (int i = 0; i < NR; ++i) acc[i] = 0.0;
+    // ---------------- short range (from the last warp down) ----------------
+    {
+      const size_t ti = (size_t)iw * per + pr;
+      const int cnt = a.srcnt[ti];
+      const double *tab = reinterpret_cast<const double *>(a.srtab) + ti * NEV * (size_t)a.srmax;
+      const double *pts = a.srpts + ti * 2 * (size_t)a.srmax;
+      for (int p = kEThreads - 1 - tid; p < cnt; p += kEThreads) {
+        double sb, cb;
+        sincos(bx * pts[2 * p] + by * pts[2 * p + 1], &sb, &cb);
+        const double *t = tab + p;
+        int e = 0;
+#pragma unroll
+        for (int m = 0; m <= LE; ++m)
+#pragma unroll
+          for (int n = m; n <= LE; n += 2) {
+            const double tc = *t;
+            t += a.srmax;
+            acc[e] = fma(tc, cb, acc[e]);
+            acc[e + 1] = fma(tc, sb, acc[e + 1]);
+            e += 2;
+            if (m) {
+              const double ts = *t;
+              t += a.srmax;
+              acc[e] = fma(ts, cb, acc[e]);
+              acc[e + 1] = fma(ts, sb, acc[e + 1]);
+              e += 2;
+            }
+          }
+      }
+    }
+    // ---------------- long range ----------------
+    {
+      const double k2 = k * k, rk = 1.0 / k, cut = 56.0 * 4 * eta * eta;
+      const double Kc = sqrt(k2 + cut) + sqrt(bx * bx + by * by);
+      const int I1 = (int)ceil(Kc * c_ew.bn[0] / (2 * M_PI)) + 1;
+      const int I2 = (int)ceil(Kc * c_ew.bn[1] / (2 * M_PI)) + 1;
+      const int W1 = 2 * I1 + 1, W2 = 2 * I2 + 1;
+      const bool ok = (long)W1 * W2 <= kEwMaxPoints && I1 >= 0 && I2 >= 0;
+      if (!ok && tid == 0) atomicOr(a.err, 1);
+      const double lrfac = rk * rk / c_ew.area, k2eta = k / (2 * eta);
+      const int WW = ok ? W1 * W2 : 0;
+      for (int t0 = 0; t0 < WW; t0 += kEThreads * kELChunks) {
+        // classes (0 past the cutoff, 1 evanescent, 2 propagating), compacted in grid order
+        __syncthreads();
+        if (tid == 0) {
+          lcnt[0] = 0;
+          lcnt[1] = 0;
+        }
+        __syncthreads();
+        for (int c = 0; c < kELChunks && t0 + c * kEThreads < WW; ++c) {
+          const int t = t0 + c * kEThreads + tid;
+          int cls = 0;
+          if (t < WW) {
+            const int i = t / W2 - I1, j = t % W2 - I2;
+            const double qx = i * c_ew.rb[0] + j * c_ew.rb[2] + bx, qy = i * c_ew.rb[1] + j * c_ew.rb[3] + by;
+            const double q2 = fma(qx, qx, qy * qy), d = q2 - k2;
+            if (d <= cut) {
+              cls = d > 0 ? 1 : 2;
+              if (fabs(d) < 1e-9 * k2) cls = sqrt(q2) / k >= 1.0 ? 1 : 2;  // as gamma is formed below
+            }
+          }
+          const unsigned bA = __ballot_sync(0xffffffffu, cls == 1), bB = __ballot_sync(0xffffffffu, cls == 2);
+          if (lane == 0) {
+            lw[0][warp] = __popc(bA);
+            lw[1][warp] = __popc(bB);
+          }
+          __syncthreads();
+          int oA = lcnt[0], oB = lcnt[1];
+          for (int w = 0; w < warp; ++w) {
+            oA += lw[0][w];
+            oB += lw[1][w];
+          }
+          const unsigned lt = (1u << lane) - 1u;
+          if (cls == 1) lstA[oA + __popc(bA & lt)] = t;
+          if (cls == 2) lstB[oB + __popc(bB & lt)] = t;
+          __syncthreads();
+          if (tid == 0)
+            for (int w = 0; w < kEThreads / 32; ++w) {
+              lcnt[0] += lw[0][w];
+              lcnt[1] += lw[1][w];
+            }
+          __syncthreads();
+        }
+        const int nA = lcnt[0], nB = lcnt[1], padA = (nA + 31) & ~31;
+        for (int pidx = tid; pidx < padA + nB; pidx += kEThreads) {
+          const bool prop = pidx >= padA;  // uniform in the warp
+          if (!prop && pidx >= nA) continue;
+          const int t = prop ? lstB[pidx - padA] : lstA[pidx];
+          const int i = t / W2 - I1, j = t % W2 - I2;
+          const double Kx = i * c_ew.rb[0] + j * c_ew.rb[2], Ky = i * c_ew.rb[1] + j * c_ew.rb[3];
+          const double qx = Kx + bx, qy = Ky + by, q2 = fma(qx, qx, qy * qy), t2 = q2 * rk * rk;
+          double pr_ = lrfac, pi_ = 0.0;  // e^{i K.s} / (k^2 A)
+          if (!self) {
+            double sK, cK;
+            sincos(Kx * sx + Ky * sy, &sK, &cK);
+            pr_ = lrfac * cK;
+            pi_ = lrfac * sK;
+          }
+          // gamma from the exact difference q/k - 1 (near a Rayleigh anomaly 1 / gamma dominates)
+          const double tt = sqrt(q2) / k, g2 = fabs((tt - 1.0) * (tt + 1.0)), rg = rsqrt(g2), g = g2 * rg;
+          const double x = g * k2eta, X = x * x, rx = rg / k2eta, rX = rx * rx;
+          double Pr[NH * (NH + 1) / 2], Pi[NH * (NH + 1) / 2];
+          if (!prop) {
+            double G[NH];
+            const double emX = exp(-X);
+            G[0] = sqpi * erfc(x);  // Gamma(1/2, X)
+            double zp = rx * emX;   // X^(1/2-j) e^-X
+#pragma unroll
+            for (int jj = 1; jj < NH; ++jj) {
+              G[jj] = (G[jj - 1] - zp) * (1.0 / (0.5 - jj));
+              zp *= rX;
+            }
+            double gp = rg;
+#pragma unroll
+            for (int jj = 0; jj < NH; ++jj) {
+              G[jj] *= gp;  // gamma^(2j-1) Gamma_j
+              gp *= g2;
+            }
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+#pragma unroll
+              for (int jj = 0; jj < h; ++jj) Pr[h * (h + 1) / 2 + jj] = t2 * Pr[h * (h - 1) / 2 + jj];
+              Pr[h * (h + 1) / 2 + h] = G[h];
+            }
+            scan_orders<LMAX, false, 0, 0>(acc, Pr, Pi, pr_, pi_, qx * rk, qy * rk, 1.0, 0.0);
+          } else {
+            // gamma = -i g, x = -i c (c = x here): Gamma(1/2, -c^2) = sqrt(pi) erfc(-i c)
+            const qg_c e0 = cerfc(cmk(0.0, -x), c_wd);
+            double Gr[NH], Gi[NH];
+            Gr[0] = sqpi * e0.re;
+            Gi[0] = sqpi * e0.im;
+            double zp = rx * exp(X);  // (-1)^(j+1) c^(1-2j) e^(c^2)
+#pragma unroll
+            for (int jj = 1; jj < NH; ++jj) {
+              Gr[jj] = Gr[jj - 1] * (1.0 / (0.5 - jj));
+              Gi[jj] = (Gi[jj - 1] - zp) * (1.0 / (0.5 - jj));
+              zp *= -rX;
+            }
+            double gp = rg;  // gamma^(2j-1) = i (-1)^j g^(2j-1)
+#pragma unroll
+            for (int jj = 0; jj < NH; ++jj) {
+              const double r = -gp * Gi[jj];
+              Gi[jj] = gp * Gr[jj];
+              Gr[jj] = r;
+              gp *= -g2;
+            }
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+#pragma unroll
+              for (int jj = 0; jj < h; ++jj) {
+                Pr[h * (h + 1) / 2 + jj] = t2 * Pr[h * (h - 1) / 2 + jj];
+                Pi[h * (h + 1) / 2 + jj] = t2 * Pi[h * (h - 1) / 2 + jj];
+              }
+              Pr[h * (h + 1) / 2 + h] = Gr[h];
+              Pi[h * (h + 1) / 2 + h] = Gi[h];
+            }
+            scan_orders<LMAX, true, 0, 0>(acc, Pr, Pi, pr_, pi_, qx * rk, qy * rk, 1.0, 0.0);
+          }
+        }
+      }
+    }
+    // ---------------- reduction into sig[] ----------------
+#pragma unroll
+    for (int q = 0; q < NG; ++q) {
+      double v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = 8 * q + i < NR ? acc[8 * q + i < NR ? 8 * q + i : 0] : 0.0;
+      const double sum = fold8(v, lane);
+      if ((lane & 3) == 0) red[warp][8 * q + (lane >> 2)] = sum;
+    }
+    for (int s = tid; s < S; s += kEThreads) sig[s] = cmk(0, 0);
+    __syncthreads();
+    for (int q = tid; q < NEV; q += kEThreads) {
+      // q-th (m, n, sign): m = 0 has one, m > 0 both signs
+      int m = 0, e = q, base = 0;
+      for (int c; e >= (c = ((LE - m) / 2 + 1) * (m ? 2 : 1)); ++m) {
+        e -= c;
+        base += 2 * c;
+      }
+      const int h = m ? e / 2 : e, n = m + 2 * h, neg = m ? e & 1 : 0;
+      double v[4] = {0, 0, 0, 0};
+      for (int w = 0; w < kEThreads / 32; ++w)
+        for (int i = 0; i < (m ? 4 : 2); ++i) v[i] += red[w][base + (m ? 4 : 2) * h + i];
+      const double sg = (neg && (m & 1)) ? -1.0 : 1.0;
+      const double re = neg ? v[0] + v[3] : v[0] - v[3], im = neg ? v[1] - v[2] : v[1] + v[2];
+      sig[n * (n + 1) + (neg ? -m : m)] = cmk(sg * im, -sg * re);
+    }
+    __syncthreads();
+    if (tid == 0 && self) sig[0] = cadd(sig[0], a.sig0[(size_t)iw * per + pr]);
+    __syncthreads();
+    contract_block<LMAX>(a, T, sig, wk, per, pr, R, C, iw);
+  }
+}
+
 // Short-range tables: one CTA per (frequency w, pair) at the common eta of w.
 // Lattice points are taken in grid order, compacted with a block prefix sum
 // (deterministic order); every valid point stores R - s and its terms
-// c_nm = prefac_n |R - s|^n I_n leg0m e^{i m phi} (n + m even).
+// c_nm = prefac_n |R - s|^n I_n leg0m e^{i m phi} (n + m even); for real_k the
+// real numbers i prefac_n |R - s|^n I_n leg0m (cos, sin)(m phi), m >= 0, in
+// ewald_scan_kernel's order, and once per self pair sigma_0.
 template <int LMAX>
 __global__ void __launch_bounds__(kEThreads) ewald_sr_table_kernel(EwaldArgs a) {
   using Sh = EwShape<LMAX>;
@@ -1097,6 +1431,37 @@ __global__ void __launch_bounds__(kEThreads) ewald_sr_table_kernel(EwaldArgs a) 
           qg_c cn = cscale(cmk(rk.im, -rk.re), 2.0 / sqpi);
           const qg_c twor_k = cscale(rk, 2.0 * r);
           qg_c emn = cmk(1, 0);
+          if (a.real_k) {
+            double bn[LE + 1];
+#pragma unroll
+            for (int n = 0; n <= LE; ++n) {
+              double In = I0.re;
+              if (n > 0) {
+                In = ((2 * n - 1) * pm1.re - k2h.re * pm2.re + E.re * etap) * inv2r2;
+                pm2 = pm1;
+                pm1 = cmk(In, 0.0);
+                etap *= eta * eta;
+              }
+              bn[n] = -cn.im * In;
+              cn = cmul(cn, twor_k);
+            }
+            double *rt = reinterpret_cast<double *>(a.srtab) + u * NEV * (size_t)a.srmax + pos;
+            qg_c em = cmk(1, 0);
+#pragma unroll
+            for (int m = 0; m <= LE; ++m) {
+              if (m) em = cmul(em, e1);
+#pragma unroll
+              for (int n = m; n <= LE; n += 2) {
+                const double b = bn[n] * c_ew.leg0m[n * (n + 1) + m];
+                *rt = b * em.re;
+                rt += a.srmax;
+                if (m) {
+                  *rt = b * em.im;
+                  rt += a.srmax;
+                }
+              }
+            }
+          } else {
 #pragma unroll
           for (int n = 0; n <= LE; ++n) {
             qg_c In;
@@ -1120,6 +1485,7 @@ __global__ void __launch_bounds__(kEThreads) ewald_sr_table_kernel(EwaldArgs a) 
             emn = cmul(emn, e1c);
             cn = cmul(cn, twor_k);
           }
+          }
         }
         __syncthreads();
       }
@@ -1128,6 +1494,12 @@ __global__ void __launch_bounds__(kEThreads) ewald_sr_table_kernel(EwaldArgs a) 
     if (tid == 0) {
       if (base_s > a.srmax) atomicOr(a.err, 1);
       a.srcnt[u] = base_s < a.srmax ? base_s : a.srmax;
+    }
+    if (a.real_k && self && sz == 0.0 && tid == 32) {
+      // sigma0 = Gamma(-1/2, -(k/2eta)^2) / (2 sqrt(pi)) on the branch from below (ewald.c:260-273)
+      qg_c G[2];
+      gamma_half_down(cmk(0.0, -k.re / (2 * eta)), 1, G);
+      a.sig0[u] = cscale(G[1], 1.0 / (2 * 1.7724538509055160273));
     }
     __syncthreads();
   }
@@ -1257,7 +1629,10 @@ int launch_ew(const EwaldArgs &a, const TransDevTables &T, cudaStream_t st) {
     QG_CUDA_TRY(cudaGetLastError());
     g_launches.fetch_add(1);
   }
-  ewald_assemble_kernel<LMAX><<<(unsigned)grid, kEThreads, 0, st>>>(a, T);
+  if (a.srtab && a.real_k && !a.paired && !a.npairs)
+    ewald_scan_kernel<LMAX><<<(unsigned)grid, kEThreads, 0, st>>>(a, T);
+  else
+    ewald_assemble_kernel<LMAX><<<(unsigned)grid, kEThreads, 0, st>>>(a, T);
   QG_CUDA_TRY(cudaGetLastError());
   g_launches.fetch_add(1);
   if (a.layered) {

@@ -63,10 +63,14 @@ struct EwaldArgs {
   // the tables (formed once per (w, pair) by the table kernel) and applies
   // only the Bloch phase e^{i beta.(R - s)}: the radial integrals do not
   // depend on beta.
-  qg_c *srtab = nullptr;   // [nw][pairs][NEVEN][srmax]
+  qg_c *srtab = nullptr;   // [nw][pairs][NEVEN][srmax]; real_k: doubles, [nw][pairs][NEVEN][srmax]
   double *srpts = nullptr; // [nw][pairs][srmax][2]: R - s in the plane
   int *srcnt = nullptr;    // [nw][pairs]
   int srmax = 0;
+  // 1 (with srtab): every k is real; the single-plane pairs run through
+  // ewald_scan_kernel, whose tables are real
+  int real_k = 0;
+  qg_c *sig0 = nullptr;    // [nw][pairs]: the self term sigma_0 of self pairs (real_k)
 };
 
 // Bound on the lattice points one unit may enumerate per sum.

@@ -349,7 +349,7 @@ int periodic_assemble_device_ex(const qpms_scatsys_t *ss, int nw, const qg_c *k_
   a.M = dM;
   a.err = derr.as<int>();
   a.layered = layered_positions(pos.data(), np);
-  Dev dtab, dpts, dcnt;
+  Dev dtab, dpts, dcnt, dsig0;
   if (sr_tables) {
     for (int w = 0; w < nw; ++w)
       for (int k = 1; k < nk; ++k)
@@ -379,6 +379,13 @@ int periodic_assemble_device_ex(const qpms_scatsys_t *ss, int nw, const qg_c *k_
     a.srpts = dpts.as<double>();
     a.srcnt = dcnt.as<int>();
     a.srmax = (int)srmax;
+    a.real_k = 1;
+    for (int w = 0; w < nw; ++w)
+      if (k_host[w].im != 0.0 || !(k_host[w].re > 0.0)) a.real_k = 0;
+    if (a.real_k) {
+      if ((e = dalloc(dsig0, units * 16))) return e;
+      a.sig0 = dsig0.as<qg_c>();
+    }
   }
   const int n = (int)(ss->fecv_size / np);
   if (T_host.size() == (size_t)nw * ss->tm_count * n * n && n > 1) return ewald_assemble_dense(ss, a, n, st);
