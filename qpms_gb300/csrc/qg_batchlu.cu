@@ -747,19 +747,20 @@ void cluster_config(int C, int nm, int N, cudaStream_t st, cudaLaunchConfig_t *c
 
 // CTAs per matrix above N = 64.  The time of a matrix against its time on one
 // CTA, measured (us, GB300):
-//                            C = 1     4     8    16
-//   complex128, N 512, 2     47321 15949  7695  4321   (FP64 pipes of C - 1 SMs)
-//   complex128, N 390, 9     21790  7349  3724  4714   (two waves at 16)
-//   complex64,  N 512, 2      2788  1000   660   580   (the panels' serial chain)
-//   complex64,  N 256, 32      574   271   750  1268   (two and four waves)
+//                            C = 1     4     8     9    16
+//   complex128, N 512, 2     47321 15949  7695        4321   (FP64 pipes of C - 1 SMs)
+//   complex128, N 390, 9     21790  7349  3724  3317  4714   (two waves at 16)
+//   complex64,  N 512, 2      2788  1000   660         580   (the panels' serial chain)
+//   complex64,  N 256, 32      574   271   750        1268   (two and four waves)
 // so the choice is the least waves x relative time, a wave being the clusters
-// that the GPU holds at once (a cluster lies within one group of SMs, so 16
-// clusters of 8 no longer fit), among sizes whose CTAs all get a tile of the
+// that the GPU holds at once (a cluster lies within one group of SMs: 14 of 9
+// run at once, 16 of 8 do not), among sizes whose CTAs all get a tile of the
 // first update.  The counts are asked for once per device.
 template <typename T>
 int cluster_size(int nm, int N, int *C_out) {
-  constexpr int kN = 4, kC[kN] = {1, 4, 8, 16}, kMaxDev = 64;
-  constexpr double kCost[kN] = {1.0, sizeof(T) == 16 ? 0.34 : 0.45, sizeof(T) == 16 ? 0.17 : 0.30,
+  constexpr int kN = 6, kC[kN] = {1, 4, 6, 8, 9, 16}, kMaxDev = 64;
+  constexpr double kCost[kN] = {1.0, sizeof(T) == 16 ? 0.34 : 0.45, sizeof(T) == 16 ? 0.22 : 0.35,
+                                sizeof(T) == 16 ? 0.17 : 0.30, sizeof(T) == 16 ? 0.15 : 0.29,
                                 sizeof(T) == 16 ? 0.10 : 0.25};
   static std::atomic<int> active[kMaxDev][kN];  // 0: not asked yet
   int dev = 0;

@@ -88,25 +88,30 @@ __device__ __forceinline__ T rcp(T b) {
 }
 
 // ---------------- diagonal block: inverse by Gauss-Jordan ----------------
-// D (kb x kb, kb even and <= 32 NB, column-major in global, leading
-// dimension lda): Ainv (column-major kb x kb, leading dimension kb) receives
-// D^-1, and D is overwritten with D - I (the column-block product that follows
-// turns it into I - D^-1, the slot the back substitution reads).  info is set
-// to 1 on a singular pivot block.  Gauss-Jordan elimination without pivoting
-// (the random butterflies make it safe with high probability, as for the
-// whole LU), two columns per step: with J = {j, j + 1} and the 2 x 2 pivot
-// block P,
-//   A_JJ <- P^-1,  A_Jc <- P^-1 A_Jc,  A_rJ <- -A_rJ P^-1,
-//   A_rc <- A_rc - A_rJ P^-1 A_Jc        (r, c not in J).
-// One CTA of 512 threads with the block in registers: thread t holds the
-// NA x NB elements (t % 16 + 16 i, t / 16 + 32 j), rows-heavy so that the
-// per-column factors u = P^-1 A_Jc (the costly part of a step besides the
-// update) are formed for NB = 4 columns only.  Row r lives in the threads with
-// t % 16 == r % 16, column c in those with t / 16 == c % 32.  At each step the
-// two pivot rows and columns are published through two alternating
-// shared-memory slots (one barrier per step); every thread then forms P^-1
-// itself, updates all its elements and overwrites the pivot rows and columns.
-constexpr int kDiagMaxNb = 128, kDiagThreads = 512;
+// D (kb x kb, kb <= 32 NB, column-major in global, leading dimension lda): Ainv
+// (column-major kb x kb, leading dimension kb) receives D^-1, and D is
+// overwritten with D - I (the column-block product that follows turns it into
+// I - D^-1, the slot the back substitution reads).  info is set to 1 on a zero
+// pivot.  Gauss-Jordan elimination without pivoting (the random butterflies
+// make it safe with high probability, as for the whole LU), eight columns per
+// step: with J the step's columns and the 8 x 8 pivot block P = A_JJ,
+//   U = P^-1 A_Jc,  A_rc <- A_rc - A_rJ U          (r, c not in J)
+//   A_Jc <- U,  A_rJ <- -A_rJ P^-1,  A_JJ <- P^-1.
+// All four are one rank-8 update A <- A - F U' of every element when the pivot
+// rows and columns of A are set to zero, F to -I on the pivot rows and U' to
+// P^-1 on the pivot columns.
+// One CTA with the block in registers: of 512 threads, thread t holds the
+// NA x NB elements (t % 16 + 16 i, t / 16 + 32 j), so a warp reads 16 rows of F
+// and 2 columns of U' from shared memory at a time.  Before its update proper a
+// step forms the next pivot block's 64 elements, and a 17th warp inverts that
+// block meanwhile, which takes the chain of eight reciprocals off the path.
+// Rows and columns past kb are an identity.
+// Measured (two columns a step, every thread inverting their 2 x 2 block, before
+// -> now): 128 x 128 complex64 99 -> 79 us, 64 x 64 25.7 -> 21.6 us.  A rank-8
+// update is 4,096 issue cycles of FMAs a step at 128, of some 9,600; waits for
+// shared memory and barriers are the rest.  Packed f32x2 FMAs reach the scalar
+// rate and no more on this part, and 256 threads with twice the tile spill.
+constexpr int kDiagThreads = 512, kDiagStep = 8;
 
 // Complex multiply-add as four fused multiply-adds (no separate product and
 // sum: fewer instructions in the update loops, one rounding per term).
@@ -121,19 +126,69 @@ __device__ __forceinline__ T fms_c(T acc, T a, T b) {  // acc - a b
   return mk<T>(fmar(a.y, b.y, fmar(-a.x, b.x, acc.x)), fmar(-a.y, b.x, fmar(-a.x, b.y, acc.y)));
 }
 
+// (p, q) element of an 8 x 8 block: lane 8 (p % 4) + q, register p / 4.  Inverts
+// the block in place; true if a pivot was zero.
+template <typename T>
+__device__ __forceinline__ bool invert8(T (&x)[2], int lane) {
+  const int q = lane & 7, p0 = lane >> 3;
+  bool zero = false;
+#pragma unroll
+  for (int s = 0; s < 8; ++s) {
+    auto get = [&](const T &v, int l) {
+      return mk<T>(__shfl_sync(0xffffffffu, v.x, l), __shfl_sync(0xffffffffu, v.y, l));
+    };
+    const T d = get(x[s / 4], 8 * (s % 4) + s), u = get(x[s / 4], 8 * (s % 4) + q);
+    const T f0 = get(x[0], 8 * p0 + s), f1 = get(x[1], 8 * p0 + s);
+    const bool z = d.x == 0 && d.y == 0;
+    zero |= z;
+    const T di = z ? mk<T>(0, 0) : rcp(d);
+    const T ud = mul(u, di);  // the pivot row times 1 / d
+    const bool col = q == s;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const T f = h ? f1 : f0;
+      if (p0 + 4 * h == s)
+        x[h] = col ? di : ud;
+      else if (col)
+        x[h] = mk<T>(-(f.x * di.x - f.y * di.y), -(f.x * di.y + f.y * di.x));
+      else
+        x[h] = fms_c(x[h], f, ud);
+    }
+  }
+  return zero;
+}
+
 template <typename T, int NB>
-__global__ void __launch_bounds__(kDiagThreads, 1) diag_inv_kernel(T *D, size_t lda, int kb, T *Ainv, int *info) {
-  constexpr int NA = 2 * NB;  // row tiles per thread: 16 rows x NA, 32 columns x NB
-  __shared__ T sc[2][2][kDiagMaxNb];  // [slot][e][r] = a_(r, j+e)
-  __shared__ T sr[2][2][kDiagMaxNb];  // [slot][e][c] = a_(j+e, c)
-  const int lr = threadIdx.x & 15, lc = threadIdx.x >> 4;
+__global__ void __launch_bounds__(kDiagThreads + 32, 1) diag_inv_kernel(T *D, size_t lda, int kb, T *Ainv, int *info) {
+  constexpr int NA = 2 * NB, W = 32 * NB, B = kDiagStep;
+  __shared__ T F[2][B][W], Rw[2][B][W];  // pivot columns and rows of alternating steps
+  __shared__ T U[B][W];
+  __shared__ T P[B][B + 1], Pinv[2][B][B + 1];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int nsteps = (kb + B - 1) / B;
+  if (tid >= kDiagThreads) {  // the inverting warp
+    bool zero = false;
+    for (int b = -1; b < nsteps; ++b) {  // inverts step b + 1's pivot block during step b
+      if (b + 1 < nsteps) {
+        asm volatile("bar.sync 2, 160;" ::: "memory");  // its owners' four warps have formed it
+        T x[2] = {P[lane >> 3][lane & 7], P[(lane >> 3) + 4][lane & 7]};
+        zero |= invert8(x, lane);
+        Pinv[(b + 1) & 1][lane >> 3][lane & 7] = x[0];
+        Pinv[(b + 1) & 1][(lane >> 3) + 4][lane & 7] = x[1];
+      }
+      __syncthreads();
+    }
+    if (zero && lane == 0) atomicOr(info, 1);
+    return;
+  }
+  const int lr = tid & 15, lc = tid >> 4;
   T a[NA][NB];
 #pragma unroll
   for (int j = 0; j < NB; ++j)
 #pragma unroll
     for (int i = 0; i < NA; ++i) {
       const int r = lr + 16 * i, c = lc + 32 * j;
-      a[i][j] = mk<T>(0, 0);
+      a[i][j] = mk<T>(r == c ? 1 : 0, 0);
       if (r < kb && c < kb) {
         T v = D[(size_t)c * lda + r];
         a[i][j] = v;
@@ -141,89 +196,95 @@ __global__ void __launch_bounds__(kDiagThreads, 1) diag_inv_kernel(T *D, size_t 
         D[(size_t)c * lda + r] = v;
       }
     }
-  bool zero = false;
-  // Step (j, j + 1), j = 32 ct + 16 h + q, q even: rows j, j + 1 are tile row
-  // 2 ct + h of the threads with lr = q, q + 1; columns j, j + 1 are tile
-  // column ct of the threads with lc = 16 h + q, 16 h + q + 1.  ct and h are
-  // unrolled, so every register index is static.
+  // the pivot block of the step at column j: tile row j / 16, tile column j / 32
+  // of the threads with lr - j % 16 and lc - j % 32 in 0..7 (four warps)
+  auto pivot_block = [&](int j, int buf, bool update) {
+    const int rt = j >> 4, ct = j >> 5, p = lr - (j & 15), q = lc - (j & 31);
+    if (q < 0 || q >= B) return;  // uniform in the warp
+    if (p >= 0 && p < B) {
+      T v = mk<T>(0, 0);
 #pragma unroll
-  for (int ct = 0; ct < NB; ++ct) {
+      for (int i = 0; i < NA; ++i)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int rt = 2 * ct + h;
-      for (int q = 0; q < 16; q += 2) {
-        const int j = 32 * ct + 16 * h + q;
-        if (j >= kb) break;  // uniform
-        const int slot = (j >> 1) & 1, cl = 16 * h + q;
-        if (lr == q || lr == q + 1) {
-          const int e = lr - q;
+        for (int jj = 0; jj < NB; ++jj)
+          if (i == rt && jj == ct) v = a[i][jj];
+      if (update)
 #pragma unroll
-          for (int jj = 0; jj < NB; ++jj) {
-            const int c = lc + 32 * jj;
-            if (c < kb) sr[slot][e][c] = a[rt][jj];
-          }
-        }
-        if (lc == cl || lc == cl + 1) {
-          const int e = lc - cl;
+        for (int s = 0; s < B; ++s) v = fms_c(v, F[buf][s][j + p], U[s][j + q]);
+      P[p][q] = v;
+    }
+    __syncwarp();
+    asm volatile("bar.arrive 2, 160;" ::: "memory");
+  };
+  // publishes the rows and columns of the step at column j and clears them
+  auto publish = [&](int j, int buf) {
+    const int rt = j >> 4, ct = j >> 5, p = lr - (j & 15), q = lc - (j & 31);
+    const bool row = p >= 0 && p < B, col = q >= 0 && q < B;
+    if (col) {
+#pragma unroll
+      for (int jj = 0; jj < NB; ++jj)
+        if (jj == ct)
 #pragma unroll
           for (int i = 0; i < NA; ++i) {
             const int r = lr + 16 * i;
-            if (r < kb) sc[slot][e][r] = a[i][ct];
+            F[buf][q][r] = (row && i == rt) ? mk<T>(p == q ? -1 : 0, 0) : a[i][jj];
           }
-        }
-        __syncthreads();
-        // P = [p00 p01; p10 p11], P^-1 = [q00 q01; q10 q11]
-        const T p00 = sc[slot][0][j], p10 = sc[slot][0][j + 1], p01 = sc[slot][1][j], p11 = sc[slot][1][j + 1];
-        const T det = sub(mul(p00, p11), mul(p01, p10));
-        const bool z = (det.x == 0 && det.y == 0);
-        zero |= z;
-        const T dinv = z ? mk<T>(0, 0) : rcp(det);
-        const T q00 = mul(p11, dinv), q11 = mul(p00, dinv);
-        const T q01 = mk<T>(-(p01.x * dinv.x - p01.y * dinv.y), -(p01.x * dinv.y + p01.y * dinv.x));
-        const T q10 = mk<T>(-(p10.x * dinv.x - p10.y * dinv.y), -(p10.x * dinv.y + p10.y * dinv.x));
-        // u = P^-1 A_Jc for this thread's NB columns
-        T u0[NB], u1[NB];
-#pragma unroll
-        for (int jj = 0; jj < NB; ++jj) {
-          const int c = min(lc + 32 * jj, kb - 1);  // columns >= kb are padding, never stored
-          const T x0 = sr[slot][0][c], x1 = sr[slot][1][c];
-          u0[jj] = fma_c(mul(q00, x0), q01, x1);
-          u1[jj] = fma_c(mul(q10, x0), q11, x1);
-        }
-        // every element: a_rc -= a_rj u0_c + a_r,j+1 u1_c; the pivot rows and
-        // columns are overwritten right after
-#pragma unroll
-        for (int i = 0; i < NA; ++i) {
-          if (16 * i >= kb) continue;  // uniform
-          const int r = min(lr + 16 * i, kb - 1);  // rows >= kb are padding, never stored
-          const T f0 = sc[slot][0][r], f1 = sc[slot][1][r];
-#pragma unroll
-          for (int jj = 0; jj < NB; ++jj) a[i][jj] = fms_c(fms_c(a[i][jj], f0, u0[jj]), f1, u1[jj]);
-          if (i == rt) {  // static: the pivot rows' tile row
-            if (lr == q)
-#pragma unroll
-              for (int jj = 0; jj < NB; ++jj) a[i][jj] = u0[jj];
-            if (lr == q + 1)
-#pragma unroll
-              for (int jj = 0; jj < NB; ++jj) a[i][jj] = u1[jj];
-          }
-        }
-        if (lc == cl || lc == cl + 1) {  // columns j + e: -A_rJ P^-1, the pivot block P^-1
-          const bool e0 = lc == cl;
-          const T qa = e0 ? q00 : q01, qb = e0 ? q10 : q11;
-#pragma unroll
-          for (int i = 0; i < NA; ++i) {
-            const int r = min(lr + 16 * i, kb - 1);
-            const T g = fma_c(mul(sc[slot][0][r], qa), sc[slot][1][r], qb);
-            a[i][ct] = mk<T>(-g.x, -g.y);
-          }
-          if (lr == q) a[rt][ct] = qa;
-          if (lr == q + 1) a[rt][ct] = qb;
-        }
-      }
     }
+    if (row) {
+#pragma unroll
+      for (int i = 0; i < NA; ++i)
+        if (i == rt)
+#pragma unroll
+          for (int jj = 0; jj < NB; ++jj) {
+            Rw[buf][p][lc + 32 * jj] = a[i][jj];
+            a[i][jj] = mk<T>(0, 0);
+          }
+    }
+    if (col) {
+#pragma unroll
+      for (int jj = 0; jj < NB; ++jj)
+        if (jj == ct)
+#pragma unroll
+          for (int i = 0; i < NA; ++i) a[i][jj] = mk<T>(0, 0);
+    }
+  };
+  pivot_block(0, 0, false);
+  publish(0, 0);
+  __syncthreads();
+  for (int b = 0; b < nsteps; ++b) {
+    const int buf = b & 1, j0 = B * b, j1 = j0 + B;
+    const bool more = b + 1 < nsteps;
+    // U' = P^-1 A_Jc; P^-1 itself on the pivot columns
+#pragma unroll
+    for (int t = 0; t < B * W / kDiagThreads; ++t) {
+      const int idx = tid + kDiagThreads * t, p = idx / W, c = idx % W;
+      T u;
+      if (c >= j0 && c < j1) {
+        u = Pinv[buf][p][c - j0];
+      } else {
+        u = mul(Pinv[buf][p][0], Rw[buf][0][c]);
+#pragma unroll
+        for (int q = 1; q < B; ++q) u = fma_c(u, Pinv[buf][p][q], Rw[buf][q][c]);
+      }
+      U[p][c] = u;
+    }
+    asm volatile("bar.sync 1, 512;" ::: "memory");
+    if (more) pivot_block(j1, buf, true);
+#pragma unroll
+    for (int s = 0; s < B; ++s) {
+      T f[NA], u[NB];
+#pragma unroll
+      for (int i = 0; i < NA; ++i) f[i] = F[buf][s][lr + 16 * i];
+#pragma unroll
+      for (int jj = 0; jj < NB; ++jj) u[jj] = U[s][lc + 32 * jj];
+#pragma unroll
+      for (int i = 0; i < NA; ++i)
+#pragma unroll
+        for (int jj = 0; jj < NB; ++jj) a[i][jj] = fms_c(a[i][jj], f[i], u[jj]);
+    }
+    if (more) publish(j1, buf ^ 1);
+    __syncthreads();
   }
-  if (zero && threadIdx.x == 0) atomicOr(info, 1);
 #pragma unroll
   for (int j = 0; j < NB; ++j)
 #pragma unroll
@@ -243,9 +304,9 @@ int launch_diag(T *D, size_t lda, int kb, T *Ainv, int *info, cudaStream_t st) {
   }
   KtScope kt(KT_DIAGLU, st, 8.0 * kb * (double)kb * kb);
   if (kb <= 64)
-    diag_inv_kernel<T, 2><<<1, kDiagThreads, 0, st>>>(D, lda, kb, Ainv, info);
+    diag_inv_kernel<T, 2><<<1, kDiagThreads + 32, 0, st>>>(D, lda, kb, Ainv, info);
   else
-    diag_inv_kernel<T, kMaxNb><<<1, kDiagThreads, 0, st>>>(D, lda, kb, Ainv, info);
+    diag_inv_kernel<T, kMaxNb><<<1, kDiagThreads + 32, 0, st>>>(D, lda, kb, Ainv, info);
   QG_CUDA_TRY(cudaGetLastError());
   g_launches.fetch_add(1);
   return QPMS_SUCCESS;
@@ -535,9 +596,9 @@ int lu_solve(cublasHandle_t h, int N, int nb, const T *A, size_t lda, T *B, size
 int lu_nopiv_tc(int N, int nb, float2 *A, size_t lda, float2 *Dinv, int *dinfo, int nsplit, __nv_bfloat16 *pa,
                 __nv_bfloat16 *pb, cudaStream_t st, cudaStream_t side, cudaEvent_t ev_a, cudaEvent_t ev_d,
                 int group) {
-  // Lookahead (side != nullptr): the trailing update first updates the next
-  // block column, then the next diagonal block is inverted on the side stream
-  // while the rest of the update runs; the next step waits for it before its
+  // Lookahead (side != nullptr): an update first updates the next block column,
+  // then the next diagonal block is inverted on the side stream while the rest
+  // of the update (inside a group: the product of its later block rows) runs; the next step waits for it before its
   // column-block product.  The update GEMMs leave SMs free for the single-CTA
   // inversion.
   // Groups: blocks are taken `group` at a time.  Within a group, block i's
@@ -601,7 +662,7 @@ int lu_nopiv_tc(int N, int nb, float2 *A, size_t lda, float2 *Dinv, int *dinfo, 
     for (int ki = k, b = blk; ki < ge; ki += nb, ++b) {
       const int kbi = (N - ki < nb) ? N - ki : nb, ke = ki + kbi, mi = N - ke;
       float2 *Ainv = Dinv + (size_t)b * nb * nb;
-      if (ki > k || !la || blk == 0) {
+      if (!la || b == 0) {
         if ((e = launch_diag<float2>(A + (size_t)ki * lda + ki, lda, kbi, Ainv, dinfo, st))) return e;
       } else {
         QG_CUDA_TRY(cudaStreamWaitEvent(st, ev_d, 0));
@@ -624,6 +685,13 @@ int lu_nopiv_tc(int N, int nb, float2 *A, size_t lda, float2 *Dinv, int *dinfo, 
       Q.m = mi, Q.n = wi;  // the later block columns of the group, every row below block i
       Q.b_plane = (size_t)mi * rs;
       if ((e = tc_cgemm_planes(Q, -1.f, 1.f, C, lda, C, lda, st))) return e;
+      if (la) {  // the next diagonal block is final: inverted beside the product of the later block rows
+        QG_CUDA_TRY(cudaEventRecord(ev_a, st));
+        QG_CUDA_TRY(cudaStreamWaitEvent(side, ev_a, 0));
+        if ((e = launch_diag<float2>(C, lda, wi < nb ? wi : nb, Dinv + (size_t)(b + 1) * nb * nb, dinfo, side)))
+          return e;
+        QG_CUDA_TRY(cudaEventRecord(ev_d, side));
+      }
       if (mi > wi) {  // the later block rows of the group, past the group: the first wi rows of the A planes
         Q.m = wi, Q.a_plane = (size_t)2 * mi * rs;
         Q.b = pb + (size_t)wi * rs, Q.n = mi - wi;
