@@ -27,6 +27,7 @@
 // The plain mode runs steps 1-3 in complex128 (FP64 GEMMs).
 // All matrices are column-major (LAPACK order).  The butterflies halve the
 // system twice, so it is padded internally to a multiple of 4 with identity.
+#include <cooperative_groups.h>
 #include <cublas_v2.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -46,6 +47,8 @@
 #include "qg_ktimer.h"
 #include "qg_tcgemm.h"
 #include "qg_tuned.h"
+
+namespace cg = cooperative_groups;
 
 namespace qg {
 int blas_handle_get(cublasHandle_t *h);
@@ -80,15 +83,8 @@ template <typename T>
 __device__ __forceinline__ T sub(T a, T b) {
   return mk<T>(a.x - b.x, a.y - b.y);
 }
-template <typename T>
-__device__ __forceinline__ T rcp(T b) {
-  typedef typename CTraits<T>::real R;
-  const R d = b.x * b.x + b.y * b.y;
-  return mk<T>(b.x / d, -b.y / d);
-}
-
 // ---------------- diagonal block: inverse by Gauss-Jordan ----------------
-// D (kb x kb, kb <= 32 NB, column-major in global, leading dimension lda): Ainv
+// D (kb x kb, kb <= W, column-major in global, leading dimension lda): Ainv
 // (column-major kb x kb, leading dimension kb) receives D^-1, and D is
 // overwritten with D - I (the column-block product that follows turns it into
 // I - D^-1, the slot the back substitution reads).  info is set to 1 on a zero
@@ -100,18 +96,21 @@ __device__ __forceinline__ T rcp(T b) {
 // All four are one rank-8 update A <- A - F U' of every element when the pivot
 // rows and columns of A are set to zero, F to -I on the pivot rows and U' to
 // P^-1 on the pivot columns.
-// One CTA with the block in registers: of 512 threads, thread t holds the
-// NA x NB elements (t % 16 + 16 i, t / 16 + 32 j), so a warp reads 16 rows of F
-// and 2 columns of U' from shared memory at a time.  Before its update proper a
-// step forms the next pivot block's 64 elements, and a 17th warp inverts that
-// block meanwhile, which takes the chain of eight reciprocals off the path.
+// A cluster of C CTAs holds the block in registers, W / C columns each: of 256
+// threads, thread t has the elements (t % 16 + 16 i, t / 16 + 16 j) of its CTA's
+// columns, so a warp reads 16 rows of F and 2 columns of U' from shared memory
+// at a time.  The CTA that owns a step's columns writes them into every CTA's F
+// (distributed shared memory); the pivot rows stay with their columns; one
+// cluster barrier ends a step.  Before its update proper the owner of the next
+// step's columns forms that pivot block's 64 elements, and a ninth warp inverts
+// it meanwhile, which takes the chain of eight reciprocals off the path.
 // Rows and columns past kb are an identity.
-// Measured (two columns a step, every thread inverting their 2 x 2 block, before
-// -> now): 128 x 128 complex64 99 -> 79 us, 64 x 64 25.7 -> 21.6 us.  A rank-8
-// update is 4,096 issue cycles of FMAs a step at 128, of some 9,600; waits for
-// shared memory and barriers are the rest.  Packed f32x2 FMAs reach the scalar
-// rate and no more on this part, and 256 threads with twice the tile spill.
-constexpr int kDiagThreads = 512, kDiagStep = 8;
+// Measured (one CTA of 512 threads -> four CTAs): 128 x 128 complex64 79 -> 44 us,
+// 64 x 64 21.6 -> 17.7 us, 64 x 64 complex128 405 -> 155 us (FP64 FMAs).  A step at
+// 128 is 1,024 issue cycles of FMAs in each CTA; the reciprocals' chain and the
+// cluster barrier are the rest, so eight CTAs (51 us) lose again, and two take
+// 19.7 us (64 x 64) and 234 us (complex128).
+constexpr int kDiagThreads = 256, kDiagStep = 8, kDiagCtas = 4;
 
 // Complex multiply-add as four fused multiply-adds (no separate product and
 // sum: fewer instructions in the update loops, one rounding per term).
@@ -141,7 +140,10 @@ __device__ __forceinline__ bool invert8(T (&x)[2], int lane) {
     const T f0 = get(x[0], 8 * p0 + s), f1 = get(x[1], 8 * p0 + s);
     const bool z = d.x == 0 && d.y == 0;
     zero |= z;
-    const T di = z ? mk<T>(0, 0) : rcp(d);
+    // 1 / d with one division per lane: even lanes the real part, odd ones the imaginary
+    const auto n = d.x * d.x + d.y * d.y;
+    const auto h0 = (lane & 1 ? -d.y : d.x) / n, h1 = __shfl_xor_sync(0xffffffffu, h0, 1);
+    const T di = z ? mk<T>(0, 0) : lane & 1 ? mk<T>(h1, h0) : mk<T>(h0, h1);
     const T ud = mul(u, di);  // the pivot row times 1 / d
     const bool col = q == s;
 #pragma unroll
@@ -158,25 +160,33 @@ __device__ __forceinline__ bool invert8(T (&x)[2], int lane) {
   return zero;
 }
 
-template <typename T, int NB>
-__global__ void __launch_bounds__(kDiagThreads + 32, 1) diag_inv_kernel(T *D, size_t lda, int kb, T *Ainv, int *info) {
-  constexpr int NA = 2 * NB, W = 32 * NB, B = kDiagStep;
-  __shared__ T F[2][B][W], Rw[2][B][W];  // pivot columns and rows of alternating steps
-  __shared__ T U[B][W];
-  __shared__ T P[B][B + 1], Pinv[2][B][B + 1];
+template <typename T, int W, int C>
+__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kDiagThreads + 32, 1)
+    diag_inv_kernel(T *D, size_t lda, int kb, T *Ainv, int *info) {
+  constexpr int CL = W / C, NA = W / 16, NB = CL / 16, B = kDiagStep;
+  __shared__ T F[2][B][W];           // pivot columns of alternating steps (from their owner)
+  __shared__ T Rw[2][B][CL];         // pivot rows, this CTA's columns
+  __shared__ T U[B][CL];
+  __shared__ T P[B][B + 1], Pinv[2][B][B + 1];  // Pinv: from the owner too
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank(), c0 = rank * CL;
   const int tid = threadIdx.x, lane = tid & 31;
   const int nsteps = (kb + B - 1) / B;
   if (tid >= kDiagThreads) {  // the inverting warp
     bool zero = false;
+    cl.sync();
     for (int b = -1; b < nsteps; ++b) {  // inverts step b + 1's pivot block during step b
-      if (b + 1 < nsteps) {
+      if (b + 1 < nsteps && B * (b + 1) / CL == rank) {
         asm volatile("bar.sync 2, 160;" ::: "memory");  // its owners' four warps have formed it
         T x[2] = {P[lane >> 3][lane & 7], P[(lane >> 3) + 4][lane & 7]};
         zero |= invert8(x, lane);
-        Pinv[(b + 1) & 1][lane >> 3][lane & 7] = x[0];
-        Pinv[(b + 1) & 1][(lane >> 3) + 4][lane & 7] = x[1];
+        for (int t = 0; t < C; ++t) {
+          T *dst = cl.map_shared_rank(&Pinv[(b + 1) & 1][0][0], t);
+          dst[(lane >> 3) * (B + 1) + (lane & 7)] = x[0];
+          dst[((lane >> 3) + 4) * (B + 1) + (lane & 7)] = x[1];
+        }
       }
-      __syncthreads();
+      cl.sync();
     }
     if (zero && lane == 0) atomicOr(info, 1);
     return;
@@ -187,7 +197,7 @@ __global__ void __launch_bounds__(kDiagThreads + 32, 1) diag_inv_kernel(T *D, si
   for (int j = 0; j < NB; ++j)
 #pragma unroll
     for (int i = 0; i < NA; ++i) {
-      const int r = lr + 16 * i, c = lc + 32 * j;
+      const int r = lr + 16 * i, c = c0 + lc + 16 * j;
       a[i][j] = mk<T>(r == c ? 1 : 0, 0);
       if (r < kb && c < kb) {
         T v = D[(size_t)c * lda + r];
@@ -196,10 +206,12 @@ __global__ void __launch_bounds__(kDiagThreads + 32, 1) diag_inv_kernel(T *D, si
         D[(size_t)c * lda + r] = v;
       }
     }
-  // the pivot block of the step at column j: tile row j / 16, tile column j / 32
-  // of the threads with lr - j % 16 and lc - j % 32 in 0..7 (four warps)
+  // the pivot block of the step at column j, in the CTA that holds that column:
+  // tile row j / 16 and this CTA's tile column of the threads with lr - j % 16
+  // and lc - j % 16 in 0..7 (four warps)
   auto pivot_block = [&](int j, int buf, bool update) {
-    const int rt = j >> 4, ct = j >> 5, p = lr - (j & 15), q = lc - (j & 31);
+    if (j / CL != rank) return;
+    const int rt = j >> 4, jl = j - c0, ct = jl >> 4, p = lr - (j & 15), q = lc - (jl & 15);
     if (q < 0 || q >= B) return;  // uniform in the warp
     if (p >= 0 && p < B) {
       T v = mk<T>(0, 0);
@@ -210,25 +222,33 @@ __global__ void __launch_bounds__(kDiagThreads + 32, 1) diag_inv_kernel(T *D, si
           if (i == rt && jj == ct) v = a[i][jj];
       if (update)
 #pragma unroll
-        for (int s = 0; s < B; ++s) v = fms_c(v, F[buf][s][j + p], U[s][j + q]);
+        for (int s = 0; s < B; ++s) v = fms_c(v, F[buf][s][j + p], U[s][jl + q]);
       P[p][q] = v;
     }
     __syncwarp();
     asm volatile("bar.arrive 2, 160;" ::: "memory");
   };
-  // publishes the rows and columns of the step at column j and clears them
+  // publishes the rows (here) and columns (to every CTA) of the step at column j
+  // and clears them
   auto publish = [&](int j, int buf) {
-    const int rt = j >> 4, ct = j >> 5, p = lr - (j & 15), q = lc - (j & 31);
-    const bool row = p >= 0 && p < B, col = q >= 0 && q < B;
+    const int rt = j >> 4, jl = j - c0, ct = jl >> 4, p = lr - (j & 15), q = lc - (jl & 15);
+    const bool row = p >= 0 && p < B, col = j / CL == rank && q >= 0 && q < B;
     if (col) {
+      T f[NA];
 #pragma unroll
-      for (int jj = 0; jj < NB; ++jj)
-        if (jj == ct)
+      for (int i = 0; i < NA; ++i) {
+        f[i] = a[i][0];
 #pragma unroll
-          for (int i = 0; i < NA; ++i) {
-            const int r = lr + 16 * i;
-            F[buf][q][r] = (row && i == rt) ? mk<T>(p == q ? -1 : 0, 0) : a[i][jj];
-          }
+        for (int jj = 1; jj < NB; ++jj)
+          if (jj == ct) f[i] = a[i][jj];
+        if (row && i == rt) f[i] = mk<T>(p == q ? -1 : 0, 0);
+      }
+#pragma unroll
+      for (int t = 0; t < C; ++t) {
+        T *dst = cl.map_shared_rank(&F[buf][q][lr], t);
+#pragma unroll
+        for (int i = 0; i < NA; ++i) dst[16 * i] = f[i];
+      }
     }
     if (row) {
 #pragma unroll
@@ -236,7 +256,7 @@ __global__ void __launch_bounds__(kDiagThreads + 32, 1) diag_inv_kernel(T *D, si
         if (i == rt)
 #pragma unroll
           for (int jj = 0; jj < NB; ++jj) {
-            Rw[buf][p][lc + 32 * jj] = a[i][jj];
+            Rw[buf][p][lc + 16 * jj] = a[i][jj];
             a[i][jj] = mk<T>(0, 0);
           }
     }
@@ -249,18 +269,19 @@ __global__ void __launch_bounds__(kDiagThreads + 32, 1) diag_inv_kernel(T *D, si
     }
   };
   pivot_block(0, 0, false);
+  cl.sync();  // every CTA has started: its shared memory may be written
   publish(0, 0);
-  __syncthreads();
+  cl.sync();
   for (int b = 0; b < nsteps; ++b) {
     const int buf = b & 1, j0 = B * b, j1 = j0 + B;
     const bool more = b + 1 < nsteps;
     // U' = P^-1 A_Jc; P^-1 itself on the pivot columns
 #pragma unroll
-    for (int t = 0; t < B * W / kDiagThreads; ++t) {
-      const int idx = tid + kDiagThreads * t, p = idx / W, c = idx % W;
+    for (int idx = tid; idx < B * CL; idx += kDiagThreads) {
+      const int p = idx / CL, c = idx % CL;
       T u;
-      if (c >= j0 && c < j1) {
-        u = Pinv[buf][p][c - j0];
+      if (c0 + c >= j0 && c0 + c < j1) {
+        u = Pinv[buf][p][c0 + c - j0];
       } else {
         u = mul(Pinv[buf][p][0], Rw[buf][0][c]);
 #pragma unroll
@@ -268,7 +289,7 @@ __global__ void __launch_bounds__(kDiagThreads + 32, 1) diag_inv_kernel(T *D, si
       }
       U[p][c] = u;
     }
-    asm volatile("bar.sync 1, 512;" ::: "memory");
+    asm volatile("bar.sync 1, 256;" ::: "memory");
     if (more) pivot_block(j1, buf, true);
 #pragma unroll
     for (int s = 0; s < B; ++s) {
@@ -276,20 +297,20 @@ __global__ void __launch_bounds__(kDiagThreads + 32, 1) diag_inv_kernel(T *D, si
 #pragma unroll
       for (int i = 0; i < NA; ++i) f[i] = F[buf][s][lr + 16 * i];
 #pragma unroll
-      for (int jj = 0; jj < NB; ++jj) u[jj] = U[s][lc + 32 * jj];
+      for (int jj = 0; jj < NB; ++jj) u[jj] = U[s][lc + 16 * jj];
 #pragma unroll
       for (int i = 0; i < NA; ++i)
 #pragma unroll
         for (int jj = 0; jj < NB; ++jj) a[i][jj] = fms_c(a[i][jj], f[i], u[jj]);
     }
     if (more) publish(j1, buf ^ 1);
-    __syncthreads();
+    cl.sync();
   }
 #pragma unroll
   for (int j = 0; j < NB; ++j)
 #pragma unroll
     for (int i = 0; i < NA; ++i) {
-      const int r = lr + 16 * i, c = lc + 32 * j;
+      const int r = lr + 16 * i, c = c0 + lc + 16 * j;
       if (r < kb && c < kb) Ainv[c * kb + r] = a[i][j];
     }
 }
@@ -297,16 +318,16 @@ __global__ void __launch_bounds__(kDiagThreads + 32, 1) diag_inv_kernel(T *D, si
 // Invert one diagonal block (kb <= 128; complex128 blocks up to 64).
 template <typename T>
 int launch_diag(T *D, size_t lda, int kb, T *Ainv, int *info, cudaStream_t st) {
-  constexpr int kMaxNb = sizeof(T) == 16 ? 2 : 4;  // complex128 blocks: nb <= 64
-  if (kb <= 0 || kb > 32 * kMaxNb || (kb & 1)) {
+  constexpr int kMaxNb = sizeof(T) == 16 ? 64 : 128;
+  if (kb <= 0 || kb > kMaxNb || (kb & 1)) {
     set_error("diagonal block of size %d not supported", kb);
     return QPMS_EINVAL;
   }
   KtScope kt(KT_DIAGLU, st, 8.0 * kb * (double)kb * kb);
   if (kb <= 64)
-    diag_inv_kernel<T, 2><<<1, kDiagThreads + 32, 0, st>>>(D, lda, kb, Ainv, info);
+    diag_inv_kernel<T, 64, kDiagCtas><<<kDiagCtas, kDiagThreads + 32, 0, st>>>(D, lda, kb, Ainv, info);
   else
-    diag_inv_kernel<T, kMaxNb><<<1, kDiagThreads + 32, 0, st>>>(D, lda, kb, Ainv, info);
+    diag_inv_kernel<T, kMaxNb, kDiagCtas><<<kDiagCtas, kDiagThreads + 32, 0, st>>>(D, lda, kb, Ainv, info);
   QG_CUDA_TRY(cudaGetLastError());
   g_launches.fetch_add(1);
   return QPMS_SUCCESS;
@@ -599,8 +620,8 @@ int lu_nopiv_tc(int N, int nb, float2 *A, size_t lda, float2 *Dinv, int *dinfo, 
   // Lookahead (side != nullptr): an update first updates the next block column,
   // then the next diagonal block is inverted on the side stream while the rest
   // of the update (inside a group: the product of its later block rows) runs; the next step waits for it before its
-  // column-block product.  The update GEMMs leave SMs free for the single-CTA
-  // inversion.
+  // column-block product.  The update GEMMs leave SMs free for the inversion's
+  // four CTAs.
   // Groups: blocks are taken `group` at a time.  Within a group, block i's
   // update is applied at once only to the group's later block columns (every
   // row below block i) and to the group's later block rows (the columns past

@@ -506,8 +506,8 @@ int launch_gemm(const CUtensorMap &ma, const CUtensorMap &mb, const GemmArgs &g,
                                     S::kBytes);
   });
   QG_CUDA_TRY(attr_err);
-  // Persistent CTAs on all but kReservedSms SMs: the single-CTA kernels of the
-  // dense LU (diagonal blocks) and the small launches of concurrent solves on
+  // Persistent CTAs on all but kReservedSms SMs: the dense LU's diagonal
+  // inversions (four CTAs) and the small launches of concurrent solves on
   // other streams always find an SM instead of waiting for a whole GEMM.
   const int ntiles = ((g.Md + BM - 1) / BM) * ((g.Nd + BN - 1) / BN);
   const int slots = g_num_sms > 2 * kReservedSms ? g_num_sms - kReservedSms : g_num_sms;
