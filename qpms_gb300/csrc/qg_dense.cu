@@ -1204,12 +1204,14 @@ size_t tc_plane_bytes(int Np, int nrhs_max, int nb) {
 }  // namespace
 
 // Block size of the LU: complex128 factors use 64; complex64 factors use 128
-// for large systems (the trailing updates carry the time) and 64 below the
-// tuned size kTunedNb64Below (the chain of diagonal-block inversions carries
-// it there: an inversion costs nb^3).  With many right-hand sides the
+// except below the tuned size kTunedNb64Below, where two blocks of 64 take less
+// than one of 128 (128 unknowns 443 us with 64-wide blocks, 554 with 128; 256
+// 723 : 658; 1,024 1,548 : 1,335; 3,072 4.33 : 3.48 ms; 14,400 51.4 : 42.5): an
+// inversion of 128 columns takes 2.5 times one of 64, and there are half as many
+// steps, launches and hops of the substitutions.  With many right-hand sides the
 // substitutions' chain, two launches per block and sweep, is the longer one:
-// 128 at every size (six contour nodes with 64 columns at 5,776 unknowns 119.7 ms
-// with 64-wide blocks, 108.5 with 128; 32 columns at 1,600 unknowns 24.2 : 22.7).
+// 128 at every size (six contour nodes with 64 columns at 5,776 unknowns 92 ms
+// with 64-wide blocks, 78 with 128).
 // QPMS_GB300_LU_NB = 64 / 128 overrides.
 int lu_block_size(int N, int mode, int nrhs) {
   if (!mode) return 64;
@@ -1540,7 +1542,12 @@ int DenseSolver::lu_group() const {
     const int g = e ? atoi(e) : 0;
     return g >= 1 && g <= kMaxLuGroup ? g : 0;
   }();
-  return v ? v : std::max(1, std::min(group, kMaxLuGroup));
+  // Pairs of blocks for small systems, where a third inversion in a row lengthens
+  // the chain; groups of 3 where the passes over the trailing matrix carry the
+  // time (pairs : 3 : 4 at 2,000 unknowns 2.36 : 2.37 : 2.37 ms, 4,500
+  // 5.75 : 5.66 : 5.69, 8,192 14.0 : 13.7 : 13.8, 14,400 42.7 : 41.8 : 42.0).
+  const int g = group ? group : N < 4096 ? 2 : 3;
+  return v ? v : std::max(1, std::min(g, kMaxLuGroup));
 }
 
 int DenseSolver::check_info(cudaStream_t st) {

@@ -82,8 +82,9 @@ struct DenseSolver {
   bool sweeps = true;
   // tensor-core LU by groups of `group` blocks (1 .. kMaxLuGroup): one
   // trailing update with K = group x nb per group (QPMS_GB300_LU_GROUP
-  // overrides); set before init(), which sizes the operand planes for it
-  int group = 2;
+  // overrides); 0 = by size (lu_group); set before init(), which sizes the
+  // operand planes for it
+  int group = 0;
   // block size of the complex64 LU: 0 = the tuned choice (lu_block_size), else
   // 64 or 128; set before init()
   int nb_pref = 0;

@@ -329,7 +329,7 @@ struct qpms_gpu_server {
     ds.lookahead = nworkers == 1;
     // and 128-wide blocks at every size: the trailing updates, not the
     // inversion chain, bound a loaded server (107.5 solves/s against 104.4
-    // with the single-solve tuning's 64-wide blocks below 6144 unknowns)
+    // with 64-wide blocks below 6,144 unknowns)
     ds.nb_pref = 128;
     // and the substitutions as one launch per block and sweep: the one-launch
     // sweeps' waiting warps hold SM slots the other requests' kernels could
@@ -338,7 +338,7 @@ struct qpms_gpu_server {
     // and groups of 3 blocks in the LU: without the lookahead the in-group
     // inversions cost nothing extra here (136.0 / 137.0 solves/s with pairs,
     // 138.1 with groups of 3, 138.2 / 137.0 with groups of 4)
-    ds.group = nworkers == 1 ? 2 : 3;
+    ds.group = nworkers == 1 ? 0 : 3;
     if ((e = ds.init((int)N, 1, mode, 0x5eed ^ j->id, pool, st))) return e;
     if ((e = ds.factorize(dM, N, st, true))) return e;
     if ((e = ds.solve(dM, N, db, dx, 1, kRefineTol, kMaxRefine, &res, &it, st))) return e;

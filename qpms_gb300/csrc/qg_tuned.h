@@ -8,7 +8,7 @@ namespace qg {
 
 // The mixed dense LU uses 64-wide diagonal blocks below this many unknowns
 // and 128-wide ones from it on.
-constexpr int kTunedNb64Below = 6144;
+constexpr int kTunedNb64Below = 256;
 
 // Operand stages and tensor-memory accumulators of the 128-wide GEMM tile,
 // as 10 x stages + accumulators.

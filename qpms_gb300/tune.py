@@ -26,11 +26,11 @@ import time
 import numpy as np
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SIZES = (1024, 2048, 3072, 4096, 6144, 8192, 11008, 14400)
+SIZES = (128, 256, 512, 1024, 2048, 3072, 4096, 6144, 8192, 11008, 14400)
 NBS = (64, 128)
 
 
-def measure(sizes=SIZES, reps=3):
+def measure(sizes=SIZES, reps=9):
     import torch
     from . import _lib
     L = _lib.lib()
@@ -147,7 +147,7 @@ def main():
     rows = measure()
     n64 = crossover(rows)
     with open(os.path.join(HERE, "tuning.json"), "w") as f:
-        json.dump({"dense_solve": {"what": "mixed dense solve, 1 right-hand side, seconds (min of 3)", "rows": rows},
+        json.dump({"dense_solve": {"what": "mixed dense solve, 1 right-hand side, seconds (min of 9)", "rows": rows},
                    "gemm": {"what": "tensor-core GEMM, microseconds per trailing update (m, n, k, digits): %s"
                             % (GEMM_SHAPES,), "variants": gemm},
                    "kTunedNb64Below": n64, "kTunedGemmPipe": pipe, "kTunedGemmWide": wide}, f, indent=1)
