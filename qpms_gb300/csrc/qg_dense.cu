@@ -869,35 +869,35 @@ int lu_solve_small(int N, int nb, const T *A, size_t lda, T *B, size_t ldb, int 
 }
 
 // ---------------- the same sweeps in one launch each ----------------
-// The two substitutions of lu_solve_small as one launch per sweep, over tiles
-// of kSweepRows rows, one warp per tile (nb a multiple of kSweepRows, at most
-// 128):
-//   forward, tile rows r of block j:  b_r <- b_r - sum_{k<j} P_k(r, :) b_k
-//   backward:                          b_r <- b_r - sum_{k>j} Q_k(r, :) b_k,
-// then a third launch writes every block's solution x_j = b_j - (I - D_j^-1)
-// b_j (no dependencies left).  b_k is final once every tile of block k has
-// written its rows (per-block completion counters, released after a fence,
-// read with acquire loads; b_k itself is read through L2).  A tile keeps its
-// sums over all k in registers and writes its rows once; the panel entries of
-// step k + 1 are requested before step k's wait.
+// The two substitutions of lu_solve_small as one launch per sweep, a CTA of four
+// warps per tile of kSweepRows rows (nb a multiple of kSweepRows, at most 128):
+//   forward, tile rows r of block j:  y_r = b_r - sum_{k<j} P_k(r, :) y_k
+//   backward:                          z_r = y_r - sum_{k>j} Q_k(r, :) z_k,
+// then a third launch writes every block's solution x_j = z_j - (I - D_j^-1)
+// z_j (no dependencies left).  What bounds a sweep is the chain from block to
+// block, so an entry of y or z is its own flag: the buffers start as all ones
+// (a NaN that no result has, see sweep_put), an entry is one 64-bit store (two
+// for complex128), and whoever needs it loads it until it has arrived: one L2
+// write and one L2 read per hop, with no fence, counter or second read between.
+// The threads of a CTA fetch one entry of block k each and share them through
+// shared memory; a tile keeps its sums over all k in registers and writes its
+// rows once.  The panel entries of step k + 1 and a first look at its block are
+// requested before step k's wait.
 // Tiles are handed out in dependency order by an atomic ticket (ascending
 // rows forward, descending backward): a tile only waits for tiles with earlier
-// tickets, which warps already running hold, so the waits end whatever number
+// tickets, which CTAs already running hold, so the waits end whatever number
 // of CTAs is resident (the argument of single-pass decoupled look-back scans).
-// Blocks also finish in sweep order (block k's tiles wait for block k - 1
-// forward, k + 1 backward), so a warp that has seen block k final knows the
-// earlier ones are.  Every wait is bounded (kSweepWaitNs); a wait that runs
-// out sets the error word, which makes the other warps leave too.  Warps are
-// independent (no CTA barrier), and a CTA of 4 warps at about 100 registers
-// fits on an SM beside a tensor-core GEMM CTA.
-// Sync words of one pair of sweeps (sweep_words): [0] error, [1] forward
-// ticket, [2] backward ticket, [3, 3 + nblk) forward block counters,
-// [3 + nblk, 3 + 2 nblk) backward block counters.
-// Lane 8 r + s of a warp handles row r of the tile and the columns
-// l = s + 8 q of each block: the eight partial sums of a row sit in eight
-// adjacent lanes and meet by shuffles; a column's four rows are one 32-byte
-// sector (complex64).
-constexpr int kSweepRows = 4, kSweepThreads = 128;
+// Every wait is bounded (kSweepWaitNs); a wait that runs out sets the error
+// word, which makes the other CTAs leave too.  A CTA of 4 warps at about 100
+// registers fits on an SM beside a tensor-core GEMM CTA.
+// Lane 8 r + s of a warp handles row r of its four and the columns l = s + 8 q
+// of each block: the eight partial sums of a row sit in eight adjacent lanes and
+// meet by shuffles; a column's four rows are one 32-byte sector (complex64).
+// Measured (counters released after a fence, a warp per tile of 4 rows, before ->
+// now): one mixed solve, three pairs of sweeps, 1,000 unknowns 1.35 -> 1.24 ms,
+// 3,000 3.51 -> 3.13, 6,000 8.59 -> 7.65, 14,400 41.8 -> 39.5; 8 right-hand sides at
+// 6,000 20.9 -> 17.7 ms.
+constexpr int kSweepRows = 16, kSweepThreads = 128;
 // complex64: at most 102 registers, so that a sweep CTA fits on an SM beside a
 // tensor-core GEMM CTA (320 threads x 160 registers)
 template <typename T>
@@ -905,54 +905,59 @@ struct SweepMinCtas {
   static constexpr int v = sizeof(T) == 8 ? 5 : 2;
 };
 constexpr unsigned long long kSweepWaitNs = 2000000000ull;  // 2 s
-size_t sweep_words(int nblk) { return 3 + 2 * (size_t)nblk; }
 
-__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ unsigned long long sweep_clock() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-// Wait until *cnt >= need; false if the error word is set or the wait ran out
-// (which sets it).
-__device__ bool sweep_wait(const unsigned *cnt, unsigned need, unsigned *err) {
-  if (ld_acquire(cnt) >= need) return true;
+// An entry as it stands in memory; false while it (or a half of it) is missing.
+__device__ __forceinline__ bool sweep_look(const float2 *p, float2 &v) {
+  unsigned long long u;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(u) : "l"(p) : "memory");
+  v = make_float2(__uint_as_float((unsigned)u), __uint_as_float((unsigned)(u >> 32)));
+  return u != ~0ull;
+}
+__device__ __forceinline__ bool sweep_look(const double2 *p, double2 &v) {
+  unsigned long long u, w;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(u) : "l"(p) : "memory");
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(&p->y) : "memory");
+  v = make_double2(__longlong_as_double((long long)u), __longlong_as_double((long long)w));
+  return u != ~0ull && w != ~0ull;
+}
+// stores an entry; the NaN that marks a missing one becomes another NaN
+__device__ __forceinline__ void sweep_put(float2 *p, float2 v) {
+  unsigned long long u = (unsigned long long)__float_as_uint(v.y) << 32 | __float_as_uint(v.x);
+  if (u == ~0ull) u >>= 1;
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(u) : "memory");
+}
+__device__ __forceinline__ void sweep_put(double2 *p, double2 v) {
+  unsigned long long u = (unsigned long long)__double_as_longlong(v.x), w = (unsigned long long)__double_as_longlong(v.y);
+  if (u == ~0ull) u >>= 1;
+  if (w == ~0ull) w >>= 1;
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(u) : "memory");
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(&p->y), "l"(w) : "memory");
+}
+// Loads *p until it has arrived; false if the error word is set or the wait ran
+// out (which sets it).  `pause`: nanoseconds between looks, for tiles whose
+// turn is not next.
+template <typename T>
+__device__ __forceinline__ bool sweep_wait(const T *p, T &v, int pause, unsigned *err) {
   const unsigned long long t0 = sweep_clock();
   for (;;) {
-    __nanosleep(32);
-    if (ld_acquire(cnt) >= need) return true;
-    if (ld_acquire(err)) return false;
+#pragma unroll 1
+    for (int i = 0; i < 16; ++i) {
+      if (pause) __nanosleep(pause);
+      if (sweep_look(p, v)) return true;
+    }
+    unsigned e;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(e) : "l"(err) : "memory");
+    if (e) return false;
     if (sweep_clock() - t0 > kSweepWaitNs) {
       atomicExch(err, 1u);
       return false;
     }
   }
-}
-// lane 0 waits, the warp follows (the barrier orders the other lanes' loads
-// after lane 0's acquire)
-__device__ __forceinline__ bool warp_wait(const unsigned *cnt, unsigned need, unsigned *err, int lane) {
-  int ok = 1;
-  if (lane == 0) ok = sweep_wait(cnt, need, err) ? 1 : 0;
-  ok = __shfl_sync(0xffffffffu, ok, 0);
-  __syncwarp();
-  return ok != 0;
-}
-// lane 0 looks once (no wait): is *cnt >= need?
-__device__ __forceinline__ bool warp_peek(const unsigned *cnt, unsigned need, int lane) {
-  int ok = 0;
-  if (lane == 0) ok = ld_acquire(cnt) >= need ? 1 : 0;
-  ok = __shfl_sync(0xffffffffu, ok, 0);
-  __syncwarp();
-  return ok != 0;
-}
-__device__ __forceinline__ int warp_ticket(unsigned *ticket, int lane) {
-  int t = 0;
-  if (lane == 0) t = (int)atomicAdd(ticket, 1u);
-  return __shfl_sync(0xffffffffu, t, 0);
 }
 
 // the 16 entries l = sl + 8 q < kb of one row of a block column (col0: its
@@ -965,25 +970,11 @@ __device__ __forceinline__ void sweep_load(const T *col0, size_t lda, int kb, bo
     pv[q] = (rowok && l < kb) ? col0[(size_t)l * lda] : mk<T>(0, 0);
   }
 }
-// acc[c] += sum_l pv[l] b_k(l, c), b_k (kb x nrhs from Bk) read through L2
-template <typename T>
-__device__ __forceinline__ void sweep_fma(const T (&pv)[16], const T *Bk, size_t ldb, int kb, int nrhs, int sl,
-                                          T (&acc)[kSmallRhs]) {
-#pragma unroll
-  for (int c = 0; c < kSmallRhs; ++c)
-    if (c < nrhs) {
-#pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        const int l = sl + 8 * q;
-        if (l < kb) acc[c] = fma_c(acc[c], pv[q], __ldcg(Bk + (size_t)c * ldb + l));
-      }
-    }
-}
 // sums over the eight lanes of a row (every lane gets the total)
-template <typename T>
-__device__ __forceinline__ void sweep_reduce(T (&acc)[kSmallRhs], int nrhs) {
+template <typename T, int NR>
+__device__ __forceinline__ void sweep_reduce(T (&acc)[NR], int nrhs) {
 #pragma unroll
-  for (int c = 0; c < kSmallRhs; ++c)
+  for (int c = 0; c < NR; ++c)
     if (c < nrhs) {
 #pragma unroll
       for (int o = 1; o < 8; o <<= 1) {
@@ -992,145 +983,148 @@ __device__ __forceinline__ void sweep_reduce(T (&acc)[kSmallRhs], int nrhs) {
       }
     }
 }
-// the tile's rows: b_r <- b_r - acc, then the tile is counted in its block
-template <typename T>
-__device__ __forceinline__ void sweep_finish(T *B, size_t ldb, int row, bool rowok, int sl, int nrhs,
-                                             const T (&acc)[kSmallRhs], unsigned *cnt, int lane) {
-  if (sl == 0 && rowok) {
-#pragma unroll
-    for (int c = 0; c < kSmallRhs; ++c)
-      if (c < nrhs) {
-        T *d = B + (size_t)c * ldb + row;
-        *d = sub(__ldcg(d), acc[c]);
-      }
-    __threadfence();
-  }
-  __syncwarp();
-  if (lane == 0) atomicAdd(cnt, 1u);
-}
 
-template <typename T>
-__global__ void __launch_bounds__(kSweepThreads, SweepMinCtas<T>::v) sweep_fwd_kernel(const T *__restrict__ A, size_t lda, int N, int nb,
-                                                                  T *B, size_t ldb, int nrhs, unsigned *sync) {
-  const int lane = threadIdx.x & 31, sl = lane & 7, rr = lane >> 3;
-  const int ntiles = (N + kSweepRows - 1) / kSweepRows;
-  const unsigned need = (unsigned)(nb / kSweepRows);  // tiles of a full block
-  unsigned *err = sync, *ticket = sync + 1, *cnt = sync + 3;
-  int known = -1;  // blocks 0..known are final
-  for (;;) {
-    const int t = warp_ticket(ticket, lane);
-    if (t >= ntiles) return;
-    const int row0 = t * kSweepRows, j = row0 / nb, row = row0 + rr;
-    const bool rowok = row < N;
-    T acc[kSmallRhs];
-#pragma unroll
-    for (int c = 0; c < kSmallRhs; ++c) acc[c] = mk<T>(0, 0);
-    if (j - 1 > known && warp_peek(cnt + j - 1, need, lane)) known = j - 1;
-    T pv[16];
-    if (j > 0) sweep_load(A + row, lda, nb, rowok, sl, pv);
-    for (int k = 0; k < j; ++k) {  // the blocks above are full: kb = nb
-      T pn[16];
-      if (k + 1 < j) sweep_load(A + (size_t)(k + 1) * nb * lda + row, lda, nb, rowok, sl, pn);
-      if (k > known) {
-        if (!warp_wait(cnt + k, need, err, lane)) return;
-        known = k;
-      }
-      sweep_fma(pv, B + (size_t)k * nb, ldb, nb, nrhs, sl, acc);
-      if (k + 1 < j) {
-#pragma unroll
-        for (int q = 0; q < 16; ++q) pv[q] = pn[q];
-      }
-    }
-    sweep_reduce(acc, nrhs);
-    sweep_finish(B, ldb, row, rowok, sl, nrhs, acc, cnt + j, lane);
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kSweepThreads, SweepMinCtas<T>::v) sweep_bwd_kernel(const T *__restrict__ A, size_t lda, int N, int nb,
-                                                                  T *B, size_t ldb, int nrhs, unsigned *sync) {
-  const int lane = threadIdx.x & 31, sl = lane & 7, rr = lane >> 3;
+// One sweep (BWD: backward) of nrhs <= NR right-hand sides: B -> Y, both with
+// leading dimension ldb; *ticket starts at -1.
+template <typename T, int NR, bool BWD>
+__device__ __forceinline__ void sweep_tiles(const T *__restrict__ A, size_t lda, int N, int nb, const T *__restrict__ B,
+                                            T *Y, size_t ldb, int nrhs, unsigned *ticket, unsigned *err) {
+  __shared__ T bs[2][NR][128];
+  __shared__ int next;
+  const int tid = threadIdx.x, lane = tid & 31, sl = lane & 7, rr = (tid >> 5) * 4 + (lane >> 3);
   const int ntiles = (N + kSweepRows - 1) / kSweepRows, nblk = (N + nb - 1) / nb;
-  unsigned *err = sync, *ticket = sync + 2, *cnt = sync + 3 + nblk;
-  auto need = [&](int k) { return (unsigned)((min(nb, N - k * nb) + kSweepRows - 1) / kSweepRows); };
-  int known = nblk;  // blocks known..nblk-1 are final
   for (;;) {
-    const int tk = warp_ticket(ticket, lane);
+    if (tid == 0) next = (int)(atomicAdd(ticket, 1u) + 1u);
+    __syncthreads();
+    const int tk = next;
+    __syncthreads();
     if (tk >= ntiles) return;
-    const int t = ntiles - 1 - tk, row0 = t * kSweepRows, j = row0 / nb, row = row0 + rr;
+    const int row0 = (BWD ? ntiles - 1 - tk : tk) * kSweepRows, j = row0 / nb, row = row0 + rr;
+    const int steps = BWD ? nblk - 1 - j : j;
     const bool rowok = row < N;
-    T acc[kSmallRhs];
+    T acc[NR], pv[16];
 #pragma unroll
-    for (int c = 0; c < kSmallRhs; ++c) acc[c] = mk<T>(0, 0);
-    if (j + 1 < known && j + 1 < nblk && warp_peek(cnt + j + 1, need(j + 1), lane)) known = j + 1;
-    T pv[16];
-    if (j < nblk - 1) sweep_load(A + (size_t)(nblk - 1) * nb * lda + row, lda, N - (nblk - 1) * nb, rowok, sl, pv);
-    for (int k = nblk - 1; k > j; --k) {
-      const int k0 = k * nb, kb = min(nb, N - k0);
+    for (int c = 0; c < NR; ++c) acc[c] = mk<T>(0, 0);
+    // lane s of a row has the row's entry of right-hand side s
+    const T own = rowok && sl < nrhs ? B[(size_t)sl * ldb + row] : mk<T>(0, 0);
+    T first = mk<T>(0, 0);  // a first look at this thread's entry of the step's block
+    bool have = true;
+    auto look = [&](int k) { have = tid >= min(nb, N - k * nb) || sweep_look(Y + k * nb + tid, first); };
+    if (steps) {
+      const int k = BWD ? nblk - 1 : 0;
+      sweep_load(A + (size_t)k * nb * lda + row, lda, min(nb, N - k * nb), rowok, sl, pv);
+      look(k);
+    }
+    for (int i = 0; i < steps; ++i) {
+      const int k = BWD ? nblk - 1 - i : i, k0 = k * nb, kb = min(nb, N - k0), kn = BWD ? k - 1 : k + 1;
       T pn[16];
-      if (k - 1 > j) sweep_load(A + (size_t)(k0 - nb) * lda + row, lda, nb, rowok, sl, pn);  // block k - 1 is full
-      if (k < known) {
-        if (!warp_wait(cnt + k, need(k), err, lane)) return;
-        known = k;
+      if (i + 1 < steps) sweep_load(A + (size_t)kn * nb * lda + row, lda, nb, rowok, sl, pn);  // a full block
+      bool ok = true;
+      const int pause = i + 1 == steps ? 0 : 64;
+      if (tid < kb) {
+        if (!have) ok = sweep_wait(Y + k0 + tid, first, pause, err);
+        bs[i & 1][0][tid] = first;
+#pragma unroll 1
+        for (int c = 1; c < nrhs; ++c) {
+          const T *p = Y + (size_t)c * ldb + k0 + tid;
+          T v;
+          if (!sweep_look(p, v)) ok = ok && sweep_wait(p, v, pause, err);
+          bs[i & 1][c][tid] = v;
+        }
       }
-      sweep_fma(pv, B + k0, ldb, kb, nrhs, sl, acc);
-      if (k - 1 > j) {
+      if (__syncthreads_or(!ok)) return;
+      if (i + 1 < steps) look(kn);
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        const int l = sl + 8 * q;
+        if (l < kb)
+#pragma unroll
+          for (int c = 0; c < NR; ++c)
+            if (c < nrhs) acc[c] = fma_c(acc[c], pv[q], bs[i & 1][c][l]);
+      }
+      if (i + 1 < steps) {
 #pragma unroll
         for (int q = 0; q < 16; ++q) pv[q] = pn[q];
       }
     }
-    sweep_reduce(acc, nrhs);
-    sweep_finish(B, ldb, row, rowok, sl, nrhs, acc, cnt + j, lane);
+    sweep_reduce<T, NR>(acc, nrhs);
+    T sum = acc[0];
+#pragma unroll
+    for (int c = 1; c < NR; ++c)
+      if (c == sl) sum = acc[c];
+    if (rowok && sl < nrhs) sweep_put(Y + (size_t)sl * ldb + row, sub(own, sum));
   }
 }
+template <typename T, int NR>
+__global__ void __launch_bounds__(kSweepThreads, SweepMinCtas<T>::v)
+    sweep_fwd_kernel(const T *__restrict__ A, size_t lda, int N, int nb, const T *__restrict__ B, T *Y, size_t ldb,
+                     int nrhs, unsigned *ticket, unsigned *err) {
+  sweep_tiles<T, NR, false>(A, lda, N, nb, B, Y, ldb, nrhs, ticket, err);
+}
+template <typename T, int NR>
+__global__ void __launch_bounds__(kSweepThreads, SweepMinCtas<T>::v)
+    sweep_bwd_kernel(const T *__restrict__ A, size_t lda, int N, int nb, const T *__restrict__ B, T *Y, size_t ldb,
+                     int nrhs, unsigned *ticket, unsigned *err) {
+  sweep_tiles<T, NR, true>(A, lda, N, nb, B, Y, ldb, nrhs, ticket, err);
+}
 
-// x_j = b_j - (I - D_j^-1) b_j for every block, one warp per tile of rows
+// x_j = z_j - (I - D_j^-1) z_j for every block, one warp per four rows
 template <typename T>
 __global__ void __launch_bounds__(kSweepThreads) sweep_diag_kernel(const T *__restrict__ A, size_t lda, int N, int nb,
-                                                                   const T *B, size_t ldb, T *X, size_t ldx,
+                                                                   const T *__restrict__ Z, T *X, size_t ld,
                                                                    int nrhs) {
   const int lane = threadIdx.x & 31, sl = lane & 7, rr = lane >> 3;
-  const int ntiles = (N + kSweepRows - 1) / kSweepRows;
+  const int ntiles = (N + 3) / 4;
   const int nwarps = (int)(gridDim.x * blockDim.x) >> 5;
   for (int t = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntiles; t += nwarps) {
-    const int row0 = t * kSweepRows, j0 = row0 / nb * nb, kbj = min(nb, N - j0), row = row0 + rr;
+    const int row0 = t * 4, j0 = row0 / nb * nb, kbj = min(nb, N - j0), row = row0 + rr;
     const bool rowok = row < N;
     T pv[16], acc[kSmallRhs];
 #pragma unroll
     for (int c = 0; c < kSmallRhs; ++c) acc[c] = mk<T>(0, 0);
     sweep_load(A + (size_t)j0 * lda + row, lda, kbj, rowok, sl, pv);
-    sweep_fma(pv, B + j0, ldb, kbj, nrhs, sl, acc);
-    sweep_reduce(acc, nrhs);
+#pragma unroll
+    for (int c = 0; c < kSmallRhs; ++c)
+      if (c < nrhs) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+          const int l = sl + 8 * q;
+          if (l < kbj) acc[c] = fma_c(acc[c], pv[q], Z[(size_t)c * ld + j0 + l]);
+        }
+      }
+    sweep_reduce<T, kSmallRhs>(acc, nrhs);
     if (sl == 0 && rowok) {
 #pragma unroll
       for (int c = 0; c < kSmallRhs; ++c)
-        if (c < nrhs) X[(size_t)c * ldx + row] = sub(B[(size_t)c * ldb + row], acc[c]);
+        if (c < nrhs) X[(size_t)c * ld + row] = sub(Z[(size_t)c * ld + row], acc[c]);
     }
   }
 }
 
-// lu_solve_small's result in three launches.  sync: sweep_words(nblk) words
-// whose error word is zero; the others are cleared here.
+// lu_solve_small's result in three launches: B (kept) -> X, both with leading
+// dimension N.  X is followed by 2 nrhs N elements and two words of scratch
+// (y, z and the tickets); err: a word that is zero.
 template <typename T>
-int lu_solve_sweep(int N, int nb, const T *A, size_t lda, T *B, size_t ldb, int nrhs, T *X, unsigned *sync,
-                   cudaStream_t st) {
-  if (nb % kSweepRows || nb > 128) return lu_solve_small<T>(N, nb, A, lda, B, ldb, nrhs, X, st);
-  const int nblk = (N + nb - 1) / nb, ntiles = (N + kSweepRows - 1) / kSweepRows;
-  const int wpc = kSweepThreads / 32, ctas = (ntiles + wpc - 1) / wpc;
+int lu_solve_sweep(int N, int nb, const T *A, size_t lda, T *B, int nrhs, T *X, unsigned *err, cudaStream_t st) {
+  if (nb % kSweepRows || nb > 128) return lu_solve_small<T>(N, nb, A, lda, B, N, nrhs, X, st);
+  const int ntiles = (N + kSweepRows - 1) / kSweepRows;
   int dev = 0, sms = 0;
   QG_CUDA_TRY(cudaGetDevice(&dev));
   QG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   sms = std::max(sms, 1);
-  QG_CUDA_TRY(cudaMemsetAsync(sync + 1, 0, (sweep_words(nblk) - 1) * sizeof(unsigned), st));
-  // two CTAs (8 warps) per SM: at 8,192 unknowns 345 us per forward sweep,
-  // against 398 us with a warp for every tile (512 CTAs), whose extra waiting
-  // warps only add polls of the block counters
-  const int grid = std::min(ctas, 2 * sms);
-  sweep_fwd_kernel<T><<<grid, kSweepThreads, 0, st>>>(A, lda, N, nb, B, ldb, nrhs, sync);
+  const size_t n = (size_t)N * nrhs;
+  T *Y = X + n, *Z = Y + n;
+  unsigned *ticket = (unsigned *)(Z + n);
+  QG_CUDA_TRY(cudaMemsetAsync(Y, 0xff, 2 * n * sizeof(T) + 2 * sizeof(unsigned), st));
+  // two CTAs per SM: three and four change nothing at 3,000 to 14,400 unknowns
+  const int grid = std::min(ntiles, 2 * sms);
+  auto fwd = nrhs == 1 ? sweep_fwd_kernel<T, 1> : sweep_fwd_kernel<T, kSmallRhs>;
+  auto bwd = nrhs == 1 ? sweep_bwd_kernel<T, 1> : sweep_bwd_kernel<T, kSmallRhs>;
+  fwd<<<grid, kSweepThreads, 0, st>>>(A, lda, N, nb, B, Y, (size_t)N, nrhs, ticket, err);
   QG_CUDA_TRY(cudaGetLastError());
-  sweep_bwd_kernel<T><<<grid, kSweepThreads, 0, st>>>(A, lda, N, nb, B, ldb, nrhs, sync);
+  bwd<<<grid, kSweepThreads, 0, st>>>(A, lda, N, nb, Y, Z, (size_t)N, nrhs, ticket + 1, err);
   QG_CUDA_TRY(cudaGetLastError());
-  sweep_diag_kernel<T><<<std::min(ctas, 8 * sms), kSweepThreads, 0, st>>>(A, lda, N, nb, B, ldb, X, ldb, nrhs);
+  sweep_diag_kernel<T><<<std::min((N + 15) / 16, 8 * sms), kSweepThreads, 0, st>>>(A, lda, N, nb, Z, X, (size_t)N, nrhs);
   QG_CUDA_TRY(cudaGetLastError());
   g_launches.fetch_add(3);
   return QPMS_SUCCESS;
@@ -1247,8 +1241,6 @@ int DenseSolver::init(int N_, int nrhs_max_, int mode_, unsigned long long seed,
   // a mixed solver that falls back to complex128 factors uses the same work
   // buffer for nb = 64 complex128 column blocks (N x 64 x 16 bytes)
   if (mode) wsz = std::max<size_t>(wsz, (size_t)std::max(Np, nrhs_max) * 64 * 16);
-  // sized for 64-wide blocks (the complex128 fallback's), the larger count
-  const size_t sweep_bytes = sweep_words((Np + 63) / 64) * sizeof(unsigned);
   // K up to group x nb: the combined update of a group of blocks
   const int kmax = lu_group() * nb;
   // one allocation for all buffers that every solver of this mode has (each by
@@ -1268,7 +1260,7 @@ int DenseSolver::init(int N_, int nrhs_max_, int mode_, unsigned long long seed,
       {(void **)&dinfo, 16},
       {(void **)&rs, (size_t)4 * Np * sizeof(double)},
       {(void **)&res_nrm, (size_t)2 * kOzakiMinRhs * sizeof(double)},
-      {(void **)&sweep, sweep_bytes},
+      {(void **)&sweep, sizeof(unsigned)},
       {&tc_pa, tc_split ? tc_planes_bytes_a(Np, kmax, 3) : 0},
       {&tc_pb, tc_split ? tc_planes_bytes_b(std::max(Np, nrhs_max), kmax, 3) : 0},
   };
@@ -1280,7 +1272,7 @@ int DenseSolver::init(int N_, int nrhs_max_, int mode_, unsigned long long seed,
     *q.p = q.bytes ? (char *)block + off : nullptr;
     off += (q.bytes + 255) / 256 * 256;
   }
-  QG_CUDA_TRY(cudaMemsetAsync(sweep, 0, sweep_bytes, ast));
+  QG_CUDA_TRY(cudaMemsetAsync(sweep, 0, sizeof(unsigned), ast));
   if (tc_split) {
     const char *la = getenv("QPMS_GB300_LOOKAHEAD");
     if (lookahead && !(la && !strcmp(la, "0")) && Np > nb) {
@@ -1330,7 +1322,7 @@ size_t DenseSolver::footprint(int N, int nrhs, int mode) {
   b += std::max<size_t>(std::max<size_t>(Np * nb, nb * std::max<size_t>(Np, nrhs)) * esz,
                         mode ? std::max<size_t>(Np, nrhs) * 64 * 16 : 0);
   b += Np * nrhs * (8 + 16) + (size_t)N * nrhs * 32 + 16 + 4 * Np * 8 + 2 * kOzakiMinRhs * 8;
-  b += sweep_words((int)((Np + 63) / 64)) * sizeof(unsigned);
+  b += sizeof(unsigned);
   if (ozaki_wanted(nrhs)) b += ozaki_matrix_bytes(N) + ozaki_work_bytes(N, nrhs);
   if (mode && tc_digits(nrhs)) b += tc_plane_bytes((int)Np, nrhs, kMaxLuGroup * (int)nb);
   if (mode && tc_digits(nrhs) && nrhs > kSmallRhs && fac_planes_wanted()) b += tc_planes_bytes_a((int)Np, (int)Np, 3);
@@ -1532,9 +1524,12 @@ int DenseSolver::factor_launch(const void *M64, size_t ldm, cudaStream_t st) {
                            CUBLAS_COMPUTE_64F, st);
 }
 
+// Few right-hand sides: one launch per sweep; QPMS_GB300_SUBST=steps takes one
+// launch per block and sweep instead (a serving mix of 24 requests with 8 workers:
+// sweeps 81.2 ms, steps 83.3 ms).
 bool DenseSolver::use_sweeps() const {
   static const int v = env_choice("QPMS_GB300_SUBST", "sweep", "steps");
-  return v < 0 ? sweeps : v == 1;
+  return v != 0;
 }
 int DenseSolver::lu_group() const {
   static const int v = [] {
@@ -1590,7 +1585,7 @@ int DenseSolver::apply_launch(const void *R, size_t ldr, void *Y, size_t ldy, in
     if (nrhs <= kSmallRhs) {
       e = !use_sweeps() ? lu_solve_small<float2>(Np, nb, (const float2 *)A, Np, (float2 *)rhs_lo, Np, nrhs,
                                                  (float2 *)work, st)
-                        : lu_solve_sweep<float2>(Np, nb, (const float2 *)A, Np, (float2 *)rhs_lo, Np, nrhs,
+                        : lu_solve_sweep<float2>(Np, nb, (const float2 *)A, Np, (float2 *)rhs_lo, nrhs,
                                                  (float2 *)work, sweep, st);
       sol = (const float2 *)work;
     } else if (tc_split) {
@@ -1608,7 +1603,7 @@ int DenseSolver::apply_launch(const void *R, size_t ldr, void *Y, size_t ldy, in
     if (nrhs <= kSmallRhs) {
       e = !use_sweeps() ? lu_solve_small<double2>(Np, nb, (const double2 *)T64, Np, (double2 *)rp, Np, nrhs,
                                                   (double2 *)work, st)
-                        : lu_solve_sweep<double2>(Np, nb, (const double2 *)T64, Np, (double2 *)rp, Np, nrhs,
+                        : lu_solve_sweep<double2>(Np, nb, (const double2 *)T64, Np, (double2 *)rp, nrhs,
                                                   (double2 *)work, sweep, st);
       if (!e)
         QG_CUDA_TRY(cudaMemcpyAsync(rp, work, n * 16, cudaMemcpyDeviceToDevice, st));

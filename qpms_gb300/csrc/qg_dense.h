@@ -74,12 +74,6 @@ struct DenseSolver {
   // turns it off; so does lookahead = false before init(): a serving loop with
   // several workers already overlaps the inversions with other requests' work)
   bool lookahead = true;
-  // few-right-hand-side substitutions as one launch per sweep (tiles that wait
-  // on per-block counters) rather than one launch per block and sweep; a
-  // serving loop with several workers turns it off: the waiting CTAs would hold
-  // SMs that other requests' GEMMs need (QPMS_GB300_SUBST=sweep / steps
-  // overrides either way)
-  bool sweeps = true;
   // tensor-core LU by groups of `group` blocks (1 .. kMaxLuGroup): one
   // trailing update with K = group x nb per group (QPMS_GB300_LU_GROUP
   // overrides); 0 = by size (lu_group); set before init(), which sizes the

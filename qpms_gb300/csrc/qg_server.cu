@@ -331,10 +331,6 @@ struct qpms_gpu_server {
     // inversion chain, bound a loaded server (107.5 solves/s against 104.4
     // with 64-wide blocks below 6,144 unknowns)
     ds.nb_pref = 128;
-    // and the substitutions as one launch per block and sweep: the one-launch
-    // sweeps' waiting warps hold SM slots the other requests' kernels could
-    // use (135.4 / 135.6 solves/s with them, 138.2 / 137.7 without, 8 workers)
-    ds.sweeps = nworkers == 1;
     // and groups of 3 blocks in the LU: without the lookahead the in-group
     // inversions cost nothing extra here (136.0 / 137.0 solves/s with pairs,
     // 138.1 with groups of 3, 138.2 / 137.0 with groups of 4)
