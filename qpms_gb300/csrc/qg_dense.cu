@@ -873,6 +873,7 @@ int lu_solve_small(int N, int nb, const T *A, size_t lda, T *B, size_t ldb, int 
 // warps per tile of kSweepRows rows (nb a multiple of kSweepRows, at most 128):
 //   forward, tile rows r of block j:  y_r = b_r - sum_{k<j} P_k(r, :) y_k
 //   backward:                          z_r = y_r - sum_{k>j} Q_k(r, :) z_k,
+// for up to NR right-hand sides per tile (NR = 1, 2, 4, 8; more by chunks),
 // then a third launch writes every block's solution x_j = z_j - (I - D_j^-1)
 // z_j (no dependencies left).  What bounds a sweep is the chain from block to
 // block, so an entry of y or z is its own flag: the buffers start as all ones
@@ -888,21 +889,20 @@ int lu_solve_small(int N, int nb, const T *A, size_t lda, T *B, size_t ldb, int 
 // tickets, which CTAs already running hold, so the waits end whatever number
 // of CTAs is resident (the argument of single-pass decoupled look-back scans).
 // Every wait is bounded (kSweepWaitNs); a wait that runs out sets the error
-// word, which makes the other CTAs leave too.  A CTA of 4 warps at about 100
-// registers fits on an SM beside a tensor-core GEMM CTA.
+// word, which makes the other CTAs leave too.
 // Lane 8 r + s of a warp handles row r of its four and the columns l = s + 8 q
 // of each block: the eight partial sums of a row sit in eight adjacent lanes and
 // meet by shuffles; a column's four rows are one 32-byte sector (complex64).
 // Measured (counters released after a fence, a warp per tile of 4 rows, before ->
 // now): one mixed solve, three pairs of sweeps, 1,000 unknowns 1.35 -> 1.24 ms,
-// 3,000 3.51 -> 3.13, 6,000 8.59 -> 7.65, 14,400 41.8 -> 39.5; 8 right-hand sides at
-// 6,000 20.9 -> 17.7 ms.
+// 3,000 3.51 -> 3.12, 6,000 8.59 -> 7.69, 14,400 41.8 -> 39.7; 8 right-hand sides at
+// 6,000 20.9 -> 16.7 ms.
 constexpr int kSweepRows = 16, kSweepThreads = 128;
-// complex64: at most 102 registers, so that a sweep CTA fits on an SM beside a
-// tensor-core GEMM CTA (320 threads x 160 registers)
-template <typename T>
+// complex64, one right-hand side: at most 102 registers, so that a sweep CTA fits
+// on an SM beside a tensor-core GEMM CTA (320 threads x 160 registers)
+template <typename T, int NR>
 struct SweepMinCtas {
-  static constexpr int v = sizeof(T) == 8 ? 5 : 2;
+  static constexpr int v = sizeof(T) == 16 ? 2 : NR == 1 ? 5 : 4;
 };
 constexpr unsigned long long kSweepWaitNs = 2000000000ull;  // 2 s
 
@@ -984,22 +984,31 @@ __device__ __forceinline__ void sweep_reduce(T (&acc)[NR], int nrhs) {
     }
 }
 
-// One sweep (BWD: backward) of nrhs <= NR right-hand sides: B -> Y, both with
-// leading dimension ldb; *ticket starts at -1.
+// One sweep (BWD: backward): B -> Y, both with leading dimension ldb; *ticket
+// starts at -1.  More than NR right-hand sides go by chunks of NR, whose chains
+// are independent: consecutive tickets are the chunks of one row tile (their
+// panel entries come from memory once).
 template <typename T, int NR, bool BWD>
-__device__ __forceinline__ void sweep_tiles(const T *__restrict__ A, size_t lda, int N, int nb, const T *__restrict__ B,
-                                            T *Y, size_t ldb, int nrhs, unsigned *ticket, unsigned *err) {
-  __shared__ T bs[2][NR][128];
+__device__ __forceinline__ void sweep_tiles(const T *__restrict__ A, size_t lda, int N, int nb, const T *__restrict__ B_all,
+                                            T *Y_all, size_t ldb, int nrhs_all, unsigned *ticket, unsigned *err) {
+  // a column's right-hand sides side by side, padded so that eight columns'
+  // 16-byte reads fall on different banks
+  constexpr int LD = NR < 4 ? NR : NR + 16 / (int)sizeof(T);
+  __shared__ __align__(16) T bs[2][128 * LD];
   __shared__ int next;
   const int tid = threadIdx.x, lane = tid & 31, sl = lane & 7, rr = (tid >> 5) * 4 + (lane >> 3);
   const int ntiles = (N + kSweepRows - 1) / kSweepRows, nblk = (N + nb - 1) / nb;
+  const int nch = (nrhs_all + NR - 1) / NR;
   for (;;) {
     if (tid == 0) next = (int)(atomicAdd(ticket, 1u) + 1u);
     __syncthreads();
     const int tk = next;
     __syncthreads();
-    if (tk >= ntiles) return;
-    const int row0 = (BWD ? ntiles - 1 - tk : tk) * kSweepRows, j = row0 / nb, row = row0 + rr;
+    if (tk >= ntiles * nch) return;
+    const int tr = tk / nch, ch = tk - tr * nch, nrhs = min(NR, nrhs_all - NR * ch);
+    const T *B = B_all + (size_t)(NR * ch) * ldb;
+    T *Y = Y_all + (size_t)(NR * ch) * ldb;
+    const int row0 = (BWD ? ntiles - 1 - tr : tr) * kSweepRows, j = row0 / nb, row = row0 + rr;
     const int steps = BWD ? nblk - 1 - j : j;
     const bool rowok = row < N;
     T acc[NR], pv[16];
@@ -1007,41 +1016,56 @@ __device__ __forceinline__ void sweep_tiles(const T *__restrict__ A, size_t lda,
     for (int c = 0; c < NR; ++c) acc[c] = mk<T>(0, 0);
     // lane s of a row has the row's entry of right-hand side s
     const T own = rowok && sl < nrhs ? B[(size_t)sl * ldb + row] : mk<T>(0, 0);
-    T first = mk<T>(0, 0);  // a first look at this thread's entry of the step's block
-    bool have = true;
-    auto look = [&](int k) { have = tid >= min(nb, N - k * nb) || sweep_look(Y + k * nb + tid, first); };
+    T first[NR];  // a first look at this thread's entries of the step's block
+    bool have[NR];
+#pragma unroll
+    for (int c = 0; c < NR; ++c) first[c] = mk<T>(0, 0);
+    auto look = [&](int k) {
+      const bool mine = tid < min(nb, N - k * nb);
+#pragma unroll
+      for (int c = 0; c < NR; ++c) {
+        have[c] = true;
+        first[c] = mk<T>(0, 0);
+        if (mine && c < nrhs) have[c] = sweep_look(Y + (size_t)c * ldb + k * nb + tid, first[c]);
+      }
+    };
     if (steps) {
       const int k = BWD ? nblk - 1 : 0;
       sweep_load(A + (size_t)k * nb * lda + row, lda, min(nb, N - k * nb), rowok, sl, pv);
       look(k);
     }
     for (int i = 0; i < steps; ++i) {
-      const int k = BWD ? nblk - 1 - i : i, k0 = k * nb, kb = min(nb, N - k0), kn = BWD ? k - 1 : k + 1;
+      const int k = BWD ? nblk - 1 - i : i, k0 = k * nb, kn = BWD ? k - 1 : k + 1;
       T pn[16];
       if (i + 1 < steps) sweep_load(A + (size_t)kn * nb * lda + row, lda, nb, rowok, sl, pn);  // a full block
       bool ok = true;
       const int pause = i + 1 == steps ? 0 : 64;
-      if (tid < kb) {
-        if (!have) ok = sweep_wait(Y + k0 + tid, first, pause, err);
-        bs[i & 1][0][tid] = first;
-#pragma unroll 1
-        for (int c = 1; c < nrhs; ++c) {
-          const T *p = Y + (size_t)c * ldb + k0 + tid;
-          T v;
-          if (!sweep_look(p, v)) ok = ok && sweep_wait(p, v, pause, err);
-          bs[i & 1][c][tid] = v;
-        }
+#pragma unroll
+      for (int c = 0; c < NR; ++c) {
+        if (!have[c]) ok = ok && sweep_wait(Y + (size_t)c * ldb + k0 + tid, first[c], pause, err);
+        bs[i & 1][tid * LD + c] = first[c];
       }
       if (__syncthreads_or(!ok)) return;
       if (i + 1 < steps) look(kn);
+      auto fma8 = [&](int q0) {  // zeros past the block's columns and right-hand sides
 #pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        const int l = sl + 8 * q;
-        if (l < kb)
+        for (int q = q0; q < q0 + 8; ++q) {
+          const T *p = bs[i & 1] + (sl + 8 * q) * LD;
+          if constexpr (sizeof(T) == 8 && NR > 1) {
 #pragma unroll
-          for (int c = 0; c < NR; ++c)
-            if (c < nrhs) acc[c] = fma_c(acc[c], pv[q], bs[i & 1][c][l]);
-      }
+            for (int c = 0; c < NR; c += 2) {
+              const float4 v = *(const float4 *)(p + c);
+              acc[c] = fma_c(acc[c], pv[q], mk<T>(v.x, v.y));
+              acc[c + 1] = fma_c(acc[c + 1], pv[q], mk<T>(v.z, v.w));
+            }
+          } else {
+#pragma unroll
+            for (int c = 0; c < NR; ++c) acc[c] = fma_c(acc[c], pv[q], p[c]);
+          }
+        }
+      };
+      fma8(0);
+      if (nb > 64) fma8(8);
       if (i + 1 < steps) {
 #pragma unroll
         for (int q = 0; q < 16; ++q) pv[q] = pn[q];
@@ -1056,13 +1080,13 @@ __device__ __forceinline__ void sweep_tiles(const T *__restrict__ A, size_t lda,
   }
 }
 template <typename T, int NR>
-__global__ void __launch_bounds__(kSweepThreads, SweepMinCtas<T>::v)
+__global__ void __launch_bounds__(kSweepThreads, SweepMinCtas<T, NR>::v)
     sweep_fwd_kernel(const T *__restrict__ A, size_t lda, int N, int nb, const T *__restrict__ B, T *Y, size_t ldb,
                      int nrhs, unsigned *ticket, unsigned *err) {
   sweep_tiles<T, NR, false>(A, lda, N, nb, B, Y, ldb, nrhs, ticket, err);
 }
 template <typename T, int NR>
-__global__ void __launch_bounds__(kSweepThreads, SweepMinCtas<T>::v)
+__global__ void __launch_bounds__(kSweepThreads, SweepMinCtas<T, NR>::v)
     sweep_bwd_kernel(const T *__restrict__ A, size_t lda, int N, int nb, const T *__restrict__ B, T *Y, size_t ldb,
                      int nrhs, unsigned *ticket, unsigned *err) {
   sweep_tiles<T, NR, true>(A, lda, N, nb, B, Y, ldb, nrhs, ticket, err);
@@ -1073,6 +1097,9 @@ template <typename T>
 __global__ void __launch_bounds__(kSweepThreads) sweep_diag_kernel(const T *__restrict__ A, size_t lda, int N, int nb,
                                                                    const T *__restrict__ Z, T *X, size_t ld,
                                                                    int nrhs) {
+  Z += (size_t)blockIdx.y * kSmallRhs * ld;  // one chunk of right-hand sides
+  X += (size_t)blockIdx.y * kSmallRhs * ld;
+  nrhs = min(kSmallRhs, nrhs - (int)blockIdx.y * kSmallRhs);
   const int lane = threadIdx.x & 31, sl = lane & 7, rr = lane >> 3;
   const int ntiles = (N + 3) / 4;
   const int nwarps = (int)(gridDim.x * blockDim.x) >> 5;
@@ -1106,8 +1133,11 @@ __global__ void __launch_bounds__(kSweepThreads) sweep_diag_kernel(const T *__re
 // (y, z and the tickets); err: a word that is zero.
 template <typename T>
 int lu_solve_sweep(int N, int nb, const T *A, size_t lda, T *B, int nrhs, T *X, unsigned *err, cudaStream_t st) {
-  if (nb % kSweepRows || nb > 128) return lu_solve_small<T>(N, nb, A, lda, B, N, nrhs, X, st);
-  const int ntiles = (N + kSweepRows - 1) / kSweepRows;
+  if (nb % kSweepRows || nb > 128) {
+    set_error("substitution sweeps: block size %d not supported", nb);
+    return QPMS_EINVAL;
+  }
+  const int ntiles = (N + kSweepRows - 1) / kSweepRows, nch = (nrhs + kSmallRhs - 1) / kSmallRhs;
   int dev = 0, sms = 0;
   QG_CUDA_TRY(cudaGetDevice(&dev));
   QG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -1116,15 +1146,19 @@ int lu_solve_sweep(int N, int nb, const T *A, size_t lda, T *B, int nrhs, T *X, 
   T *Y = X + n, *Z = Y + n;
   unsigned *ticket = (unsigned *)(Z + n);
   QG_CUDA_TRY(cudaMemsetAsync(Y, 0xff, 2 * n * sizeof(T) + 2 * sizeof(unsigned), st));
-  // two CTAs per SM: three and four change nothing at 3,000 to 14,400 unknowns
-  const int grid = std::min(ntiles, 2 * sms);
-  auto fwd = nrhs == 1 ? sweep_fwd_kernel<T, 1> : sweep_fwd_kernel<T, kSmallRhs>;
-  auto bwd = nrhs == 1 ? sweep_bwd_kernel<T, 1> : sweep_bwd_kernel<T, kSmallRhs>;
+  // one chunk: two CTAs per SM (three and four change nothing at 3,000 to 14,400
+  // unknowns); several: four (32 columns at 5,776 unknowns, six contour nodes: 65.0 ms
+  // with two, 64.2 with four)
+  const int grid = std::min(ntiles * nch, (nch > 1 ? 4 : 2) * sms);
+  auto fwd = nrhs == 1 ? sweep_fwd_kernel<T, 1> : nrhs == 2 ? sweep_fwd_kernel<T, 2>
+             : nrhs <= 4 ? sweep_fwd_kernel<T, 4> : sweep_fwd_kernel<T, kSmallRhs>;
+  auto bwd = nrhs == 1 ? sweep_bwd_kernel<T, 1> : nrhs == 2 ? sweep_bwd_kernel<T, 2>
+             : nrhs <= 4 ? sweep_bwd_kernel<T, 4> : sweep_bwd_kernel<T, kSmallRhs>;
   fwd<<<grid, kSweepThreads, 0, st>>>(A, lda, N, nb, B, Y, (size_t)N, nrhs, ticket, err);
   QG_CUDA_TRY(cudaGetLastError());
   bwd<<<grid, kSweepThreads, 0, st>>>(A, lda, N, nb, Y, Z, (size_t)N, nrhs, ticket + 1, err);
   QG_CUDA_TRY(cudaGetLastError());
-  sweep_diag_kernel<T><<<std::min((N + 15) / 16, 8 * sms), kSweepThreads, 0, st>>>(A, lda, N, nb, Z, X, (size_t)N, nrhs);
+  sweep_diag_kernel<T><<<dim3(std::min((N + 15) / 16, 8 * sms), nch), kSweepThreads, 0, st>>>(A, lda, N, nb, Z, X, (size_t)N, nrhs);
   QG_CUDA_TRY(cudaGetLastError());
   g_launches.fetch_add(3);
   return QPMS_SUCCESS;
@@ -1137,6 +1171,30 @@ int env_choice(const char *name, const char *yes, const char *no) {
   if (e && !strcmp(e, yes)) return 1;
   if (e && !strcmp(e, no)) return 0;
   return -1;
+}
+
+// Few right-hand sides: one launch per sweep; QPMS_GB300_SUBST=steps takes one
+// launch per block and sweep instead (a serving mix of 24 requests with 8 workers:
+// sweeps 81.2 ms, steps 83.3 ms).
+bool sweeps_chosen() {
+  static const int v = env_choice("QPMS_GB300_SUBST", "sweep", "steps");
+  return v != 0;
+}
+// Most right-hand sides that the complex64 factors of the tensor-core LU take as
+// sweeps.  The sweeps are FP32 FMAs by chunks of eight columns, the alternative two
+// tensor-core products of digit planes per block: many columns pay for its chain,
+// and the chain is short where there are few blocks.  Six contour nodes, two at a
+// time, products : sweeps: 2,400 unknowns with 12 columns 18.5 : 14.8 ms, 32
+// 21.2 : 18.2, 64 24.4 : 22.6; 5,776 with 12 columns 58.3 : 50.3, 32 67.6 : 64.2, 48
+// 74.1 : 75.1, 64 78.8 : 83.9.  One solve with 128 columns at 1,600 unknowns
+// 4.90 : 4.34, at 5,776 26.8 : 28.1; with 32 at 14,400 110.0 : 103.5.
+int sweep_rhs_limit(int Np) { return std::max(32, std::min(128, 200000 / std::max(Np, 1))); }
+// y, z and the tickets of lu_solve_sweep behind its result
+size_t sweep_scratch(int Np, int nrhs_max, int mode) {
+  const int n = std::min(nrhs_max, mode ? sweep_rhs_limit(Np) : kSmallRhs);
+  // a mixed solver's complex128 fallback sweeps up to kSmallRhs
+  const size_t e = std::max<size_t>((size_t)n * (mode ? 8 : 16), (size_t)std::min(n, kSmallRhs) * 16);
+  return 3 * (size_t)Np * e + 2 * sizeof(unsigned);
 }
 
 }  // namespace
@@ -1241,6 +1299,7 @@ int DenseSolver::init(int N_, int nrhs_max_, int mode_, unsigned long long seed,
   // a mixed solver that falls back to complex128 factors uses the same work
   // buffer for nb = 64 complex128 column blocks (N x 64 x 16 bytes)
   if (mode) wsz = std::max<size_t>(wsz, (size_t)std::max(Np, nrhs_max) * 64 * 16);
+  wsz = std::max(wsz, sweep_scratch(Np, nrhs_max, mode));
   // K up to group x nb: the combined update of a group of blocks
   const int kmax = lu_group() * nb;
   // one allocation for all buffers that every solver of this mode has (each by
@@ -1286,7 +1345,7 @@ int DenseSolver::init(int N_, int nrhs_max_, int mode_, unsigned long long seed,
   // many right-hand sides on the tensor cores: the factors' digit planes, cut
   // once per factorisation instead of per substitution step (skipped when
   // they do not fit: the steps then cut their panels themselves)
-  if (tc_split && nrhs_max > kSmallRhs && fac_planes_wanted()) {
+  if (tc_split && fac_planes_wanted(Np, nrhs_max)) {
     if (dev_alloc(&fac_planes, tc_planes_bytes_a(Np, Np, 3)) != cudaSuccess) {
       cudaGetLastError();
       fac_planes = nullptr;
@@ -1321,17 +1380,18 @@ size_t DenseSolver::footprint(int N, int nrhs, int mode) {
   size_t b = (mode ? Np * Np * esz : Np * Np * 16) + nblk * 2 * nb * nb * esz;
   b += std::max<size_t>(std::max<size_t>(Np * nb, nb * std::max<size_t>(Np, nrhs)) * esz,
                         mode ? std::max<size_t>(Np, nrhs) * 64 * 16 : 0);
+  b += sweep_scratch((int)Np, nrhs, mode);
   b += Np * nrhs * (8 + 16) + (size_t)N * nrhs * 32 + 16 + 4 * Np * 8 + 2 * kOzakiMinRhs * 8;
   b += sizeof(unsigned);
   if (ozaki_wanted(nrhs)) b += ozaki_matrix_bytes(N) + ozaki_work_bytes(N, nrhs);
   if (mode && tc_digits(nrhs)) b += tc_plane_bytes((int)Np, nrhs, kMaxLuGroup * (int)nb);
-  if (mode && tc_digits(nrhs) && nrhs > kSmallRhs && fac_planes_wanted()) b += tc_planes_bytes_a((int)Np, (int)Np, 3);
+  if (mode && tc_digits(nrhs) && fac_planes_wanted((int)Np, nrhs)) b += tc_planes_bytes_a((int)Np, (int)Np, 3);
   return b + 13 * 512;  // allocation rounding
 }
 
-bool fac_planes_wanted() {
+bool fac_planes_wanted(int Np, int nrhs_max) {
   static const int v = env_choice("QPMS_GB300_FACTOR_PLANES", "1", "0");
-  return v != 0;
+  return v != 0 && nrhs_max > (sweeps_chosen() ? sweep_rhs_limit(Np) : kSmallRhs);
 }
 
 bool ozaki_wanted(int nrhs_max) {
@@ -1524,12 +1584,10 @@ int DenseSolver::factor_launch(const void *M64, size_t ldm, cudaStream_t st) {
                            CUBLAS_COMPUTE_64F, st);
 }
 
-// Few right-hand sides: one launch per sweep; QPMS_GB300_SUBST=steps takes one
-// launch per block and sweep instead (a serving mix of 24 requests with 8 workers:
-// sweeps 81.2 ms, steps 83.3 ms).
-bool DenseSolver::use_sweeps() const {
-  static const int v = env_choice("QPMS_GB300_SUBST", "sweep", "steps");
-  return v != 0;
+// The substitutions of nrhs right-hand sides as sweeps?  The complex64 factors of
+// the tensor-core LU up to sweep_rhs_limit, everything else up to kSmallRhs.
+bool DenseSolver::use_sweeps(int nrhs) const {
+  return sweeps_chosen() && nrhs <= (mode && tc_split ? sweep_rhs_limit(Np) : kSmallRhs);
 }
 int DenseSolver::lu_group() const {
   static const int v = [] {
@@ -1582,11 +1640,11 @@ int DenseSolver::apply_launch(const void *R, size_t ldr, void *Y, size_t ldy, in
     QG_CUDA_TRY(cudaGetLastError());
     g_launches.fetch_add(1);
     const float2 *sol = (const float2 *)rhs_lo;
-    if (nrhs <= kSmallRhs) {
-      e = !use_sweeps() ? lu_solve_small<float2>(Np, nb, (const float2 *)A, Np, (float2 *)rhs_lo, Np, nrhs,
-                                                 (float2 *)work, st)
-                        : lu_solve_sweep<float2>(Np, nb, (const float2 *)A, Np, (float2 *)rhs_lo, nrhs,
-                                                 (float2 *)work, sweep, st);
+    if (use_sweeps(nrhs) || nrhs <= kSmallRhs) {
+      e = use_sweeps(nrhs) ? lu_solve_sweep<float2>(Np, nb, (const float2 *)A, Np, (float2 *)rhs_lo, nrhs,
+                                                    (float2 *)work, sweep, st)
+                           : lu_solve_small<float2>(Np, nb, (const float2 *)A, Np, (float2 *)rhs_lo, Np, nrhs,
+                                                    (float2 *)work, st);
       sol = (const float2 *)work;
     } else if (tc_split) {
       e = lu_solve_tc(Np, nb, (const float2 *)A, Np, (float2 *)rhs_lo, Np, nrhs, 3, (__nv_bfloat16 *)tc_pa,
@@ -1601,10 +1659,10 @@ int DenseSolver::apply_launch(const void *R, size_t ldr, void *Y, size_t ldy, in
     g_launches.fetch_add(1);
   } else {
     if (nrhs <= kSmallRhs) {
-      e = !use_sweeps() ? lu_solve_small<double2>(Np, nb, (const double2 *)T64, Np, (double2 *)rp, Np, nrhs,
-                                                  (double2 *)work, st)
-                        : lu_solve_sweep<double2>(Np, nb, (const double2 *)T64, Np, (double2 *)rp, nrhs,
-                                                  (double2 *)work, sweep, st);
+      e = use_sweeps(nrhs) ? lu_solve_sweep<double2>(Np, nb, (const double2 *)T64, Np, (double2 *)rp, nrhs,
+                                                     (double2 *)work, sweep, st)
+                           : lu_solve_small<double2>(Np, nb, (const double2 *)T64, Np, (double2 *)rp, Np, nrhs,
+                                                     (double2 *)work, st);
       if (!e)
         QG_CUDA_TRY(cudaMemcpyAsync(rp, work, n * 16, cudaMemcpyDeviceToDevice, st));
     } else {
@@ -1672,7 +1730,7 @@ int DenseSolver::solve(const void *M64, size_t ldm, const void *B, void *X, int 
     norm2_kernel<<<grid1(n), 256, 0, st>>>(n, (const double2 *)r64, nrm);
     QG_CUDA_TRY(cudaMemcpyAsync(&hr, nrm, 8, cudaMemcpyDeviceToHost, st));
     unsigned sweep_err = 0;
-    if (nrhs <= kSmallRhs) QG_CUDA_TRY(cudaMemcpyAsync(&sweep_err, sweep, 4, cudaMemcpyDeviceToHost, st));
+    if (use_sweeps(nrhs)) QG_CUDA_TRY(cudaMemcpyAsync(&sweep_err, sweep, 4, cudaMemcpyDeviceToHost, st));
     QG_CUDA_TRY(cudaStreamSynchronize(st));
     g_launches.fetch_add(1);
     if (sweep_err) {

@@ -15,9 +15,9 @@ constexpr int kOzakiMinRhs = 8;
 // Largest group of blocks of the tensor-core LU (DenseSolver::group).
 constexpr int kMaxLuGroup = 4;
 bool ozaki_wanted(int nrhs_max);
-// Whether a solver for many right-hand sides keeps the digit planes of its
-// factors (QPMS_GB300_FACTOR_PLANES=0 turns it off).
-bool fac_planes_wanted();
+// Whether a solver for more right-hand sides than the sweeps take keeps the digit
+// planes of its factors (QPMS_GB300_FACTOR_PLANES=0 turns it off).
+bool fac_planes_wanted(int Np, int nrhs_max);
 
 // The system is padded to Np = N rounded up to a multiple of 4 (identity on the
 // padding), the size the two butterfly levels halve.
@@ -109,7 +109,7 @@ struct DenseSolver {
  private:
   cudaError_t dev_alloc(void *ptr, size_t bytes);
   int check_info(cudaStream_t st);  // zero-pivot flag of the last factorisation
-  bool use_sweeps() const;
+  bool use_sweeps(int nrhs) const;
   int lu_group() const;
   int factor_launch(const void *M64, size_t ldm, cudaStream_t st);  // factorize_current's launches
   int apply_launch(const void *R, size_t ldr, void *Y, size_t ldy, int nrhs, cudaStream_t st);

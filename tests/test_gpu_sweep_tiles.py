@@ -1,6 +1,9 @@
 """The one-launch substitution sweeps at the edges of their tiles and blocks:
 last tiles of fewer than 16 rows, one block, last blocks of a few rows, one and
-several right-hand sides, complex64 and complex128 factors.
+several right-hand sides (instances for 1, 2, 4 and 8), more of them by chunks of
+eight with a short last one, both sides of the line to the tensor-core products
+(32 columns, or 200,000 divided by the unknowns up to 128), complex64 and complex128
+factors.
 
 Tolerances: the systems are 2 I plus a random matrix of norm about 2 / sqrt(2),
 and an FP64 refinement takes the residual to 1e-13: within 1e-10 of numpy's.
@@ -25,9 +28,9 @@ def test_sweep_tiles(N, mode):
     rng = np.random.default_rng(N)
     M = (rng.normal(size=(N, N)) + 1j * rng.normal(size=(N, N))) / (2 * np.sqrt(N)) + 2 * np.eye(N)
     tM = torch.from_numpy(M.reshape(-1, order="F").copy()).cuda()
-    Ball = rng.normal(size=(N, 8)) + 1j * rng.normal(size=(N, 8))
+    Ball = rng.normal(size=(N, 131)) + 1j * rng.normal(size=(N, 131))
     ref = np.linalg.solve(M, Ball)
-    for nrhs in (1, 2, 7, 8):
+    for nrhs in (1, 2, 3, 4, 7, 8, 9, 32, 33, 77, 81, 128, 131):
         tB = torch.from_numpy(Ball[:, :nrhs].reshape(-1, order="F").copy()).cuda()
         tX = torch.empty_like(tB)
         res, it = np.zeros(1), np.zeros(1, dtype=np.int32)
