@@ -75,6 +75,18 @@ __device__ __forceinline__ T crcp(T b) {
   return cmk<T>(b.x * s, -b.y * s);
 }
 
+// a / b with r = crcp(b) at hand.  complex64: corrected by the remainder, which
+// makes it as good as a division; complex128: a r, whose results measured the
+// same as a division's.  (Mixed solves of up to 40 unknowns, error after the
+// refinement relative to divisions and tree sums: 1.37 with a r and plain chains,
+// 0.8 to 1.0 with this and RowSum below.)
+template <typename T>
+__device__ __forceinline__ T cquo(T a, T b, T r) {
+  const T q = cmul(a, r);
+  if (sizeof(T) == 16) return q;
+  return cfma(q, cfms(a, q, b), r);
+}
+
 // Pivot search over |Re| + |Im| (LAPACK's izamax measure), first of equals.
 // A key orders candidates as unsigned integers: 0 for a NaN, else the bits of
 // the measure plus one.
@@ -173,7 +185,7 @@ __global__ void __launch_bounds__(kSmallThreads) getrf_small_kernel(int N, T *A_
       if (r < N) {
         T v = r == c ? d : (r == p ? s_old : S[r * LD + c]);
         if (r > c) {
-          if (!zero) v = cmul(v, s_rinv);
+          if (!zero) v = cquo(v, d, s_rinv);
           lcol[r] = v;
         }
         S[r * LD + c] = v;
@@ -348,7 +360,7 @@ __device__ __forceinline__ void factor_panel(int N, int k, int pw, T *Lp, int *p
         for (int i = 0; i < RPT; ++i) {
           const int r = tid + PT * i;
           if (PT * i < rows && r > c) {  // rows past the matrix hold zeros
-            const T l = cmul(a[i][c], rinv);
+            const T l = cquo(a[i][c], u[c], rinv);
             a[i][c] = l;
 #pragma unroll
             for (int j = c + 1; j < PW; ++j) a[i][j] = cfms(a[i][j], l, u[j]);
@@ -542,6 +554,34 @@ __global__ void __launch_bounds__(kThreads) getrf_cluster_kernel(int N, int C, T
 // ---------------- substitutions, one right-hand side ----------------
 // N <= 64: one warp per system, the factors staged in shared memory, lane l
 // holding unknowns l and l + 32.
+// x - sum a b term by term: complex128 as it is, complex64 with the roundings of
+// the products and differences summed beside it, since a lane's chain of up to
+// 63 terms would round more often than a sum over a tree.
+template <typename T>
+struct RowSum {
+  T h;
+  __device__ __forceinline__ explicit RowSum(T b) : h(b) {}
+  __device__ __forceinline__ void sub(T a, T b) { h = cfms(h, a, b); }
+  __device__ __forceinline__ T get() const { return h; }
+};
+template <>
+struct RowSum<float2> {
+  float2 h, l;
+  __device__ __forceinline__ explicit RowSum(float2 b) : h(b), l(make_float2(0, 0)) {}
+  static __device__ __forceinline__ void term(float &h, float &l, float a, float b) {  // h + l -= a b
+    const float p = __fmul_rn(a, b), e = __fmaf_rn(a, b, -p), s = __fsub_rn(h, p), z = __fsub_rn(s, h);
+    l = __fadd_rn(l, __fsub_rn(__fsub_rn(__fsub_rn(h, __fsub_rn(s, z)), __fadd_rn(p, z)), e));
+    h = s;
+  }
+  __device__ __forceinline__ void sub(float2 a, float2 b) {
+    term(h.x, l.x, a.x, b.x);
+    term(h.x, l.x, -a.y, b.y);
+    term(h.y, l.y, a.x, b.y);
+    term(h.y, l.y, a.y, b.x);
+  }
+  __device__ __forceinline__ float2 get() const { return make_float2(h.x + l.x, h.y + l.y); }
+};
+
 template <typename T>
 __global__ void __launch_bounds__(32) getrs_small_kernel(int N, const T *LU_all, const int *piv_all, T *b_all) {
   extern __shared__ __align__(16) unsigned char sm[];
@@ -574,26 +614,26 @@ __global__ void __launch_bounds__(32) getrs_small_kernel(int N, const T *LU_all,
   }
   __syncwarp();
   const T z = cmk<T>(0, 0);
-  T x0 = r0 < N ? xs[r0] : z, x1 = r1 < N ? xs[r1] : z;
+  RowSum<T> x0(r0 < N ? xs[r0] : z), x1(r1 < N ? xs[r1] : z);
   const int q0 = min(r0, N - 1), q1 = min(r1, N - 1);
   const T d0 = crcp(S[q0 * LD + q0]), d1 = N > 32 ? crcp(S[q1 * LD + q1]) : z;
   for (int j = 0; j < N; ++j) {  // L y = P b, unit lower
-    const T y = shfl_c(j < 32 ? x0 : x1, j & 31);
-    if (j < 31 && r0 > j) x0 = cfms(x0, S[q0 * LD + j], y);
-    if (N > 32 && r1 > j) x1 = cfms(x1, S[q1 * LD + j], y);
+    const T y = shfl_c(j < 32 ? x0.get() : x1.get(), j & 31);
+    if (j < 31 && r0 > j) x0.sub(S[q0 * LD + j], y);
+    if (N > 32 && r1 > j) x1.sub(S[q1 * LD + j], y);
   }
   for (int j = N - 1; j >= 0; --j) {  // U x = y
     if (j < 32) {
-      if (r0 == j) x0 = cmul(x0, d0);
+      if (r0 == j) x0 = RowSum<T>(cquo(x0.get(), S[q0 * LD + q0], d0));
     } else if (r1 == j) {
-      x1 = cmul(x1, d1);
+      x1 = RowSum<T>(cquo(x1.get(), S[q1 * LD + q1], d1));
     }
-    const T y = shfl_c(j < 32 ? x0 : x1, j & 31);
-    if (r0 < j) x0 = cfms(x0, S[q0 * LD + j], y);
-    if (j > 32 && r1 < j) x1 = cfms(x1, S[q1 * LD + j], y);
+    const T y = shfl_c(j < 32 ? x0.get() : x1.get(), j & 31);
+    if (r0 < j) x0.sub(S[q0 * LD + j], y);
+    if (j > 32 && r1 < j) x1.sub(S[q1 * LD + j], y);
   }
-  if (r0 < N) b[r0] = x0;
-  if (r1 < N) b[r1] = x1;
+  if (r0 < N) b[r0] = x0.get();
+  if (r1 < N) b[r1] = x1.get();
 }
 
 // Above: one CTA per system, blocks of 32 unknowns.  Warp 0 solves a block's
@@ -677,7 +717,7 @@ __global__ void __launch_bounds__(kRsThreads) getrs_block_kernel(int N, const T 
       } else {
         const T di = dinv[i0 + r];
         for (int j = bs - 1; j >= 0; --j) {
-          if (r == j) v = cmul(v, di);
+          if (r == j) v = cquo(v, tl[r][r], di);
           const T y = shfl_c(v, j);
           if (r < j) v = cfms(v, tl[r][j], y);
         }
