@@ -532,9 +532,13 @@ def _trans_bytes(nvec, lMax):
 
 
 def _trans_flops(lMax):
+    """FP64 flops of one translation's dot products, two FMAs per nonzero real
+    coefficient x complex term; elements (n, m; nu, mu) and (nu, -mu; n, -m) share
+    one dot product (an element with n = nu, m = -mu is its own partner)."""
     from qpms_gb300.translations import multipliers_export
     A, B = multipliers_export(lMax)
-    return 4 * (A.size + B.size)  # two FP64 FMAs per real-coefficient x complex term
+    own = sum(2 * (n - abs(m)) + 1 for n in range(1, lMax + 1) for m in range(-n, n + 1))
+    return 2 * (int(np.count_nonzero(A)) + int(np.count_nonzero(B)) + own)
 
 
 def section_translation(args):
@@ -695,7 +699,7 @@ def section_dispersion(args):
                 d[name]["kernels_ms"] = {k: v[0] for k, v in kt.items()}
                 if "ewald" in kt:
                     ms, work, n = kt["ewald"]
-                    d["roofline"] = {"bound": "fp64", "kernel": "ewald_assemble_kernel<3> (+ sr table)",
+                    d["roofline"] = {"bound": "fp64", "kernel": "ewald_scan_kernel<3> (+ sr table)",
                                      "ms": ms, "launches": n, "share_of_scan": ms / (dt * 1e3),
                                      "note": "FP64-pipe bound (special functions per lattice point); "
                                              "output bytes %.2f GB/s" % (work / (ms * 1e-3) / 1e9)}

@@ -11,8 +11,8 @@
 //      randomization techniques", ACM TOMS 39 (2013)), after which Gaussian
 //      elimination without pivoting is stable with high probability;
 //   2. factorises A' without pivoting by blocks in Schur-complement form: at
-//      step k the nb x nb diagonal block D is inverted by one CTA
-//      (Gauss-Jordan in registers), the whole column block k is multiplied
+//      step k the nb x nb diagonal block D is inverted by a cluster of
+//      four CTAs (Gauss-Jordan in registers), the whole column block k is multiplied
 //      by D^-1 (below the block this is P = A21 D^-1, above it
 //      Q = A_0:k,k D^-1, the block itself becomes I - D^-1) and the trailing
 //      matrix is updated, A22 -= P A12, with the row panel A12 kept as it is;

@@ -48,13 +48,17 @@
 //  * eta is lowered to 1 / |w| where eta |w| > 1, which keeps the cancellation
 //    in the series below e^2 (the sums do not depend on eta);
 //  * distant layers, |k w| >= 2.5 (where eta <= 1 / |w| would let the short-
-//    and long-range parts cancel by e^(k^2 / 4 eta^2)): the eta -> infinity
+//    and long-range parts cancel by e^(k^2 / 4 eta^2)), and nearer ones whose
+//    reciprocal points are few enough (spectral_passes): the eta -> infinity
 //    limit, a pure reciprocal-lattice sum (no short range) with
 //    Delta_j(0, z) = 2 (a/2)^(1/2-j) K_(j-1/2)(a), a = gamma k |w|, in closed
 //    form by the half-integer Bessel K recurrence; it converges like
 //    e^(-|beta + K| |w|);
 //  * the (n, m) accumulators are split into passes of at most 36 entries to
 //    stay in registers.
+//
+// Scans at real wavenumbers with their short-range terms in tables take
+// ewald_scan_kernel, which keeps real what is real there.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>

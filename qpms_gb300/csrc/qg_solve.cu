@@ -2,8 +2,8 @@
 // pipeline (assembly -> incident field -> T a -> LU solve -> sigma_ext).
 //
 // Two solve modes for the batched pipeline:
-//   mode 0 ("plain FP64"): complex128 LU with partial pivoting (cuBLAS
-//          getrf/getrs batched) -- the plain FP64 GPU path;
+//   mode 0 ("plain FP64"): complex128 LU with partial pivoting (the batched
+//          LU of qg_batchlu.cu up to 512 unknowns, the dense solver above);
 //   mode 1 ("mixed"):      complex64 LU of the same matrices, then FP64
 //          iterative refinement x += LU64^{-1} (b - M x) with the residual
 //          formed in FP64 from the FP64 matrix, until ||b - M x|| / ||b||
