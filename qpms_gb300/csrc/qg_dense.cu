@@ -896,7 +896,7 @@ int lu_solve_small(int N, int nb, const T *A, size_t lda, T *B, size_t ldb, int 
 // Measured (counters released after a fence, a warp per tile of 4 rows, before ->
 // now): one mixed solve, three pairs of sweeps, 1,000 unknowns 1.35 -> 1.24 ms,
 // 3,000 3.51 -> 3.12, 6,000 8.59 -> 7.69, 14,400 41.8 -> 39.7; 8 right-hand sides at
-// 6,000 20.9 -> 16.7 ms.
+// 6,000 20.9 -> 16.7 ms.  A sweep at 8,192 unknowns 345 -> 143 us, 2.2 us a hop.
 constexpr int kSweepRows = 16, kSweepThreads = 128;
 // complex64, one right-hand side: at most 102 registers, so that a sweep CTA fits
 // on an SM beside a tensor-core GEMM CTA (320 threads x 160 registers)
