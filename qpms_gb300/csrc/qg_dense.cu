@@ -1378,9 +1378,8 @@ size_t DenseSolver::footprint(int N, int nrhs, int mode) {
   const size_t Np = (size_t)(N + 3) / 4 * 4, nb = mode ? 128 : 64, esz = mode ? 8 : 16;
   const size_t nblk = (Np + nb - 1) / nb;
   size_t b = (mode ? Np * Np * esz : Np * Np * 16) + nblk * 2 * nb * nb * esz;
-  b += std::max<size_t>(std::max<size_t>(Np * nb, nb * std::max<size_t>(Np, nrhs)) * esz,
-                        mode ? std::max<size_t>(Np, nrhs) * 64 * 16 : 0);
-  b += sweep_scratch((int)Np, nrhs, mode);
+  b += std::max({std::max<size_t>(Np * nb, nb * std::max<size_t>(Np, nrhs)) * esz,
+                 mode ? std::max<size_t>(Np, nrhs) * 64 * 16 : 0, sweep_scratch((int)Np, nrhs, mode)});
   b += Np * nrhs * (8 + 16) + (size_t)N * nrhs * 32 + 16 + 4 * Np * 8 + 2 * kOzakiMinRhs * 8;
   b += sizeof(unsigned);
   if (ozaki_wanted(nrhs)) b += ozaki_matrix_bytes(N) + ozaki_work_bytes(N, nrhs);
