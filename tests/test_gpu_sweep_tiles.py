@@ -40,3 +40,43 @@ def test_sweep_tiles(N, mode):
         X = tX.cpu().numpy().reshape((N, nrhs), order="F")
         assert np.linalg.norm(X - ref[:, :nrhs]) <= 1e-10 * np.linalg.norm(ref[:, :nrhs])
         assert res[0] <= 1e-12 and it[0] <= (5 if mode else 2)
+
+
+_CHILD = r"""
+import sys, numpy as np, torch
+sys.path.insert(0, sys.argv[1])
+import qpms_gb300
+N, nrhs = 1500, 136
+rng = np.random.default_rng(7)
+M = (rng.normal(size=(N, N)) + 1j * rng.normal(size=(N, N))) / (2 * np.sqrt(N)) + 2 * np.eye(N)
+B = rng.normal(size=(N, nrhs)) + 1j * rng.normal(size=(N, nrhs))
+tM, tB = (torch.from_numpy(a.reshape(-1, order="F").copy()).cuda() for a in (M, B))
+tX = torch.empty_like(tB)
+res, it = np.zeros(1), np.zeros(1, dtype=np.int32)
+rc = qpms_gb300.lib().qpms_gpu_dense_solve(N, nrhs, tM.data_ptr(), tB.data_ptr(), tX.data_ptr(), 1,
+                                           res.ctypes.data, it.ctypes.data)
+assert rc == 0, qpms_gb300.last_error()
+X = tX.cpu().numpy().reshape((N, nrhs), order="F")
+ref = np.linalg.solve(M, B)
+assert np.linalg.norm(X - ref) <= 1e-10 * np.linalg.norm(ref) and it[0] <= 5
+np.save(sys.argv[2], X)
+"""
+
+
+def test_products_past_the_line(tmp_path):
+    """136 columns at 1,500 unknowns take the tensor-core products: the factors'
+    digit planes cut once give bit for bit the result of cutting each step's panel."""
+    import os
+    import subprocess
+    import sys
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = []
+    for flag in ("1", "0"):
+        f = str(tmp_path / ("x%s.npy" % flag))
+        subprocess.run([sys.executable, "-c", _CHILD, root, f], env=dict(os.environ, QPMS_GB300_FACTOR_PLANES=flag),
+                       check=True, timeout=600)
+        out.append(np.load(f))
+    assert np.array_equal(out[0], out[1])
