@@ -703,24 +703,26 @@ static void sigma_long_z(const e3c_t *c, int csphase, double complex *target, do
  * outgoing for the branch of gamma above), so
  *   gamma^(2j-1) Delta_j = sqrt(pi) 2^j (k|z|)^-j e^-a gamma^(j-1) kappa_j(a),
  * kappa_j = sqrt(2a/pi) e^a K_(j-1/2)(a) (kappa_0 = kappa_1 = 1,
- * kappa_(j+1) = kappa_(j-1) + (2j - 1) kappa_j / a).  Converges like
- * e^(-|beta + K| |z|). */
+ * kappa_(j+1) = kappa_(j-1) + (2j - 1) kappa_j / a).  An order decays as
+ * e^(-sqrt(|beta + K|^2 - k^2) |z|), the propagating ones not at all: all orders
+ * up to |beta + K|^2 = (Re k)^2 + (80 / |z|)^2 are taken. */
 static void sigma_spectral_z(const e3c_t *c, int csphase, double complex *target, double complex k, double A,
                              orc_c2 rb1, orc_c2 rb2, orc_c2 beta, orc_c2 shift, double shift_z) {
   const int nelem_sc = c->nelem_sc, lMax = c->lMax;
   double complex *tc = calloc(nelem_sc, sizeof(double complex));
   memset(target, 0, sizeof(double complex) * nelem_sc);
   const double aw = fabs(shift_z);
-  const double maxK = 80.0 / aw + sqrt(dot2(beta, beta));
+  const double maxq = hypot(creal(k), 80.0 / aw), maxK = maxq + sqrt(dot2(beta, beta));
+  const double det = fabs(rb1.x * rb2.y - rb1.y * rb2.x);
+  const long I1 = (long)(maxK * sqrt(dot2(rb2, rb2)) / det), I2 = (long)(maxK * sqrt(dot2(rb1, rb1)) / det);
   const double complex commonfac = 1 / (k * k * A);
   const double complex kw = k * (-shift_z), kaw = k * aw;
-  xyweb g;
-  xyweb_init(&g, rb1, rb2, 1e-13, 0, 1, maxK, 0);
-  orc_c2 K;
   double complex Kt[lMax + 2];
-  while (xyweb_next(&g, &K)) {
+  for (long t = 0; t < (2 * I1 + 1) * (2 * I2 + 1); ++t) {
+    const orc_c2 K = add2(scale2((double)(t % (2 * I1 + 1) - I1), rb1), scale2((double)(t / (2 * I1 + 1) - I2), rb2));
     orc_c2 bK = add2(K, beta);
     const double rbeta = sqrt(dot2(bK, bK));
+    if (rbeta > maxq) continue;
     const double arg = atan2(bK.y, bK.x);
     const double complex phasefac = cexp(I * dot2(K, shift));
     const double complex gamma_pq = clilgamma(rbeta / k);
