@@ -50,10 +50,8 @@
 //  * distant layers, |k w| >= 2.5 (where eta <= 1 / |w| would let the short-
 //    and long-range parts cancel by e^(k^2 / 4 eta^2)), and nearer ones whose
 //    reciprocal points are few enough (spectral_passes): the eta -> infinity
-//    limit, a pure reciprocal-lattice sum (no short range) with
-//    Delta_j(0, z) = 2 (a/2)^(1/2-j) K_(j-1/2)(a), a = gamma k |w|, in closed
-//    form by the half-integer Bessel K recurrence; it converges like
-//    e^(-|beta + K| |w|);
+//    limit, a pure reciprocal-lattice sum of plane waves (no short range), over
+//    every order up to |beta + K|^2 = (Re k)^2 + (C / |w|)^2;
 //  * the (n, m) accumulators are split into passes of at most 36 entries to
 //    stay in registers.
 //
@@ -197,8 +195,11 @@ __device__ __forceinline__ int lr_class(qg_c k, bool kreal, double eta, double r
 // obeys Q_{j+1} = x Q_j - c Q_{j-1}; at x = i sgn(w) gamma it is
 // (i sgn w)^j q_j with q_{j+1} = gamma q_j + c q_{j-1}, a sum of positive real
 // numbers for the evanescent orders of a real k (all but a few), two FP64
-// operations per (n, m).  The terms are taken up to q |w| = C(lMax), past which
-// q^(2 lMax + 1) e^{-q |w|} sums to less than 1e-20 of the whole.
+// operations per (n, m).  An order decays as e^{-Re(gamma k) |w|}, Re(gamma k)
+// >= sqrt(q^2 - (Re k)^2), and propagating orders do not decay: the orders up to
+// q^2 = (Re k)^2 + (C(lMax) / |w|)^2 are taken.  Past it the terms
+// (q / k)^(2 lMax + 1) e^{-gamma k |w|} sum to less than 1e-20 of the whole at
+// any k |w| (near planes are the worst: q |w| near 2 lMax + 1 carries the sum).
 //
 // Bound: the FP64 pipe, about 220 operations per reciprocal point at lMax 2
 // against some 2,700 for Kambe's double sum over (j, s) at each point.
@@ -1540,7 +1541,7 @@ __global__ void __launch_bounds__(kEThreads) ewald_layers_kernel(EwaldArgs a, Tr
     // eta <= 1 / |sz| for the Delta series, which keeps k / (2 eta) <= 1.25.  A scan of
     // 100 (omega, k), reciprocal sum against Ewald (ms): lMax 2, 4,752 points 1.62 : 1.57,
     // 7,425 1.99 : 1.56; lMax 4, 6,236 4.57 : 4.72, 17,324 8.9 : 6.0.
-    const double pcut = SpecShape<LMAX>::kCut / fabs(sz);
+    const double pcut = hypot(k.re, SpecShape<LMAX>::kCut / sz);
     const bool spectral = hypot(k.re, k.im) * fabs(sz) >= 2.5 || pcut * pcut * c_ew.area <= kSpecPoints * 4 * M_PI;
     if (spectral) {
       SpecUnit su;
