@@ -196,7 +196,10 @@ struct FiniteSource : MSource {
       opos = in->upload(pos.data(), pos.size() * 8);
       oT = in->add(T.size() * 16);
       ok = in->add(16);
-      if ((e = in->alloc(st))) return e;
+      if ((e = in->alloc(st))) {
+        in.reset();
+        return e;
+      }
     }
     const size_t N = ss->fecv_size;
     if (iri >= 0 && !full) QG_CUDA_TRY(cudaMalloc(&full, N * N * 16));
@@ -360,19 +363,15 @@ int beyn_quadrature(MSource &src, beyn_function_M_inv_Vhat_t minv, void *minv_pa
     return QPMS_ERROR;
   }
   // lanes of nodes, each with a source, solver, stream and sums of its own
-  int lanes = 1;
+  int most = 1;
   std::vector<std::unique_ptr<MSource>> clones;
-  if (!minv && mode == 1 && ne - nb > 1) {
-    lanes = lanes_that_fit((int)std::min<size_t>(kBeynLanes, ne - nb),
-                           m * m * 16 + DenseSolver::footprint((int)m, (int)l, mode) + 5 * nml * 16);
-    for (int i = 1; i < lanes; ++i) {
+  if (!minv && mode == 1)
+    for (; most < kBeynLanes && (size_t)most < ne - nb; ++most) {
       clones.emplace_back(src.clone());
-      if (!clones.back()) {
-        clones.clear();
-        lanes = 1;
-      }
+      if (!clones.back()) break;
     }
-  }
+  LaneGrant grant(most, m * m * 16 + DenseSolver::footprint((int)m, (int)l, mode) + 5 * nml * 16);
+  const int lanes = grant.lanes();
   struct Sums {
     DevPtr dX, dA[4];
     double max_res = 0;
@@ -397,18 +396,22 @@ int beyn_quadrature(MSource &src, beyn_function_M_inv_Vhat_t minv, void *minv_pa
     }
     const cudaStream_t st = ns.s;
     Sums &S = sums[lane];
-    if (cudaMalloc(&S.dX.p, nml * 16) != cudaSuccess) {
+    // what a lane that starts over has allocated already is taken again
+    if (!S.dX.p && cudaMalloc(&S.dX.p, nml * 16) != cudaSuccess) {
       set_error("Beyn: out of device memory (m = %zu, l = %zu)", m, l);
       return QPMS_ENOMEM;
     }
     for (auto &a : S.dA)
-      if (cudaMalloc(&a.p, nml * 16) != cudaSuccess || cudaMemsetAsync(a.p, 0, nml * 16, st) != cudaSuccess) {
+      if ((!a.p && cudaMalloc(&a.p, nml * 16) != cudaSuccess) ||
+          cudaMemsetAsync(a.p, 0, nml * 16, st) != cudaSuccess) {
         set_error("Beyn: out of device memory (m = %zu, l = %zu)", m, l);
         return QPMS_ENOMEM;
       }
+    S.max_res = 0;
+    S.max_it = 0;
     MSource &so = lane ? *clones[lane - 1] : src;
     int e;
-    if (lane && (e = so.init_stage())) return e;
+    if (lane && !so.stage && (e = so.init_stage())) return e;
     DenseSolver ds;
     if (!minv && (e = ds.init((int)m, (int)l, mode, seed ^ 0x9e3779b97f4a7c15ULL, nullptr, st))) return e;
     ds.graphs = true;
@@ -452,7 +455,7 @@ int beyn_quadrature(MSource &src, beyn_function_M_inv_Vhat_t minv, void *minv_pa
     return QPMS_SUCCESS;
   };
   int e;
-  if ((e = run_lanes(lanes, run))) return e;
+  if ((e = run_lanes(grant, run))) return e;
   for (int i = 1; i < lanes; ++i) {  // in the lanes' order
     for (int c = 0; c < 4; ++c)
       beyn_add_kernel<<<grid1(nml), 256>>>(nml, (const double2 *)sums[i].dA[c].p, (double2 *)sums[0].dA[c].p);

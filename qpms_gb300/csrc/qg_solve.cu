@@ -118,7 +118,8 @@ int finite_scatter_dense(const qpms_scatsys_t *ss, int W, const std::vector<qg_c
   size_t namax = 0;
   for (int i = 0; i < nir; ++i) namax = std::max(namax, sym_size(ss, i));
   // the complex128 path fills the GPU by itself
-  const int lanes = nir == 0 && mode == 1 ? lanes_that_fit(scatter_lanes(N, W), N2 * 16 + DenseSolver::footprint((int)N, 1, 1)) : 1;
+  LaneGrant grant(nir == 0 && mode == 1 ? scatter_lanes(N, W) : 1, N2 * 16 + DenseSolver::footprint((int)N, 1, 1));
+  const int lanes = grant.lanes();
   if (lanes > 1) QG_CUDA_TRY(cudaStreamSynchronize(0));  // the inputs are there for every lane's stream
   auto run = [&](int lane) -> int {
     LaneStream ls;
@@ -214,7 +215,7 @@ int finite_scatter_dense(const qpms_scatsys_t *ss, int W, const std::vector<qg_c
     }
     return QPMS_SUCCESS;
   };
-  return run_lanes(lanes, run);
+  return run_lanes(grant, run);
 }
 
 }  // namespace
