@@ -362,24 +362,83 @@ int beyn_quadrature(MSource &src, beyn_function_M_inv_Vhat_t minv, void *minv_pa
     set_error("Beyn: host to device copy failed");
     return QPMS_ERROR;
   }
-  // lanes of nodes, each with a source, solver, stream and sums of its own
-  int most = 1;
+  // Every kBeynLanes-th node adds to one of kBeynLanes sums, on however many
+  // lanes: each lane, with a source, solver and stream of its own, takes whole
+  // sums, so the result does not depend on how many fit the free memory.
+  int nsums = 1;
   std::vector<std::unique_ptr<MSource>> clones;
   if (!minv && mode == 1)
-    for (; most < kBeynLanes && (size_t)most < ne - nb; ++most) {
+    for (; nsums < kBeynLanes && (size_t)nsums < ne - nb; ++nsums) {
       clones.emplace_back(src.clone());
       if (!clones.back()) break;
     }
-  LaneGrant grant(most, m * m * 16 + DenseSolver::footprint((int)m, (int)l, mode) + 5 * nml * 16);
+  LaneGrant grant(nsums, m * m * 16 + DenseSolver::footprint((int)m, (int)l, mode) + 5 * nml * 16);
   const int lanes = grant.lanes();
   struct Sums {
-    DevPtr dX, dA[4];
+    DevPtr dA[4];
     double max_res = 0;
     int max_it = 0;
   };
-  std::vector<Sums> sums(lanes);
+  std::vector<Sums> sums(nsums);
   const cd z0 = to_cd(contour->centre);
   if (lanes > 1) QG_CUDA_TRY(cudaStreamSynchronize(0));  // dV is there for every lane's stream
+  // the nodes of sum j
+  auto add_nodes = [&](int j, MSource &so, cudaStream_t st) -> int {
+    Sums &S = sums[j];
+    DevPtr dX;
+    bool memory = cudaMalloc(&dX.p, nml * 16) == cudaSuccess;
+    for (auto &a : S.dA)  // there already where the lane starts over
+      memory = memory && (a.p || cudaMalloc(&a.p, nml * 16) == cudaSuccess) &&
+               cudaMemsetAsync(a.p, 0, nml * 16, st) == cudaSuccess;
+    if (!memory) {
+      set_error("Beyn: out of device memory (m = %zu, l = %zu)", m, l);
+      return QPMS_ENOMEM;
+    }
+    S.max_res = 0;
+    S.max_it = 0;
+    int e;
+    DenseSolver ds;
+    if (!minv && (e = ds.init((int)m, (int)l, mode, seed ^ 0x9e3779b97f4a7c15ULL, nullptr, st))) return e;
+    ds.graphs = true;
+    std::vector<qpms_complex_t> hx;
+    for (size_t i = nb + j; i < ne; i += nsums) {
+      const cd z = to_cd(contour->z_dz[i][0]), dz = to_cd(contour->z_dz[i][1]);
+      if (minv) {  // user-supplied M(z)^-1 Vhat (row-major m x l)
+        hx.resize(nml);
+        const int rc = minv(hx.data(), m, l, (const qpms_complex_t *)Vh.data(), from_cd(z), minv_params);
+        if (rc) {
+          set_error("M^-1 Vhat callback returned %d", rc);
+          return rc;
+        }
+        for (size_t r = 0; r < m; ++r)
+          for (size_t c = 0; c < l; ++c) Vc[r + c * m] = to_cd(hx[r * l + c]);
+        if (cudaMemcpy(dX.p, Vc.data(), nml * 16, cudaMemcpyHostToDevice) != cudaSuccess) {
+          set_error("Beyn: host to device copy failed");
+          return QPMS_ERROR;
+        }
+      } else {
+        double res = 0;
+        int it = 0;
+        if ((e = so.build_rowmajor(z, st))) return e;
+        // the staged row-major M(z) goes straight to the solver (transposed on the fly)
+        if ((e = ds.factorize(so.stage, m, st, true))) return e;
+        if ((e = ds.solve(so.stage, m, dV.p, dX.p, (int)l, refine_tol, kMaxRefine, &res, &it, st))) return e;
+        if (!(res <= S.max_res)) S.max_res = res;  // NaN-propagating max
+        if (it > S.max_it) S.max_it = it;
+      }
+      beyn_accumulate_kernel<<<grid1(nml), 256, 0, st>>>(
+          nml, (const double2 *)dX.p, make_double2(dz.real(), dz.imag()),
+          make_double2((z - z0).real(), (z - z0).imag()), (i % 2) == 0, (double2 *)S.dA[0].p, (double2 *)S.dA[1].p,
+          (double2 *)S.dA[2].p, (double2 *)S.dA[3].p);
+      if (cudaGetLastError() != cudaSuccess) {
+        set_error("Beyn: accumulation kernel launch failed");
+        return QPMS_ERROR;
+      }
+      g_launches.fetch_add(1);
+    }
+    QG_CUDA_TRY(cudaStreamSynchronize(st));
+    return QPMS_SUCCESS;
+  };
   auto run = [&](int lane) -> int {
     // the nodes run on a stream of their own, so that the solver's repeated
     // launch sequences can be captured as CUDA graphs and replayed node after
@@ -394,69 +453,15 @@ int beyn_quadrature(MSource &src, beyn_function_M_inv_Vhat_t minv, void *minv_pa
       set_error("Beyn: stream creation failed");
       return QPMS_ERROR;
     }
-    const cudaStream_t st = ns.s;
-    Sums &S = sums[lane];
-    // what a lane that starts over has allocated already is taken again
-    if (!S.dX.p && cudaMalloc(&S.dX.p, nml * 16) != cudaSuccess) {
-      set_error("Beyn: out of device memory (m = %zu, l = %zu)", m, l);
-      return QPMS_ENOMEM;
-    }
-    for (auto &a : S.dA)
-      if ((!a.p && cudaMalloc(&a.p, nml * 16) != cudaSuccess) ||
-          cudaMemsetAsync(a.p, 0, nml * 16, st) != cudaSuccess) {
-        set_error("Beyn: out of device memory (m = %zu, l = %zu)", m, l);
-        return QPMS_ENOMEM;
-      }
-    S.max_res = 0;
-    S.max_it = 0;
     MSource &so = lane ? *clones[lane - 1] : src;
-    int e;
+    int e = QPMS_SUCCESS;
     if (lane && !so.stage && (e = so.init_stage())) return e;
-    DenseSolver ds;
-    if (!minv && (e = ds.init((int)m, (int)l, mode, seed ^ 0x9e3779b97f4a7c15ULL, nullptr, st))) return e;
-    ds.graphs = true;
-    std::vector<qpms_complex_t> hx;
-    for (size_t i = nb + lane; i < ne; i += lanes) {
-      const cd z = to_cd(contour->z_dz[i][0]), dz = to_cd(contour->z_dz[i][1]);
-      if (minv) {  // user-supplied M(z)^-1 Vhat (row-major m x l)
-        hx.resize(nml);
-        const int rc = minv(hx.data(), m, l, (const qpms_complex_t *)Vh.data(), from_cd(z), minv_params);
-        if (rc) {
-          set_error("M^-1 Vhat callback returned %d", rc);
-          return rc;
-        }
-        for (size_t r = 0; r < m; ++r)
-          for (size_t c = 0; c < l; ++c) Vc[r + c * m] = to_cd(hx[r * l + c]);
-        if (cudaMemcpy(S.dX.p, Vc.data(), nml * 16, cudaMemcpyHostToDevice) != cudaSuccess) {
-          set_error("Beyn: host to device copy failed");
-          return QPMS_ERROR;
-        }
-      } else {
-        double res = 0;
-        int it = 0;
-        if ((e = so.build_rowmajor(z, st))) return e;
-        // the staged row-major M(z) goes straight to the solver (transposed on the fly)
-        if ((e = ds.factorize(so.stage, m, st, true))) return e;
-        if ((e = ds.solve(so.stage, m, dV.p, S.dX.p, (int)l, refine_tol, kMaxRefine, &res, &it, st))) return e;
-        if (!(res <= S.max_res)) S.max_res = res;  // NaN-propagating max
-        if (it > S.max_it) S.max_it = it;
-      }
-      beyn_accumulate_kernel<<<grid1(nml), 256, 0, st>>>(
-          nml, (const double2 *)S.dX.p, make_double2(dz.real(), dz.imag()),
-          make_double2((z - z0).real(), (z - z0).imag()), (i % 2) == 0, (double2 *)S.dA[0].p, (double2 *)S.dA[1].p,
-          (double2 *)S.dA[2].p, (double2 *)S.dA[3].p);
-      if (cudaGetLastError() != cudaSuccess) {
-        set_error("Beyn: accumulation kernel launch failed");
-        return QPMS_ERROR;
-      }
-      g_launches.fetch_add(1);
-    }
-    QG_CUDA_TRY(cudaStreamSynchronize(st));
-    return QPMS_SUCCESS;
+    for (int j = lane; j < nsums && !e; j += lanes) e = add_nodes(j, so, ns.s);
+    return e;
   };
   int e;
   if ((e = run_lanes(grant, run))) return e;
-  for (int i = 1; i < lanes; ++i) {  // in the lanes' order
+  for (int i = 1; i < nsums; ++i) {
     for (int c = 0; c < 4; ++c)
       beyn_add_kernel<<<grid1(nml), 256>>>(nml, (const double2 *)sums[i].dA[c].p, (double2 *)sums[0].dA[c].p);
     QG_CUDA_TRY(cudaGetLastError());
