@@ -922,6 +922,11 @@ const char *qpms_gpu_last_error(void);
 int qpms_gpu_measure_fp64_peak(double *tflops);
 /* Host evaluation of the library's complex erfc (Weideman Faddeeva), for tests. */
 int qpms_gpu_debug_cerfc(double re, double im, double *out);
+/* The batched pivoted LU and substitution (N <= 512) on the caller's host arrays,
+ * for tests: nm row-major N x N complex128 (is_double) or complex64 matrices A are
+ * replaced with their factors, the nm vectors b with the solutions, piv gets the
+ * 0-based row exchanged with row i at step i. */
+int qpms_gpu_debug_batch_lu(int is_double, int nm, int N, void *A, int *piv, void *b);
 /* Number of kernels this library launched since load (for benchmarks); the
  * launches inside a replayed CUDA graph count as well. */
 unsigned long long qpms_gpu_kernel_launch_count(void);

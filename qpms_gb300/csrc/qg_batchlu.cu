@@ -74,17 +74,29 @@ __device__ __forceinline__ T crcp(T b) {
   const R s = R(1) / fmar(b.x, b.x, b.y * b.y);
   return cmk<T>(b.x * s, -b.y * s);
 }
+// 1 / b with a Newton step.
+template <typename T>
+__device__ __forceinline__ T crcp_near(T b) {
+  typedef typename BL<T>::R R;
+  const T r = crcp(b), e = cfms(cmk<T>(R(1), R(0)), b, r);
+  return cfma(r, r, e);
+}
 
-// a / b with r = crcp(b) at hand.  complex64: corrected by the remainder, which
-// makes it as good as a division; complex128: a r, whose results measured the
-// same as a division's.  (Mixed solves of up to 40 unknowns, error after the
-// refinement relative to divisions and tree sums: 1.37 with a r and plain chains,
-// 0.8 to 1.0 with this and RowSum below.)
+// a / b with r = crcp(b) at hand: a r corrected by the remainder, as good as a
+// division; or a r alone for the complex128 multipliers, which are small against
+// the pivot.  Errors of solves by the two factorisations and substitutions against
+// divisions and tree sums, geometric mean over 200 to 400 matrices I - T S of
+// clusters: complex64 0.93 to 1.01, complex128 0.97 to 1.00, at 12 to 512 unknowns
+// (a r in place of every quotient and plain chains in the substitutions: up to
+// 1.29 and 1.60).
+template <typename T>
+__device__ __forceinline__ T cquo_near(T a, T b, T r) {
+  const T q = cmul(a, r);
+  return cfma(q, cfms(a, q, b), r);
+}
 template <typename T>
 __device__ __forceinline__ T cquo(T a, T b, T r) {
-  const T q = cmul(a, r);
-  if (sizeof(T) == 16) return q;
-  return cfma(q, cfms(a, q, b), r);
+  return sizeof(T) == 16 ? cmul(a, r) : cquo_near(a, b, r);
 }
 
 // Pivot search over |Re| + |Im| (LAPACK's izamax measure), first of equals.
@@ -554,15 +566,43 @@ __global__ void __launch_bounds__(kThreads) getrf_cluster_kernel(int N, int C, T
 // ---------------- substitutions, one right-hand side ----------------
 // N <= 64: one warp per system, the factors staged in shared memory, lane l
 // holding unknowns l and l + 32.
-// x - sum a b term by term: complex128 as it is, complex64 with the roundings of
-// the products and differences summed beside it, since a lane's chain of up to
-// 63 terms would round more often than a sum over a tree.
+// b - sum x y, a term at a time, with no more roundings at the size of b than a
+// sum over a tree: the products are summed apart from b, against which they are
+// small in a mode problem, by K partial sums in turn, term q of K to sum q.
+// get(q): the value after a term q; the other sums are added while term q is
+// formed.  K: at 64 unknowns a general matrix's residual is 1.36 times that of
+// divisions and tree sums with the products taken off b one by one, 1.28 with two
+// sums, 1.13 with four, which cost 50 us of a scan of 4,096 matrices of 30.
+template <typename T, int K>
+struct PartSum {
+  T b, a[K];
+  __device__ __forceinline__ PartSum(T b_, T known) : b(b_) {
+    a[0] = known;
+#pragma unroll
+    for (int i = 1; i < K; ++i) a[i] = cmk<T>(0, 0);
+  }
+  __device__ __forceinline__ void add(int q, T x, T y) { a[q] = cfma(a[q], x, y); }
+  __device__ __forceinline__ T get(int q) const {
+    T s[K];
+#pragma unroll
+    for (int i = 0; i < K - 1; ++i) s[i] = a[i < q ? i : i + 1];
+#pragma unroll
+    for (int n = K - 1; n > 1; n = (n + 1) / 2)
+#pragma unroll
+      for (int i = 0; i < n / 2; ++i) s[i] = cmk<T>(s[i].x + s[n - 1 - i].x, s[i].y + s[n - 1 - i].y);
+    return cmk<T>(b.x - (a[q].x + s[0].x), b.y - (a[q].y + s[0].y));
+  }
+};
+constexpr int kPart = 2;
+
+// The same for the small substitutions: complex128 as above, complex64 with the
+// roundings of the products and differences summed beside them (the error-free
+// transformations of Knuth's TwoSum and of the product by FMA, as in Ogita, Rump
+// and Oishi, Accurate Sum and Dot Product, 2005), since a lane's chain has up to 63
+// terms.
 template <typename T>
-struct RowSum {
-  T h;
-  __device__ __forceinline__ explicit RowSum(T b) : h(b) {}
-  __device__ __forceinline__ void sub(T a, T b) { h = cfms(h, a, b); }
-  __device__ __forceinline__ T get() const { return h; }
+struct RowSum : PartSum<T, kPart> {
+  __device__ __forceinline__ explicit RowSum(T b) : PartSum<T, kPart>(b, cmk<T>(0, 0)) {}
 };
 template <>
 struct RowSum<float2> {
@@ -573,13 +613,13 @@ struct RowSum<float2> {
     l = __fadd_rn(l, __fsub_rn(__fsub_rn(__fsub_rn(h, __fsub_rn(s, z)), __fadd_rn(p, z)), e));
     h = s;
   }
-  __device__ __forceinline__ void sub(float2 a, float2 b) {
+  __device__ __forceinline__ void add(int, float2 a, float2 b) {
     term(h.x, l.x, a.x, b.x);
     term(h.x, l.x, -a.y, b.y);
     term(h.y, l.y, a.x, b.y);
     term(h.y, l.y, a.y, b.x);
   }
-  __device__ __forceinline__ float2 get() const { return make_float2(h.x + l.x, h.y + l.y); }
+  __device__ __forceinline__ float2 get(int) const { return make_float2(h.x + l.x, h.y + l.y); }
 };
 
 template <typename T>
@@ -617,23 +657,37 @@ __global__ void __launch_bounds__(32) getrs_small_kernel(int N, const T *LU_all,
   RowSum<T> x0(r0 < N ? xs[r0] : z), x1(r1 < N ? xs[r1] : z);
   const int q0 = min(r0, N - 1), q1 = min(r1, N - 1);
   const T d0 = crcp(S[q0 * LD + q0]), d1 = N > 32 ? crcp(S[q1 * LD + q1]) : z;
-  for (int j = 0; j < N; ++j) {  // L y = P b, unit lower
-    const T y = shfl_c(j < 32 ? x0.get() : x1.get(), j & 31);
-    if (j < 31 && r0 > j) x0.sub(S[q0 * LD + j], y);
-    if (N > 32 && r1 > j) x1.sub(S[q1 * LD + j], y);
-  }
-  for (int j = N - 1; j >= 0; --j) {  // U x = y
-    if (j < 32) {
-      if (r0 == j) x0 = RowSum<T>(cquo(x0.get(), S[q0 * LD + q0], d0));
-    } else if (r1 == j) {
-      x1 = RowSum<T>(cquo(x1.get(), S[q1 * LD + q1], d1));
+  // terms j = j0 + q
+  for (int j0 = 0; j0 < N; j0 += kPart)  // L y = P b, unit lower
+#pragma unroll
+    for (int q = 0; q < kPart; ++q) {
+      const int j = j0 + q, last = (q + kPart - 1) % kPart;
+      if (j < N) {
+        const T y = shfl_c((j < 32 ? x0 : x1).get(last), j & 31);
+        if (j < 31 && r0 > j) x0.add(q, S[q0 * LD + j], y);
+        if (N > 32 && r1 > j) x1.add(q, S[q1 * LD + j], y);
+      }
     }
-    const T y = shfl_c(j < 32 ? x0.get() : x1.get(), j & 31);
-    if (r0 < j) x0.sub(S[q0 * LD + j], y);
-    if (j > 32 && r1 < j) x1.sub(S[q1 * LD + j], y);
-  }
-  if (r0 < N) b[r0] = x0.get();
-  if (r1 < N) b[r1] = x1.get();
+  T u0 = x0.get(0), u1 = x1.get(0);
+  x0 = RowSum<T>(u0);
+  x1 = RowSum<T>(u1);
+  for (int j0 = (N - 1) / kPart * kPart; j0 >= 0; j0 -= kPart)  // U x = y
+#pragma unroll
+    for (int q = kPart - 1; q >= 0; --q) {
+      const int j = j0 + q, last = (q + 1) % kPart;
+      if (j < N) {
+        if (j < 32) {
+          if (r0 == j) u0 = cquo_near(x0.get(last), S[q0 * LD + q0], d0);
+        } else if (r1 == j) {
+          u1 = cquo_near(x1.get(last), S[q1 * LD + q1], d1);
+        }
+        const T y = shfl_c(j < 32 ? u0 : u1, j & 31);
+        if (r0 < j) x0.add(q, S[q0 * LD + j], y);
+        if (j > 32 && r1 < j) x1.add(q, S[q1 * LD + j], y);
+      }
+    }
+  if (r0 < N) b[r0] = u0;
+  if (r1 < N) b[r1] = u1;
 }
 
 // Above: one CTA per system, blocks of 32 unknowns.  Warp 0 solves a block's
@@ -677,7 +731,7 @@ __global__ void __launch_bounds__(kRsThreads) getrs_block_kernel(int N, const T 
     x[i] = b[i];
     sp[i] = piv_all[(size_t)blockIdx.x * N + i];
     moved |= sp[i] != i;
-    dinv[i] = crcp(A[(size_t)i * N + i]);
+    dinv[i] = sizeof(T) == 16 ? crcp_near(A[(size_t)i * N + i]) : crcp(A[(size_t)i * N + i]);
   }
   const int nb = (N + kRsB - 1) / kRsB;
   // stage q of 2 nb: the forward blocks in order, then the backward blocks
@@ -706,23 +760,37 @@ __global__ void __launch_bounds__(kRsThreads) getrs_block_kernel(int N, const T 
     T acc[kRsRows];
     if (warp == 0) {
       const int r = min(lane, bs - 1);
-      T v = x[i0 + r];
-      v = cmk<T>(v.x - part[r].x, v.y - part[r].y);
+      PartSum<T, kPart> v(x[i0 + r], part[r]);
+      T u = cmk<T>(0, 0);
       const T(*tl)[kRsB + 1] = tri[q & 1];
       if (q < nb) {
-        for (int j = 0; j < bs; ++j) {
-          const T y = shfl_c(v, j);
-          if (r > j) v = cfms(v, tl[r][j], y);
-        }
+        for (int j0 = 0; j0 < bs; j0 += kPart)
+#pragma unroll
+          for (int p = 0; p < kPart; ++p) {
+            const int j = j0 + p;
+            if (j < bs) {
+              if (r == j) u = v.get((p + kPart - 1) % kPart);
+              const T y = shfl_c(u, j);
+              if (r > j) v.add(p, tl[r][j], y);
+            }
+          }
       } else {
         const T di = dinv[i0 + r];
-        for (int j = bs - 1; j >= 0; --j) {
-          if (r == j) v = cquo(v, tl[r][r], di);
-          const T y = shfl_c(v, j);
-          if (r < j) v = cfms(v, tl[r][j], y);
-        }
+        for (int j0 = (bs - 1) / kPart * kPart; j0 >= 0; j0 -= kPart)
+#pragma unroll
+          for (int p = kPart - 1; p >= 0; --p) {
+            const int j = j0 + p;
+            if (j < bs) {
+              if (r == j) {
+                const T w = v.get((p + 1) % kPart);
+                u = sizeof(T) == 16 ? cmul(w, di) : cquo_near(w, tl[r][r], di);
+              }
+              const T y = shfl_c(u, j);
+              if (r < j) v.add(p, tl[r][j], y);
+            }
+          }
       }
-      if (lane < bs) x[i0 + lane] = v;
+      if (lane < bs) x[i0 + lane] = u;
     } else if (more) {
       // the next triangle and the square beside it: lane = column, loads in flight together
       const int w0 = (warp - 1) * kRsRows;
@@ -905,3 +973,30 @@ int batch_getrs_c128(int nm, int N, const void *LU, const int *piv, void *b, cud
 }
 
 }  // namespace qg
+
+extern "C" int qpms_gpu_debug_batch_lu(int is_double, int nm, int N, void *A, int *piv, void *b) {
+  using namespace qg;
+  clear_error();
+  if (nm <= 0 || N <= 0 || !A || !piv || !b) {
+    set_error("batched LU: empty or NULL argument");
+    return QPMS_EINVAL;
+  }
+  const size_t sz = is_double ? 16 : 8, na = (size_t)nm * N * N * sz, nb = (size_t)nm * N * sz, np = (size_t)nm * N * 4;
+  char *d = nullptr;
+  QG_CUDA_TRY(cudaMalloc(&d, na + nb + np));
+  auto run = [&]() -> int {
+    int *dp = (int *)(d + na + nb);
+    QG_CUDA_TRY(cudaMemcpy(d, A, na, cudaMemcpyHostToDevice));
+    QG_CUDA_TRY(cudaMemcpy(d + na, b, nb, cudaMemcpyHostToDevice));
+    int e = is_double ? batch_getrf_c128(nm, N, d, dp, nullptr, 0) : batch_getrf_c64(nm, N, d, dp, nullptr, 0);
+    if (e) return e;
+    if ((e = is_double ? batch_getrs_c128(nm, N, d, dp, d + na, 0) : batch_getrs_c64(nm, N, d, dp, d + na, 0))) return e;
+    QG_CUDA_TRY(cudaMemcpy(A, d, na, cudaMemcpyDeviceToHost));
+    QG_CUDA_TRY(cudaMemcpy(b, d + na, nb, cudaMemcpyDeviceToHost));
+    QG_CUDA_TRY(cudaMemcpy(piv, dp, np, cudaMemcpyDeviceToHost));
+    return QPMS_SUCCESS;
+  };
+  const int e = run();
+  cudaFree(d);
+  return e;
+}
