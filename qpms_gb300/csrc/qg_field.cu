@@ -32,7 +32,9 @@
 // Bound: the FP64 pipe (1/64 of the FP32 rate), so the FP64 instructions per
 // pair count.  Through spherical components (radial, polar and azimuthal parts
 // of N and M per (l, m), a complex product per coefficient) lMax 3 took 790 of
-// them and @MEAS@
+// them and 20.7 ms for 1.6e7 pairs (400 particles, 40,001 points); now 306 and
+// 9.1 ms.  Six of them add a particle's field to the sum once all its waves are
+// summed (8.9 ms without, with an error 1.03 to 1.06 times as large).
 #include <math.h>
 #include <string.h>
 
@@ -218,6 +220,7 @@ __global__ void __launch_bounds__(kFieldThreads) scattered_field_kernel(const Fi
       A[0] = 1.0;
       B[0] = 0.0;
       const qg_c(*C)[3] = sC[p];
+      qg_c e[3];  // this particle's field: one rounding at the size of the sum per particle
 #pragma unroll
       for (int l = 0; l <= LP; ++l) {
         if (l == 1) {
@@ -252,9 +255,12 @@ __global__ void __launch_bounds__(kFieldThreads) scattered_field_kernel(const Fi
         }
 #pragma unroll
         for (int c = 0; c < 3; ++c)
-          E[c] = cmk(fma(-z[l].im, S[c].im, fma(z[l].re, S[c].re, E[c].re)),
-                     fma(z[l].im, S[c].re, fma(z[l].re, S[c].im, E[c].im)));
+          e[c] = l ? cmk(fma(-z[l].im, S[c].im, fma(z[l].re, S[c].re, e[c].re)),
+                         fma(z[l].im, S[c].re, fma(z[l].re, S[c].im, e[c].im)))
+                   : cmul(z[0], S[c]);
       }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) E[c] = cadd(E[c], e[c]);
     }
   }
   if (q0 >= a.npts) return;
