@@ -68,12 +68,37 @@ template <typename T>
 __device__ __forceinline__ T cmul(T a, T b) {
   return cmk<T>(fmar(-a.y, b.y, a.x * b.x), fmar(a.y, b.x, a.x * b.y));
 }
+// The largest exponent of b's parts, in units of 2^23 (FP32) or 2^20 (FP64).
+__device__ __forceinline__ unsigned cexponent(float2 b) {
+  return max(__float_as_uint(b.x) & 0x7fffffffu, __float_as_uint(b.y) & 0x7fffffffu);
+}
+__device__ __forceinline__ unsigned cexponent(double2 b) {
+  return max((unsigned)__double2hiint(b.x) & 0x7fffffffu, (unsigned)__double2hiint(b.y) & 0x7fffffffu);
+}
 template <typename T>
-__device__ __forceinline__ T crcp(T b) {
+__device__ __forceinline__ T crcp_plain(T b) {
   typedef typename BL<T>::R R;
   const R s = R(1) / fmar(b.x, b.x, b.y * b.y);
   return cmk<T>(b.x * s, -b.y * s);
 }
+template <typename T>
+__device__ __noinline__ T crcp_scaled(T b, bool small) {
+  typedef typename BL<T>::R R;
+  const R up = R(sizeof(R) == 4 ? 0x1p75 : 0x1p600), f = small ? up : R(1) / up;
+  const T r = crcp_plain(cmk<T>(b.x * f, b.y * f));
+  return cmk<T>(r.x * f, r.y * f);
+}
+// 1 / b over the whole range of b: outside of 2^+-60 (FP32) or 2^+-500 (FP64), where
+// |b|^2 may leave the type's range, b is scaled by a power of two.
+template <typename T>
+__device__ __forceinline__ T crcp(T b) {
+  constexpr bool kF = sizeof(T) == 8;
+  constexpr unsigned kOne = kF ? 127u << 23 : 1023u << 20, kSpan = kF ? 60u << 23 : 500u << 20;
+  const unsigned x = cexponent(b);
+  if (x - (kOne - kSpan) > 2 * kSpan) return crcp_scaled(b, x < kOne);  // rare
+  return crcp_plain(b);
+}
+
 // 1 / b with a Newton step.
 template <typename T>
 __device__ __forceinline__ T crcp_near(T b) {
