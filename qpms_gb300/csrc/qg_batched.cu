@@ -78,9 +78,9 @@ int resolve_fp64(cudaStream_t st, const std::vector<int> &idx, size_t N, const q
   return e;
 }
 
-int batched_solve(cublasHandle_t h, cudaStream_t st, int nm, size_t N, const qg_c *dM, const qg_c *db, qg_c *dx,
-                  int mode, double tol, int max_iter, void *scratch, double *resid_host, int *iters_host,
-                  int *info_host, double *logabsdet, int *fallback_host) {
+int batched_solve(cudaStream_t st, int nm, size_t N, const qg_c *dM, const qg_c *db, qg_c *dx, int mode, double tol,
+                  int max_iter, void *scratch, double *resid_host, int *iters_host, int *info_host,
+                  double *logabsdet, int *fallback_host) {
   if (nm <= 0) return QPMS_SUCCESS;
   max_iter = max_refine_steps(max_iter);
   const size_t m = (size_t)nm, N2 = N * N;
@@ -96,7 +96,6 @@ int batched_solve(cublasHandle_t h, cudaStream_t st, int nm, size_t N, const qg_
   qg_c *r = (qg_c *)p;
   p += al(m * N * 16);
   double *rn2 = (double *)p, *bn2 = rn2 + m;
-  (void)h;
   std::vector<double> hr(m), hb(m);
   std::vector<int> its(m, 0);
   int e;

@@ -1,6 +1,5 @@
 // Batched solve of many small mode-problem systems (qg_batched.cu).
 #pragma once
-#include <cublas_v2.h>
 #include <cuda_runtime.h>
 
 #include <vector>
@@ -25,9 +24,9 @@ size_t batched_solve_bytes(int nm, size_t N, int mode);
 // logabsdet (device, may be NULL): log|det M_i| from the diagonal of complex128
 // factors; with it, mode 1 solves through those complex128 factors as mode 0
 // does (the factors it needs solve the systems too).
-int batched_solve(cublasHandle_t h, cudaStream_t st, int nm, size_t N, const qg_c *dM, const qg_c *db, qg_c *dx,
-                  int mode, double tol, int max_iter, void *scratch, double *resid_host, int *iters_host,
-                  int *info_host, double *logabsdet, int *fallback_host = nullptr);
+int batched_solve(cudaStream_t st, int nm, size_t N, const qg_c *dM, const qg_c *db, qg_c *dx, int mode, double tol,
+                  int max_iter, void *scratch, double *resid_host, int *iters_host, int *info_host,
+                  double *logabsdet, int *fallback_host = nullptr);
 
 // Systems idx of a contiguous batch solved again in complex128 (partial
 // pivoting), x overwritten: the fallback of a stalled complex64 refinement.

@@ -128,8 +128,10 @@ __device__ __forceinline__ T cquo(T a, T b, T r) {
 // A key orders candidates as unsigned integers, 0 for a NaN.  complex128: the bits
 // of the measure plus one.  complex64: the measure with all its bits, as the FP32
 // sum plus one and, below it, the sum's rounding error (TwoSum), which orders equal
-// sums: the exact sums' order without FP64 instructions (1 % of a batch of 32 of 480
-// unknowns; the FP32 sum alone takes the first of sums equal in 24 bits).
+// sums: the exact sums' order without FP64 instructions.  (32 LUs of 256 unknowns
+// 278 us, with the FP32 sum alone, which takes the first of sums equal in 24 bits,
+// 254 us; forming the low word only where the high words are equal, behind branches
+// in the unrolled columns, 342 us.)
 typedef unsigned long long PivKey;
 __device__ __forceinline__ PivKey pivot_key(float2 z) {
   const float a = fabsf(z.x), b = fabsf(z.y), s = __fadd_rn(a, b), t = __fsub_rn(s, a);
@@ -721,24 +723,6 @@ constexpr int kRsB = 32;
 
 constexpr int kRsFar = 8, kRsThreads = 32 * (1 + kRsFar), kRsRows = kRsB / kRsFar;
 
-// Sums of the 8 values over the warp's lanes, folded so that each exchange
-// halves the values (9 additions instead of 40; FP64 additions are the cost):
-// returns the sum of v[lane >> 2 & 7] (bits 4, 3, 2 of the lane).
-template <typename R>
-__device__ __forceinline__ R fold8(R (&v)[8], int lane) {
-#pragma unroll
-  for (int h = 4, o = 16; h; h >>= 1, o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int i = 0; i < h; ++i) {
-      const R keep = up ? v[i + h] : v[i], give = up ? v[i] : v[i + h];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-    }
-  }
-  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
-}
-
 template <typename T>
 __global__ void __launch_bounds__(kRsThreads) getrs_block_kernel(int N, const T *LU_all, const int *piv_all, T *b_all) {
   typedef typename BL<T>::R R;
@@ -875,17 +859,19 @@ void cluster_config(int C, int nm, int N, cudaStream_t st, cudaLaunchConfig_t *c
   cfg->numAttrs = 1;
 }
 
-// CTAs per matrix above N = 64.  The time of a matrix against its time on one
-// CTA, measured (us, GB300):
-//                            C = 1     4     8     9    16
-//   complex128, N 512, 2     47321 15949  7695        4321   (FP64 pipes of C - 1 SMs)
-//   complex128, N 390, 9     21790  7349  3724  3317  4714   (two waves at 16)
-//   complex64,  N 512, 2      2788  1000   660         580   (the panels' serial chain)
-//   complex64,  N 256, 32      574   271   750        1268   (two and four waves)
-// so the choice is the least waves x relative time, a wave being the clusters
-// that the GPU holds at once (a cluster lies within one group of SMs: 14 of 9
-// run at once, 16 of 8 do not), among sizes whose CTAs all get a tile of the
-// first update.  The counts are asked for once per device.
+// CTAs per matrix above N = 64.  The time of a batch, measured (us, GB300; diagonally
+// dominant matrices, so without row exchanges):
+//                            C = 1     4     6     8     9    16
+//   complex128, N 512, 2     47300 15870 10080  7650  6815  4270  (FP64 pipes of C - 1 SMs)
+//   complex128, N 390, 9     21710  7310  4770  3700  3300  4680  (two waves at 16)
+//   complex128, N 200, 40     3310  2310  1740  2250  2190        (two, two, three and three waves)
+//   complex64,  N 512, 2      2790   985   734   652   624   600  (the panels' serial chain)
+//   complex64,  N 256, 32      570   278   533   786              (two and three waves)
+// so the choice is the least waves x relative time, a wave being the clusters that the
+// GPU holds at once (152, 36, 23, 15, 15, 7: a cluster lies within one group of SMs),
+// among sizes whose CTAs all get a tile of the first update.  Relative times:
+// complex128 as at N 512; complex64 between those of N 512 and N 256 (4 CTAs 0.35 and
+// 0.49, 8 CTAs 0.23 and 0.46).  The counts are asked for once per device.
 template <typename T>
 int cluster_size(int nm, int N, int *C_out) {
   constexpr int kN = 6, kC[kN] = {1, 4, 6, 8, 9, 16}, kMaxDev = 64;

@@ -39,8 +39,6 @@ int sym_nirreps(const qpms_scatsys_t *ss);
 void scatsys_tdiag(const qpms_scatsys_t *ss, int t, double om_re, double om_im, std::vector<qg_c> &out);
 qg_c scatsys_wavenumber(const qpms_scatsys_t *ss, double om_re, double om_im);
 int blas_handle_get(cublasHandle_t *h);
-int assemble_modeproblem_device(const qpms_scatsys_t *ss, int nw, const std::vector<qg_c> &T_host, bool dense,
-                                const std::vector<qg_c> &k_host, int J, qg_c *dM, cudaStream_t st);
 int periodic_assemble_device(const qpms_scatsys_t *ss, int nw, const qg_c *k_host, const std::vector<qg_c> &T_host,
                              int nk, const double *beta_host, const double *eta_host, qg_c *dM, cudaStream_t st);
 

@@ -34,6 +34,23 @@ __device__ __forceinline__ double xor_sign(double x, unsigned long long mask) {
   return __longlong_as_double(__double_as_longlong(x) ^ (long long)mask);
 }
 constexpr unsigned long long kSignBit = 0x8000000000000000ull;
+// Sums of the 8 values over the warp's lanes, folded so that each exchange
+// halves the values (9 additions instead of 40; FP64 additions are the cost):
+// returns the sum of v[lane >> 2 & 7] (bits 4, 3, 2 of the lane).
+template <typename R>
+__device__ __forceinline__ R fold8(R (&v)[8], int lane) {
+#pragma unroll
+  for (int h = 4, o = 16; h; h >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const R keep = up ? v[i + h] : v[i], give = up ? v[i] : v[i + h];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
 #endif
 QG_HD double cabs2(qg_c a) { return a.re * a.re + a.im * a.im; }
 QG_HD double cabsd(qg_c a) { return hypot(a.re, a.im); }

@@ -1039,21 +1039,6 @@ struct ScanShape {
   static constexpr int NH = LE / 2 + 1;                // (n - |m|) / 2 + 1 at most
 };
 
-// Sums of the 8 values over the warp's lanes; lane l gets the sum of v[l >> 2].
-__device__ __forceinline__ double fold8(double (&v)[8], int lane) {
-#pragma unroll
-  for (int h = 4, o = 16; h; h >>= 1, o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int i = 0; i < h; ++i) {
-      const double keep = up ? v[i + h] : v[i], give = up ? v[i] : v[i + h];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-    }
-  }
-  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
-}
-
 // acc[e..] += i^r j (p1, p2, p3, p4): the products of order m's phase
 template <int R>
 __device__ __forceinline__ void acc4(double *acc, double j, double p1, double p2, double p3, double p4) {

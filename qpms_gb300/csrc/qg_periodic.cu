@@ -609,9 +609,7 @@ int qpms_gpu_periodic_scan(const qpms_scatsys_t *ss, size_t nw, const double *om
   if (!nw || !nk) return QPMS_SUCCESS;
   const int lMax = scatsys_lmax(ss), np = ss->p_count, ntm = ss->tm_count, n = 2 * lMax * (lMax + 2);
   const size_t N = ss->fecv_size, N2 = N * N;
-  cublasHandle_t h;
   int e;
-  if ((e = blas_handle_get(&h))) return e;
   // process in chunks of whole frequencies, <= ~2 GiB of matrices per chunk
   const size_t per_w = nk * N2 * 16;
   const int wchunk = (int)std::max<size_t>(1, std::min<size_t>(nw, (size_t(2) << 30) / per_w));
@@ -672,7 +670,7 @@ int qpms_gpu_periodic_scan(const qpms_scatsys_t *ss, size_t nw, const double *om
         (e = launch_apply_t((int)nm, np, n, ntm, scatsys_dense(ss) ? 1 : 0, dtm, dTw, da, db, 0, (int)nk)))
       return e;
     // LU (complex128, or complex64 + FP64 refinement), log|det| from the factors
-    if ((e = batched_solve(h, 0, (int)nm, N, dM, db, dx, mode, 1e-13, 12, ar.at<char>(oscr), res.data(), its.data(),
+    if ((e = batched_solve(0, (int)nm, N, dM, db, dx, mode, 1e-13, 12, ar.at<char>(oscr), res.data(), its.data(),
                            info.data(), dlog)))
       return e;
     QG_CUDA_TRY(cudaMemcpy(logdet + w0 * nk, dlog, nm * 8, cudaMemcpyDeviceToHost));

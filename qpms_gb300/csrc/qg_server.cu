@@ -19,7 +19,6 @@
 // device and the workers' kernels overlap.  The per-lMax translation tables
 // are resident (shared calculators); per-system particle data are uploaded
 // once and kept, keyed by content.
-#include <cublas_v2.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <string.h>
@@ -49,7 +48,6 @@ void scatsys_tdiag(const qpms_scatsys_t *ss, int t, double om_re, double om_im, 
 qg_c scatsys_wavenumber(const qpms_scatsys_t *ss, double om_re, double om_im);
 void planewave_direction_coeffs(int lMax, const double k_dir[3], const qpms_complex_t E_cart[3],
                                 std::vector<qg_c> &coef);
-int blas_handle_get(cublasHandle_t *h);
 int ewald_assemble_locked(const qpms_scatsys_t *ss, const EwaldArgs &a, cudaStream_t st);
 int ewald_assemble_dense(const qpms_scatsys_t *ss, const EwaldArgs &a, int n, cudaStream_t st);
 int layered_system(const qpms_scatsys_t *ss);
@@ -298,9 +296,6 @@ struct qpms_gpu_server {
     SysDev sd;
     int e;
     if ((e = system_dev(ss, st, &sd))) return e;
-    cublasHandle_t h;
-    if ((e = blas_handle_get(&h))) return e;
-    QG_BLAS_TRY(cublasSetStream(h, st));
     PoolBufs B(st);
     qg_c *dM, *dT, *dk, *dcoef, *da, *db, *dx;
     double *dkv, *dsig, *dbeta, *deta;
@@ -381,8 +376,6 @@ struct qpms_gpu_server {
     SysDev sd;
     int e;
     if ((e = system_dev(ss, st, &sd))) return e;
-    cublasHandle_t h;
-    if ((e = blas_handle_get(&h))) return e;
     PoolBufs B(st);
     qg_c *dM, *dT, *dk, *dcoef, *da, *db, *dx;
     double *dkv, *dsig, *dbeta, *deta;
@@ -406,7 +399,7 @@ struct qpms_gpu_server {
     if ((e = launch_apply_t(nb, np, n, ntm, scatsys_dense(ss) ? 1 : 0, sd.tmid, dT, da, db, st))) return e;
     std::vector<double> res(nb), sig(nb);
     std::vector<int> its(nb), info(nb), fb(nb);
-    if ((e = batched_solve(h, st, nb, N, dM, db, dx, mode, kRefineTol, kMaxRefine, scratch, res.data(), its.data(),
+    if ((e = batched_solve(st, nb, N, dM, db, dx, mode, kRefineTol, kMaxRefine, scratch, res.data(), its.data(),
                            info.data(), nullptr, fb.data())))
       return e;
     if ((e = launch_sigma_ext(nb, N, da, dx, dk, dsig, st))) return e;

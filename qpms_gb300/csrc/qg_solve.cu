@@ -492,10 +492,7 @@ int qpms_gpu_finite_planewave_scatter_ext(const qpms_scatsys_t *ss, size_t nw, c
   if (N > kBatchedMaxN)
     return finite_scatter_dense(ss, W, T, k, kvec, coef, mode, f_out, sigma_ext, sigma_scat, resid_out, iters_out);
   cudaStream_t st = 0;
-  cublasHandle_t h;
   int e;
-  if ((e = blas_handle_get(&h))) return e;
-  QG_BLAS_TRY(cublasSetStream(h, st));
   std::vector<double> pos(3 * np);
   std::vector<int> tm(np);
   for (int i = 0; i < np; ++i) {
