@@ -372,16 +372,16 @@ int periodic_assemble_device_ex(const qpms_scatsys_t *ss, int nw, const qg_c *k_
       }
     const int lMax = scatsys_lmax(ss), LE = 2 * lMax + 1, nev = (LE + 1) * (LE + 2) / 2;
     const size_t units = (size_t)nw * np * np;
-    if ((e = dalloc(dtab, units * nev * srmax * 16)) || (e = dalloc(dpts, units * srmax * 16)) ||
+    a.real_k = 1;
+    for (int w = 0; w < nw; ++w)
+      if (k_host[w].im != 0.0 || !(k_host[w].re > 0.0)) a.real_k = 0;
+    if ((e = dalloc(dtab, units * nev * srmax * (a.real_k ? 8 : 16))) || (e = dalloc(dpts, units * srmax * 16)) ||
         (e = dalloc(dcnt, units * 4)))
       return e;
     a.srtab = dtab.as<qg_c>();
     a.srpts = dpts.as<double>();
     a.srcnt = dcnt.as<int>();
     a.srmax = (int)srmax;
-    a.real_k = 1;
-    for (int w = 0; w < nw; ++w)
-      if (k_host[w].im != 0.0 || !(k_host[w].re > 0.0)) a.real_k = 0;
     if (a.real_k) {
       if ((e = dalloc(dsig0, units * 16))) return e;
       a.sig0 = dsig0.as<qg_c>();
