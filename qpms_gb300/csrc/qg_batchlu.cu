@@ -99,14 +99,6 @@ __device__ __forceinline__ T crcp(T b) {
   return crcp_plain(b);
 }
 
-// 1 / b with a Newton step.
-template <typename T>
-__device__ __forceinline__ T crcp_near(T b) {
-  typedef typename BL<T>::R R;
-  const T r = crcp(b), e = cfms(cmk<T>(R(1), R(0)), b, r);
-  return cfma(r, r, e);
-}
-
 // a / b with r = crcp(b) at hand: a r corrected by the remainder, as good as a
 // division; or a r alone for the complex128 multipliers, which are small against
 // the pivot.  Errors of solves by the two factorisations and substitutions against
@@ -746,7 +738,7 @@ __global__ void __launch_bounds__(kRsThreads) getrs_block_kernel(int N, const T 
     x[i] = b[i];
     sp[i] = piv_all[(size_t)blockIdx.x * N + i];
     moved |= sp[i] != i;
-    dinv[i] = sizeof(T) == 16 ? crcp_near(A[(size_t)i * N + i]) : crcp(A[(size_t)i * N + i]);
+    dinv[i] = crcp(A[(size_t)i * N + i]);
   }
   const int nb = (N + kRsB - 1) / kRsB;
   // stage q of 2 nb: the forward blocks in order, then the backward blocks
@@ -791,19 +783,21 @@ __global__ void __launch_bounds__(kRsThreads) getrs_block_kernel(int N, const T 
           }
       } else {
         const T di = dinv[i0 + r];
+        T w = u;
         for (int j0 = (bs - 1) / kPart * kPart; j0 >= 0; j0 -= kPart)
 #pragma unroll
           for (int p = kPart - 1; p >= 0; --p) {
             const int j = j0 + p;
             if (j < bs) {
               if (r == j) {
-                const T w = v.get((p + 1) % kPart);
-                u = sizeof(T) == 16 ? cmul(w, di) : cquo_near(w, tl[r][r], di);
+                w = v.get((p + 1) % kPart);
+                u = cmul(w, di);
               }
               const T y = shfl_c(u, j);
               if (r < j) v.add(p, tl[r][j], y);
             }
           }
+        u = cfma(u, cfms(w, u, tl[r][r]), di);  // the quotient's correction, off the chain
       }
       if (lane < bs) x[i0 + lane] = u;
     } else if (more) {
