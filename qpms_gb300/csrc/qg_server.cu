@@ -317,18 +317,16 @@ struct qpms_gpu_server {
     double res = 0;
     int it = 0;
     // with several workers the diagonal-block inversions already overlap other
-    // requests' work; the LU's own lookahead then only costs launches
-    // (measured on the serving trace: 94.5 solves/s with it, 100.7 without)
-    // (also measured: lookahead only for requests above 4,096 / 8,192 / 12,000
-    // unknowns, 106-109 solves/s against 116 without)
+    // requests' work; the LU's own lookahead then only costs launches (the
+    // 60-request trace, 8 workers, median of 8 passes: 132 solves/s with it, 158
+    // without)
     ds.lookahead = nworkers == 1;
     // and 128-wide blocks at every size: the trailing updates, not the
-    // inversion chain, bound a loaded server (107.5 solves/s against 104.4
-    // with 64-wide blocks below 6,144 unknowns)
+    // inversion chain, bound a loaded server (158 solves/s, 141 with 64-wide ones)
     ds.nb_pref = 128;
     // and groups of 3 blocks in the LU: without the lookahead the in-group
-    // inversions cost nothing extra here (136.0 / 137.0 solves/s with pairs,
-    // 138.1 with groups of 3, 138.2 / 137.0 with groups of 4)
+    // inversions cost nothing extra here (138 solves/s one block at a time, 155
+    // with pairs, 158 with groups of 3 and of 4)
     ds.group = nworkers == 1 ? 0 : 3;
     if ((e = ds.init((int)N, 1, mode, 0x5eed ^ j->id, pool, st))) return e;
     if ((e = ds.factorize(dM, N, st, true))) return e;

@@ -506,9 +506,10 @@ int launch_gemm(const CUtensorMap &ma, const CUtensorMap &mb, const GemmArgs &g,
                                     S::kBytes);
   });
   QG_CUDA_TRY(attr_err);
-  // Persistent CTAs on all but kReservedSms SMs: the dense LU's diagonal
-  // inversions (four CTAs) and the small launches of concurrent solves on
-  // other streams always find an SM instead of waiting for a whole GEMM.
+  // Persistent CTAs on all but kReservedSms SMs, where the small launches of
+  // other streams start instead of waiting for a whole GEMM.  The dense LU's
+  // diagonal inversions need room for a cluster of four CTAs within one group of
+  // SMs; which SMs stay free is not under control, so they may still wait.
   const int ntiles = ((g.Md + BM - 1) / BM) * ((g.Nd + BN - 1) / BN);
   const int slots = g_num_sms > 2 * kReservedSms ? g_num_sms - kReservedSms : g_num_sms;
   const int grid = ntiles < slots ? ntiles : slots;
