@@ -126,7 +126,7 @@ __device__ __forceinline__ T fms_c(T acc, T a, T b) {  // acc - a b
 }
 
 // (p, q) element of an 8 x 8 block: lane 8 (p % 4) + q, register p / 4.  Inverts
-// the block in place; true if a pivot was zero.
+// the block in place; true if a pivot, or its square, was zero.
 template <typename T>
 __device__ __forceinline__ bool invert8(T (&x)[2], int lane) {
   const int q = lane & 7, p0 = lane >> 3;
@@ -138,10 +138,10 @@ __device__ __forceinline__ bool invert8(T (&x)[2], int lane) {
     };
     const T d = get(x[s / 4], 8 * (s % 4) + s), u = get(x[s / 4], 8 * (s % 4) + q);
     const T f0 = get(x[0], 8 * p0 + s), f1 = get(x[1], 8 * p0 + s);
-    const bool z = d.x == 0 && d.y == 0;
+    const auto n = d.x * d.x + d.y * d.y;
+    const bool z = n == 0;  // also a pivot whose square leaves the type's range: its reciprocal would be infinite
     zero |= z;
     // 1 / d with one division per lane: even lanes the real part, odd ones the imaginary
-    const auto n = d.x * d.x + d.y * d.y;
     const auto h0 = (lane & 1 ? -d.y : d.x) / n, h1 = __shfl_xor_sync(0xffffffffu, h0, 1);
     const T di = z ? mk<T>(0, 0) : lane & 1 ? mk<T>(h1, h0) : mk<T>(h0, h1);
     const T ud = mul(u, di);  // the pivot row times 1 / d
