@@ -1419,9 +1419,10 @@ void DenseSolver::release() {
     *g = Graph();
   }
   if (side) cudaStreamDestroy(side);
+  if (capture) cudaStreamDestroy(capture);
   if (ev_a) cudaEventDestroy(ev_a);
   if (ev_d) cudaEventDestroy(ev_d);
-  side = nullptr;
+  side = capture = nullptr;
   ev_a = ev_d = nullptr;
   block = A = T64 = Dinv = work = rhs_lo = rp = nullptr;
   r64 = y64 = nullptr;
@@ -1459,7 +1460,7 @@ template <class F>
 int DenseSolver::run_graph(Graph &g, const unsigned long long (&key)[6], bool capturable, cudaStream_t st, F body) {
   const char *ev = getenv("QPMS_GB300_GRAPHS");
   const bool env_off = ev && !strcmp(ev, "0");
-  if (!graphs || env_off || !capturable || st == 0 || kt_on()) return body();
+  if (!graphs || env_off || !capturable || st == 0 || kt_on()) return body(st);
   bool same = g.keyed;
   for (int i = 0; i < 6 && same; ++i) same = g.key[i] == key[i];
   if (same && g.exec) {
@@ -1474,14 +1475,15 @@ int DenseSolver::run_graph(Graph &g, const unsigned long long (&key)[6], bool ca
     g.exec = nullptr;
     for (int i = 0; i < 6; ++i) g.key[i] = key[i];
     g.keyed = true;
-    return body();
+    return body(st);
   }
   // second call with the same buffers: capture, then launch the graph
   cudaGraph_t graph = nullptr;
   const unsigned long long l0 = g_launches.load();
-  QG_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-  const int e = body();
-  const cudaError_t ce = cudaStreamEndCapture(st, &graph);
+  if (!capture) QG_CUDA_TRY(cudaStreamCreateWithFlags(&capture, cudaStreamNonBlocking));
+  QG_CUDA_TRY(cudaStreamBeginCapture(capture, cudaStreamCaptureModeThreadLocal));
+  const int e = body(capture);
+  const cudaError_t ce = cudaStreamEndCapture(capture, &graph);
   if (e || ce != cudaSuccess) {
     if (graph) cudaGraphDestroy(graph);
     cudaGetLastError();
@@ -1512,10 +1514,10 @@ int DenseSolver::factorize(const void *M64, size_t ldm, cudaStream_t st, bool ro
   const unsigned long long key[6] = {(unsigned long long)(uintptr_t)M64, ldm, rowmaj ? 1ull : 0ull,
                                      (unsigned long long)mode, (unsigned long long)tc_split,
                                      use_ozaki ? 1ull : 0ull};
-  int e = run_graph(gf, key, mode == 1 && tc_split != 0, st, [&]() -> int {
+  int e = run_graph(gf, key, mode == 1 && tc_split != 0, st, [&](cudaStream_t s) -> int {
     int e2;
-    if (use_ozaki && (e2 = ozaki_split_matrix(M64, ldm, row_major, N, oz_mat, &oz, st))) return e2;
-    return factor_launch(M64, ldm, st);
+    if (use_ozaki && (e2 = ozaki_split_matrix(M64, ldm, row_major, N, oz_mat, &oz, s))) return e2;
+    return factor_launch(M64, ldm, s);
   });
   if (e) return e;
   return check_info(st);
@@ -1619,7 +1621,8 @@ int DenseSolver::apply_inverse(const void *R, size_t ldr, void *Y, size_t ldy, i
                                      (unsigned long long)nrhs,
                                      (unsigned long long)mode | ((unsigned long long)tc_split << 8)};
   const bool capturable = mode == 1 && (nrhs <= kSmallRhs || tc_split != 0);
-  return run_graph(gs, key, capturable, st, [&]() { return apply_launch(R, ldr, Y, ldy, nrhs, st); });
+  return run_graph(gs, key, capturable, st,
+                   [&](cudaStream_t s) { return apply_launch(R, ldr, Y, ldy, nrhs, s); });
 }
 
 int DenseSolver::apply_launch(const void *R, size_t ldr, void *Y, size_t ldy, int nrhs, cudaStream_t st) {

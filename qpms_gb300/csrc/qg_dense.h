@@ -69,6 +69,10 @@ struct DenseSolver {
   };
   bool graphs = false;
   Graph gf, gs;
+  // Launch sequences are captured on a non-blocking stream of their own: while a
+  // blocking stream captures, another thread's work on the legacy default stream
+  // fails, and the capture with it.
+  cudaStream_t capture = nullptr;
   // lookahead of the tensor-core LU: the next diagonal block is inverted on
   // `side` (high priority) while the trailing update runs (QPMS_GB300_LOOKAHEAD=0
   // turns it off; so does lookahead = false before init(): a serving loop with
